@@ -285,6 +285,12 @@ typedef struct {
 } ulm_ce_bwd_args;
 int ulm_ce_bwd(const ulm_ce_bwd_args* a);
 
+/* Mean over the rows of the loss the two forms above and below return (train.py:2069-2082): *loss = sum of
+ * rows_loss / n and *inv = 1 / n in fp32, n = *denom_dev if that is non-NULL, else denom if it is positive, else the
+ * number of targets != ignore_index (at least 1).  Fixed summation order. */
+int ulm_loss_mean(const float* rows_loss, const int64_t* target, int64_t rows, int64_t ignore_index, const float* denom_dev,
+                  float denom, float* loss, float* inv, void* stream);
+
 /* ---- lm-head GEMM with the loss statistics in its epilogue -----------------
  * Forward of the reference's `F.cross_entropy(self.fc_out(h), t)` (train.py:2075-2079) as ONE tensor-core
  * kernel plus a per-row finishing kernel: z = h w^T rounded to the 16-bit dtype (what the autocast linear

@@ -6,6 +6,9 @@ next to the sources, never raise at import time, and report a failed build
 through ``build_error()``.  The library is plain ``nvcc -shared`` output with
 ``extern "C"`` entry points (include/ulm_b200.h); it does not link against
 torch.  There is no fallback: every op raises if the library is unavailable.
+
+Beside it stands ``_ulm_torch.so`` (csrc/torch_ops.cpp), the autograd functions over the same entry points as a
+CPython extension: a host compiler builds it against torch's headers, and `ext` loads it.
 """
 from __future__ import annotations
 
@@ -23,7 +26,11 @@ _SOURCES = ['attn_bwd.cu', 'attn_fwd.cu', 'lmhead.cu', 'lib.cu', 'tc_host.cu', '
             'grad_post.cu', 'selftest.cu']          # slowest first: they are compiled in parallel
 _HEADERS = ['common.cuh', 'tc.cuh', 'rope_math.cuh', os.path.join('..', '..', 'include', 'ulm_b200.h')]
 
+_EXT_PATH = os.path.join(_HERE, '_ulm_torch.so')
+_EXT_SOURCE = 'torch_ops.cpp'
+
 _lock = threading.Lock()
+_ext = None
 _lib = None
 _error = None
 
@@ -117,6 +124,7 @@ EXPORTS = {
     'ulm_lmhead_lse': (C.c_int, [C.POINTER(LmHeadLseArgs)]),
     'ulm_lmhead_lse_parts': (C.c_int64, [C.c_int32]),
     'ulm_ce_bwd': (C.c_int, [C.POINTER(CeBwdArgs)]),
+    'ulm_loss_mean': (C.c_int, [vp, vp, i64, i64, vp, f32, vp, vp, vp]),
     'ulm_swiglu_fwd': (C.c_int, [C.POINTER(SwigluArgs)]),
     'ulm_swiglu_bwd': (C.c_int, [C.POINTER(SwigluArgs)]),
     'ulm_grad_unscale_sumsq': (C.c_int, [vp, i64, vp, vp, vp, vp]),
@@ -139,40 +147,83 @@ def nvcc_commands(obj_dir, out_path=_LIB_PATH, extra=()):
     objs = [os.path.join(obj_dir, s[:-3] + '.o') for s in _SOURCES]
     compile_cmds = [[_nvcc(), *extra, *_ARCH, *_CFLAGS, '-c', os.path.join(_CSRC, s), '-o', o]
                     for s, o in zip(_SOURCES, objs)]
-    link = [_nvcc(), *_ARCH, '-shared', '-Xcompiler', '-fPIC', '-cudart', 'static', *objs, '-o', out_path]
+    link = [_nvcc(), *_ARCH, '-shared', '-Xcompiler', '-fPIC', '-cudart', 'static', '-Xlinker', '-soname=libulm_b200.so', *objs, '-o', out_path]
     return compile_cmds, link
 
 
-def _stale():
-    if not os.path.exists(_LIB_PATH):
+def ext_commands(obj_path, out_path):
+    """Compile and link commands of the torch extension (the link needs the library beside it)."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as X
+    cxx = 'g++'          # exceptions cross between torch and this library: both must share one C++ runtime (no $CXX wrapper with its own)
+    inc = [*X.include_paths(), os.path.join(X.CUDA_HOME or '/usr/local/cuda', 'include'), sysconfig.get_paths()['include']]
+    comp = [cxx, '-O2', '-std=c++17', '-fPIC', '-fvisibility=hidden', f'-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}',
+            *(a for d in inc for a in ('-isystem', d)), '-c', os.path.join(_CSRC, _EXT_SOURCE), '-o', obj_path]
+    link = [cxx, '-shared', obj_path, '-o', out_path, f'-L{_HERE}', '-lulm_b200', '-Wl,-rpath,$ORIGIN',
+            *(f'-L{d}' for d in X.library_paths()), '-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch', '-ltorch_python']
+    return comp, link
+
+
+def _older(path, deps):
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(_LIB_PATH)
-    deps = [os.path.join(_CSRC, s) for s in _SOURCES + _HEADERS]
+    t = os.path.getmtime(path)
     return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
 
 
+def _stale():
+    return _older(_LIB_PATH, [os.path.join(_CSRC, s) for s in _SOURCES + _HEADERS])
+
+
+def _ext_stale():
+    return _older(_EXT_PATH, [os.path.join(_CSRC, s) for s in (_EXT_SOURCE, _HEADERS[-1])])
+
+
 def build(force=False, verbose=False):
-    """Compile csrc/*.cu for sm_100a into libulm_b200.so beside this file."""
-    if not force and not _stale():
-        return _LIB_PATH
+    """Compile csrc/*.cu for sm_100a into libulm_b200.so beside this file, and csrc/torch_ops.cpp into _ulm_torch.so."""
+    do_lib, do_ext = force or _stale(), force or _ext_stale()
+    with concurrent.futures.ThreadPoolExecutor(max_workers=1) as ex:
+        lib_job = ex.submit(_build_lib, verbose) if do_lib else None
+        if do_ext:
+            _build_ext(verbose, before_link=lib_job.result if lib_job else None)
+        elif lib_job:
+            lib_job.result()
+    return _LIB_PATH
+
+
+def _run(cmd, verbose):
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode:
+        print(' '.join(cmd))
+        print(r.stdout, r.stderr)
+    if r.returncode:
+        raise RuntimeError(f'{os.path.basename(cmd[0])} failed ({r.returncode}):\n{r.stderr[-4000:]}')
+
+
+def _build_ext(verbose=False, before_link=None):
+    tmp_path = f'{_EXT_PATH}.{os.getpid()}.tmp'
+    with tempfile.TemporaryDirectory(prefix='ulm_b200_build_') as obj_dir:
+        comp, link = ext_commands(os.path.join(obj_dir, 'torch_ops.o'), tmp_path)
+        _run(comp, verbose)
+        if before_link is not None:
+            before_link()
+        _run(link, verbose)
+    os.replace(tmp_path, _EXT_PATH)
+
+
+def _build_lib(verbose=False):
     # Several ranks may find the library stale at once: each links into a file of its own
     # and the rename is atomic, so a reader never sees a half-written library.
     tmp_path = f'{_LIB_PATH}.{os.getpid()}.tmp'
     with tempfile.TemporaryDirectory(prefix='ulm_b200_build_') as obj_dir:
         compile_cmds, link = nvcc_commands(obj_dir, tmp_path)
 
-        def run(cmd):
-            r = subprocess.run(cmd, capture_output=True, text=True)
-            if verbose or r.returncode:
-                print(' '.join(cmd))
-                print(r.stdout, r.stderr)
-            if r.returncode:
-                raise RuntimeError(f'nvcc failed ({r.returncode}):\n{r.stderr[-4000:]}')
         with concurrent.futures.ThreadPoolExecutor(max_workers=min(len(compile_cmds), os.cpu_count() or 1)) as ex:
-            list(ex.map(run, compile_cmds))
-        run(link)
+            list(ex.map(lambda c: _run(c, verbose), compile_cmds))
+        _run(link, verbose)
     os.replace(tmp_path, _LIB_PATH)
-    return _LIB_PATH
 
 
 def _load():
@@ -184,7 +235,7 @@ def _load():
             # Sources are newer than the library only on a developer's machine; the
             # shipped .so is used as is when no compiler is around.
             if _stale() and os.path.exists(_nvcc()):
-                build()
+                _build_lib()
             lib = C.CDLL(_LIB_PATH)
             for name, (res, args) in EXPORTS.items():
                 fn = getattr(lib, name)
@@ -202,6 +253,28 @@ def lib():
     if _lib is None:
         raise RuntimeError(f'libulm_b200.so is unavailable: {_error}')
     return _lib
+
+
+def ext():
+    """The torch extension over the library (csrc/torch_ops.cpp), or raise."""
+    return _ext if _ext is not None else _load_ext()
+
+
+def _load_ext():
+    global _ext
+    lib()                                                  # builds and checks the library it links
+    with _lock:
+        if _ext is None:
+            if _ext_stale() and os.path.exists(_nvcc()):
+                _build_ext()
+            import importlib.util
+
+            import torch  # noqa: F401 - the extension's symbols resolve against the loaded torch libraries
+            spec = importlib.util.spec_from_file_location('_ulm_torch', _EXT_PATH)
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            _ext = mod
+    return _ext
 
 
 def available() -> bool:

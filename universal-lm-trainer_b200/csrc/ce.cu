@@ -135,6 +135,39 @@ ce_bwd_kernel(T* __restrict__ logits, const int64_t* __restrict__ target, const 
   }
 }
 
+// Mean of the row losses in one CTA and a fixed order: loss = sum / denominator, inv = 1 / denominator; the
+// denominator is *denom_dev, denom when that is positive, or the number of targets != ignore_index (at least 1).
+// One launch for what took a compare, two reductions, a clamp, a cast and a division; 12 bytes per row, so one CTA's
+// latency (about 5 us at 32768 rows) is all it costs.
+constexpr int kMeanThreads = 1024;
+__global__ void __launch_bounds__(kMeanThreads)
+loss_mean_kernel(const float* __restrict__ rows_loss, const int64_t* __restrict__ target, int64_t rows, int64_t ignore_index,
+                 const float* __restrict__ denom_dev, float denom, float* __restrict__ loss, float* __restrict__ inv) {
+  float s = 0.f;
+  int n = 0;
+  const bool count = !denom_dev && !(denom > 0.f);
+#pragma unroll 4
+  for (int64_t r = threadIdx.x; r < rows; r += kMeanThreads) {
+    s += rows_loss[r];
+    if (count) n += target[r] != ignore_index;
+  }
+  s = warp_sum(s);
+  n = __reduce_add_sync(0xffffffffu, n);
+  __shared__ float ss[kMeanThreads / 32];
+  __shared__ int sn[kMeanThreads / 32];
+  if ((threadIdx.x & 31) == 0) { ss[threadIdx.x >> 5] = s; sn[threadIdx.x >> 5] = n; }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = warp_sum(ss[threadIdx.x]);
+    n = __reduce_add_sync(0xffffffffu, sn[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      const float d = denom_dev ? *denom_dev : count ? (float)(n > 0 ? n : 1) : denom;
+      *loss = s / d;
+      *inv = 1.f / d;
+    }
+  }
+}
+
 int check(const char* who, const void* logits, const void* target, const void* lse, int64_t row_stride,
           int64_t rows, int V, int dtype) {
   if (dtype != ULM_F16 && dtype != ULM_BF16 && dtype != ULM_F32) return fail(ULM_ERR_ARG, "%s: bad dtype", who);
@@ -174,4 +207,14 @@ extern "C" int ulm_ce_bwd(const ulm_ce_bwd_args* a) {
   if (a->dtype == ULM_F16) ULM_CE_BWD(__half); else if (a->dtype == ULM_BF16) ULM_CE_BWD(__nv_bfloat16); else ULM_CE_BWD(float);
 #undef ULM_CE_BWD
   return check_launch("ulm_ce_bwd");
+}
+
+extern "C" int ulm_loss_mean(const float* rows_loss, const int64_t* target, int64_t rows, int64_t ignore_index, const float* denom_dev,
+                             float denom, float* loss, float* inv, void* stream) {
+  using namespace ulm;
+  if (rows < 0) return fail(ULM_ERR_ARG, "ulm_loss_mean: negative rows");
+  if (rows > 0x7fffffffLL) return fail(ULM_ERR_TOO_LARGE, "ulm_loss_mean: more than 2^31-1 rows");
+  if ((rows > 0 && (!rows_loss || !target)) || !loss || !inv) return fail(ULM_ERR_ARG, "ulm_loss_mean: null pointer");
+  loss_mean_kernel<<<1, kMeanThreads, 0, (cudaStream_t)stream>>>(rows_loss, target, rows, ignore_index, denom_dev, denom, loss, inv);
+  return check_launch("ulm_loss_mean");
 }

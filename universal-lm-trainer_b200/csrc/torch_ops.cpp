@@ -1,0 +1,839 @@
+// The host side of the ops as native autograd functions: argument checks, output allocation, the C-ABI call
+// (include/ulm_b200.h) and the backward's node, without the interpreter.
+//
+// What bounds a small call is this path and not the kernels: at 4 x 201 tokens the six kernels of RoPE + attention
+// forward and backward take 35 us on the device, while the same ops written as Python autograd functions over
+// ctypes kept the host busy for 310 us (argument structs, shape and stride queries, an interpreter lock per
+// backward node).  The Python modules keep their functions and their documentation and forward to this file; the
+// semantics of every op are documented there.
+//
+// Nothing here computes: every kernel is the library's, plus the library GEMMs of the linear layers.
+#include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <atomic>
+#include <memory>
+#include <mutex>
+#include <unordered_map>
+#include <utility>
+#include <vector>
+
+#include "../../include/ulm_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+void check(int rc, const char* what) {
+  if (rc == ULM_OK) return;
+  const char* msg = ulm_last_error();
+  TORCH_CHECK_VALUE(rc != ULM_ERR_ARG, what, ": ", msg);
+  TORCH_CHECK(false, what, ": ", msg, " (code ", rc, ")");
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+bool is_16bit(at::ScalarType t) { return t == at::kHalf || t == at::kBFloat16; }
+int code_of(at::ScalarType t) { return t == at::kHalf ? ULM_F16 : t == at::kBFloat16 ? ULM_BF16 : ULM_F32; }
+bool known(at::ScalarType t) { return is_16bit(t) || t == at::kFloat; }
+
+// Device tensors straight from the caching allocator: no dispatcher round trip.
+Tensor empty_strided(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType dtype, const Tensor& like) {
+  return at::detail::empty_strided_cuda(sizes, strides, dtype, like.device());
+}
+Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType dtype, const Tensor& like) {
+  return at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt);
+}
+// (B,H,S,64) stored as (B,S,H,64)
+Tensor empty_bshd(int64_t B, int64_t H, int64_t S, const Tensor& like) {
+  return empty_strided({B, H, S, 64}, {S * H * 64, 64, H * 64, 1}, like.scalar_type(), like);
+}
+
+// True when the call will not be differentiated: the op then runs without a graph node.
+template <typename... Ts>
+bool no_graph(const Ts&... ts) {
+  return !at::GradMode::is_enabled() || !(ts.requires_grad() || ...);
+}
+
+// Base of the ops' backward nodes: the tensors they keep, unpacked through autograd's own saved variables (version
+// checks, saved-tensor hooks, release after the backward).
+struct OpNode : torch::autograd::Node {
+  std::vector<torch::autograd::SavedVariable> saved;
+  void keep(const Tensor& t, bool is_output = false) { saved.emplace_back(t, is_output); }
+  Tensor kept(size_t i) { return saved[i].unpack(getptr()); }
+  void release_variables() override {
+    for (auto& s : saved) s.reset_data();
+  }
+};
+// The node's edges to the inputs that may receive a gradient, in the order `apply` returns them.
+template <typename N, typename... Ts>
+std::shared_ptr<N> make_node(const Ts&... inputs) {
+  std::shared_ptr<N> n(new N(), torch::autograd::deleteNode);
+  n->set_next_edges(torch::autograd::collect_next_edges(inputs...));
+  return n;
+}
+// What surrounds every op's own work: no recording below it and no autocast of the tensors it has already cast.
+struct OpScope {
+  at::NoGradGuard no_grad;
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
+};
+
+// ---------------------------------------------------------------------------
+// status word: one int32 per device that the kernels OR their timeout bits into
+// ---------------------------------------------------------------------------
+constexpr int kMaxDevices = 64;
+std::mutex g_status_mu;
+std::atomic<uint32_t*> g_status_ptr[kMaxDevices];
+Tensor* g_status[kMaxDevices];                   // never destroyed: no exit-order hazards
+
+Tensor status_tensor(int64_t index) {
+  TORCH_CHECK(index >= 0 && index < kMaxDevices, "device index ", index, " beyond ", kMaxDevices - 1);
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  if (!g_status[index]) {
+    g_status[index] = new Tensor(at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, (c10::DeviceIndex)index)));
+    g_status_ptr[index].store(static_cast<uint32_t*>(g_status[index]->data_ptr()), std::memory_order_release);
+  }
+  return *g_status[index];
+}
+uint32_t* status_ptr(const Tensor& t) {
+  const int i = t.device().index();
+  uint32_t* p = g_status_ptr[i].load(std::memory_order_acquire);
+  return p ? p : (status_tensor(i), g_status_ptr[i].load(std::memory_order_acquire));
+}
+
+// ---------------------------------------------------------------------------
+// attention and RoPE
+// ---------------------------------------------------------------------------
+// (B,H,S,64) 16-bit, innermost contiguous, 32-byte aligned base and strides
+bool fa_ready(const Tensor& t) {
+  if (!t.is_cuda() || !is_16bit(t.scalar_type()) || t.dim() != 4) return false;
+  const auto n = t.sizes(), s = t.strides();
+  if (n[3] != 64 || s[3] != 1 || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 31)) return false;
+  for (int i = 0; i < 3; ++i)
+    if (s[i] % 16 || (s[i] <= 0 && n[i] != 1)) return false;
+  return n[2] == 1 || s[2] >= 64;
+}
+bool can_use(const Tensor& q, const Tensor& k, const Tensor& v) {
+  return fa_ready(q) && fa_ready(k) && fa_ready(v) && q.sizes() == k.sizes() && k.sizes() == v.sizes() &&
+         q.scalar_type() == k.scalar_type() && k.scalar_type() == v.scalar_type();
+}
+bool table_ok(const Tensor& t, int64_t rows, const Tensor& like) {
+  return t.scalar_type() == at::kFloat && t.device() == like.device() && t.dim() == 2 && t.size(0) == rows && t.size(1) == 64 &&
+         t.stride(1) == 1 && t.stride(0) % 4 == 0 && !(reinterpret_cast<uintptr_t>(t.data_ptr()) & 15);
+}
+bool rope_can_use(const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin) {
+  return fa_ready(q) && fa_ready(k) && q.sizes() == k.sizes() && q.scalar_type() == k.scalar_type() &&
+         table_ok(cos, q.size(2), q) && table_ok(sin, q.size(2), q);
+}
+
+// Dense output in the input's memory order: fused-qkv views come back as (B,S,H,64)-ordered tensors
+Tensor rope_out_like(at::IntArrayRef n, at::IntArrayRef s, const Tensor& like) {
+  int64_t extent = 1, numel = 1;
+  for (int i = 0; i < 4; ++i) { extent += (n[i] - 1) * s[i]; numel *= n[i]; }
+  if (extent == numel) return empty_strided(n, s, like.scalar_type(), like);
+  if (s[1] == n[3] && s[2] >= n[1] * n[3]) return empty_bshd(n[0], n[1], n[2], like);
+  return empty_cuda(n, like.scalar_type(), like);
+}
+
+// q (and qo) may be undefined: only k is rotated then
+void rope_launch(const Tensor& q, const Tensor& k, const Tensor& qo, const Tensor& ko, const Tensor& cos, const Tensor& sin, bool backward) {
+  ulm_rope_args a{};
+  a.k = k.data_ptr(); a.ko = ko.data_ptr();
+  a.k_sb = k.stride(0); a.k_sh = k.stride(1); a.k_ss = k.stride(2);
+  a.ko_sb = ko.stride(0); a.ko_sh = ko.stride(1); a.ko_ss = ko.stride(2);
+  if (q.defined()) {
+    a.q = q.data_ptr(); a.qo = qo.data_ptr();
+    a.q_sb = q.stride(0); a.q_sh = q.stride(1); a.q_ss = q.stride(2);
+    a.qo_sb = qo.stride(0); a.qo_sh = qo.stride(1); a.qo_ss = qo.stride(2);
+  }
+  a.cos_tab = cos.data_ptr<float>(); a.sin_tab = sin.data_ptr<float>();
+  a.cos_stride = cos.stride(0); a.sin_stride = sin.stride(0);
+  a.B = (int32_t)k.size(0); a.H = (int32_t)k.size(1); a.S = (int32_t)k.size(2);
+  a.dtype = code_of(k.scalar_type()); a.backward = backward;
+  a.stream = stream_of(k);
+  check(ulm_rope(&a), "rope");
+}
+
+struct AttnArgs {
+  double dropout_p; bool causal; double scale; int64_t seed;
+};
+
+// -> (o, lse); with tables q comes unrotated and, where q_rot is defined, its rotated copy is written there
+void attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const AttnArgs& p,
+                  const Tensor& cos = Tensor(), const Tensor& sin = Tensor(), const Tensor& q_rot = Tensor()) {
+  ulm_attn_fwd_args a{};
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.lse = lse.data_ptr<float>();
+  a.q_sb = q.stride(0); a.q_sh = q.stride(1); a.q_ss = q.stride(2);
+  a.k_sb = k.stride(0); a.k_sh = k.stride(1); a.k_ss = k.stride(2);
+  a.v_sb = v.stride(0); a.v_sh = v.stride(1); a.v_ss = v.stride(2);
+  a.o_sb = o.stride(0); a.o_sh = o.stride(1); a.o_ss = o.stride(2);
+  a.B = (int32_t)q.size(0); a.H = (int32_t)q.size(1); a.S = (int32_t)q.size(2);
+  a.dtype = code_of(q.scalar_type()); a.causal = p.causal;
+  a.softmax_scale = (float)p.scale; a.dropout_p = (float)p.dropout_p; a.seed = (uint32_t)p.seed;
+  a.status_dev = status_ptr(q); a.stream = stream_of(q);
+  if (cos.defined()) {
+    a.cos_tab = cos.data_ptr<float>(); a.sin_tab = sin.data_ptr<float>();
+    a.cos_stride = cos.stride(0); a.sin_stride = sin.stride(0);
+    if (q_rot.defined()) {
+      a.q_rot = q_rot.data_ptr();
+      a.qr_sb = q_rot.stride(0); a.qr_sh = q_rot.stride(1); a.qr_ss = q_rot.stride(2);
+    }
+  }
+  check(ulm_attn_fwd(&a), "flash_attn_v100 forward");
+}
+
+void attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o_in, const Tensor& lse, const Tensor& do_in,
+                   const Tensor& dq, const Tensor& dk, const Tensor& dv, const AttnArgs& p, const Tensor& cos = Tensor(), const Tensor& sin = Tensor()) {
+  const Tensor go = fa_ready(do_in) ? do_in : do_in.contiguous(), o = fa_ready(o_in) ? o_in : o_in.contiguous();
+  const Tensor delta = empty_cuda({q.size(0), q.size(1), q.size(2)}, at::kFloat, q);
+  ulm_attn_bwd_args a{};
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.d_o = go.data_ptr();
+  a.lse = lse.data_ptr<float>(); a.delta = delta.data_ptr<float>();
+  a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr();
+  a.q_sb = q.stride(0); a.q_sh = q.stride(1); a.q_ss = q.stride(2);
+  a.k_sb = k.stride(0); a.k_sh = k.stride(1); a.k_ss = k.stride(2);
+  a.v_sb = v.stride(0); a.v_sh = v.stride(1); a.v_ss = v.stride(2);
+  a.o_sb = o.stride(0); a.o_sh = o.stride(1); a.o_ss = o.stride(2);
+  a.do_sb = go.stride(0); a.do_sh = go.stride(1); a.do_ss = go.stride(2);
+  a.dq_sb = dq.stride(0); a.dq_sh = dq.stride(1); a.dq_ss = dq.stride(2);
+  a.dk_sb = dk.stride(0); a.dk_sh = dk.stride(1); a.dk_ss = dk.stride(2);
+  a.dv_sb = dv.stride(0); a.dv_sh = dv.stride(1); a.dv_ss = dv.stride(2);
+  a.B = (int32_t)q.size(0); a.H = (int32_t)q.size(1); a.S = (int32_t)q.size(2);
+  a.dtype = code_of(q.scalar_type()); a.causal = p.causal; a.mode = 7;
+  a.softmax_scale = (float)p.scale; a.dropout_p = (float)p.dropout_p; a.seed = (uint32_t)p.seed;
+  a.status_dev = status_ptr(q); a.stream = stream_of(q);
+  if (cos.defined()) {
+    a.cos_tab = cos.data_ptr<float>(); a.sin_tab = sin.data_ptr<float>();
+    a.cos_stride = cos.stride(0); a.sin_stride = sin.stride(0);
+  }
+  check(ulm_attn_bwd(&a), "flash_attn_v100 backward");
+}
+
+Tensor empty_lse(const Tensor& q) { return empty_cuda({q.size(0), q.size(1), q.size(2)}, at::kFloat, q); }
+
+// dq, dk, dv of one allocation, each (B,H,S,64) stored as (B,S,H,64)
+std::array<Tensor, 3> empty_grads(const Tensor& q) {
+  const int64_t B = q.size(0), H = q.size(1), S = q.size(2), n = B * H * S * 64;
+  const Tensor buf = empty_cuda({3 * n}, q.scalar_type(), q);
+  std::array<Tensor, 3> out;
+  for (int i = 0; i < 3; ++i) out[i] = buf.as_strided({B, H, S, 64}, {S * H * 64, 64, H * 64, 1}, i * n);
+  return out;
+}
+
+struct RopeBwd : OpNode {
+  std::vector<int64_t> n, qs, ks;                          // shape and input strides
+  variable_list apply(variable_list&& g) override {
+    OpScope scope;
+    const bool has_q = g[0].defined(), has_k = g[1].defined();
+    if (!has_q && !has_k) return {Tensor(), Tensor()};
+    auto ready = [](const Tensor& t) {
+      return t.stride(3) == 1 && !(reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && t.stride(2) % 8 == 0;
+    };
+    const Tensor cos = kept(0), sin = kept(1);
+    Tensor in[2], out[2];
+    for (int i = 0; i < 2; ++i)
+      if (g[i].defined()) {
+        in[i] = ready(g[i]) ? g[i] : g[i].contiguous();
+        out[i] = rope_out_like(n, i ? ks : qs, in[i]);
+      }
+    // a branch whose output went unused has a zero gradient: only the other one is rotated
+    if (has_k) rope_launch(in[0], in[1], out[0], out[1], cos, sin, true);
+    else rope_launch(Tensor(), in[0], Tensor(), out[0], cos, sin, true);
+    for (int i = 0; i < 2; ++i)
+      if (!out[i].defined() && task_should_compute_output(i)) out[i] = rope_out_like(n, i ? ks : qs, in[1 - i]).zero_();
+    return {out[0], out[1]};
+  }
+};
+
+std::tuple<Tensor, Tensor> rope(const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin) {
+  TORCH_CHECK_VALUE(q.is_cuda() && k.is_cuda() && is_16bit(q.scalar_type()) && q.dim() == 4 && k.dim() == 4 && q.sizes() == k.sizes() && q.scalar_type() == k.scalar_type(),
+                    "rope needs CUDA fp16/bf16 (B,H,S,64) tensors of one shape");
+  Tensor qo, ko;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(q.device());
+    qo = rope_out_like(q.sizes(), q.strides(), q);
+    ko = rope_out_like(k.sizes(), k.strides(), k);
+    rope_launch(q, k, qo, ko, cos, sin, false);
+  }
+  if (!no_graph(q, k)) {
+    auto node = make_node<RopeBwd>(q, k);
+    node->n = q.sizes().vec(); node->qs = q.strides().vec(); node->ks = k.strides().vec();
+    node->keep(cos); node->keep(sin);
+    torch::autograd::set_history(qo, node);
+    torch::autograd::set_history(ko, node);
+  }
+  return {qo, ko};
+}
+
+struct FlashBwd : OpNode {
+  AttnArgs p{};
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    OpScope scope;
+    const Tensor q = kept(0);
+    auto d = empty_grads(q);
+    attn_backward(q, kept(1), kept(2), kept(3), kept(4), g[0], d[0], d[1], d[2], p);
+    return {d[0], d[1], d[2]};
+  }
+};
+
+Tensor flash_attn(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, double dropout_p, bool causal, double scale, int64_t seed) {
+  TORCH_CHECK_VALUE(q_in.is_cuda() && is_16bit(q_in.scalar_type()) && q_in.dim() == 4 && q_in.size(3) == 64,
+                    "flash_attn_v100 needs CUDA fp16/bf16 inputs with head_dim 64");
+  const Tensor q = fa_ready(q_in) ? q_in : q_in.contiguous(), k = fa_ready(k_in) ? k_in : k_in.contiguous(), v = fa_ready(v_in) ? v_in : v_in.contiguous();
+  const AttnArgs p{dropout_p, causal, scale, seed};
+  Tensor o, lse;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(q.device());
+    o = empty_bshd(q.size(0), q.size(1), q.size(2), q);
+    lse = empty_lse(q);
+    attn_forward(q, k, v, o, lse, p);
+  }
+  if (!no_graph(q, k, v)) {
+    auto node = make_node<FlashBwd>(q, k, v);
+    node->p = p;
+    torch::autograd::set_history(o, node);
+    node->keep(q); node->keep(k); node->keep(v); node->keep(o, true); node->keep(lse);
+  }
+  return o;
+}
+
+// Where the RoPE work runs: 0 stand-alone kernels, 1 Q rotated inside the forward, 2 also the adjoint behind the
+// backward kernels.  All give the same bits.
+enum Fuse : int64_t { kFuseNone = 0, kFuseFwd = 1, kFuseAll = 2 };
+
+// o and lse are written; returns the rotated (q, k)
+std::pair<Tensor, Tensor> rope_attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cos, const Tensor& sin,
+                                            const Tensor& o, const Tensor& lse, const AttnArgs& p, int64_t fuse) {
+  const Tensor ko = rope_out_like(k.sizes(), k.strides(), k);
+  Tensor qo;
+  if (fuse == kFuseNone) {
+    qo = rope_out_like(q.sizes(), q.strides(), q);
+    rope_launch(q, k, qo, ko, cos, sin, false);
+    attn_forward(qo, ko, v, o, lse, p);
+  } else {
+    qo = empty_bshd(q.size(0), q.size(1), q.size(2), q);
+    rope_launch(Tensor(), k, Tensor(), ko, cos, sin, false);
+    attn_forward(q, ko, v, o, lse, p, cos, sin, qo);
+  }
+  return {qo, ko};
+}
+
+// gradients of the UNROTATED q, k and of v.  The stand-alone adjoint runs in place: a thread reads both halves of
+// what it rotates before it writes them, and the 16-bit gradients need no second buffer.
+void rope_attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go,
+                        const Tensor& cos, const Tensor& sin, const Tensor& dq, const Tensor& dk, const Tensor& dv, const AttnArgs& p, int64_t fuse) {
+  if (!cos.defined()) { attn_backward(q, k, v, o, lse, go, dq, dk, dv, p); return; }
+  if (fuse == kFuseAll) { attn_backward(q, k, v, o, lse, go, dq, dk, dv, p, cos, sin); return; }
+  attn_backward(q, k, v, o, lse, go, dq, dk, dv, p);
+  rope_launch(dq, dk, dq, dk, cos, sin, true);
+}
+
+struct RopeFlashBwd : OpNode {
+  AttnArgs p{};
+  int64_t fuse = 0;
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    OpScope scope;
+    const Tensor q = kept(0);
+    auto d = empty_grads(q);
+    rope_attn_backward(q, kept(1), kept(2), kept(3), kept(4), g[0], kept(5), kept(6), d[0], d[1], d[2], p, fuse);
+    return {d[0], d[1], d[2]};
+  }
+};
+
+Tensor rope_flash_attn(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cos, const Tensor& sin, double dropout_p, bool causal,
+                       double scale, int64_t seed, int64_t fuse) {
+  TORCH_CHECK_VALUE(rope_can_use(q, k, cos, sin) && can_use(q, k, v), "rope_flash_attn needs 16-bit (B,H,S,64) CUDA views and fp32 (S,64) tables");
+  const AttnArgs p{dropout_p, causal, scale, seed};
+  Tensor o, lse, qr, kr;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(q.device());
+    o = empty_bshd(q.size(0), q.size(1), q.size(2), q);
+    lse = empty_lse(q);
+    std::tie(qr, kr) = rope_attn_forward(q, k, v, cos, sin, o, lse, p, fuse);
+  }
+  if (!no_graph(q, k, v)) {
+    auto node = make_node<RopeFlashBwd>(q, k, v);
+    node->p = p; node->fuse = fuse;
+    torch::autograd::set_history(o, node);
+    node->keep(qr); node->keep(kr); node->keep(v); node->keep(o, true); node->keep(lse); node->keep(cos); node->keep(sin);
+  }
+  return o;
+}
+
+// Third `i` (0 q, 1 k, 2 v) of the first B*S rows of a contiguous [.., 3*H*64] tensor as a (B,H,S,64) view
+Tensor qkv_part(const Tensor& qkv, int i, int64_t B, int64_t S, int64_t H) {
+  const int64_t w = 3 * H * 64;
+  return qkv.as_strided({B, H, S, 64}, {S * w, 64, w, 1}, qkv.storage_offset() + i * H * 64);
+}
+// the first B*S rows of a contiguous [.., H*64] tensor as a (B,H,S,64) view
+Tensor heads_of(const Tensor& x, int64_t B, int64_t S, int64_t H) {
+  return x.as_strided({B, H, S, 64}, {S * H * 64, 64, H * 64, 1}, x.storage_offset());
+}
+
+struct QkvBwd : OpNode {
+  AttnArgs p{};
+  int64_t fuse = 0, B = 0, S = 0, H = 0, rows = -1;        // rows >= 0: the flattened form with padding rows
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor()};
+    OpScope scope;
+    const Tensor qkv = kept(0), cos = kept(5), sin = kept(6);
+    const Tensor q = cos.defined() ? kept(1) : qkv_part(qkv, 0, B, S, H), k = cos.defined() ? kept(2) : qkv_part(qkv, 1, B, S, H);
+    const Tensor go = heads_of(g[0].contiguous(), B, S, H);
+    const Tensor d = empty_cuda(qkv.sizes(), qkv.scalar_type(), qkv);
+    if (rows > B * S) d.narrow(0, B * S, rows - B * S).zero_();
+    rope_attn_backward(q, k, qkv_part(qkv, 2, B, S, H), heads_of(kept(3), B, S, H), kept(4), go, cos, sin,
+                       qkv_part(d, 0, B, S, H), qkv_part(d, 1, B, S, H), qkv_part(d, 2, B, S, H), p, fuse);
+    return {d};
+  }
+};
+
+Tensor qkv_attn(const Tensor& qkv, int64_t H, const OptTensor& cos_o, const OptTensor& sin_o, double dropout_p, bool causal, double scale,
+                int64_t seed, int64_t fuse, int64_t flat_b, int64_t flat_s) {
+  const bool flat = flat_b >= 0;
+  TORCH_CHECK_VALUE(!flat || (qkv.dim() == 2 && qkv.size(0) >= flat_b * flat_s), "flat_shape=(n, L) needs a 2-D qkv with at least n*L rows");
+  TORCH_CHECK_VALUE(qkv.is_cuda() && is_16bit(qkv.scalar_type()) && (flat || qkv.dim() == 3) && qkv.is_contiguous() && qkv.size(-1) == 3 * H * 64 &&
+                        !(reinterpret_cast<uintptr_t>(qkv.data_ptr()) & 31),
+                    "qkv_rope_flash_attn needs a contiguous CUDA fp16/bf16 [n, L, 3*n_heads*64] tensor");
+  const int64_t B = flat ? flat_b : qkv.size(0), S = flat ? flat_s : qkv.size(1), rows = flat ? qkv.size(0) : -1;
+  const Tensor cos = cos_o.value_or(Tensor()), sin = sin_o.value_or(Tensor());
+  TORCH_CHECK_VALUE(cos.defined() == sin.defined(), "cos2d and sin2d must be given together");
+  TORCH_CHECK_VALUE(!cos.defined() || (table_ok(cos, S, qkv) && table_ok(sin, S, qkv)),
+                    "RoPE tables must be fp32 (L,64) views on the same device, 16-byte aligned rows");
+  const AttnArgs p{dropout_p, causal, scale, seed};
+  Tensor out, lse, qr, kr;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(qkv.device());
+    out = flat ? empty_cuda({rows, H * 64}, qkv.scalar_type(), qkv) : empty_cuda({B, S, H * 64}, qkv.scalar_type(), qkv);
+    if (rows > B * S) out.narrow(0, B * S, rows - B * S).zero_();
+    const Tensor o = heads_of(out, B, S, H), v = qkv_part(qkv, 2, B, S, H);
+    const Tensor q = qkv_part(qkv, 0, B, S, H), k = qkv_part(qkv, 1, B, S, H);
+    lse = empty_lse(q);
+    if (cos.defined()) std::tie(qr, kr) = rope_attn_forward(q, k, v, cos, sin, o, lse, p, fuse);
+    else attn_forward(q, k, v, o, lse, p);
+  }
+  if (!no_graph(qkv)) {
+    auto node = make_node<QkvBwd>(qkv);
+    node->p = p; node->fuse = fuse; node->B = B; node->S = S; node->H = H; node->rows = rows;
+    torch::autograd::set_history(out, node);
+    node->keep(qkv); node->keep(qr); node->keep(kr); node->keep(out, true); node->keep(lse); node->keep(cos); node->keep(sin);
+  }
+  return out;
+}
+
+// Forward alone, nothing kept: Q is rotated inside the kernel and its rotated copy is never written.
+std::tuple<Tensor, Tensor, Tensor> causal_attention(const Tensor& qkv_in, int64_t H, const OptTensor& cos_o, const OptTensor& sin_o, double scale) {
+  OpScope scope;
+  const Tensor qkv = qkv_in.detach();
+  TORCH_CHECK_VALUE(qkv.is_cuda() && is_16bit(qkv.scalar_type()) && qkv.dim() == 3 && qkv.is_contiguous() && qkv.size(2) == 3 * H * 64,
+                    "causal_attention needs a contiguous CUDA fp16/bf16 [n, L, 3*n_heads*64] tensor");
+  c10::cuda::CUDAGuard dev(qkv.device());
+  const int64_t B = qkv.size(0), S = qkv.size(1);
+  const Tensor q = qkv_part(qkv, 0, B, S, H), v = qkv_part(qkv, 2, B, S, H), out = empty_cuda({B, S, H * 64}, qkv.scalar_type(), qkv);
+  Tensor k = qkv_part(qkv, 1, B, S, H), cos, sin;
+  const Tensor lse = empty_lse(q);
+  const AttnArgs p{0.0, true, scale, 0};
+  if (cos_o) {
+    // the model's [1, L, >=64] or [L, >=64] tables
+    auto table = [&](const Tensor& t) {
+      const Tensor t2 = t.reshape({-1, t.size(-1)});
+      return t2.size(0) >= S && t2.size(1) >= 64 ? t2.narrow(0, 0, S).narrow(1, 0, 64) : t2;
+    };
+    cos = table(*cos_o); sin = table(*sin_o);
+    TORCH_CHECK_VALUE(rope_can_use(q, k, cos, sin), "causal_attention needs fp32 RoPE tables of at least 64 columns on the same device");
+    const Tensor ko = rope_out_like(k.sizes(), k.strides(), k);
+    rope_launch(Tensor(), k, Tensor(), ko, cos, sin, false);
+    k = ko;
+  }
+  attn_forward(q, k, v, heads_of(out, B, S, H), lse, p, cos, sin);
+  return {out, k, v};
+}
+
+// ---------------------------------------------------------------------------
+// RMSNorm, SwiGLU
+// ---------------------------------------------------------------------------
+// [.., d] as [rows, d] with contiguous 16-byte aligned rows
+Tensor rows_of(const Tensor& x) {
+  const Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
+  const bool ok = x2.stride(1) == 1 && !(reinterpret_cast<uintptr_t>(x2.data_ptr()) & 15) && (x2.stride(0) * x2.element_size()) % 16 == 0;
+  return ok ? x2 : x2.contiguous();
+}
+int y_kind(at::ScalarType y, at::ScalarType x) { return y == x ? ULM_Y_SAME : y == at::kHalf ? ULM_Y_F16 : ULM_Y_BF16; }
+
+// dx (and d_branch) and dw of one norm; ga: the gradient reaching the normalised tensor from elsewhere
+Tensor norm_backward(const Tensor& x, const Tensor& w, const Tensor& rstd, const Tensor& dy, double eps, int kind, const Tensor& dx,
+                     const Tensor& ga, const Tensor& d_branch) {
+  const int64_t rows = x.size(0), d = x.size(1);
+  const Tensor dw = empty_cuda({d}, at::kFloat, x);
+  const Tensor partial = empty_cuda({ulm_rmsnorm_bwd_partial_rows(rows), d}, at::kFloat, x);
+  ulm_rmsnorm_bwd_args a{};
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.dy = dy.data_ptr(); a.rstd = rstd.data_ptr<float>();
+  a.dx = dx.data_ptr(); a.dw = dw.data_ptr<float>(); a.partial = partial.data_ptr<float>();
+  a.x_stride = x.stride(0); a.dy_stride = dy.stride(0); a.dx_stride = dx.stride(0);
+  a.rows = rows; a.d = (int32_t)d; a.x_dtype = code_of(x.scalar_type()); a.w_dtype = code_of(w.scalar_type());
+  a.eps = (float)eps; a.stream = stream_of(x); a.dy_kind = kind;
+  if (ga.defined()) { a.g_add = ga.data_ptr(); a.gadd_stride = ga.stride(0); }
+  if (d_branch.defined()) { a.d_branch = d_branch.data_ptr(); a.dbranch_stride = d_branch.stride(0); }
+  check(ulm_rmsnorm_bwd(&a), d_branch.defined() ? "add_rms_norm backward" : "rms_norm backward");
+  return dw;
+}
+
+struct NormBwd : OpNode {
+  double eps = 0;
+  std::vector<int64_t> shape;
+  at::ScalarType wdtype, ydtype;
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor(), Tensor()};
+    OpScope scope;
+    const Tensor x = kept(0), w = kept(1), rstd = kept(2);
+    const Tensor dy = rows_of(g[0].to(ydtype)), dx = empty_cuda({x.size(0), x.size(1)}, x.scalar_type(), x);
+    const Tensor dw = norm_backward(x, w, rstd, dy, eps, y_kind(ydtype, x.scalar_type()), dx, Tensor(), Tensor());
+    return {dx.view(shape), dw.to(wdtype)};
+  }
+};
+
+Tensor rms_norm(const Tensor& x, const Tensor& weight, double eps, std::optional<at::ScalarType> out_dtype) {
+  TORCH_CHECK_VALUE(x.is_cuda() && known(x.scalar_type()), "rms_norm needs a CUDA fp16/bf16/fp32 tensor");
+  at::ScalarType yt = x.scalar_type();
+  if (out_dtype) yt = *out_dtype;
+  else if (yt == at::kFloat && at::autocast::is_autocast_enabled(at::kCUDA)) yt = at::autocast::get_autocast_dtype(at::kCUDA);
+  TORCH_CHECK_VALUE(yt == x.scalar_type() || (x.scalar_type() == at::kFloat && is_16bit(yt)),
+                    "rms_norm: a different output dtype needs an fp32 input and a 16-bit output");
+  Tensor y, x2, w, rstd;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(x.device());
+    x2 = rows_of(x);
+    const int64_t rows = x2.size(0), d = x2.size(1);
+    y = empty_cuda(x.sizes(), yt, x);
+    rstd = empty_cuda({rows}, at::kFloat, x);
+    w = weight.scalar_type() == x.scalar_type() || weight.scalar_type() == at::kFloat ? weight : weight.to(at::kFloat);
+    w = w.contiguous();
+    ulm_rmsnorm_fwd_args a{};
+    a.x = x2.data_ptr(); a.w = w.data_ptr(); a.y = y.data_ptr(); a.rstd = rstd.data_ptr<float>();
+    a.x_stride = x2.stride(0); a.y_stride = d; a.rows = rows; a.d = (int32_t)d;
+    a.x_dtype = code_of(x.scalar_type()); a.w_dtype = code_of(w.scalar_type()); a.eps = (float)eps; a.stream = stream_of(x);
+    a.y_kind = y_kind(yt, x.scalar_type());
+    check(ulm_rmsnorm_fwd(&a), "rms_norm forward");
+  }
+  if (!no_graph(x, weight)) {
+    auto node = make_node<NormBwd>(x, weight);
+    node->eps = eps; node->shape = x.sizes().vec(); node->wdtype = weight.scalar_type(); node->ydtype = yt;
+    node->keep(x2); node->keep(w); node->keep(rstd);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+struct AddNormBwd : OpNode {
+  double eps = 0;
+  std::vector<int64_t> shape;
+  at::ScalarType wdtype, bdtype;
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined() && !g[1].defined()) return {Tensor(), Tensor(), Tensor()};
+    OpScope scope;
+    if (!g[1].defined()) return {g[0], g[0].to(bdtype), Tensor()};          // the normalised output went unused
+    const Tensor x = kept(0), w = kept(1), rstd = kept(2);
+    const int64_t rows = x.size(0), d = x.size(1);
+    const Tensor dy = rows_of(g[1].to(bdtype)), ga = g[0].defined() ? rows_of(g[0].to(at::kFloat)) : Tensor();
+    const Tensor dx = empty_cuda({rows, d}, at::kFloat, x), db = empty_cuda({rows, d}, bdtype, x);
+    const Tensor dw = norm_backward(x.view({rows, d}), w, rstd, dy, eps, y_kind(bdtype, at::kFloat), dx, ga, db);
+    return {dx.view(shape), db.view(shape), dw.to(wdtype)};
+  }
+};
+
+std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const Tensor& branch, const Tensor& weight, double eps) {
+  TORCH_CHECK_VALUE(x.is_cuda() && x.scalar_type() == at::kFloat && is_16bit(branch.scalar_type()) && branch.sizes() == x.sizes(),
+                    "add_rms_norm needs an fp32 CUDA x and a 16-bit branch of the same shape");
+  TORCH_CHECK_VALUE(x.size(-1) <= 1024 && x.size(-1) % 4 == 0, "add_rms_norm takes rows of at most 1024 elements, a multiple of 4");
+  Tensor x_new, y, w, rstd;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(x.device());
+    const Tensor x2 = rows_of(x), b2 = rows_of(branch);
+    const int64_t rows = x2.size(0), d = x2.size(1);
+    x_new = empty_cuda(x.sizes(), at::kFloat, x);
+    y = empty_cuda(x.sizes(), branch.scalar_type(), x);
+    rstd = empty_cuda({rows}, at::kFloat, x);
+    w = weight.to(at::kFloat).contiguous();
+    ulm_rmsnorm_fwd_args a{};
+    a.x = x2.data_ptr(); a.w = w.data_ptr(); a.y = y.data_ptr(); a.rstd = rstd.data_ptr<float>();
+    a.x_stride = x2.stride(0); a.y_stride = d; a.rows = rows; a.d = (int32_t)d;
+    a.x_dtype = ULM_F32; a.w_dtype = ULM_F32; a.eps = (float)eps; a.stream = stream_of(x); a.y_kind = y_kind(branch.scalar_type(), at::kFloat);
+    a.branch = b2.data_ptr(); a.x_out = x_new.data_ptr(); a.branch_stride = b2.stride(0); a.xout_stride = d;
+    check(ulm_rmsnorm_fwd(&a), "add_rms_norm forward");
+  }
+  if (!no_graph(x, branch, weight)) {
+    auto node = make_node<AddNormBwd>(x, branch, weight);
+    node->eps = eps; node->shape = x.sizes().vec(); node->wdtype = weight.scalar_type(); node->bdtype = branch.scalar_type();
+    torch::autograd::set_history(x_new, node);
+    torch::autograd::set_history(y, node);
+    node->keep(x_new, true); node->keep(w); node->keep(rstd);
+  }
+  return {x_new, y};
+}
+
+struct SwigluBwd : OpNode {
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor(), Tensor()};
+    OpScope scope;
+    const Tensor a = kept(0), b = kept(1), dy = g[0].to(a.scalar_type()).contiguous();
+    const Tensor da = empty_cuda(a.sizes(), a.scalar_type(), a), db = empty_cuda(a.sizes(), a.scalar_type(), a);
+    ulm_swiglu_args p{a.data_ptr(), b.data_ptr(), nullptr, dy.data_ptr(), da.data_ptr(), db.data_ptr(), a.numel(), code_of(a.scalar_type()), 0, stream_of(a)};
+    check(ulm_swiglu_bwd(&p), "swiglu backward");
+    return {da, db};
+  }
+};
+
+Tensor swiglu(const Tensor& a_in, const Tensor& b_in) {
+  TORCH_CHECK_VALUE(a_in.is_cuda() && known(a_in.scalar_type()) && b_in.scalar_type() == a_in.scalar_type() && b_in.sizes() == a_in.sizes(),
+                    "swiglu needs two CUDA tensors of one shape and one of fp16/bf16/fp32");
+  Tensor a, b, y;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(a_in.device());
+    a = a_in.contiguous(); b = b_in.contiguous();
+    y = empty_cuda(a.sizes(), a.scalar_type(), a);
+    ulm_swiglu_args p{a.data_ptr(), b.data_ptr(), y.data_ptr(), nullptr, nullptr, nullptr, a.numel(), code_of(a.scalar_type()), 0, stream_of(a)};
+    check(ulm_swiglu_fwd(&p), "swiglu forward");
+  }
+  if (!no_graph(a_in, b_in)) {
+    auto node = make_node<SwigluBwd>(a_in, b_in);
+    node->keep(a); node->keep(b);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+// ---------------------------------------------------------------------------
+// linear layers
+// ---------------------------------------------------------------------------
+std::atomic<bool> g_wgrad_in_place{false};
+
+// Scopes in which the 16-bit copy of a weight is made once and reused (the innermost one counts; an empty stack:
+// nothing is cached).  Keyed by the parameter's implementation object, which a cache entry keeps alive.
+struct CastScope {
+  std::unordered_map<const c10::TensorImpl*, std::pair<Tensor, Tensor>> made;      // parameter, its copy
+};
+std::mutex g_cast_mu;
+std::vector<std::unique_ptr<CastScope>> g_cast_scopes;
+void cast_scope_push() {
+  std::lock_guard<std::mutex> lock(g_cast_mu);
+  g_cast_scopes.push_back(std::make_unique<CastScope>());
+}
+void cast_scope_pop() {
+  std::unique_ptr<CastScope> gone;                       // its tensors are released outside the lock
+  std::lock_guard<std::mutex> lock(g_cast_mu);
+  TORCH_CHECK(!g_cast_scopes.empty(), "no weight-cast scope is active");
+  gone = std::move(g_cast_scopes.back());
+  g_cast_scopes.pop_back();
+}
+Tensor cast_cached(const Tensor& weight, at::ScalarType dtype) {
+  if (weight.scalar_type() == dtype) return weight;
+  const c10::TensorImpl* key = weight.unsafeGetTensorImpl();
+  CastScope* scope = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_cast_mu);
+    if (!g_cast_scopes.empty()) {
+      scope = g_cast_scopes.back().get();
+      auto it = scope->made.find(key);
+      if (it != scope->made.end() && it->second.second.scalar_type() == dtype && it->second.second.device() == weight.device()) return it->second.second;
+    }
+  }
+  const Tensor c = weight.detach().to(dtype);
+  if (scope) {
+    std::lock_guard<std::mutex> lock(g_cast_mu);
+    if (!g_cast_scopes.empty() && g_cast_scopes.back().get() == scope) scope->made[key] = {weight, c};
+  }
+  return c;
+}
+
+// dW = dy^T x for autograd, or an undefined tensor after adding it into weight.grad in place
+Tensor weight_grad(const Tensor& weight, const Tensor& dy, const Tensor& x) {
+  const bool half_gemm = dy.is_cuda() && is_16bit(dy.scalar_type());
+  if (g_wgrad_in_place.load(std::memory_order_relaxed) && half_gemm) {
+    Tensor g = weight.grad();
+    if (g.defined() && g.scalar_type() == at::kFloat && g.is_contiguous()) {
+      at::addmm_out(g, g, dy.t(), x, at::kFloat);
+      return Tensor();
+    }
+  }
+  // fp32 parameters get the fp32 sums directly: no 16-bit rounding and no cast pass
+  if (half_gemm && weight.scalar_type() == at::kFloat) return at::mm(dy.t(), x, at::kFloat);
+  return at::mm(dy.t(), x).to(weight.scalar_type());
+}
+
+struct LinearBwd : OpNode {
+  at::ScalarType cd, x_dtype;
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor(), Tensor()};
+    OpScope scope;
+    const Tensor x = kept(0), weight = kept(1);
+    const Tensor dy = g[0].reshape({-1, g[0].size(-1)}).to(cd);
+    Tensor dx, dw;
+    if (task_should_compute_output(0)) dx = at::mm(dy, cast_cached(weight, cd)).view(x.sizes()).to(x_dtype);
+    if (task_should_compute_output(1)) dw = weight_grad(weight, dy, x.reshape({-1, x.size(-1)}));
+    return {dx, dw};
+  }
+};
+
+Tensor linear(const Tensor& x, const Tensor& weight) {
+  at::ScalarType cd = x.scalar_type();
+  if (x.is_cuda() && at::autocast::is_autocast_enabled(at::kCUDA)) cd = at::autocast::get_autocast_dtype(at::kCUDA);
+  Tensor xc, y;
+  {
+    OpScope scope;
+    c10::OptionalDeviceGuard dev(x.device());
+    xc = x.to(cd);
+    const Tensor wt = cast_cached(weight, cd).t();
+    if (xc.dim() == 2) {
+      y = at::mm(xc, wt);
+    } else {
+      auto n = xc.sizes().vec();
+      n.back() = weight.size(0);
+      y = at::mm(xc.reshape({-1, xc.size(-1)}), wt).view(n);
+    }
+  }
+  if (!no_graph(x, weight)) {
+    auto node = make_node<LinearBwd>(x, weight);
+    node->cd = cd; node->x_dtype = x.scalar_type();
+    node->keep(xc); node->keep(weight);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+// ---------------------------------------------------------------------------
+// lm head + cross-entropy, the form that keeps the 16-bit logits between forward and backward
+// ---------------------------------------------------------------------------
+// -> lse, loss rows (undefined without targets or logits), logits (undefined unless kept)
+std::tuple<Tensor, Tensor, Tensor> lm_head_lse(const Tensor& h, const Tensor& w, const OptTensor& target, int64_t ignore_index, bool keep_logits) {
+  TORCH_CHECK_VALUE(is_16bit(h.scalar_type()) && w.scalar_type() == h.scalar_type(), "lm_head_lse takes fp16 or bf16 operands of one dtype");
+  TORCH_CHECK_VALUE(h.dim() == 2 && w.dim() == 2 && h.size(1) == w.size(1) && h.stride(1) == 1 && w.stride(1) == 1,
+                    "lm_head_lse takes hidden [rows, d] and weight [V, d] with contiguous rows");
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(h.device());
+  const int64_t rows = h.size(0), d = h.size(1), V = w.size(0);
+  const Tensor lse = empty_cuda({rows}, at::kFloat, h);
+  Tensor logits, loss;
+  if (keep_logits) logits = empty_cuda({rows, V}, h.scalar_type(), h);
+  if (keep_logits && target) loss = empty_cuda({rows}, at::kFloat, h);
+  const int64_t n_part = std::max<int64_t>(rows, 1) * ulm_lmhead_lse_parts((int32_t)V);
+  const Tensor part = empty_cuda({2, n_part}, at::kFloat, h);
+  ulm_lmhead_lse_args a{};
+  a.h = h.data_ptr(); a.w = w.data_ptr(); a.lse = lse.data_ptr<float>();
+  if (keep_logits) { a.logits = logits.data_ptr(); a.z_stride = V; }
+  if (loss.defined()) { a.loss = loss.data_ptr<float>(); a.target = target->data_ptr<int64_t>(); }
+  a.part_m = part.data_ptr<float>(); a.part_s = a.part_m + n_part;
+  a.h_stride = h.stride(0); a.w_stride = w.stride(0);
+  a.rows = rows; a.V = (int32_t)V; a.d = (int32_t)d; a.dtype = code_of(h.scalar_type());
+  a.ignore_index = ignore_index; a.status_dev = status_ptr(h); a.stream = stream_of(h);
+  check(ulm_lmhead_lse(&a), "lm-head GEMM + LSE");
+  return {lse, loss, logits};
+}
+
+struct KeptCeBwd : OpNode {
+  int64_t ignore_index = 0;
+  at::ScalarType cd;
+  std::atomic<bool> consumed{false};
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor(), Tensor()};
+    OpScope scope;
+    const Tensor hidden = kept(0), weight = kept(1), target = kept(2), lse = kept(3), logits = kept(4), inv = kept(5), wc = kept(6), hc = kept(7);
+    TORCH_CHECK(!consumed.exchange(true),
+                "chunked_cross_entropy: the kept logits were turned into their gradient in place by the first backward; a second "
+                "backward through the same graph is not supported");
+    const Tensor gs = g[0].to(at::kFloat).mul(inv);                            // d loss / d row loss
+    ulm_ce_bwd_args a{};
+    a.logits = logits.data_ptr(); a.target = target.data_ptr<int64_t>(); a.lse = lse.data_ptr<float>();
+    a.gscale_dev = gs.data_ptr<float>(); a.gscale = 1.f;
+    a.row_stride = logits.stride(0); a.rows = logits.size(0); a.V = (int32_t)logits.size(1); a.dtype = code_of(cd);
+    a.ignore_index = ignore_index; a.stream = stream_of(logits);
+    check(ulm_ce_bwd(&a), "cross-entropy backward");                             // in place over the kept logits
+    Tensor dh, dw;
+    if (task_should_compute_output(0)) dh = at::mm(logits, wc).to(hidden.scalar_type());
+    if (task_should_compute_output(1)) dw = weight_grad(weight, logits, hc);
+    return {dh, dw};
+  }
+};
+
+Tensor kept_cross_entropy(const Tensor& hidden, const Tensor& weight, const Tensor& target, int64_t ignore_index, at::ScalarType cd,
+                          const OptTensor& denom_dev, double denom, bool fused) {
+  Tensor loss, lse, rows_loss, logits, inv, wc, hc;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(hidden.device());
+    wc = cast_cached(weight, cd);
+    hc = hidden.to(cd);
+    if (fused && is_16bit(cd) && hc.size(1) % 64 == 0 && wc.size(0) % 64 == 0 && hc.is_contiguous() && wc.is_contiguous()) {
+      std::tie(lse, rows_loss, logits) = lm_head_lse(hc, wc, target, ignore_index, true);
+    } else {
+      logits = at::mm(hc, wc.t());
+      lse = empty_cuda({logits.size(0)}, at::kFloat, hc);
+      rows_loss = empty_cuda({logits.size(0)}, at::kFloat, hc);
+      ulm_ce_fwd_args a{logits.data_ptr(), target.data_ptr<int64_t>(), lse.data_ptr<float>(), rows_loss.data_ptr<float>(),
+                        logits.stride(0), logits.size(0), (int32_t)logits.size(1), code_of(cd), ignore_index, stream_of(hc)};
+      check(ulm_ce_fwd(&a), "cross-entropy forward");
+    }
+    loss = empty_cuda({}, at::kFloat, hc);                  // sum of the row losses / denominator
+    inv = empty_cuda({}, at::kFloat, hc);                   // 1 / denominator
+    Tensor dd;
+    if (denom_dev) dd = denom_dev->to(hidden.device(), at::kFloat);
+    check(ulm_loss_mean(rows_loss.data_ptr<float>(), target.data_ptr<int64_t>(), rows_loss.size(0), ignore_index,
+                        dd.defined() ? dd.data_ptr<float>() : nullptr, (float)denom, loss.data_ptr<float>(), inv.data_ptr<float>(), stream_of(hc)),
+          "loss mean");
+  }
+  if (!no_graph(hidden, weight)) {
+    auto node = make_node<KeptCeBwd>(hidden, weight);
+    node->ignore_index = ignore_index; node->cd = cd;
+    node->keep(hidden); node->keep(weight); node->keep(target); node->keep(lse); node->keep(logits); node->keep(inv); node->keep(wc); node->keep(hc);
+    torch::autograd::set_history(loss, node);
+  }
+  return loss;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_ulm_torch, m) {
+  namespace py = pybind11;
+  using no_gil = py::call_guard<py::gil_scoped_release>;
+  m.def("status_tensor", &status_tensor, no_gil());
+  m.def("fa_ready", &fa_ready);
+  m.def("can_use", &can_use);
+  m.def("rope_can_use", &rope_can_use);
+  m.def("rope", &rope, no_gil());
+  m.def("flash_attn", &flash_attn, no_gil());
+  m.def("rope_flash_attn", &rope_flash_attn, no_gil());
+  m.def("qkv_attn", &qkv_attn, no_gil());
+  m.def("causal_attention", &causal_attention, no_gil());
+  m.def("rms_norm", &rms_norm, no_gil());
+  m.def("add_rms_norm", &add_rms_norm, no_gil());
+  m.def("swiglu", &swiglu, no_gil());
+  m.def("set_wgrad_in_place", [](bool on) { return g_wgrad_in_place.exchange(on); });
+  m.def("cast_scope_push", &cast_scope_push);
+  m.def("cast_scope_pop", &cast_scope_pop, no_gil());
+  m.def("cast_cached", &cast_cached, no_gil());
+  m.def("weight_grad", [](const Tensor& w, const Tensor& dy, const Tensor& x) -> OptTensor {
+    OpScope scope;
+    Tensor g = weight_grad(w, dy, x);
+    return g.defined() ? OptTensor(g) : std::nullopt;
+  }, no_gil());
+  m.def("linear", &linear, no_gil());
+  m.def("lm_head_lse", &lm_head_lse, no_gil());
+  m.def("kept_cross_entropy", &kept_cross_entropy, no_gil());
+}

@@ -3,7 +3,7 @@
 Same names, arguments and error behaviour as flash_attn_v100_cuda.py of
 sunyi9161/Universal-LM-Trainer (the module train.py:82 imports and calls at
 train.py:90,94,100,1912,1913,1950), backed by the sm_100a library
-``libulm_b200.so`` through ctypes instead of a torch C++ extension:
+``libulm_b200.so``; the autograd functions are native (csrc/torch_ops.cpp):
 
     is_available()  build_error()  can_use(q,k,v)
     rope_can_use(q,k,cos2d,sin2d)  rope(q,k,cos2d,sin2d)
@@ -65,7 +65,7 @@ def _status(dev):
     index = dev.index if dev.index is not None else torch.cuda.current_device()
     s = _STATUS.get(index)
     if s is None:
-        s = _STATUS[index] = torch.zeros(1, dtype=torch.int32, device=torch.device('cuda', index))
+        s = _STATUS[index] = N.ext().status_tensor(index)
     return s
 
 
@@ -74,9 +74,7 @@ def check_status(device=None):
     call (synchronises; meant for step boundaries and tests)."""
     dev = torch.device('cuda', torch.cuda.current_device()) if device is None else torch.device(device)
     index = dev.index if dev.index is not None else torch.cuda.current_device()
-    s = _STATUS.get(index)
-    if s is None:
-        return
+    s = _status(torch.device('cuda', index))
     bits = int(s.item())
     if bits:
         s.zero_()
@@ -86,17 +84,11 @@ def check_status(device=None):
 def _fa_ready(t):
     """flash_attn_v100_cuda.py:97-102, with bf16 admitted: (B,H,S,64), innermost
     contiguous, 32-byte aligned base and strides."""
-    return (t.is_cuda and t.dtype in _16BIT and t.dim() == 4
-            and t.size(3) == 64 and t.stride(3) == 1
-            and t.data_ptr() % 32 == 0
-            and all((s * 2) % 32 == 0 for s in t.stride()[:3])
-            and all(s > 0 or n == 1 for s, n in zip(t.stride()[:3], t.shape[:3]))
-            and (t.size(2) == 1 or t.stride(2) >= 64))
+    return N.ext().fa_ready(t)
 
 
 def can_use(q, k, v):
-    return (_fa_ready(q) and _fa_ready(k) and _fa_ready(v)
-            and q.shape == k.shape == v.shape and q.dtype == k.dtype == v.dtype)
+    return N.ext().can_use(q, k, v)
 
 
 def _empty_bshd(B, H, S, like):
@@ -135,24 +127,20 @@ def attn_forward(q, k, v, dropout_p, causal, softmax_scale, seed, cos=None, sin=
     return o, lse, q_rot
 
 
-class _FlashAttnV100Cuda(torch.autograd.Function):
-    """flash_attn_v100_cuda.py:69-94."""
+def _seed_for(dropout_p):
+    """The seed of the next forward; without dropout nothing reads it, so only the sequence advances."""
+    if dropout_p:
+        return _next_seed()
+    next(_SEED_COUNTER)
+    return 0
+
+
+class _FlashAttnV100Cuda:
+    """flash_attn_v100_cuda.py:69-94: the op itself, without the wrapper's defaults."""
 
     @staticmethod
-    def forward(ctx, q, k, v, dropout_p, causal, softmax_scale):
-        seed = _next_seed()
-        o, lse, _ = attn_forward(q, k, v, dropout_p, causal, softmax_scale, seed)
-        ctx.save_for_backward(q, k, v, o, lse)
-        ctx.dropout_p, ctx.causal = float(dropout_p), bool(causal)
-        ctx.softmax_scale, ctx.seed = float(softmax_scale), seed
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        q, k, v, o, lse = ctx.saved_tensors
-        dq, dk, dv = attn_backward(q, k, v, o, lse, do, ctx.dropout_p, ctx.causal,
-                                   ctx.softmax_scale, ctx.seed)
-        return dq, dk, dv, None, None, None
+    def apply(q, k, v, dropout_p, causal, softmax_scale):
+        return N.ext().flash_attn(q, k, v, float(dropout_p), bool(causal), float(softmax_scale), _next_seed())
 
 
 def attn_backward(q, k, v, o, lse, do, dropout_p, causal, softmax_scale, seed, mode=7,
@@ -225,60 +213,30 @@ def _rope_launch(q, k, cos, sin, backward, shape_like=None, out=None):
     return qo, ko
 
 
-class _RopeV100Cuda(torch.autograd.Function):
+class _RopeV100Cuda:
     """flash_attn_v100_cuda.py:111-138: fused RoPE, one kernel each way."""
 
     @staticmethod
-    def forward(ctx, q, k, cos, sin):
-        qo, ko = _rope_launch(q, k, cos, sin, backward=False)
-        ctx.save_for_backward(q, k, cos, sin)
-        return qo, ko
-
-    @staticmethod
-    def backward(ctx, dqo, dko):
-        q, k, cos, sin = ctx.saved_tensors
-        # A branch whose output went unused arrives as None: run the kernel on
-        # zeros for it but hand None back (flash_attn_v100_cuda.py:124-138).
-        q_unused, k_unused = dqo is None, dko is None
-        if q_unused and k_unused:
-            return None, None, None, None
-        dqo = torch.zeros_like(q) if q_unused else (dqo if _rope_grad_ready(dqo) else dqo.contiguous())
-        dko = torch.zeros_like(k) if k_unused else (dko if _rope_grad_ready(dko) else dko.contiguous())
-        dq, dk = _rope_launch(dqo, dko, cos, sin, backward=True, shape_like=(q, k))
-        return (None if q_unused else dq), (None if k_unused else dk), None, None
-
-
-def _rope_grad_ready(t):
-    return (t.stride(3) == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in t.stride()[:3]))
+    def apply(q, k, cos, sin):
+        return N.ext().rope(q, k, cos, sin)
 
 
 def rope_can_use(q, k, cos, sin):
     """flash_attn_v100_cuda.py:141-147 (plus the 16-byte table alignment the
     vector loads here need)."""
-    return (_fa_ready(q) and _fa_ready(k)
-            and q.shape == k.shape and q.dtype == k.dtype
-            and cos.dtype == torch.float32 and sin.dtype == torch.float32
-            and cos.device == q.device and sin.device == q.device
-            and cos.shape == (q.size(2), 64) and sin.shape == cos.shape
-            and cos.stride(1) == 1 and sin.stride(1) == 1
-            and cos.stride(0) % 4 == 0 and sin.stride(0) % 4 == 0
-            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0)
+    return N.ext().rope_can_use(q, k, cos, sin)
 
 
 def rope(q, k, cos2d, sin2d):
     """q,k: (B,H,S,64) 16-bit views of any stride; cos2d/sin2d: fp32 (S,64), rows may be padded."""
-    return _RopeV100Cuda.apply(q, k, cos2d, sin2d)
+    return N.ext().rope(q, k, cos2d, sin2d)
 
 
 def flash_attn_v100(q, k, v, dropout_p: float = 0.0, causal: bool = True, softmax_scale=None):
     """flash_attn_v100_cuda.py:155-166."""
-    if not (q.is_cuda and q.dtype in _16BIT and q.size(3) == 64):
-        raise ValueError('flash_attn_v100 needs CUDA fp16/bf16 inputs with head_dim 64')
-    if not _fa_ready(q) or not _fa_ready(k) or not _fa_ready(v):
-        q, k, v = (t if _fa_ready(t) else t.contiguous() for t in (q, k, v))
     if softmax_scale is None:
         softmax_scale = q.shape[-1] ** -0.5
-    return _FlashAttnV100Cuda.apply(q, k, v, float(dropout_p), bool(causal), float(softmax_scale))
+    return N.ext().flash_attn(q, k, v, dropout_p, bool(causal), softmax_scale, _seed_for(dropout_p))
 
 
 # Where the RoPE work of rope_flash_attn / qkv_rope_flash_attn runs.  All three give the same bits.
@@ -289,6 +247,7 @@ def flash_attn_v100(q, k, v, dropout_p: float = 0.0, causal: bool = True, softma
 # CTA's start-up path) and the backward fusion costs more than the launch it removes (the epilogue of a
 # persistent in-order pipeline is on its critical path), so 'none' is the default; profiles/ has the numbers.
 ROPE_FUSION = 'none'
+_FUSE = {'none': 0, 'fwd': 1, 'all': 2}
 
 
 def _rope_attn_forward(q, k, v, cos, sin, dropout_p, causal, softmax_scale, seed, fuse, o_out=None):
@@ -318,100 +277,20 @@ def _rope_attn_backward(q_rot, k_rot, v, o, lse, do, cos, sin, dropout_p, causal
     return out
 
 
-class _RopeFlashAttn(torch.autograd.Function):
-    """RoPE + attention as one differentiable op: what ``_RopeV100Cuda`` followed by
-    ``_FlashAttnV100Cuda`` compute (flash_attn_v100_cuda.py:111-138, 69-94).  Saves the rotated
-    q and k (the backward recomputes the scores from them), not the unrotated ones."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, cos, sin, dropout_p, causal, softmax_scale, fuse):
-        seed = _next_seed()
-        o, lse, q_rot, k_rot = _rope_attn_forward(q, k, v, cos, sin, dropout_p, causal, softmax_scale, seed, fuse)
-        ctx.save_for_backward(q_rot, k_rot, v, o, lse, cos, sin)
-        ctx.args = (float(dropout_p), bool(causal), float(softmax_scale), seed, fuse)
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        q_rot, k_rot, v, o, lse, cos, sin = ctx.saved_tensors
-        dq, dk, dv = _rope_attn_backward(q_rot, k_rot, v, o, lse, do, cos, sin, *ctx.args)
-        return dq, dk, dv, None, None, None, None, None, None
+def _fuse_code(fuse):
+    code = _FUSE.get(ROPE_FUSION if fuse is None else fuse)
+    if code is None:
+        raise ValueError("fuse must be 'none', 'fwd' or 'all'")
+    return code
 
 
 def rope_flash_attn(q, k, v, cos2d, sin2d, dropout_p: float = 0.0, causal: bool = True, softmax_scale=None, fuse=None):
     """``flash_attn_v100(*rope(q, k, cos2d, sin2d), v, ...)`` as one op (see the module docstring);
     ``fuse`` picks where the RoPE work runs (default: ROPE_FUSION).  Inputs must satisfy
     ``rope_can_use`` and ``can_use``; there is no other path."""
-    if not (rope_can_use(q, k, cos2d, sin2d) and can_use(q, k, v)):
-        raise ValueError('rope_flash_attn needs 16-bit (B,H,S,64) CUDA views and fp32 (S,64) tables')
-    fuse = ROPE_FUSION if fuse is None else fuse
-    if fuse not in ('none', 'fwd', 'all'):
-        raise ValueError("fuse must be 'none', 'fwd' or 'all'")
     if softmax_scale is None:
         softmax_scale = q.shape[-1] ** -0.5
-    return _RopeFlashAttn.apply(q, k, v, cos2d, sin2d, float(dropout_p), bool(causal), float(softmax_scale), fuse)
-
-
-class _QkvRopeFlashAttn(torch.autograd.Function):
-    """The attention block between the two projections of train.py:1934-1964 as one op on the FUSED
-    projection output: qkv [n, L, 3*H*64] -> chunk into q, k, v (train.py:1935-1939), RoPE on q and k,
-    causal attention, heads merged back to [n, L, H*64] (train.py:1963).  Nothing is copied that the
-    reference copies around the kernels: q, k, v are strided views of qkv, the output comes out of the
-    kernel in (n, L, H, 64) order, and the backward kernels write dq, dk, dv straight into the three
-    slices of one [n, L, 3*H*64] gradient tensor (autograd would otherwise concatenate them)."""
-
-    @staticmethod
-    def forward(ctx, qkv, cos, sin, n_heads, dropout_p, causal, softmax_scale, fuse, flat_shape=None):
-        # flat_shape = (B, S): qkv is the flattened [T', 3*H*64] projection with T' >= B*S; the rows beyond B*S
-        # are padding -- the output gets zero rows there and so does the gradient, without any copy
-        if flat_shape is not None:
-            B, S = flat_shape
-            rows = qkv.shape[0]
-            qkv3 = qkv[:B * S].view(B, S, qkv.shape[-1])
-        else:
-            B, S, _ = qkv.shape
-            rows = None
-            qkv3 = qkv
-        q, k, v = (t.view(B, S, n_heads, 64).transpose(1, 2) for t in qkv3.chunk(3, dim=-1))
-        seed = _next_seed()
-        o_out = out2d = None
-        if rows is not None:
-            out2d = torch.empty((rows, n_heads * 64), dtype=qkv.dtype, device=qkv.device)
-            out2d[B * S:].zero_()
-            o_out = out2d[:B * S].view(B, S, n_heads, 64).transpose(1, 2)
-        if cos is not None:
-            o, lse, q, k = _rope_attn_forward(q, k, v, cos, sin, dropout_p, causal, softmax_scale, seed, fuse, o_out=o_out)
-        else:
-            o, lse, _ = attn_forward(q, k, v, dropout_p, causal, softmax_scale, seed, o_out=o_out)
-        ctx.save_for_backward(q, k, v, o, lse, cos, sin)
-        ctx.args = (float(dropout_p), bool(causal), float(softmax_scale), seed, fuse)
-        ctx.rows = rows
-        if rows is not None:
-            return out2d
-        return o.transpose(1, 2).reshape(B, S, n_heads * 64)          # a view: o is stored (B,S,H,64)
-
-    @staticmethod
-    def backward(ctx, d_out):
-        q, k, v, o, lse, cos, sin = ctx.saved_tensors
-        B, H, S, _ = q.shape
-        rows = ctx.rows
-        if not d_out.is_contiguous():
-            d_out = d_out.contiguous()
-        do = (d_out if rows is None else d_out[:B * S]).view(B, S, H, 64).transpose(1, 2)
-        if rows is None:
-            d_qkv = torch.empty((B, S, 3, H, 64), dtype=q.dtype, device=q.device)
-            d3 = d_qkv
-        else:
-            d_qkv = torch.empty((rows, 3, H, 64), dtype=q.dtype, device=q.device)
-            d_qkv[B * S:].zero_()
-            d3 = d_qkv[:B * S].view(B, S, 3, H, 64)
-        out = tuple(d3[:, :, i].transpose(1, 2) for i in range(3))
-        if cos is not None:
-            _rope_attn_backward(q, k, v, o, lse, do, cos, sin, *ctx.args, out=out)
-        else:
-            attn_backward(q, k, v, o, lse, do, *ctx.args[:4], out=out)
-        d_flat = d_qkv.view(B, S, 3 * H * 64) if rows is None else d_qkv.view(rows, 3 * H * 64)
-        return d_flat, None, None, None, None, None, None, None, None
+    return N.ext().rope_flash_attn(q, k, v, cos2d, sin2d, dropout_p, bool(causal), softmax_scale, _seed_for(dropout_p), _fuse_code(fuse))
 
 
 def qkv_rope_flash_attn(qkv, n_heads, cos2d=None, sin2d=None, dropout_p: float = 0.0, causal: bool = True,
@@ -419,37 +298,20 @@ def qkv_rope_flash_attn(qkv, n_heads, cos2d=None, sin2d=None, dropout_p: float =
     """qkv [n, L, 3*n_heads*64] (the fused projection, 16-bit, contiguous) -> attention output
     [n, L, n_heads*64]; RoPE with the fp32 (L,64) tables when they are given.  With ``flat_shape=(n, L)``
     qkv is the flattened [T', 3*n_heads*64] tensor with T' >= n*L (padding rows at the end) and the output is
-    [T', n_heads*64] with zero padding rows: no copy either way."""
-    if flat_shape is not None:
-        n_, L_ = flat_shape
-        if not (qkv.dim() == 2 and qkv.shape[0] >= n_ * L_):
-            raise ValueError('flat_shape=(n, L) needs a 2-D qkv with at least n*L rows')
-        probe = qkv[:n_ * L_].view(n_, L_, qkv.shape[-1])
-    else:
-        probe = qkv
-    if not (qkv.is_cuda and qkv.dtype in _16BIT and probe.dim() == 3 and qkv.is_contiguous()
-            and qkv.shape[-1] == 3 * n_heads * 64 and qkv.data_ptr() % 32 == 0):
-        raise ValueError('qkv_rope_flash_attn needs a contiguous CUDA fp16/bf16 [n, L, 3*n_heads*64] tensor')
-    if (cos2d is None) != (sin2d is None):
-        raise ValueError('cos2d and sin2d must be given together')
-    if cos2d is not None:
-        L = probe.shape[1]
-        ok = (cos2d.dtype == torch.float32 and sin2d.dtype == torch.float32 and cos2d.device == qkv.device
-              and sin2d.device == qkv.device and cos2d.shape == (L, 64) and sin2d.shape == (L, 64)
-              and cos2d.stride(1) == 1 and sin2d.stride(1) == 1 and cos2d.stride(0) % 4 == 0 and sin2d.stride(0) % 4 == 0
-              and cos2d.data_ptr() % 16 == 0 and sin2d.data_ptr() % 16 == 0)
-        if not ok:
-            raise ValueError('RoPE tables must be fp32 (L,64) views on the same device, 16-byte aligned rows')
-    fuse = ROPE_FUSION if fuse is None else fuse
-    if fuse not in ('none', 'fwd', 'all'):
-        raise ValueError("fuse must be 'none', 'fwd' or 'all'")
+    [T', n_heads*64] with zero padding rows: no copy either way.
+
+    This is the attention block between the two projections of train.py:1934-1964 as one op: chunk into q, k, v
+    (train.py:1935-1939), RoPE on q and k, causal attention, heads merged back (train.py:1963).  Nothing is copied
+    that the reference copies around the kernels: q, k, v are strided views of qkv, the output comes out of the kernel
+    in (n, L, H, 64) order, and the backward kernels write dq, dk, dv straight into the three slices of one gradient
+    tensor (autograd would otherwise concatenate them)."""
+    n, L = (-1, -1) if flat_shape is None else flat_shape
+    code = _fuse_code(fuse)
     if softmax_scale is None:
         softmax_scale = 64 ** -0.5
-    if probe.shape[0] == 0 or probe.shape[1] == 0:
-        shape = (qkv.shape[0], n_heads * 64) if flat_shape is not None else (qkv.shape[0], qkv.shape[1], n_heads * 64)
-        return qkv.new_zeros(shape) + 0 * qkv.sum()
-    return _QkvRopeFlashAttn.apply(qkv, cos2d, sin2d, int(n_heads), float(dropout_p), bool(causal), float(softmax_scale), fuse,
-                                   None if flat_shape is None else (int(flat_shape[0]), int(flat_shape[1])))
+    if qkv.numel() == 0 or (flat_shape is not None and n * L == 0):
+        return qkv.new_zeros((*qkv.shape[:-1], n_heads * 64)) + 0 * qkv.sum()
+    return N.ext().qkv_attn(qkv, n_heads, cos2d, sin2d, dropout_p, bool(causal), softmax_scale, _seed_for(dropout_p), code, n, L)
 
 
 def selftest_wait_timeout(limit_ns=2_000_000, device=None):

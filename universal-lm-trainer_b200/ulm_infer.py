@@ -18,7 +18,7 @@ import types
 
 import torch
 
-import flash_attn_v100_cuda as _fa
+import _native as N
 import ulm_ops
 
 
@@ -27,19 +27,7 @@ def causal_attention(qkv, n_heads, cos=None, sin=None, softmax_scale=None):
     rotated, both as (n, n_heads, L, 64) views.  ``cos``/``sin``: the model's [1, L, >=64] or [L, >=64]
     fp32 RoPE tables (None: no rotation).  No autograd graph is built and nothing is saved: Q is rotated
     inside the kernel and its rotated copy is never written."""
-    B, S, _ = qkv.shape
-    q, k, v = (t.view(B, S, n_heads, 64).transpose(1, 2) for t in qkv.detach().chunk(3, dim=-1))
-    scale = 64 ** -0.5 if softmax_scale is None else float(softmax_scale)
-    if cos is not None:
-        cos2d = cos.reshape(-1, cos.shape[-1])[:S, :64]
-        sin2d = sin.reshape(-1, sin.shape[-1])[:S, :64]
-        if not _fa.rope_can_use(q, k, cos2d, sin2d):
-            raise ValueError('causal_attention needs fp32 RoPE tables of at least 64 columns on the same device')
-        _, k = _fa._rope_launch(None, k, cos2d, sin2d, backward=False)
-        o, _, _ = _fa.attn_forward(q, k, v, 0.0, True, scale, 0, cos=cos2d, sin=sin2d, want_q_rot=False)
-    else:
-        o, _, _ = _fa.attn_forward(q, k, v, 0.0, True, scale, 0)
-    return o.transpose(1, 2).reshape(B, S, n_heads * 64), k, v
+    return N.ext().causal_attention(qkv, n_heads, cos, sin, 64 ** -0.5 if softmax_scale is None else float(softmax_scale))
 
 
 def _eligible(module, x, mask, past, is_causal):
