@@ -366,11 +366,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  const uint32_t tmem_base = ctl->tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);   // warp-uniform
   constexpr uint32_t cQ = 128 * kBufs;
 
   if (warp == kProducerWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
       if (FUSE_DELTA) tma_prefetch_desc(&tmO);
       ItemIter items(n_items);
@@ -416,7 +416,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == kMmaWarp || warp == kMma2Warp) {
-    if (lane == 0) {                                     // score MMAs: S_j = Q K_j^T (first issuer), dP_j = dO V_j^T (second)
+    if (elect_one()) {                                     // score MMAs: S_j = Q K_j^T (first issuer), dP_j = dO V_j^T (second)
       const bool second = warp == kMma2Warp;
       constexpr uint32_t idesc_s = make_idesc(Fmt<T>::v, BR, BT, 0);   // 128 x 64, both K-major
       ItemIter items(n_items);
@@ -445,7 +445,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == kGradWarp) {
-    if (lane == 0) {                                     // gradient MMAs: dQ += dS_j K_j
+    if (elect_one()) {                                     // gradient MMAs: dQ += dS_j K_j
       constexpr uint32_t idesc_q = make_idesc(Fmt<T>::v, BR, HD, 1);   // 128 x 64, B = K tile read MN-major
       ItemIter items(n_items);
       uint32_t t = 0;
@@ -714,11 +714,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  const uint32_t tmem_base = ctl->tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);   // warp-uniform
   constexpr uint32_t cV = 128 * kBufs, cK = 128 * kBufs + 64;
 
   if (warp == kProducerWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
       ItemIter items(n_items);
       uint32_t t = 0;                                     // tiles issued so far, over all items
@@ -762,7 +762,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
   } else if (warp == kMmaWarp || warp == kMma2Warp) {
-    if (lane == 0) {                                     // score MMAs: S^T = K Q_i^T (first issuer), dP^T = V dO_i^T (second)
+    if (elect_one()) {                                     // score MMAs: S^T = K Q_i^T (first issuer), dP^T = V dO_i^T (second)
       const bool second = warp == kMma2Warp;
       constexpr uint32_t idesc_s = make_idesc(Fmt<T>::v, BR, BT, 0);   // 128 keys x 64 queries
       ItemIter items(n_items);
@@ -791,7 +791,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
   } else if (warp == kGradWarp || (warp == kGrad2Warp && kGradIssuers == 2)) {
-    if (lane == 0) {                                     // gradient MMAs: dV += P^T dO_i (first issuer), dK += dS^T Q_i (second)
+    if (elect_one()) {                                     // gradient MMAs: dV += P^T dO_i (first issuer), dK += dS^T Q_i (second)
       const bool second = warp == kGrad2Warp;
       constexpr uint32_t idesc_a = make_idesc(Fmt<T>::v, BR, HD, 1);   // B = dO / Q tile read MN-major
       ItemIter items(n_items);

@@ -134,9 +134,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
   if (threadIdx.x == 0) {
     mbar_init(&ctl->q_full, 1);
-    mbar_init(&ctl->q_ready, 256);
+    mbar_init(&ctl->q_ready, 8);
     for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->k_full[s], 1); mbar_init(&ctl->v_full[s], 1); mbar_init(&ctl->kv_empty[s], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&ctl->s_full[i], 1); mbar_init(&ctl->p_ready[i], 256); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&ctl->s_full[i], 1); mbar_init(&ctl->p_ready[i], 8); }
     mbar_init(&ctl->o_done, 1);
     ctl->abort = 0;
     ctl->fail_bits = 0;
@@ -146,11 +146,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  const uint32_t tmem_base = ctl->tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);   // warp-uniform
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
       mbar_expect_tx(&ctl->q_full, kQBytes);
       tma_load_4d(sQ, &tmQ, &ctl->q_full, 0, m0, h, b);
@@ -179,7 +179,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == 9) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr int fmt = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
       constexpr uint32_t idesc_s = make_idesc(fmt, BM, BN, 0);
       constexpr uint32_t idesc_o = make_idesc(fmt, BM, HD, 1);
@@ -256,7 +256,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         // generic-proxy writes -> visible to the tensor core's (async proxy) operand reads
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(&ctl->q_ready);
+        warp_arrive(&ctl->q_ready);
       }
     }
     uint32_t sv[32];
@@ -338,7 +338,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       tmem_wait_st();
       fence_before_sync();
-      mbar_arrive(&ctl->p_ready[j & 1]);
+      warp_arrive(&ctl->p_ready[j & 1]);
     }
     // epilogue: merge the two key halves, O / l -> 16-bit, LSE
     ctl->m_half[hf][r] = m;

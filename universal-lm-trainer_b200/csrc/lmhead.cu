@@ -122,11 +122,11 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  const uint32_t tmem_base = ctl->tmem_base;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);   // warp-uniform
 
   if (warp == kLmEpiWarps) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmH); tma_prefetch_desc(&tmW);
       ItemIter it_items(n_items);
       uint32_t it = 0;                                   // k-blocks issued so far, over all tiles
@@ -160,7 +160,7 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
     }
   } else if (warp == kLmEpiWarps + 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(LmFmt<T>::v, LM_BM, LM_BN, 0);   // 128 x 256, both operands K-major
       ItemIter it_items(n_items);
       uint32_t it = 0, tt = 0;                           // k-blocks / tiles so far
