@@ -300,7 +300,7 @@ int ulm_loss_mean(const float* rows_loss, const int64_t* target, int64_t rows, i
  * multiple of 64, base pointers 16-byte aligned.  logits: optional [rows, V] buffer of the same dtype that
  * receives z for the backward (needs V % 64 == 0, z_stride a multiple of 8); NULL: nothing is stored and
  * loss must be NULL too (lse only).  part_m, part_s: fp32 scratch of rows * ulm_lmhead_lse_parts(V) floats
- * each.  status_dev: optional, see ULM_STATUS_*.
+ * each (or rows * ulm_lmhead_parts(rows, V)).  status_dev: optional, see ULM_STATUS_*.
  */
 typedef struct {
   const void* h; const void* w;
@@ -317,6 +317,12 @@ typedef struct {
 } ulm_lmhead_lse_args;
 int ulm_lmhead_lse(const ulm_lmhead_lse_args* a);
 int64_t ulm_lmhead_lse_parts(int32_t V);
+/* What exactly `rows` rows need (ulm_lmhead_lse_parts: the most any row count does). */
+int64_t ulm_lmhead_parts(int64_t rows, int32_t V);
+/* The same GEMM for scoring (inf.py:866-937): no logits are stored (a->logits NULL); loss and target are required, lse
+ * is optional; hit[r] = 1 where target[r] has row r's largest logit (the lowest column on ties), 0 elsewhere and on
+ * ignored rows.  part_i: int32 scratch of the size of part_m. */
+int ulm_lmhead_score(const ulm_lmhead_lse_args* a, uint8_t* hit, int32_t* part_i);
 
 /* ---- gradient post-processing after the data-parallel all-reduce ----------
  * No counterpart kernel in the reference: fuses what scaler.unscale_ and

@@ -123,6 +123,8 @@ EXPORTS = {
     'ulm_ce_fwd': (C.c_int, [C.POINTER(CeFwdArgs)]),
     'ulm_lmhead_lse': (C.c_int, [C.POINTER(LmHeadLseArgs)]),
     'ulm_lmhead_lse_parts': (C.c_int64, [C.c_int32]),
+    'ulm_lmhead_parts': (C.c_int64, [i64, C.c_int32]),
+    'ulm_lmhead_score': (C.c_int, [C.POINTER(LmHeadLseArgs), vp, vp]),
     'ulm_ce_bwd': (C.c_int, [C.POINTER(CeBwdArgs)]),
     'ulm_loss_mean': (C.c_int, [vp, vp, i64, i64, vp, f32, vp, vp, vp]),
     'ulm_swiglu_fwd': (C.c_int, [C.POINTER(SwigluArgs)]),

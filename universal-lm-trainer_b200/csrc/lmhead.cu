@@ -77,13 +77,29 @@ __device__ __forceinline__ bool half_sync_any(int half, bool fail) {
   return any != 0;
 }
 
+// Column tiles per work item: the count whose rounds of items over the SMs take the fewest tile times, an item's own
+// cost (pipeline fill, statistics) being worth about a quarter of a tile.  At 32768 x 32000 that is 5 (220 tile times,
+// 216 ideal; the fixed 25 of before took 225); with 2048 rows x 4096 columns, 1 instead of 16: 256 items on 148 SMs
+// where 16 SMs had one each.
+int lm_group_tiles(int64_t rows, int V) {
+  const int64_t n_rb = (rows + LM_BM - 1) / LM_BM, n_ct = (V + LM_BN - 1) / LM_BN;
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int want = 1; want <= kLmGroupTiles; ++want) {
+    const int64_t groups = (n_ct + want - 1) / want, tiles = (n_ct + groups - 1) / groups;
+    const int64_t cost = ((n_rb * groups + kNumSMs - 1) / kNumSMs) * (4 * tiles + 1);
+    if (cost < best_cost) { best_cost = cost; best = (int)tiles; }
+  }
+  return best;
+}
+
 struct LmItems {
   int n_rb, n_ct, n_groups, group_tiles;
-  __host__ __device__ LmItems(int64_t rows, int V) {
+  __host__ __device__ LmItems(int64_t rows, int V, int tiles) {
     n_rb = (int)((rows + LM_BM - 1) / LM_BM);
     n_ct = (V + LM_BN - 1) / LM_BN;
-    n_groups = (n_ct + kLmGroupTiles - 1) / kLmGroupTiles;
-    group_tiles = (n_ct + n_groups - 1) / n_groups;
+    group_tiles = tiles;
+    n_groups = (n_ct + tiles - 1) / tiles;
   }
   __host__ __device__ int n_items() const { return n_rb * n_groups; }
   // all CTAs are on one column group at a time: its W tiles are read from L2 by everyone
@@ -95,11 +111,20 @@ struct LmItems {
   }
 };
 
-template <typename T, bool KEEP>
+// TOP1 (scoring): instead of storing the logits the epilogue picks out what a score needs of them, the target's logit
+// (into z_target) and the column of the largest one (part_i, the lowest on ties).
+struct LmTop1 {
+  const int64_t* target;
+  int64_t ignore_index;
+  float* z_target;
+  int32_t* part_i;
+};
+
+template <typename T, bool KEEP, bool TOP1>
 __global__ void __launch_bounds__(kLmThreads, 1)
 lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmW,
                   const __grid_constant__ CUtensorMap tmZ, float* __restrict__ part_m, float* __restrict__ part_s,
-                  int64_t rows, int V, int n_kb, uint32_t* status) {
+                  int64_t rows, int V, int n_kb, int group_tiles, uint32_t* status, const LmTop1 top) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stages = base;                                             // [stage][H tile | W tile]
@@ -108,7 +133,7 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
   volatile int* abort_flag = &ctl->abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const LmItems items(rows, V);
+  const LmItems items(rows, V, group_tiles);
   const int n_items = items.n_items();
 
   if (threadIdx.x == 0) {
@@ -204,6 +229,15 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
       int rb, g, ct0, nct;
       items.decode(idx, rb, g, ct0, nct);
       float m = -INFINITY, ssum = 0.f;                   // base-2 domain: m = max(z) * log2e
+      const int64_t grow = (int64_t)rb * LM_BM + r;
+      [[maybe_unused]] float best = -INFINITY;
+      [[maybe_unused]] int best_i = V, tgt = -1;
+      if constexpr (TOP1) {
+        if (grow < rows) {
+          const int64_t t = top.target[grow];
+          if (t != top.ignore_index && t >= 0 && t < V) tgt = (int)t;
+        }
+      }
       for (int t = 0; ok && t < nct; ++t, ++tt) {
         const uint32_t b = tt & 1;
         const bool waited = __all_sync(0xffffffffu, mbar_wait(&ctl->acc_full[b], (tt >> 1) & 1, abort_flag));
@@ -256,6 +290,21 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
               bulk_commit();
             }
           }
+          if constexpr (TOP1) {
+            if (mx > best) {                             // strictly: the lowest column keeps a tie
+              int at = 0;
+#pragma unroll
+              for (int c = 63; c >= 0; --c) at = __uint_as_float(acc[c]) == mx ? c : at;
+              best = mx;
+              best_i = col0 + at;
+            }
+            if ((unsigned)(tgt - col0) < 64u) {          // one block of one thread holds the row's target
+              float z = 0.f;
+#pragma unroll
+              for (int c = 0; c < 64; ++c) z = tgt - col0 == c ? __uint_as_float(acc[c]) : z;
+              top.z_target[grow] = z;
+            }
+          }
           // running statistics over the rounded values
           const float m_new = fmaxf(m, mx * kLmLog2e);
           if (m_new > -INFINITY) {
@@ -275,12 +324,12 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
         }
       }
       if (!ok) break;
-      const int64_t grow = (int64_t)rb * LM_BM + r;
       if (grow < rows) {
         // [row][group][half]: the finishing kernel merges 2 * n_groups pairs per row
         const int64_t o = (grow * items.n_groups + g) * 2 + half;
         part_m[o] = m;
         part_s[o] = ssum;
+        if constexpr (TOP1) top.part_i[o] = best_i;
       }
     }
     if (KEEP && tg == 0) bulk_wait0();                   // our stores must be complete before the CTA ends
@@ -292,86 +341,129 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
   if (threadIdx.x == 0 && ctl->fail_bits && status) atomicOr(status, ctl->fail_bits);
 }
 
-// lse[r] = ln sum_c exp(z[r,c]) from the per-group (max, sum) pairs; loss[r] = lse[r] - z[r, target[r]]
-// (0 for ignored rows), z read from the stored logits.  One thread per row.
-template <typename T>
-__global__ void lmhead_finish_kernel(const float* __restrict__ part_m, const float* __restrict__ part_s, int n_parts,
-                                     const T* __restrict__ logits, int64_t row_stride, const int64_t* __restrict__ target,
-                                     int64_t ignore_index, int V, float* __restrict__ lse, float* __restrict__ loss, int64_t rows) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// lse[r] = ln sum_c exp(z[r,c]) from the per-group (max, sum) pairs; loss[r] = lse[r] - z[r, target[r]] (0 for ignored
+// rows), z read from the stored logits, or with TOP1 from loss[r] itself, where the epilogue left it; TOP1 also says
+// whether the target has the row's largest logit.  One warp per row: there are up to one pair per 128 columns.
+template <typename T, bool TOP1>
+__global__ void __launch_bounds__(256)
+lmhead_finish_kernel(const float* __restrict__ part_m, const float* __restrict__ part_s, const int32_t* __restrict__ part_i,
+                     int n_parts, const T* __restrict__ logits, int64_t row_stride, const int64_t* __restrict__ target,
+                     int64_t ignore_index, int V, float* __restrict__ lse, float* loss, uint8_t* __restrict__ hit, int64_t rows) {
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
   if (r >= rows) return;
   float m = -INFINITY;
-  for (int i = 0; i < n_parts; ++i) m = fmaxf(m, part_m[r * n_parts + i]);
+  [[maybe_unused]] int at = V;
+  for (int i = lane; i < n_parts; i += 32) {
+    const float mi = part_m[r * n_parts + i];
+    if constexpr (TOP1) {
+      const int ai = part_i[r * n_parts + i];
+      if (mi > m || (mi == m && ai < at)) at = ai;
+    }
+    m = fmaxf(m, mi);
+  }
+  if constexpr (TOP1) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float mo = __shfl_xor_sync(0xffffffffu, m, o);
+      const int ao = __shfl_xor_sync(0xffffffffu, at, o);
+      if (mo > m || (mo == m && ao < at)) at = ao;
+      m = fmaxf(m, mo);
+    }
+  } else {
+    m = warp_max(m);
+  }
   float s = 0.f;
-  for (int i = 0; i < n_parts; ++i) {
+  for (int i = lane; i < n_parts; i += 32) {
     const float mi = part_m[r * n_parts + i];
     if (mi > -INFINITY) s += part_s[r * n_parts + i] * exp2f(mi - m);
   }
+  s = warp_sum(s);
+  if (lane) return;
   const float l = (m + log2f(s)) * kLmLn2;
-  lse[r] = l;
+  if (lse) lse[r] = l;
   if (loss) {
     const int64_t t = target[r];
-    loss[r] = (t == ignore_index || t < 0 || t >= V) ? 0.f : l - Cvt<T>::to_f(logits[r * row_stride + t]);
+    const bool none = t == ignore_index || t < 0 || t >= V;
+    if constexpr (TOP1) {
+      loss[r] = none ? 0.f : l - loss[r];
+      hit[r] = !none && at == (int)t;
+    } else {
+      loss[r] = none ? 0.f : l - Cvt<T>::to_f(logits[r * row_stride + t]);
+    }
   }
 }
 
-template <typename T, bool KEEP>
-int launch_lmhead(const ulm_lmhead_lse_args* a, const CUtensorMap& mh, const CUtensorMap& mw, const CUtensorMap& mz, int device) {
+template <typename T, bool KEEP, bool TOP1>
+int launch_lmhead(const ulm_lmhead_lse_args* a, const LmTop1& top, uint8_t* hit, const CUtensorMap& mh, const CUtensorMap& mw, const CUtensorMap& mz,
+                  int device, const char* who) {
   static std::atomic<bool> attr_set[kMaxDevices];
-  auto kern = lmhead_lse_kernel<T, KEEP>;
-  if (int rc = ensure_smem_attr(kern, kLmSmem, device, attr_set, "ulm_lmhead_lse")) return rc;
-  const LmItems items(a->rows, a->V);
+  auto kern = lmhead_lse_kernel<T, KEEP, TOP1>;
+  if (int rc = ensure_smem_attr(kern, kLmSmem, device, attr_set, who)) return rc;
+  const LmItems items(a->rows, a->V, lm_group_tiles(a->rows, a->V));
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const int grid = items.n_items() < sms ? items.n_items() : sms;
-  kern<<<grid, kLmThreads, kLmSmem, (cudaStream_t)a->stream>>>(mh, mw, mz, a->part_m, a->part_s, a->rows, a->V, a->d / LM_BK, a->status_dev);
-  return ULM_OK;
+  cudaStream_t st = (cudaStream_t)a->stream;
+  kern<<<grid, kLmThreads, kLmSmem, st>>>(mh, mw, mz, a->part_m, a->part_s, a->rows, a->V, a->d / LM_BK, items.group_tiles, a->status_dev, top);
+  if (int rc = check_launch(who)) return rc;
+  lmhead_finish_kernel<T, TOP1><<<(unsigned)((a->rows + 7) / 8), 256, 0, st>>>(
+      a->part_m, a->part_s, top.part_i, 2 * items.n_groups, static_cast<const T*>(a->logits), a->z_stride, a->target, a->ignore_index, a->V, a->lse,
+      a->loss, hit, a->rows);
+  return check_launch(who);
 }
 
-}  // namespace
-}  // namespace ulm
-
-extern "C" int64_t ulm_lmhead_lse_parts(int32_t V) {
-  const ulm::LmItems items(1, V);
-  return 2 * (int64_t)items.n_groups;
-}
-
-extern "C" int ulm_lmhead_lse(const ulm_lmhead_lse_args* a) {
-  using namespace ulm;
-  const char* who = "ulm_lmhead_lse";
-  if (!a) return fail(ULM_ERR_ARG, "%s: null args", who);
+// Checks and tensor maps of both entry points; hit and part_i are the scoring form's.
+int lmhead(const ulm_lmhead_lse_args* a, uint8_t* hit, int32_t* part_i, const char* who) {
+  const bool top1 = hit != nullptr, keep = a->logits != nullptr;
   if (a->dtype != ULM_F16 && a->dtype != ULM_BF16) return fail(ULM_ERR_ARG, "%s: dtype must be fp16 or bf16", who);
   if (a->rows < 0 || a->V <= 0 || a->d <= 0 || a->d % LM_BK) return fail(ULM_ERR_ARG, "%s: need rows >= 0, V > 0, d a positive multiple of %d", who, LM_BK);
   if (a->rows == 0) return ULM_OK;
-  if (!a->h || !a->w || !a->part_m || !a->part_s || !a->lse) return fail(ULM_ERR_ARG, "%s: null tensor", who);
+  if (!a->h || !a->w || !a->part_m || !a->part_s || (!a->lse && !top1)) return fail(ULM_ERR_ARG, "%s: null tensor", who);
   if (a->h_stride < a->d || a->w_stride < a->d || a->h_stride % 8 || a->w_stride % 8)
     return fail(ULM_ERR_ARG, "%s: row strides must be multiples of 8 elements and at least d", who);
-  const bool keep = a->logits != nullptr;
-  if (a->loss && (!keep || !a->target)) return fail(ULM_ERR_ARG, "%s: loss needs the logits buffer and the targets", who);
+  if (!top1 && a->loss && (!keep || !a->target)) return fail(ULM_ERR_ARG, "%s: loss needs the logits buffer and the targets", who);
   if (keep && (a->V % 64 || a->z_stride < a->V || a->z_stride % 8))
     return fail(ULM_ERR_ARG, "%s: storing the logits needs V a multiple of 64 and a row stride that is a multiple of 8 and at least V", who);
-  tc::DeviceScope scope(a->h, who);
+  DeviceScope scope(a->h, who);
   if (scope.rc) return scope.rc;
   int rc;
   // the matrices as [row][block of 64 columns][64]: the tensor-map encoder's (S, H, 64) with B = 1
   CUtensorMap mh, mw, mz;
   const int n_kb = a->d / LM_BK;
-  if ((rc = tc::encode_bhsd_map(&mh, a->h, a->dtype, 1, n_kb, (int)a->rows, 0, 64, a->h_stride, LM_BM, who))) return rc;
-  if ((rc = tc::encode_bhsd_map(&mw, a->w, a->dtype, 1, n_kb, a->V, 0, 64, a->w_stride, LM_BN, who))) return rc;
+  if ((rc = encode_bhsd_map(&mh, a->h, a->dtype, 1, n_kb, (int)a->rows, 0, 64, a->h_stride, LM_BM, who))) return rc;
+  if ((rc = encode_bhsd_map(&mw, a->w, a->dtype, 1, n_kb, a->V, 0, 64, a->w_stride, LM_BN, who))) return rc;
   mz = mh;
-  if (keep && (rc = tc::encode_bhsd_map(&mz, a->logits, a->dtype, 1, a->V / 64, (int)a->rows, 0, 64, a->z_stride, 128, who))) return rc;
-  if (a->dtype == ULM_BF16) rc = keep ? launch_lmhead<__nv_bfloat16, true>(a, mh, mw, mz, scope.device) : launch_lmhead<__nv_bfloat16, false>(a, mh, mw, mz, scope.device);
-  else rc = keep ? launch_lmhead<__half, true>(a, mh, mw, mz, scope.device) : launch_lmhead<__half, false>(a, mh, mw, mz, scope.device);
-  if (rc) return rc;
-  if ((rc = check_launch(who))) return rc;
-  const int n_parts = (int)ulm_lmhead_lse_parts(a->V);
-  const int threads = 128;
-  const unsigned blocks = (unsigned)((a->rows + threads - 1) / threads);
-  if (a->dtype == ULM_BF16)
-    lmhead_finish_kernel<__nv_bfloat16><<<blocks, threads, 0, (cudaStream_t)a->stream>>>(
-        a->part_m, a->part_s, n_parts, static_cast<const __nv_bfloat16*>(a->logits), a->z_stride, a->target, a->ignore_index, a->V, a->lse, a->loss, a->rows);
-  else
-    lmhead_finish_kernel<__half><<<blocks, threads, 0, (cudaStream_t)a->stream>>>(
-        a->part_m, a->part_s, n_parts, static_cast<const __half*>(a->logits), a->z_stride, a->target, a->ignore_index, a->V, a->lse, a->loss, a->rows);
-  return check_launch(who);
+  if (keep && (rc = encode_bhsd_map(&mz, a->logits, a->dtype, 1, a->V / 64, (int)a->rows, 0, 64, a->z_stride, 128, who))) return rc;
+  const LmTop1 top{a->target, a->ignore_index, a->loss, part_i};
+  auto go = [&](auto t) {
+    using T = decltype(t);
+    if (top1) return launch_lmhead<T, false, true>(a, top, hit, mh, mw, mz, scope.device, who);
+    return keep ? launch_lmhead<T, true, false>(a, top, hit, mh, mw, mz, scope.device, who)
+                : launch_lmhead<T, false, false>(a, top, hit, mh, mw, mz, scope.device, who);
+  };
+  return a->dtype == ULM_BF16 ? go(__nv_bfloat16()) : go(__half());
+}
+
+}  // namespace
+}  // namespace ulm
+
+// the most any row count needs: one column tile per work item
+extern "C" int64_t ulm_lmhead_lse_parts(int32_t V) { return 2 * (((int64_t)V + ulm::LM_BN - 1) / ulm::LM_BN); }
+
+extern "C" int64_t ulm_lmhead_parts(int64_t rows, int32_t V) { return 2 * (int64_t)ulm::LmItems(rows, V, ulm::lm_group_tiles(rows, V)).n_groups; }
+
+extern "C" int ulm_lmhead_lse(const ulm_lmhead_lse_args* a) {
+  using namespace ulm;
+  if (!a) return fail(ULM_ERR_ARG, "ulm_lmhead_lse: null args");
+  return lmhead(a, nullptr, nullptr, "ulm_lmhead_lse");
+}
+
+extern "C" int ulm_lmhead_score(const ulm_lmhead_lse_args* a, uint8_t* hit, int32_t* part_i) {
+  using namespace ulm;
+  if (!a) return fail(ULM_ERR_ARG, "ulm_lmhead_score: null args");
+  if (a->logits) return fail(ULM_ERR_ARG, "ulm_lmhead_score: stores no logits");
+  if (a->rows > 0 && (!hit || !part_i || !a->loss || !a->target)) return fail(ULM_ERR_ARG, "ulm_lmhead_score: null tensor");
+  if (a->rows == 0) return ULM_OK;
+  return lmhead(a, hit, part_i, "ulm_lmhead_score");
 }

@@ -721,30 +721,48 @@ Tensor linear(const Tensor& x, const Tensor& weight) {
 // ---------------------------------------------------------------------------
 // lm head + cross-entropy, the form that keeps the 16-bit logits between forward and backward
 // ---------------------------------------------------------------------------
-// -> lse, loss rows (undefined without targets or logits), logits (undefined unless kept)
-std::tuple<Tensor, Tensor, Tensor> lm_head_lse(const Tensor& h, const Tensor& w, const OptTensor& target, int64_t ignore_index, bool keep_logits) {
+// operands, scratch and stream of one lm-head launch; `part` holds the fp32 scratch
+ulm_lmhead_lse_args lmhead_args(const Tensor& h, const Tensor& w, int64_t ignore_index, Tensor& part) {
   TORCH_CHECK_VALUE(is_16bit(h.scalar_type()) && w.scalar_type() == h.scalar_type(), "lm_head_lse takes fp16 or bf16 operands of one dtype");
   TORCH_CHECK_VALUE(h.dim() == 2 && w.dim() == 2 && h.size(1) == w.size(1) && h.stride(1) == 1 && w.stride(1) == 1,
                     "lm_head_lse takes hidden [rows, d] and weight [V, d] with contiguous rows");
-  OpScope scope;
-  c10::cuda::CUDAGuard dev(h.device());
   const int64_t rows = h.size(0), d = h.size(1), V = w.size(0);
-  const Tensor lse = empty_cuda({rows}, at::kFloat, h);
-  Tensor logits, loss;
-  if (keep_logits) logits = empty_cuda({rows, V}, h.scalar_type(), h);
-  if (keep_logits && target) loss = empty_cuda({rows}, at::kFloat, h);
-  const int64_t n_part = std::max<int64_t>(rows, 1) * ulm_lmhead_lse_parts((int32_t)V);
-  const Tensor part = empty_cuda({2, n_part}, at::kFloat, h);
+  const int64_t n_part = std::max<int64_t>(rows, 1) * ulm_lmhead_parts(rows, (int32_t)V);
+  part = empty_cuda({3, n_part}, at::kFloat, h);
   ulm_lmhead_lse_args a{};
-  a.h = h.data_ptr(); a.w = w.data_ptr(); a.lse = lse.data_ptr<float>();
-  if (keep_logits) { a.logits = logits.data_ptr(); a.z_stride = V; }
-  if (loss.defined()) { a.loss = loss.data_ptr<float>(); a.target = target->data_ptr<int64_t>(); }
+  a.h = h.data_ptr(); a.w = w.data_ptr();
   a.part_m = part.data_ptr<float>(); a.part_s = a.part_m + n_part;
   a.h_stride = h.stride(0); a.w_stride = w.stride(0);
   a.rows = rows; a.V = (int32_t)V; a.d = (int32_t)d; a.dtype = code_of(h.scalar_type());
   a.ignore_index = ignore_index; a.status_dev = status_ptr(h); a.stream = stream_of(h);
+  return a;
+}
+
+// -> lse, loss rows (undefined without targets or logits), logits (undefined unless kept)
+std::tuple<Tensor, Tensor, Tensor> lm_head_lse(const Tensor& h, const Tensor& w, const OptTensor& target, int64_t ignore_index, bool keep_logits) {
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(h.device());
+  Tensor part, logits, loss;
+  ulm_lmhead_lse_args a = lmhead_args(h, w, ignore_index, part);
+  const Tensor lse = empty_cuda({a.rows}, at::kFloat, h);
+  a.lse = lse.data_ptr<float>();
+  if (keep_logits) { logits = empty_cuda({a.rows, a.V}, h.scalar_type(), h); a.logits = logits.data_ptr(); a.z_stride = a.V; }
+  if (keep_logits && target) { loss = empty_cuda({a.rows}, at::kFloat, h); a.loss = loss.data_ptr<float>(); a.target = target->data_ptr<int64_t>(); }
   check(ulm_lmhead_lse(&a), "lm-head GEMM + LSE");
   return {lse, loss, logits};
+}
+
+// -> loss rows, whether the target has the row's largest logit (uint8)
+std::tuple<Tensor, Tensor> lm_head_score(const Tensor& h, const Tensor& w, const Tensor& target, int64_t ignore_index) {
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(h.device());
+  TORCH_CHECK_VALUE(target.scalar_type() == at::kLong && target.is_contiguous() && target.numel() == h.size(0), "lm_head_score takes one int64 target per row");
+  Tensor part;
+  ulm_lmhead_lse_args a = lmhead_args(h, w, ignore_index, part);
+  const Tensor loss = empty_cuda({a.rows}, at::kFloat, h), hit = empty_cuda({a.rows}, at::kByte, h);
+  a.loss = loss.data_ptr<float>(); a.target = target.data_ptr<int64_t>();
+  check(ulm_lmhead_score(&a, hit.data_ptr<uint8_t>(), reinterpret_cast<int32_t*>(a.part_s + part.size(1))), "lm-head GEMM + score");
+  return {loss, hit};
 }
 
 struct KeptCeBwd : OpNode {
@@ -835,5 +853,6 @@ PYBIND11_MODULE(_ulm_torch, m) {
   }, no_gil());
   m.def("linear", &linear, no_gil());
   m.def("lm_head_lse", &lm_head_lse, no_gil());
+  m.def("lm_head_score", &lm_head_score, no_gil());
   m.def("kept_cross_entropy", &kept_cross_entropy, no_gil());
 }

@@ -126,6 +126,13 @@ def lm_head_lse(hidden, weight, target=None, ignore_index=0, keep_logits=True):
     return N.ext().lm_head_lse(hidden, weight, target, int(ignore_index), bool(keep_logits))
 
 
+def lm_head_score(hidden, weight, target, ignore_index=-100):
+    """`lm_head_lse` for scoring: the per-row loss lse - z[target] (fp32, 0 on ignored rows) and whether the target has
+    the row's largest logit (uint8; the lowest column counts on ties, as in ``argmax``).  The logits are never stored:
+    the epilogue picks the target's and the largest out of the accumulator."""
+    return N.ext().lm_head_score(hidden, weight, target, int(ignore_index))
+
+
 def ce_rows_backward_(logits, target, lse, gscale_dev, ignore_index, gscale=1.0):
     """In place: logits <- (softmax - onehot) * gscale * gscale_dev[0] (0 on ignored rows)."""
     lib = N.lib()
