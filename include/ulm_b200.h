@@ -256,6 +256,9 @@ typedef struct {
 } ulm_swiglu_args;
 int ulm_swiglu_fwd(const ulm_swiglu_args* a);
 int ulm_swiglu_bwd(const ulm_swiglu_args* a);
+/* The same gate on column blocks: a and b (backward: and da, db) are rows of d elements, row_stride elements apart -- the
+ * two halves of one [rows, 2d] projection; y and dy are dense, n = rows * d.  d and row_stride: whole 16-byte vectors. */
+int ulm_swiglu_rows(const ulm_swiglu_args* a, int32_t backward, int64_t d, int64_t row_stride);
 
 /* ---- chunked cross-entropy row kernels -----------------------------------
  * The reference loops fc_out + F.cross_entropy(reduction='sum') over chunks of

@@ -75,17 +75,28 @@ __device__ __forceinline__ void sigmoid_silu(float a, float& s, float& u) {
 template <typename T> constexpr int kVecsFwd = 2;
 template <typename T> constexpr int kVecsBwd = 1;
 
-template <typename T>
+// Where vector v of the gate's operands lies: a and b (da and db) are dense, or column blocks of a wider matrix (the two
+// halves of one projection's output): rows of vpr vectors, `stride` vectors apart.
+struct Rows { uint32_t vpr; int64_t stride; };
+template <bool ROWS>
+__device__ __forceinline__ int64_t operand_vec(int64_t v, const Rows& rw) {
+  if constexpr (!ROWS) return v;
+  const uint32_t u = (uint32_t)v, r = u / rw.vpr;        // fewer than 2^32 vectors (checked by the host)
+  return (int64_t)r * rw.stride + (u - r * rw.vpr);
+}
+
+template <typename T, bool ROWS>
 __global__ void __launch_bounds__(kThreads)
-swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, int64_t nvec, int64_t n) {
+swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, int64_t nvec, int64_t n, const Rows rw) {
   constexpr int N = VecN<T>::N, K = kVecsFwd<T>;
   const int64_t v0 = (int64_t)blockIdx.x * (kThreads * K) + threadIdx.x;
   uint4 ra[K], rb[K];
 #pragma unroll
   for (int k = 0; k < K; ++k)
     if (v0 + k * kThreads < nvec) {
-      ra[k] = __ldg(reinterpret_cast<const uint4*>(a) + v0 + k * kThreads);
-      rb[k] = __ldg(reinterpret_cast<const uint4*>(b) + v0 + k * kThreads);
+      const int64_t o = operand_vec<ROWS>(v0 + k * kThreads, rw);
+      ra[k] = __ldg(reinterpret_cast<const uint4*>(a) + o);
+      rb[k] = __ldg(reinterpret_cast<const uint4*>(b) + o);
     }
 #pragma unroll
   for (int k = 0; k < K; ++k)
@@ -118,18 +129,19 @@ __device__ __forceinline__ void bwd_one(float fa, float fb, float fg, float& da,
   da = rnd<T>(fg * fb) * (s * (1.f + fa * (1.f - s)));
 }
 
-template <typename T>
+template <typename T, bool ROWS>
 __global__ void __launch_bounds__(kThreads)
 swiglu_bwd_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ dy,
-                  T* __restrict__ da, T* __restrict__ db, int64_t nvec, int64_t n) {
+                  T* __restrict__ da, T* __restrict__ db, int64_t nvec, int64_t n, const Rows rw) {
   constexpr int N = VecN<T>::N, K = kVecsBwd<T>;
   const int64_t v0 = (int64_t)blockIdx.x * (kThreads * K) + threadIdx.x;
   uint4 ra[K], rb[K], rg[K];
 #pragma unroll
   for (int k = 0; k < K; ++k)
     if (v0 + k * kThreads < nvec) {
-      ra[k] = __ldg(reinterpret_cast<const uint4*>(a) + v0 + k * kThreads);
-      rb[k] = __ldg(reinterpret_cast<const uint4*>(b) + v0 + k * kThreads);
+      const int64_t o = operand_vec<ROWS>(v0 + k * kThreads, rw);
+      ra[k] = __ldg(reinterpret_cast<const uint4*>(a) + o);
+      rb[k] = __ldg(reinterpret_cast<const uint4*>(b) + o);
       rg[k] = __ldg(reinterpret_cast<const uint4*>(dy) + v0 + k * kThreads);
     }
 #pragma unroll
@@ -141,8 +153,9 @@ swiglu_bwd_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* __r
       unpack<T>(rg[k], fg);
 #pragma unroll
       for (int i = 0; i < N; ++i) bwd_one<T>(fa[i], fb[i], fg[i], oa[i], ob[i]);
-      reinterpret_cast<uint4*>(da)[v0 + k * kThreads] = pack<T>(oa);
-      reinterpret_cast<uint4*>(db)[v0 + k * kThreads] = pack<T>(ob);
+      const int64_t o = operand_vec<ROWS>(v0 + k * kThreads, rw);
+      reinterpret_cast<uint4*>(da)[o] = pack<T>(oa);
+      reinterpret_cast<uint4*>(db)[o] = pack<T>(ob);
     }
   if (blockIdx.x == 0 && threadIdx.x < (int)(n - nvec * N)) {
     const int64_t i = nvec * N + threadIdx.x;
@@ -161,45 +174,52 @@ bool too_many(int64_t n) { return n / 4 / kThreads > 0x7ffffff0LL; }      // blo
 
 bool aligned16(const void* p) { return p && !(reinterpret_cast<uintptr_t>(p) & 15); }
 
+// d == 0: dense operands; otherwise rows of d elements, `stride` elements apart (y and dy are dense either way)
+int check_swiglu(const ulm_swiglu_args* p, int64_t d, int64_t stride, const char* who) {
+  if (!p) return fail(ULM_ERR_ARG, "%s: null args", who);
+  if (p->dtype != ULM_F16 && p->dtype != ULM_BF16 && p->dtype != ULM_F32) return fail(ULM_ERR_ARG, "%s: bad dtype", who);
+  if (p->n < 0) return fail(ULM_ERR_ARG, "%s: negative size", who);
+  if (too_many(p->n)) return fail(ULM_ERR_TOO_LARGE, "%s: too many elements", who);
+  if (d) {
+    const int64_t vec = p->dtype == ULM_F32 ? 4 : 8;
+    if (d < 0 || d % vec || stride % vec || stride < d || p->n % d) return fail(ULM_ERR_ARG, "%s: rows and their stride must be whole 16-byte vectors", who);
+    if (p->n / vec > 0xffffffffLL || d / vec > 0xffffffffLL) return fail(ULM_ERR_TOO_LARGE, "%s: too many elements", who);
+  }
+  return ULM_OK;
+}
+
+template <typename T>
+void swiglu_launch(const ulm_swiglu_args* p, bool bwd, int64_t d, int64_t stride) {
+  cudaStream_t st = (cudaStream_t)p->stream;
+  const int64_t nvec = p->n / VecN<T>::N;
+  const Rows rw{(uint32_t)(d / VecN<T>::N), stride / VecN<T>::N};
+  const T *a = (const T*)p->a, *b = (const T*)p->b, *dy = (const T*)p->dy;
+  T *y = (T*)p->y, *da = (T*)p->da, *db = (T*)p->db;
+  const unsigned grid = grid_for(nvec, bwd ? kVecsBwd<T> : kVecsFwd<T>);
+  if (bwd && d) swiglu_bwd_kernel<T, true><<<grid, kThreads, 0, st>>>(a, b, dy, da, db, nvec, p->n, rw);
+  else if (bwd) swiglu_bwd_kernel<T, false><<<grid, kThreads, 0, st>>>(a, b, dy, da, db, nvec, p->n, rw);
+  else if (d) swiglu_fwd_kernel<T, true><<<grid, kThreads, 0, st>>>(a, b, y, nvec, p->n, rw);
+  else swiglu_fwd_kernel<T, false><<<grid, kThreads, 0, st>>>(a, b, y, nvec, p->n, rw);
+}
+
+int swiglu(const ulm_swiglu_args* p, bool bwd, int64_t d, int64_t stride, const char* who) {
+  if (int rc = check_swiglu(p, d, stride, who)) return rc;
+  if (p->n == 0) return ULM_OK;
+  if (!aligned16(p->a) || !aligned16(p->b) || (bwd ? !aligned16(p->dy) || !aligned16(p->da) || !aligned16(p->db) : !aligned16(p->y)))
+    return fail(ULM_ERR_ARG, "%s: %s must be non-null and 16-byte aligned", who, bwd ? "a, b, dy, da, db" : "a, b, y");
+  if (p->dtype == ULM_F16) swiglu_launch<__half>(p, bwd, d, stride);
+  else if (p->dtype == ULM_BF16) swiglu_launch<__nv_bfloat16>(p, bwd, d, stride);
+  else swiglu_launch<float>(p, bwd, d, stride);
+  return check_launch(who);
+}
+
 }  // namespace
 }  // namespace ulm
 
-extern "C" int ulm_swiglu_fwd(const ulm_swiglu_args* p) {
-  using namespace ulm;
-  if (!p) return fail(ULM_ERR_ARG, "ulm_swiglu_fwd: null args");
-  if (p->dtype != ULM_F16 && p->dtype != ULM_BF16 && p->dtype != ULM_F32) return fail(ULM_ERR_ARG, "ulm_swiglu_fwd: bad dtype");
-  if (p->n < 0) return fail(ULM_ERR_ARG, "ulm_swiglu_fwd: negative size");
-  if (too_many(p->n)) return fail(ULM_ERR_TOO_LARGE, "ulm_swiglu_fwd: too many elements");
-  if (p->n == 0) return ULM_OK;
-  if (!aligned16(p->a) || !aligned16(p->b) || !aligned16(p->y)) return fail(ULM_ERR_ARG, "ulm_swiglu_fwd: a, b, y must be non-null and 16-byte aligned");
-  cudaStream_t st = (cudaStream_t)p->stream;
-#define ULM_GO(T)                                                                                   \
-  do {                                                                                              \
-    const int64_t nvec = p->n / VecN<T>::N;                                                          \
-    swiglu_fwd_kernel<T><<<grid_for(nvec, kVecsFwd<T>), kThreads, 0, st>>>((const T*)p->a, (const T*)p->b, (T*)p->y, nvec, p->n); \
-  } while (0)
-  if (p->dtype == ULM_F16) ULM_GO(__half); else if (p->dtype == ULM_BF16) ULM_GO(__nv_bfloat16); else ULM_GO(float);
-#undef ULM_GO
-  return check_launch("ulm_swiglu_fwd");
-}
+extern "C" int ulm_swiglu_fwd(const ulm_swiglu_args* p) { return ulm::swiglu(p, false, 0, 0, "ulm_swiglu_fwd"); }
+extern "C" int ulm_swiglu_bwd(const ulm_swiglu_args* p) { return ulm::swiglu(p, true, 0, 0, "ulm_swiglu_bwd"); }
 
-extern "C" int ulm_swiglu_bwd(const ulm_swiglu_args* p) {
-  using namespace ulm;
-  if (!p) return fail(ULM_ERR_ARG, "ulm_swiglu_bwd: null args");
-  if (p->dtype != ULM_F16 && p->dtype != ULM_BF16 && p->dtype != ULM_F32) return fail(ULM_ERR_ARG, "ulm_swiglu_bwd: bad dtype");
-  if (p->n < 0) return fail(ULM_ERR_ARG, "ulm_swiglu_bwd: negative size");
-  if (too_many(p->n)) return fail(ULM_ERR_TOO_LARGE, "ulm_swiglu_bwd: too many elements");
-  if (p->n == 0) return ULM_OK;
-  if (!aligned16(p->a) || !aligned16(p->b) || !aligned16(p->dy) || !aligned16(p->da) || !aligned16(p->db))
-    return fail(ULM_ERR_ARG, "ulm_swiglu_bwd: a, b, dy, da, db must be non-null and 16-byte aligned");
-  cudaStream_t st = (cudaStream_t)p->stream;
-#define ULM_GO(T)                                                                                   \
-  do {                                                                                              \
-    const int64_t nvec = p->n / VecN<T>::N;                                                          \
-    swiglu_bwd_kernel<T><<<grid_for(nvec, kVecsBwd<T>), kThreads, 0, st>>>((const T*)p->a, (const T*)p->b, (const T*)p->dy, \
-                                                               (T*)p->da, (T*)p->db, nvec, p->n);    \
-  } while (0)
-  if (p->dtype == ULM_F16) ULM_GO(__half); else if (p->dtype == ULM_BF16) ULM_GO(__nv_bfloat16); else ULM_GO(float);
-#undef ULM_GO
-  return check_launch("ulm_swiglu_bwd");
+extern "C" int ulm_swiglu_rows(const ulm_swiglu_args* p, int32_t backward, int64_t d, int64_t row_stride) {
+  if (d <= 0) return ulm::fail(ULM_ERR_ARG, "ulm_swiglu_rows: d must be positive");
+  return ulm::swiglu(p, backward != 0, d, row_stride, "ulm_swiglu_rows");
 }

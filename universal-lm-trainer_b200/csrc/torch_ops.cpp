@@ -632,9 +632,38 @@ struct CastScope {
 };
 std::mutex g_cast_mu;
 std::vector<std::unique_ptr<CastScope>> g_cast_scopes;
-void cast_scope_push() {
+// 16-bit copies of a fixed set of fp32 weights in one buffer, in the given order: one fused cast fills them all where a
+// scope would otherwise make each on first use (a launch and about 12 us of host time per weight), and weights that
+// follow one another in the list do so in memory, so that two projections of one input can run as one GEMM.  A training
+// program keeps the object and refreshes it once per step.
+struct WeightCopies {
+  std::vector<Tensor> params, views;
+  WeightCopies(std::vector<Tensor> ps, at::ScalarType dtype) : params(std::move(ps)) {
+    if (params.empty()) return;
+    OpScope scope;
+    int64_t n = 0;
+    for (const Tensor& p : params) n += (p.numel() + 7) / 8 * 8;              // 16-byte aligned starts
+    const Tensor flat = at::empty({n}, params[0].options().dtype(dtype).requires_grad(false));
+    int64_t off = 0;
+    for (const Tensor& p : params) {
+      views.push_back(flat.narrow(0, off, p.numel()).view(p.sizes()));
+      off += (p.numel() + 7) / 8 * 8;
+    }
+  }
+  void refresh() {
+    if (params.empty()) return;
+    OpScope scope;
+    at::_foreach_copy_(views, params);
+  }
+};
+
+// `copies` (already refreshed) seeds the scope
+void cast_scope_push(const std::shared_ptr<WeightCopies>& copies) {
+  auto scope = std::make_unique<CastScope>();
+  if (copies)
+    for (size_t i = 0; i < copies->params.size(); ++i) scope->made[copies->params[i].unsafeGetTensorImpl()] = {copies->params[i], copies->views[i]};
   std::lock_guard<std::mutex> lock(g_cast_mu);
-  g_cast_scopes.push_back(std::make_unique<CastScope>());
+  g_cast_scopes.push_back(std::move(scope));
 }
 void cast_scope_pop() {
   std::unique_ptr<CastScope> gone;                       // its tensors are released outside the lock
@@ -713,6 +742,98 @@ Tensor linear(const Tensor& x, const Tensor& weight) {
     auto node = make_node<LinearBwd>(x, weight);
     node->cd = cd; node->x_dtype = x.scalar_type();
     node->keep(xc); node->keep(weight);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+// ---------------------------------------------------------------------------
+// gated projections: silu(x w1^T) * (x w3^T)
+// ---------------------------------------------------------------------------
+// Two equal-shaped contiguous matrices that follow one another in one storage, as one matrix; undefined otherwise
+Tensor stacked(const Tensor& a, const Tensor& b) {
+  if (!a.is_contiguous() || !b.is_contiguous() || a.scalar_type() != b.scalar_type() || !a.storage().is_alias_of(b.storage()) ||
+      b.storage_offset() != a.storage_offset() + a.numel())
+    return Tensor();
+  return a.as_strided({a.size(0) + b.size(0), a.size(1)}, {a.size(1), 1}, a.storage_offset());
+}
+
+void swiglu_rows(const Tensor& ab, const Tensor& y, const Tensor& dy, const Tensor& dab, bool backward) {
+  const int64_t d = ab.size(1) / 2, half = d * ab.element_size();
+  auto at_half = [&](const Tensor& t, int h) -> void* { return t.defined() ? static_cast<char*>(t.data_ptr()) + h * half : nullptr; };
+  ulm_swiglu_args p{at_half(ab, 0), at_half(ab, 1), at_half(y, 0), at_half(dy, 0), at_half(dab, 0), at_half(dab, 1), ab.size(0) * d,
+                    code_of(ab.scalar_type()), 0, stream_of(ab)};
+  check(ulm_swiglu_rows(&p, backward, d, 2 * d), backward ? "swiglu backward" : "swiglu forward");
+}
+
+struct GatedBwd : OpNode {
+  at::ScalarType cd, x_dtype;
+  variable_list apply(variable_list&& g) override {
+    if (!g[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    OpScope scope;
+    const Tensor x = kept(0), w1 = kept(1), w3 = kept(2), ab = kept(3);
+    const Tensor dy = g[0].reshape({-1, g[0].size(-1)}).to(cd).contiguous(), x2 = x.reshape({-1, x.size(-1)});
+    const Tensor dab = empty_cuda(ab.sizes(), cd, ab);
+    swiglu_rows(ab, Tensor(), dy, dab, true);
+    const int64_t ff = w1.size(0);
+    const Tensor da = dab.narrow(1, 0, ff), db = dab.narrow(1, ff, ff);
+    Tensor dx, dw1, dw3;
+    if (task_should_compute_output(0)) {
+      const Tensor c1 = cast_cached(w1, cd), c3 = cast_cached(w3, cd), both = stacked(c1, c3);
+      dx = both.defined() ? at::mm(dab, both) : at::mm(da, c1).addmm_(db, c3);      // one GEMM sums the two branches in fp32
+      dx = dx.view(x.sizes()).to(x_dtype);
+    }
+    const bool need1 = task_should_compute_output(1), need3 = task_should_compute_output(2);
+    if (need1 && need3) {
+      const Tensor g1 = w1.grad(), g3 = w3.grad();
+      if (g_wgrad_in_place.load(std::memory_order_relaxed) && is_16bit(cd) && g1.defined() && g3.defined() && g1.scalar_type() == at::kFloat) {
+        Tensor both = stacked(g1, g3);
+        if (both.defined()) {
+          at::addmm_out(both, both, dab.t(), x2, at::kFloat);
+          return {dx, Tensor(), Tensor()};
+        }
+      } else if (is_16bit(cd) && w1.scalar_type() == at::kFloat && w3.scalar_type() == at::kFloat) {
+        const Tensor dw = at::mm(dab.t(), x2, at::kFloat);
+        return {dx, dw.narrow(0, 0, ff), dw.narrow(0, ff, ff)};
+      }
+    }
+    if (need1) dw1 = weight_grad(w1, da, x2);
+    if (need3) dw3 = weight_grad(w3, db, x2);
+    return {dx, dw1, dw3};
+  }
+};
+
+// Both projections write the two halves of one [rows, 2 ff] matrix: as one GEMM where the weights' 16-bit copies lie one
+// behind the other (WeightCopies).  Against two linears and a gate that is one GEMM less forward, two less backward,
+// and no pass that adds the two branches' gradients of x.
+Tensor gated_linear(const Tensor& x, const Tensor& w1, const Tensor& w3) {
+  at::ScalarType cd = x.scalar_type();
+  if (x.is_cuda() && at::autocast::is_autocast_enabled(at::kCUDA)) cd = at::autocast::get_autocast_dtype(at::kCUDA);
+  const int64_t ff = w1.size(0);
+  if (!x.is_cuda() || !known(cd) || w3.sizes() != w1.sizes() || ff % (16 / (int64_t)c10::elementSize(cd))) return ::swiglu(::linear(x, w1), ::linear(x, w3));
+  Tensor xc, ab, y;
+  {
+    OpScope scope;
+    c10::cuda::CUDAGuard dev(x.device());
+    xc = x.to(cd);
+    const Tensor x2 = xc.reshape({-1, xc.size(-1)}), c1 = cast_cached(w1, cd), c3 = cast_cached(w3, cd), both = stacked(c1, c3);
+    if (both.defined()) {
+      ab = at::mm(x2, both.t());
+    } else {
+      ab = empty_cuda({x2.size(0), 2 * ff}, cd, x2);
+      Tensor a = ab.narrow(1, 0, ff), b = ab.narrow(1, ff, ff);
+      at::mm_out(a, x2, c1.t());
+      at::mm_out(b, x2, c3.t());
+    }
+    auto n = xc.sizes().vec();
+    n.back() = ff;
+    y = empty_cuda(n, cd, x2);
+    swiglu_rows(ab, y, Tensor(), Tensor(), false);
+  }
+  if (!no_graph(x, w1, w3)) {
+    auto node = make_node<GatedBwd>(x, w1, w3);
+    node->cd = cd; node->x_dtype = x.scalar_type();
+    node->keep(xc); node->keep(w1); node->keep(w3); node->keep(ab);
     torch::autograd::set_history(y, node);
   }
   return y;
@@ -843,7 +964,10 @@ PYBIND11_MODULE(_ulm_torch, m) {
   m.def("add_rms_norm", &add_rms_norm, no_gil());
   m.def("swiglu", &swiglu, no_gil());
   m.def("set_wgrad_in_place", [](bool on) { return g_wgrad_in_place.exchange(on); });
-  m.def("cast_scope_push", &cast_scope_push);
+  py::class_<WeightCopies, std::shared_ptr<WeightCopies>>(m, "WeightCopies")
+      .def(py::init<std::vector<Tensor>, at::ScalarType>())
+      .def("refresh", &WeightCopies::refresh, no_gil());
+  m.def("cast_scope_push", &cast_scope_push, py::arg("copies") = nullptr);
   m.def("cast_scope_pop", &cast_scope_pop, no_gil());
   m.def("cast_cached", &cast_cached, no_gil());
   m.def("weight_grad", [](const Tensor& w, const Tensor& dy, const Tensor& x) -> OptTensor {
@@ -852,6 +976,7 @@ PYBIND11_MODULE(_ulm_torch, m) {
     return g.defined() ? OptTensor(g) : std::nullopt;
   }, no_gil());
   m.def("linear", &linear, no_gil());
+  m.def("gated_linear", &gated_linear, no_gil());
   m.def("lm_head_lse", &lm_head_lse, no_gil());
   m.def("lm_head_score", &lm_head_score, no_gil());
   m.def("kept_cross_entropy", &kept_cross_entropy, no_gil());

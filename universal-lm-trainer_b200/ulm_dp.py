@@ -437,6 +437,7 @@ class DataParallelStep:
         # cast once per step instead of once per call (and not again by a checkpointed layer's recomputation).
         # 'call': one context per forward, closed before its backward, like the reference's loop (train.py:2351).
         self.amp_scope = amp_scope
+        self._copies = None                               # see _weight_copies
 
     def _arm(self):
         """Called before the backward of this rank's last micro-batch of the step."""
@@ -461,6 +462,16 @@ class DataParallelStep:
         if self._pending[bi] == 0:
             self._ready[bi] = True
             self._launch_ready()
+
+    def _weight_copies(self):
+        """The buffer of the linear layers' 16-bit weights (2 bytes per element, kept between steps and refilled by one
+        fused cast at the start of each); None where there is nothing to cast."""
+        if self._copies is None:
+            linears = {id(m.weight): m.weight for m in self.model.modules() if isinstance(m, torch.nn.Linear)}
+            ws = [w for w in linears.values() if w.is_cuda and w.dtype == torch.float32 and w.device == self.device]
+            use = ws and self.amp_scope == 'step' and self.dtype in (torch.float16, torch.bfloat16)
+            self._copies = ulm_ops.weight_copies(ws, self.dtype) if use else False
+        return self._copies or None
 
     def _forward_backward(self, ids, weight, n_tokens):
         if self.amp_scope == 'call' and self.device.type == 'cuda':
@@ -499,7 +510,7 @@ class DataParallelStep:
             dev_ids = [(rows if rows.is_pinned() else rows.pin_memory()).to(self.device, non_blocking=True) for rows, _, _ in work]
         else:
             dev_ids = [rows for rows, _, _ in work]
-        with amp, in_place, ulm_ops.weight_cast_scope():
+        with amp, in_place, ulm_ops.weight_cast_scope(self._weight_copies()):
             for i, (rows, weight, n_tokens) in enumerate(work):
                 if sharded and self.overlap and i == len(work) - 1:
                     self._arm()                           # all-reduce buckets as their gradients complete

@@ -15,7 +15,7 @@ import torch.nn.functional as F
 
 import flash_attn_v100_cuda as _fa
 import ulm_ops
-from ulm_ops import FusedRMSNorm, linear, swiglu
+from ulm_ops import FusedRMSNorm, gated_linear, linear
 
 
 @dataclass
@@ -130,7 +130,7 @@ class FeedForward(nn.Module):  # train.py:1966-1975
         self.dropout = nn.Dropout(dropout)
 
     def forward(self, x):
-        return linear(self.dropout(swiglu(linear(x, self.w1.weight), linear(x, self.w3.weight))), self.w2.weight)
+        return linear(self.dropout(gated_linear(x, self.w1.weight, self.w3.weight)), self.w2.weight)
 
 
 class DecoderOnlyBlock(nn.Module):  # train.py:1977-1994

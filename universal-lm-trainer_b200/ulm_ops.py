@@ -87,16 +87,32 @@ def wgrad_in_place(enabled=True):
 
 
 @contextlib.contextmanager
-def weight_cast_scope():
+def weight_cast_scope(copies=None):
     """While active, `linear` keeps the 16-bit copy it makes of a weight and reuses it: the caller promises
     that the weights do not change inside the scope (one optimiser step's forward/backward calls).  Nothing
     is reused across scopes or outside one -- a parameter's version counter cannot be relied on for that
-    (fused optimisers update parameters without bumping it)."""
-    N.ext().cast_scope_push()
+    (fused optimisers update parameters without bumping it).  ``copies``: a `weight_copies` object, which is
+    refreshed here; without it each weight is cast on first use."""
+    if copies is not None:
+        copies.refresh()
+    N.ext().cast_scope_push(copies)
     try:
         yield
     finally:
         N.ext().cast_scope_pop()
+
+
+def weight_copies(weights, dtype):
+    """One buffer for the 16-bit copies of ``weights`` (fp32 CUDA parameters), kept by the caller and filled by one fused
+    cast each time a `weight_cast_scope` opens with it; weights that follow one another in the list do so in the
+    buffer, so that `gated_linear` runs its two projections as one GEMM.  Holds 2 bytes per weight element."""
+    return N.ext().WeightCopies(list(weights), dtype)
+
+
+def gated_linear(x, w1, w3):
+    """``swiglu(linear(x, w1), linear(x, w3))`` (train.py:1975) as one op: both projections write the halves of one
+    [rows, 2 d_ff] matrix, which the gate's kernels read and differentiate in place of two."""
+    return N.ext().gated_linear(x, w1, w3)
 
 
 def linear(x, weight):
