@@ -122,6 +122,9 @@ typedef struct {
   int64_t qr_sb, qr_sh, qr_ss;
 } ulm_attn_fwd_args;
 int ulm_attn_fwd(const ulm_attn_fwd_args* a);
+/* The same for sequences of at most 128 rows, with k BEFORE rotation too: the one CTA of a (batch, head) rotates q and k
+ * and, where q_rot / k_rot (16-byte aligned, strides multiples of 8) are not NULL, writes the rotated tensors. */
+int ulm_attn_fwd_rope_qk(const ulm_attn_fwd_args* a, void* k_rot, int64_t kr_sb, int64_t kr_sh, int64_t kr_ss);
 
 /* ---- attention backward --------------------------------------------------
  * Replaces fa_bwd (csrc/flash_attn_v100/flash_attn_v100_bwd.cu:433-506; kernels

@@ -115,6 +115,7 @@ EXPORTS = {
     'ulm_launch_count': (C.c_uint64, []),
     'ulm_rope': (C.c_int, [C.POINTER(RopeArgs)]),
     'ulm_attn_fwd': (C.c_int, [C.POINTER(AttnFwdArgs)]),
+    'ulm_attn_fwd_rope_qk': (C.c_int, [C.POINTER(AttnFwdArgs), vp, i64, i64, i64]),
     'ulm_attn_bwd': (C.c_int, [C.POINTER(AttnBwdArgs)]),
     'ulm_rmsnorm_fwd': (C.c_int, [C.POINTER(RmsFwdArgs)]),
     'ulm_rmsnorm_bwd': (C.c_int, [C.POINTER(RmsBwdArgs)]),

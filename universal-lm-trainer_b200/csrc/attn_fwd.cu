@@ -34,7 +34,11 @@
 // the writes visible to the tensor core's shared-memory reads with a proxy fence and
 // release the MMA issuer; the rotated tile is also written out for the backward.  A
 // Q tile belongs to exactly one CTA, so nothing is rotated twice.  K tiles are read by
-// every query tile of their head and therefore come rotated by the stand-alone kernel.
+// every query tile of their head and therefore come rotated by the stand-alone kernel --
+// except when the whole sequence is one query tile (S <= 128): then K belongs to this CTA
+// alone, its rows have the positions of Q's, and it is rotated with the same table values
+// in the same pass (kRopeQK).  One launch instead of two: at these sizes launches are the cost
+// (67 tokens x 12 heads: 14.2 -> 8.3 us a call).
 // Every barrier wait is bounded; on expiry the CTA records a status bit, drains
 // its loads, frees TMEM and returns.  Waits of the softmax warps are made warp-uniform
 // by a vote, because warp-wide instructions (TMEM loads, votes) follow them.
@@ -82,12 +86,17 @@ __device__ __forceinline__ bool dropout_keep(uint32_t seed_mix, int row, int col
   return ((h >> 8) * (1.0f / 16777216.0f)) >= p;
 }
 
-// Tables and destination of the fused Q rotation (unused when ROPE is false).
+// What is rotated inside the kernel
+enum { kRopeNone = 0, kRopeQ = 1, kRopeQK = 2 };
+
+// Tables of the fused rotation and destinations of the rotated tensors, either may be null (unused with kRopeNone).
 struct RopeQ {
   const float* cos_tab; const float* sin_tab;
   int64_t cos_stride, sin_stride;
   void* q_rot;
   int64_t sb, sh, ss;
+  void* k_rot;
+  int64_t k_sb, k_sh, k_ss;
 };
 
 // All lanes of a warp learn together whether the wait succeeded.
@@ -95,7 +104,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
-template <typename T, bool CAUSAL, bool DROPOUT, bool ROPE>
+template <typename T, bool CAUSAL, bool DROPOUT, int ROPE>
 __global__ void __launch_bounds__(kThreads, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, T* __restrict__ O, float* __restrict__ LSE,
@@ -121,7 +130,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   // values first of all, so that the loads' latency runs under the barrier set-up, the TMEM allocation and
   // the Q tile's TMA load.
   [[maybe_unused]] RopeQuad rope_tab[4];
-  if constexpr (ROPE) {
+  if constexpr (ROPE != kRopeNone) {
     if (warp < 8) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -185,8 +194,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       constexpr uint32_t idesc_o = make_idesc(fmt, BM, HD, 1);
       const uint32_t tS = tmem_base + kColS, tO = tmem_base + kColO;
       // with the fused rotation the tile is usable once the softmax warps have rewritten it
-      bool ok = ROPE ? mbar_wait(&ctl->q_ready, 0, abort_flag) : mbar_wait(&ctl->q_full, 0, abort_flag);
-      if (!ok) atomicOr(&ctl->fail_bits, (uint32_t)(ROPE ? ULM_STATUS_TIMEOUT_SOFTMAX : ULM_STATUS_TIMEOUT_LOAD));
+      bool ok = ROPE != kRopeNone ? mbar_wait(&ctl->q_ready, 0, abort_flag) : mbar_wait(&ctl->q_full, 0, abort_flag);
+      if (!ok) atomicOr(&ctl->fail_bits, (uint32_t)(ROPE != kRopeNone ? ULM_STATUS_TIMEOUT_SOFTMAX : ULM_STATUS_TIMEOUT_LOAD));
       fence_after_sync();
       const uint64_t dq = make_sdesc_sw128(smem_u32(sQ));
       auto issue_scores = [&](int j) -> bool {             // S_j = Q K_j^T into score buffer j & 1
@@ -232,7 +241,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint64_t sc2 = f2_pack(scale2, scale2);
     float m = -INFINITY, l = 0.f;
     bool ok = true;
-    if constexpr (ROPE) {
+    if constexpr (ROPE != kRopeNone) {
       // Rotate the resident Q tile in place (128-byte-swizzled rows) and write the rotated rows out.
       ok = warp_wait(&ctl->q_full, 0, abort_flag);
       if (!ok && lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD);
@@ -252,6 +261,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             T* dst = qr_base + (int64_t)(m0 + row) * rq.ss;
             *reinterpret_cast<uint2*>(dst + 4 * cg) = olo;
             *reinterpret_cast<uint2*>(dst + 32 + 4 * cg) = ohi;
+          }
+        }
+        if constexpr (ROPE == kRopeQK) {
+          // Rows 0-63 of K are tile 0 (stage 0 of the ring), 64-127 tile 1: task j is row 32 j + t / 8 here too
+          T* kr_base = rq.k_rot ? reinterpret_cast<T*>(rq.k_rot) + (int64_t)b * rq.k_sb + (int64_t)h * rq.k_sh : nullptr;
+          for (int i = 0; i < nkv; ++i) ok = ok && warp_wait(&ctl->k_full[i], 0, abort_flag);
+          if (!ok && lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int row = 32 * j + ((int)threadIdx.x >> 3);
+            if (!ok || row >= nkv * BN) continue;
+            uint8_t* tile = sKV + (size_t)(row >> 6) * 2 * kTileBytes;
+            uint2* p_lo = reinterpret_cast<uint2*>(tile + swz_quad_offset(row & 63, cg));
+            uint2* p_hi = reinterpret_cast<uint2*>(tile + swz_quad_offset(row & 63, cg + 8));
+            uint2 olo, ohi;
+            rope_apply_quad<T, false>(rope_tab[j], *p_lo, *p_hi, olo, ohi);
+            *p_lo = olo;
+            *p_hi = ohi;
+            if (kr_base && row < S) {
+              T* dst = kr_base + (int64_t)row * rq.k_ss;
+              *reinterpret_cast<uint2*>(dst + 4 * cg) = olo;
+              *reinterpret_cast<uint2*>(dst + 32 + 4 * cg) = ohi;
+            }
           }
         }
         // generic-proxy writes -> visible to the tensor core's (async proxy) operand reads
@@ -386,13 +418,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (threadIdx.x == 0 && ctl->fail_bits && status) atomicOr(status, ctl->fail_bits);
 }
 
-template <typename T, bool CAUSAL, bool DROPOUT, bool ROPE>
-int launch(const ulm_attn_fwd_args* a, int device, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv) {
+// where the rotated K goes (kRopeQK)
+struct KRot { void* p; int64_t sb, sh, ss; };
+
+template <typename T, bool CAUSAL, bool DROPOUT, int ROPE>
+int launch(const ulm_attn_fwd_args* a, const KRot& kr, int device, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv) {
   static std::atomic<bool> attr_set[kMaxDevices];
   auto kern = attn_fwd_kernel<T, CAUSAL, DROPOUT, ROPE>;
   if (int rc = ensure_smem_attr(kern, kSmemBytes, device, attr_set, "ulm_attn_fwd")) return rc;
   RopeQ rq{};
-  if (ROPE) rq = RopeQ{a->cos_tab, a->sin_tab, a->cos_stride, a->sin_stride, a->q_rot, a->qr_sb, a->qr_sh, a->qr_ss};
+  if (ROPE != kRopeNone)
+    rq = RopeQ{a->cos_tab, a->sin_tab, a->cos_stride, a->sin_stride, a->q_rot, a->qr_sb, a->qr_sh, a->qr_ss, kr.p, kr.sb, kr.sh, kr.ss};
   dim3 grid((unsigned)(a->B * a->H), (unsigned)((a->S + BM - 1) / BM));
   kern<<<grid, kThreads, kSmemBytes, (cudaStream_t)a->stream>>>(
       mq, mk, mv, (T*)a->o, a->lse, a->o_sb, a->o_sh, a->o_ss, a->S, a->H,
@@ -400,19 +436,15 @@ int launch(const ulm_attn_fwd_args* a, int device, const CUtensorMap& mq, const 
   return check_launch("ulm_attn_fwd");
 }
 
-template <typename T, bool ROPE>
-int dispatch(const ulm_attn_fwd_args* a, int device, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv) {
+template <typename T, int ROPE>
+int dispatch(const ulm_attn_fwd_args* a, const KRot& kr, int device, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv) {
   const bool drop = a->dropout_p > 0.f;
-  if (a->causal) return drop ? launch<T, true, true, ROPE>(a, device, mq, mk, mv) : launch<T, true, false, ROPE>(a, device, mq, mk, mv);
-  return drop ? launch<T, false, true, ROPE>(a, device, mq, mk, mv) : launch<T, false, false, ROPE>(a, device, mq, mk, mv);
+  if (a->causal) return drop ? launch<T, true, true, ROPE>(a, kr, device, mq, mk, mv) : launch<T, true, false, ROPE>(a, kr, device, mq, mk, mv);
+  return drop ? launch<T, false, true, ROPE>(a, kr, device, mq, mk, mv) : launch<T, false, false, ROPE>(a, kr, device, mq, mk, mv);
 }
 
-}  // namespace
-}  // namespace ulm
-
-extern "C" int ulm_attn_fwd(const ulm_attn_fwd_args* a) {
-  using namespace ulm;
-  if (!a) return fail(ULM_ERR_ARG, "ulm_attn_fwd: null args");
+// kr: the destination of the rotated K when k comes unrotated too (S <= 128), else null
+int attn_fwd(const ulm_attn_fwd_args* a, const KRot* kr) {
   if (a->dtype != ULM_F16 && a->dtype != ULM_BF16) return fail(ULM_ERR_ARG, "ulm_attn_fwd: dtype must be f16 or bf16");
   if (a->B < 0 || a->H < 0 || a->S < 0) return fail(ULM_ERR_ARG, "ulm_attn_fwd: negative size");
   if (a->B == 0 || a->H == 0 || a->S == 0) return ULM_OK;
@@ -438,6 +470,29 @@ extern "C" int ulm_attn_fwd(const ulm_attn_fwd_args* a) {
   if ((rc = tc::encode_bhsd_map(&mq, a->q, a->dtype, a->B, a->H, a->S, a->q_sb, a->q_sh, a->q_ss, BM, "ulm_attn_fwd(q)"))) return rc;
   if ((rc = tc::encode_bhsd_map(&mk, a->k, a->dtype, a->B, a->H, a->S, a->k_sb, a->k_sh, a->k_ss, BN, "ulm_attn_fwd(k)"))) return rc;
   if ((rc = tc::encode_bhsd_map(&mv, a->v, a->dtype, a->B, a->H, a->S, a->v_sb, a->v_sh, a->v_ss, BN, "ulm_attn_fwd(v)"))) return rc;
-  if (a->dtype == ULM_F16) return rope ? dispatch<__half, true>(a, dev.device, mq, mk, mv) : dispatch<__half, false>(a, dev.device, mq, mk, mv);
-  return rope ? dispatch<__nv_bfloat16, true>(a, dev.device, mq, mk, mv) : dispatch<__nv_bfloat16, false>(a, dev.device, mq, mk, mv);
+  auto go = [&](auto t) {
+    using T = decltype(t);
+    if (kr) return dispatch<T, kRopeQK>(a, *kr, dev.device, mq, mk, mv);
+    return rope ? dispatch<T, kRopeQ>(a, KRot{}, dev.device, mq, mk, mv) : dispatch<T, kRopeNone>(a, KRot{}, dev.device, mq, mk, mv);
+  };
+  return a->dtype == ULM_F16 ? go(__half()) : go(__nv_bfloat16());
+}
+
+}  // namespace
+}  // namespace ulm
+
+extern "C" int ulm_attn_fwd(const ulm_attn_fwd_args* a) {
+  if (!a) return ulm::fail(ULM_ERR_ARG, "ulm_attn_fwd: null args");
+  return ulm::attn_fwd(a, nullptr);
+}
+
+extern "C" int ulm_attn_fwd_rope_qk(const ulm_attn_fwd_args* a, void* k_rot, int64_t kr_sb, int64_t kr_sh, int64_t kr_ss) {
+  using namespace ulm;
+  if (!a) return fail(ULM_ERR_ARG, "ulm_attn_fwd_rope_qk: null args");
+  if (a->S > BM) return fail(ULM_ERR_TOO_LARGE, "ulm_attn_fwd_rope_qk: takes sequences of at most %d rows", BM);
+  if (!a->cos_tab || !a->sin_tab) return fail(ULM_ERR_ARG, "ulm_attn_fwd_rope_qk: needs the RoPE tables");
+  if (k_rot && ((reinterpret_cast<uintptr_t>(k_rot) & 15) || kr_sb % 8 || kr_sh % 8 || kr_ss % 8))
+    return fail(ULM_ERR_ARG, "ulm_attn_fwd_rope_qk: k_rot must be 16-byte aligned with strides that are multiples of 8");
+  const KRot kr{k_rot, kr_sb, kr_sh, kr_ss};
+  return attn_fwd(a, &kr);
 }

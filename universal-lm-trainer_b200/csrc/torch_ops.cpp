@@ -168,9 +168,13 @@ struct AttnArgs {
   double dropout_p; bool causal; double scale; int64_t seed;
 };
 
-// -> (o, lse); with tables q comes unrotated and, where q_rot is defined, its rotated copy is written there
+// Longest sequence whose K the attention forward rotates itself (one query tile)
+constexpr int64_t kRopeQkRows = 128;
+
+// -> (o, lse); with tables q comes unrotated and, where q_rot is defined, its rotated copy is written there; with k_rot
+// (S <= kRopeQkRows) k comes unrotated too
 void attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const AttnArgs& p,
-                  const Tensor& cos = Tensor(), const Tensor& sin = Tensor(), const Tensor& q_rot = Tensor()) {
+                  const Tensor& cos = Tensor(), const Tensor& sin = Tensor(), const Tensor& q_rot = Tensor(), const Tensor& k_rot = Tensor()) {
   ulm_attn_fwd_args a{};
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.lse = lse.data_ptr<float>();
   a.q_sb = q.stride(0); a.q_sh = q.stride(1); a.q_ss = q.stride(2);
@@ -189,7 +193,8 @@ void attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
       a.qr_sb = q_rot.stride(0); a.qr_sh = q_rot.stride(1); a.qr_ss = q_rot.stride(2);
     }
   }
-  check(ulm_attn_fwd(&a), "flash_attn_v100 forward");
+  check(k_rot.defined() ? ulm_attn_fwd_rope_qk(&a, k_rot.data_ptr(), k_rot.stride(0), k_rot.stride(1), k_rot.stride(2)) : ulm_attn_fwd(&a),
+        "flash_attn_v100 forward");
 }
 
 void attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o_in, const Tensor& lse, const Tensor& do_in,
@@ -319,7 +324,10 @@ std::pair<Tensor, Tensor> rope_attn_forward(const Tensor& q, const Tensor& k, co
                                             const Tensor& o, const Tensor& lse, const AttnArgs& p, int64_t fuse) {
   const Tensor ko = rope_out_like(k.sizes(), k.strides(), k);
   Tensor qo;
-  if (fuse == kFuseNone) {
+  if (q.size(2) <= kRopeQkRows) {                        // one query tile: its CTA rotates both, and a launch is saved
+    qo = rope_out_like(q.sizes(), q.strides(), q);
+    attn_forward(q, k, v, o, lse, p, cos, sin, qo, ko);
+  } else if (fuse == kFuseNone) {
     qo = rope_out_like(q.sizes(), q.strides(), q);
     rope_launch(q, k, qo, ko, cos, sin, false);
     attn_forward(qo, ko, v, o, lse, p);
@@ -451,12 +459,17 @@ std::tuple<Tensor, Tensor, Tensor> causal_attention(const Tensor& qkv_in, int64_
   if (cos_o) {
     // the model's [1, L, >=64] or [L, >=64] tables
     auto table = [&](const Tensor& t) {
+      if (t.dim() == 2 && t.size(0) == S && t.size(1) == 64) return t;
       const Tensor t2 = t.reshape({-1, t.size(-1)});
-      return t2.size(0) >= S && t2.size(1) >= 64 ? t2.narrow(0, 0, S).narrow(1, 0, 64) : t2;
+      return t2.size(0) >= S && t2.size(1) >= 64 ? t2.as_strided({S, 64}, t2.strides(), t2.storage_offset()) : t2;
     };
     cos = table(*cos_o); sin = table(*sin_o);
     TORCH_CHECK_VALUE(rope_can_use(q, k, cos, sin), "causal_attention needs fp32 RoPE tables of at least 64 columns on the same device");
     const Tensor ko = rope_out_like(k.sizes(), k.strides(), k);
+    if (S <= kRopeQkRows) {
+      attn_forward(q, k, v, heads_of(out, B, S, H), lse, p, cos, sin, Tensor(), ko);
+      return {out, ko, v};
+    }
     rope_launch(Tensor(), k, Tensor(), ko, cos, sin, false);
     k = ko;
   }
