@@ -297,6 +297,12 @@ int ulm_ce_bwd(const ulm_ce_bwd_args* a);
 int ulm_loss_mean(const float* rows_loss, const int64_t* target, int64_t rows, int64_t ignore_index, const float* denom_dev,
                   float denom, float* loss, float* inv, void* stream);
 
+/* One micro-batch's int64 ids [n, len] (and labels, the same tensor as a rule) as `padded` >= n * len flat rows: ids_out
+ * (0 past the end) and target_out, the next token of the row's sequence, ignore_index at its end and on the padding
+ * (train.py:2063-2067's shift). */
+int ulm_token_targets(const int64_t* ids, const int64_t* labels, int64_t n, int64_t len, int64_t padded, int64_t ignore_index,
+                      int64_t* ids_out, int64_t* target_out, void* stream);
+
 /* ---- lm-head GEMM with the loss statistics in its epilogue -----------------
  * Forward of the reference's `F.cross_entropy(self.fc_out(h), t)` (train.py:2075-2079) as ONE tensor-core
  * kernel plus a per-row finishing kernel: z = h w^T rounded to the 16-bit dtype (what the autocast linear
@@ -342,6 +348,9 @@ int ulm_lmhead_score(const ulm_lmhead_lse_args* a, uint8_t* hit, int32_t* part_i
  */
 int ulm_grad_unscale_sumsq(float* grad, int64_t n, const float* inv_scale_dev,
                            float* out, float* partial, void* stream);
+/* clip_grad_norm_ (train.py:2365) on the same bucket: *norm_out = sqrt(*sumsq), g *= min(1, max_norm / (norm + 1e-6)); all
+ * on the device, without a pass over the gradients when nothing is to be clipped. */
+int ulm_grad_clip(float* grad, int64_t n, const float* sumsq, float max_norm, float* norm_out, void* stream);
 int64_t ulm_grad_sumsq_partial_count(void);
 
 /* ---- diagnostics ------------------------------------------------------------

@@ -132,6 +132,8 @@ EXPORTS = {
     'ulm_swiglu_bwd': (C.c_int, [C.POINTER(SwigluArgs)]),
     'ulm_swiglu_rows': (C.c_int, [C.POINTER(SwigluArgs), C.c_int32, i64, i64]),
     'ulm_grad_unscale_sumsq': (C.c_int, [vp, i64, vp, vp, vp, vp]),
+    'ulm_grad_clip': (C.c_int, [vp, i64, vp, f32, vp, vp]),
+    'ulm_token_targets': (C.c_int, [vp, vp, i64, i64, i64, i64, vp, vp, vp]),
     'ulm_grad_sumsq_partial_count': (C.c_int64, []),
     'ulm_tensor_map_cache_stats': (None, [C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
     'ulm_selftest_wait_timeout': (C.c_int, [C.c_uint64, vp, vp]),

@@ -168,6 +168,18 @@ loss_mean_kernel(const float* __restrict__ rows_loss, const int64_t* __restrict_
   }
 }
 
+// One micro-batch's ids as the model's flat, padded rows: ids_out[i] = ids[i] (0 past the end) and target_out[i] = the
+// label the row predicts, the next token of its sequence; ignore_index for a sequence's last position and the padding.
+__global__ void __launch_bounds__(256)
+token_targets_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__ labels, int64_t tokens, int64_t len, int64_t padded,
+                     int64_t ignore_index, int64_t* __restrict__ ids_out, int64_t* __restrict__ target_out) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= padded) return;
+  const bool in = i < tokens;
+  ids_out[i] = in ? ids[i] : 0;
+  target_out[i] = in && (i + 1) % len != 0 ? labels[i + 1] : ignore_index;
+}
+
 int check(const char* who, const void* logits, const void* target, const void* lse, int64_t row_stride,
           int64_t rows, int V, int dtype) {
   if (dtype != ULM_F16 && dtype != ULM_BF16 && dtype != ULM_F32) return fail(ULM_ERR_ARG, "%s: bad dtype", who);
@@ -207,6 +219,17 @@ extern "C" int ulm_ce_bwd(const ulm_ce_bwd_args* a) {
   if (a->dtype == ULM_F16) ULM_CE_BWD(__half); else if (a->dtype == ULM_BF16) ULM_CE_BWD(__nv_bfloat16); else ULM_CE_BWD(float);
 #undef ULM_CE_BWD
   return check_launch("ulm_ce_bwd");
+}
+
+extern "C" int ulm_token_targets(const int64_t* ids, const int64_t* labels, int64_t n, int64_t len, int64_t padded, int64_t ignore_index,
+                                 int64_t* ids_out, int64_t* target_out, void* stream) {
+  using namespace ulm;
+  if (n < 0 || len < 0 || padded < n * len) return fail(ULM_ERR_ARG, "ulm_token_targets: bad sizes");
+  if (padded == 0) return ULM_OK;
+  if (!ids_out || !target_out || (n * len > 0 && (!ids || !labels))) return fail(ULM_ERR_ARG, "ulm_token_targets: null pointer");
+  if ((padded + 255) / 256 > 0x7fffffffLL) return fail(ULM_ERR_TOO_LARGE, "ulm_token_targets: too many tokens");
+  token_targets_kernel<<<(unsigned)((padded + 255) / 256), 256, 0, (cudaStream_t)stream>>>(ids, labels, n * len, len > 0 ? len : 1, padded, ignore_index, ids_out, target_out);
+  return check_launch("ulm_token_targets");
 }
 
 extern "C" int ulm_loss_mean(const float* rows_loss, const int64_t* target, int64_t rows, int64_t ignore_index, const float* denom_dev,

@@ -479,8 +479,9 @@ class DataParallelStep:
                 loss = self.model.compute_loss(ids, ignore_index=self.pad_id, chunk_rows=self.chunk_rows, denominator=n_tokens)
         else:
             loss = self.model.compute_loss(ids, ignore_index=self.pad_id, chunk_rows=self.chunk_rows, denominator=n_tokens)
-        (loss * (weight * self.scale)).backward()
-        return loss.detach() * weight
+        # the loss scale and the micro-batch's weight enter as the gradient of the loss: no product in the graph
+        loss.backward(torch.full_like(loss, weight * self.scale))
+        return loss.detach()
 
     def _event(self):
         e = torch.cuda.Event(enable_timing=True)
@@ -514,7 +515,7 @@ class DataParallelStep:
             for i, (rows, weight, n_tokens) in enumerate(work):
                 if sharded and self.overlap and i == len(work) - 1:
                     self._arm()                           # all-reduce buckets as their gradients complete
-                loss_acc += self._forward_backward(dev_ids[i], weight, n_tokens)
+                loss_acc.add_(self._forward_backward(dev_ids[i], weight, n_tokens), alpha=weight)
         if prof:
             ev.append(self._event())
         if sharded:
@@ -545,7 +546,7 @@ class DataParallelStep:
         flat = self.grads.flat
         self.stats.zero_()
         self.grad_post(flat, self.inv_scale, self.stats)
-        norm = self.stats[0].sqrt()
+        norm = None
         t_enq = time.perf_counter() - self._prof[0] if self.profile else 0.0   # host time to enqueue everything so far
         if self.scale != 1.0:
             # the one host sync of the step (the reference's is loss_accum.item(), train.py:2375); the
@@ -555,8 +556,10 @@ class DataParallelStep:
             skipped = False
         if not skipped:
             if self.max_norm is not None:
-                flat.mul_(torch.clamp(self.max_norm / (norm + 1e-6), max=1.0))   # clip_grad_norm_'s factor
+                norm = self._clip(flat)
             self.opt.step()
+        if norm is None:
+            norm = self.stats[0].sqrt()
         if self.profile:
             t_host0, ev = self._prof
             ev.append(self._event())
@@ -577,6 +580,14 @@ class DataParallelStep:
                     self.scale, self._clean_steps = self.scale * 2.0, 0
             self.inv_scale.fill_(1.0 / self.scale)
         return loss_acc, norm, skipped
+
+    def _clip(self, flat):
+        """clip_grad_norm_ with the norm the post-pass left in ``stats``; returns the norm."""
+        if flat.is_cuda:
+            return ulm_ops.grad_clip_(flat, self.stats, self.max_norm)
+        norm = self.stats[0].sqrt()
+        flat.mul_(torch.clamp(self.max_norm / (norm + 1e-6), max=1.0))
+        return norm
 
     def gradients_of(self, micro_batches, sharded=True):
         """Loss and unscaled gradients of one step WITHOUT touching the optimiser: with

@@ -177,7 +177,7 @@ class DecoderOnlyTransformer(nn.Module):  # train.py:1996-2082
             if isinstance(m, (nn.Linear, nn.Embedding)):
                 nn.init.normal_(m.weight, mean=0.0, std=0.02)
 
-    def _forward_flat(self, ids, quantum=0):
+    def _forward_flat(self, ids, quantum=0, flat_ids=None):
         """Hidden states of the flattened tokens, [T', d] with T' = n*L rounded up to a multiple of ``quantum``
         (0: no padding).  Everything outside the attention works on rows, so the layers run on the 2-D tensor;
         the padding rows carry an arbitrary token, are seen by projections, norms and gates only, and reach
@@ -187,9 +187,10 @@ class DecoderOnlyTransformer(nn.Module):  # train.py:1996-2082
         n, L = ids.shape
         T = n * L
         Tp = T if quantum <= 1 else -(-T // quantum) * quantum
-        flat_ids = ids.reshape(-1)
-        if Tp > T:
-            flat_ids = torch.cat([flat_ids, flat_ids.new_zeros(Tp - T)])
+        if flat_ids is None:
+            flat_ids = ids.reshape(-1)
+            if Tp > T:
+                flat_ids = torch.cat([flat_ids, flat_ids.new_zeros(Tp - T)])
         x = self.embedding(flat_ids)
         cos = sin = None
         if self.config.use_rope:
@@ -218,9 +219,9 @@ class DecoderOnlyTransformer(nn.Module):  # train.py:1996-2082
         targets: the data-parallel step passes the micro-batch's global count."""
         labels = input_ids if labels is None else labels
         n, L = input_ids.shape
-        hidden, T = self._forward_flat(input_ids, TOKEN_QUANTUM)
         # position i predicts label i+1; a row's last position and the padding rows predict nothing
-        target = labels.new_full((hidden.shape[0],), ignore_index)
-        target[:T].view(n, L)[:, :-1] = labels[:, 1:]
+        Tp = n * L if TOKEN_QUANTUM <= 1 else -(-n * L // TOKEN_QUANTUM) * TOKEN_QUANTUM
+        flat_ids, target = ulm_ops.token_targets(input_ids.contiguous(), labels.contiguous(), Tp, ignore_index)
+        hidden, _ = self._forward_flat(input_ids, TOKEN_QUANTUM, flat_ids)
         return ulm_ops.chunked_cross_entropy(hidden, self.fc_out.weight, target, ignore_index=ignore_index,
                                              chunk_rows=chunk_rows, denominator=denominator)

@@ -245,6 +245,25 @@ def chunked_cross_entropy(hidden, weight, target, ignore_index=0, chunk_rows=204
     return _ChunkedCE.apply(hidden, weight, target, int(ignore_index), int(chunk_rows), compute_dtype, denominator)
 
 
+def token_targets(ids, labels, padded, ignore_index):
+    """The [n, L] int64 ``ids`` as ``padded`` flat rows (0 past the end) and the label each row predicts: the next token of
+    its sequence, ``ignore_index`` at a sequence's last position and on the padding rows."""
+    n, L = ids.shape
+    out = torch.empty((2, padded), dtype=torch.long, device=ids.device)
+    N.check(N.lib().ulm_token_targets(ids.data_ptr(), labels.data_ptr(), n, L, padded, int(ignore_index), out[0].data_ptr(),
+                                      out[1].data_ptr(), _stream(ids)), 'token_targets')
+    return out[0], out[1]
+
+
+def grad_clip_(flat_grad, sumsq, max_norm):
+    """clip_grad_norm_ on the flat gradients, given their squared norm on the device: scales them by
+    min(1, max_norm / (norm + 1e-6)) and returns the norm; no pass over memory when nothing is to be clipped."""
+    norm = torch.empty((), dtype=torch.float32, device=flat_grad.device)
+    N.check(N.lib().ulm_grad_clip(flat_grad.data_ptr(), flat_grad.numel(), sumsq.data_ptr(), float(max_norm), norm.data_ptr(),
+                                  _stream(flat_grad)), 'grad_clip')
+    return norm
+
+
 _SUMSQ_SCRATCH = {}     # device index -> fp32 scratch for the per-CTA partial sums
 
 
