@@ -109,9 +109,14 @@ __device__ __forceinline__ void load_w(const TW* w, int i, float (&out)[N]) {
   }
 }
 
-// Rows a warp works on at a time (measured on B200 at 32768 x 768: two rows and three CTAs per SM reach the
-// speed of a plain copy; four rows or more CTAs are slower).
-__host__ __device__ constexpr int rows_per_iter(int nv) { return nv <= 6 ? 2 : 1; }
+// Rows a warp works on at a time and CTAs per SM.  Plain norms, measured at 32768 x 768 16-bit: two rows and three CTAs
+// per SM reach the speed of a plain copy; four rows or more CTAs are slower.  The fused add of fp32 rows of 513-768
+// elements (six vectors a lane) holds half as many registers with one row, and four CTAs' rows keep the loads flowing better
+// than three CTAs' pairs: 32768 x 768 55.6 -> 49.5 us (6.1 TB/s), 12288 x 768 24.8 -> 18.9 us; five or six CTAs spill, and
+// wider rows (eight vectors) lose with four.
+__host__ __device__ constexpr bool single_rows(int nv, bool add) { return nv > 6 || (add && nv == 6); }
+__host__ __device__ constexpr int rows_per_iter(int nv, bool add) { return single_rows(nv, add) ? 1 : 2; }
+__host__ __device__ constexpr int fwd_ctas(int nv, bool add) { return add && nv == 6 ? 4 : 3; }
 
 struct FwdParams {
   const void* x; const void* branch; const void* w; void* x_out; void* y; float* rstd;
@@ -121,10 +126,10 @@ struct FwdParams {
 
 // T: dtype of x (and x_out); TY: dtype of y (and of branch); NV: vectors of N = 16/sizeof(T) elements per lane.
 template <typename T, typename TW, typename TY, int NV, bool ADD>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, fwd_ctas(NV, ADD))
 rmsnorm_fwd_kernel(const FwdParams p) {
   constexpr int N = Vec<T>::N;
-  constexpr int R = rows_per_iter(NV);
+  constexpr int R = rows_per_iter(NV, ADD);
   const T* __restrict__ x = static_cast<const T*>(p.x);
   const TY* __restrict__ br = static_cast<const TY*>(p.branch);
   const TW* __restrict__ w = static_cast<const TW*>(p.w);
@@ -600,9 +605,10 @@ int pick_nv(int need) {
 template <typename T, typename TW, typename TY, bool ADD>
 void launch_fwd(const FwdParams& p, int nv, cudaStream_t st) {
   auto go = [&](auto kern, int nv_) {
-    const int64_t per_cta = (int64_t)kWarps * rows_per_iter(nv_);
+    const int64_t per_cta = (int64_t)kWarps * rows_per_iter(nv_, ADD);
     int64_t blocks = (p.rows + per_cta - 1) / per_cta;
-    if (blocks > 8 * kNumSMs) blocks = 8 * kNumSMs;
+    const int64_t cap = (ADD && nv_ == 6 ? 64 : 8) * kNumSMs;
+    if (blocks > cap) blocks = cap;
     kern<<<(unsigned)blocks, kThreads, 0, st>>>(p);
   };
   switch (nv) {

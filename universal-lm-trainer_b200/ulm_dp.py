@@ -467,10 +467,7 @@ class DataParallelStep:
         """The buffer of the linear layers' 16-bit weights (2 bytes per element, kept between steps and refilled by one
         fused cast at the start of each); None where there is nothing to cast."""
         if self._copies is None:
-            linears = {id(m.weight): m.weight for m in self.model.modules() if isinstance(m, torch.nn.Linear)}
-            ws = [w for w in linears.values() if w.is_cuda and w.dtype == torch.float32 and w.device == self.device]
-            use = ws and self.amp_scope == 'step' and self.dtype in (torch.float16, torch.bfloat16)
-            self._copies = ulm_ops.weight_copies(ws, self.dtype) if use else False
+            self._copies = (self.amp_scope == 'step' and ulm_ops.linear_copies(self.model, self.dtype)) or False
         return self._copies or None
 
     def _forward_backward(self, ids, weight, n_tokens):

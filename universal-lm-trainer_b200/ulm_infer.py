@@ -14,12 +14,14 @@ attention mask, no KV cache, head_dim 64, fp16/bf16 on a B200; anything else (si
 steps with a cache, padded-mask batches, CPU tensors) goes to the module's own forward, which is the
 caller's code, not a path of this library.
 """
+import array
 import types
 
 import numpy as np
 import torch
 
 import _native as N
+import ulm_model
 import ulm_ops
 
 
@@ -84,6 +86,12 @@ def unpatch_attention(model):
             del m._ulm_original_forward
 
 
+def _ids(window):
+    """A window's token ids as an int64 array; a list of Python ints through the array module, which is twice as fast as
+    numpy's element-by-element conversion."""
+    return np.frombuffer(array.array('q', window), dtype=np.int64) if isinstance(window, (list, tuple)) else np.asarray(window, dtype=np.int64)
+
+
 def score_windows(model, windows, pad_id, device, batch_size, chunk_rows, amp_dtype=torch.float16):
     """inf.py:866-937: per-window (loss sum, token count, correct top-1 count), windows sorted by length
     into right-padded batches, ``input = w[:-1]``, ``label = w[1:]``; ``model`` provides
@@ -100,7 +108,9 @@ def score_windows(model, windows, pad_id, device, batch_size, chunk_rows, amp_dt
     order = sorted(range(n), key=lambda i: len(windows[i]))
     scored, loss_parts, hit_parts = [], [], []
     on_gpu = torch.device(device).type == 'cuda'
-    with torch.no_grad(), ulm_ops.weight_cast_scope(), torch.autocast('cuda', dtype=amp_dtype):
+    # the package's own model takes its 16-bit weights from one fused cast; others cast through autocast
+    copies = ulm_ops.linear_copies(model, amp_dtype) if isinstance(model, ulm_model.DecoderOnlyTransformer) else None
+    with torch.no_grad(), ulm_ops.weight_cast_scope(copies), torch.autocast('cuda', dtype=amp_dtype):
         w16 = None
         for start in range(0, n, batch_size):
             idxs = [i for i in order[start:start + batch_size] if tokens[i] > 0]
@@ -112,7 +122,7 @@ def score_windows(model, windows, pad_id, device, batch_size, chunk_rows, amp_dt
             v = host.numpy()
             at = g * t
             for j, i in enumerate(idxs):
-                ids, k = np.asarray(windows[i], dtype=np.int64), tokens[i]
+                ids, k = _ids(windows[i]), tokens[i]
                 v[j * t:j * t + k] = ids[:-1]
                 v[at:at + k] = ids[1:]
                 v[at + m:at + m + k] = np.arange(j * t, j * t + k)

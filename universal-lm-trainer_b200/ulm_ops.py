@@ -109,6 +109,13 @@ def weight_copies(weights, dtype):
     return N.ext().WeightCopies(list(weights), dtype)
 
 
+def linear_copies(model, dtype):
+    """`weight_copies` of the fp32 CUDA weights of ``model``'s linear layers (each once); None if there are none."""
+    ws = {id(m.weight): m.weight for m in model.modules() if isinstance(m, nn.Linear)}
+    ws = [w for w in ws.values() if w.is_cuda and w.dtype == torch.float32]
+    return weight_copies(ws, dtype) if ws and dtype in _16BIT else None
+
+
 def gated_linear(x, w1, w3):
     """``swiglu(linear(x, w1), linear(x, w3))`` (train.py:1975) as one op: both projections write the halves of one
     [rows, 2 d_ff] matrix, which the gate's kernels read and differentiate in place of two."""
