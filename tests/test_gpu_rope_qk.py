@@ -31,3 +31,18 @@ def test_same_bits_as_rope_then_attention(S, dtype):
     o, k_out, _ = ulm_infer.causal_attention(qkv.detach(), H, cos, sin)
     assert torch.equal(o, want) and torch.equal(k_out, kr)
     fa.check_status()
+
+
+@pytest.mark.parametrize('n,S', [(1, 130), (5, 4097), (6, 3600)])
+def test_prefill_same_bits_on_both_sides_of_its_size_rule(n, S):
+    """Q rotated by the stand-alone launch (up to 20 M elements) or inside the kernel (beyond): the same bits."""
+    H = 16
+    qkv = torch.randn(n, S, 3 * H * 64, generator=torch.Generator(device='cuda').manual_seed(S), device='cuda').half()
+    cos, sin = _tables(S, H)
+    q, k, v = (t.view(n, S, H, 64).transpose(1, 2) for t in qkv.chunk(3, dim=-1))
+    with torch.no_grad():
+        qr, kr = fa.rope(q, k, cos, sin)
+        want = fa.flash_attn_v100(qr, kr, v, causal=True).transpose(1, 2).reshape(n, S, H * 64)
+    o, k_out, _ = ulm_infer.causal_attention(qkv, H, cos, sin)
+    assert torch.equal(o, want) and torch.equal(k_out, kr)
+    fa.check_status()
