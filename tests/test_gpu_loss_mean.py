@@ -28,3 +28,14 @@ def test_loss_mean_matches_float64(rows, form):
     want = float(losses.double().sum()) / n
     assert abs(float(out[0]) - want) <= 2e-6 * max(want, 1e-30) + 1e-12
     assert abs(float(out[1]) * n - 1.0) <= 2e-7
+
+
+@pytest.mark.parametrize('rows', [1025, 32768, 40001, 300007])
+def test_loss_mean_is_rounded_once(rows):
+    losses = torch.rand(rows, generator=torch.Generator().manual_seed(rows)) * 12
+    lc, tc, out = losses.cuda(), torch.ones(rows, dtype=torch.long).cuda(), torch.empty(2, device='cuda')
+    N.check(N.lib().ulm_loss_mean(lc.data_ptr(), tc.data_ptr(), rows, 0, None, 0.0, out[0:].data_ptr(), out[1:].data_ptr(),
+                                  C.c_void_p(torch.cuda.current_stream().cuda_stream)), 'loss_mean')
+    # an fp64 sum is exact to 2^-53 * rows: what remains is the one rounding to fp32
+    want = float(losses.double().sum()) / rows
+    assert abs(float(out[0]) - want) <= 2.0 ** -24 * want * (1 + 1e-6)

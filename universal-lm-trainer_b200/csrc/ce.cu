@@ -138,12 +138,13 @@ ce_bwd_kernel(T* __restrict__ logits, const int64_t* __restrict__ target, const 
 // Mean of the row losses in one CTA and a fixed order: loss = sum / denominator, inv = 1 / denominator; the
 // denominator is *denom_dev, denom when that is positive, or the number of targets != ignore_index (at least 1).
 // One launch for what took a compare, two reductions, a clamp, a cast and a division; 12 bytes per row, so one CTA's
-// latency (about 5 us at 32768 rows) is all it costs.
+// latency (about 5 us at 32768 rows) is all it costs.  Each thread adds up a strided chain of rows, so the sum runs in
+// fp64 and is rounded once: in fp32 the chain's error reached the loss (one ulp more than a pairwise sum's).
 constexpr int kMeanThreads = 1024;
 __global__ void __launch_bounds__(kMeanThreads)
 loss_mean_kernel(const float* __restrict__ rows_loss, const int64_t* __restrict__ target, int64_t rows, int64_t ignore_index,
                  const float* __restrict__ denom_dev, float denom, float* __restrict__ loss, float* __restrict__ inv) {
-  float s = 0.f;
+  double s = 0.;
   int n = 0;
   const bool count = !denom_dev && !(denom > 0.f);
 #pragma unroll 4
@@ -153,7 +154,7 @@ loss_mean_kernel(const float* __restrict__ rows_loss, const int64_t* __restrict_
   }
   s = warp_sum(s);
   n = __reduce_add_sync(0xffffffffu, n);
-  __shared__ float ss[kMeanThreads / 32];
+  __shared__ double ss[kMeanThreads / 32];
   __shared__ int sn[kMeanThreads / 32];
   if ((threadIdx.x & 31) == 0) { ss[threadIdx.x >> 5] = s; sn[threadIdx.x >> 5] = n; }
   __syncthreads();
@@ -162,7 +163,7 @@ loss_mean_kernel(const float* __restrict__ rows_loss, const int64_t* __restrict_
     n = __reduce_add_sync(0xffffffffu, sn[threadIdx.x]);
     if (threadIdx.x == 0) {
       const float d = denom_dev ? *denom_dev : count ? (float)(n > 0 ? n : 1) : denom;
-      *loss = s / d;
+      *loss = (float)(s / d);
       *inv = 1.f / d;
     }
   }
