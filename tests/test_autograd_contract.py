@@ -1,0 +1,59 @@
+"""What the native ops owe autograd: checkpointing, saved-tensor hooks and the other uses a differentiable op has."""
+import pytest
+import torch
+from torch.utils.checkpoint import checkpoint
+
+import ulm_ops
+
+
+def _weights(dtype=torch.float32, device='cpu', n=2, d=16):
+    g = torch.Generator().manual_seed(3)
+    return [torch.nn.Parameter((torch.randn(d, d, generator=g) * d ** -0.5).to(dtype).to(device)) for _ in range(n)]
+
+
+BLOCKS = {
+    'relu': lambda x, w: ulm_ops.linear(ulm_ops.linear(x, w[0]).relu(), w[1]),
+    'silu gate': lambda x, w: ulm_ops.linear(torch.nn.functional.silu(ulm_ops.linear(x, w[0])) * x, w[1]),
+    'dropout': lambda x, w: ulm_ops.linear(torch.nn.functional.dropout(ulm_ops.linear(x, w[0]), 0.5), w[1]),
+    'view': lambda x, w: ulm_ops.linear(ulm_ops.linear(x, w[0]).view(2, -1, 16), w[1]),
+}
+
+
+@pytest.mark.parametrize('frozen', [False, True])
+@pytest.mark.parametrize('block', list(BLOCKS))
+def test_checkpoint_recomputes_the_same_graph(block, frozen):
+    w = _weights()
+    w[1].requires_grad_(not frozen)
+    x = torch.randn(6, 16, generator=torch.Generator().manual_seed(4))
+    wrt = [p for p in w if p.requires_grad]
+
+    def run(call):
+        torch.manual_seed(7)
+        t = x.clone().requires_grad_()
+        return torch.autograd.grad(call(t).square().sum(), [t, *wrt])
+
+    plain = run(lambda t: BLOCKS[block](t, w))
+    for a, b in zip(run(lambda t: checkpoint(BLOCKS[block], t, w, use_reentrant=False)), plain):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+def test_checkpoint_with_library_ops_between():
+    w = _weights(device='cuda')
+    n1 = torch.nn.Parameter(torch.ones(16, device='cuda'))
+
+    def block(x):
+        h = ulm_ops.rms_norm(x, n1)
+        return x + ulm_ops.linear(torch.tanh(ulm_ops.gated_linear(h, w[0], w[1])), w[0])
+
+    x = torch.randn(32, 16, device='cuda')
+
+    def run(call):
+        t = x.clone().requires_grad_()
+        with torch.autocast('cuda', dtype=torch.bfloat16):
+            y = call(t)
+        return torch.autograd.grad(y.float().square().sum(), [t, n1, *w])
+
+    plain = run(block)
+    for a, b in zip(run(lambda t: checkpoint(block, t, use_reentrant=False)), plain):
+        assert torch.equal(a, b)

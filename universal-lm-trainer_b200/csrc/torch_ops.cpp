@@ -18,6 +18,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <algorithm>
 #include <atomic>
 #include <memory>
 #include <mutex>
@@ -64,13 +65,34 @@ bool no_graph(const Ts&... ts) {
   return !at::GradMode::is_enabled() || !(ts.requires_grad() || ...);
 }
 
+// What surrounds every op's own work: no recording below it and no autocast of the tensors it has already cast.
+struct OpScope {
+  at::NoGradGuard no_grad;
+  at::AutoDispatchBelowADInplaceOrView below;
+  c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
+};
+
 // Base of the ops' backward nodes: the tensors they keep, unpacked through autograd's own saved variables (version
-// checks, saved-tensor hooks, release after the backward).
+// checks, saved-tensor hooks, release after the backward).  All are unpacked BEFORE the op's scope opens: a hook may run
+// a checkpointed forward again, which has to record its graph and to autocast as it did the first time.
 struct OpNode : torch::autograd::Node {
   std::vector<torch::autograd::SavedVariable> saved;
   void keep(const Tensor& t, bool is_output = false) { saved.emplace_back(t, is_output); }
-  Tensor kept(size_t i) { return saved[i].unpack(getptr()); }
+  // the gradients of the inputs, from those of the outputs (at least one is defined) and the tensors kept
+  virtual variable_list backward(variable_list& g, const variable_list& kept) = 0;
+  variable_list apply(variable_list&& g) final {
+    if (std::none_of(g.begin(), g.end(), [](const Tensor& t) { return t.defined(); })) return variable_list(num_outputs());
+    variable_list kept;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      kept.reserve(saved.size());
+      for (const auto& s : saved) kept.push_back(s.unpack(getptr()));
+    }
+    OpScope scope;
+    return backward(g, kept);
+  }
   void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
     for (auto& s : saved) s.reset_data();
   }
 };
@@ -81,12 +103,6 @@ std::shared_ptr<N> make_node(const Ts&... inputs) {
   n->set_next_edges(torch::autograd::collect_next_edges(inputs...));
   return n;
 }
-// What surrounds every op's own work: no recording below it and no autocast of the tensors it has already cast.
-struct OpScope {
-  at::NoGradGuard no_grad;
-  at::AutoDispatchBelowADInplaceOrView below;
-  c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
-};
 
 // ---------------------------------------------------------------------------
 // status word: one int32 per device that the kernels OR their timeout bits into
@@ -237,14 +253,12 @@ std::array<Tensor, 3> empty_grads(const Tensor& q) {
 
 struct RopeBwd : OpNode {
   std::vector<int64_t> n, qs, ks;                          // shape and input strides
-  variable_list apply(variable_list&& g) override {
-    OpScope scope;
+  variable_list backward(variable_list& g, const variable_list& kept) override {
     const bool has_q = g[0].defined(), has_k = g[1].defined();
-    if (!has_q && !has_k) return {Tensor(), Tensor()};
     auto ready = [](const Tensor& t) {
       return t.stride(3) == 1 && !(reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0 && t.stride(2) % 8 == 0;
     };
-    const Tensor cos = kept(0), sin = kept(1);
+    const Tensor cos = kept[0], sin = kept[1];
     Tensor in[2], out[2];
     for (int i = 0; i < 2; ++i)
       if (g[i].defined()) {
@@ -283,12 +297,10 @@ std::tuple<Tensor, Tensor> rope(const Tensor& q, const Tensor& k, const Tensor& 
 
 struct FlashBwd : OpNode {
   AttnArgs p{};
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor(), Tensor(), Tensor()};
-    OpScope scope;
-    const Tensor q = kept(0);
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor q = kept[0];
     auto d = empty_grads(q);
-    attn_backward(q, kept(1), kept(2), kept(3), kept(4), g[0], d[0], d[1], d[2], p);
+    attn_backward(q, kept[1], kept[2], kept[3], kept[4], g[0], d[0], d[1], d[2], p);
     return {d[0], d[1], d[2]};
   }
 };
@@ -352,12 +364,10 @@ void rope_attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const
 struct RopeFlashBwd : OpNode {
   AttnArgs p{};
   int64_t fuse = 0;
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor(), Tensor(), Tensor()};
-    OpScope scope;
-    const Tensor q = kept(0);
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor q = kept[0];
     auto d = empty_grads(q);
-    rope_attn_backward(q, kept(1), kept(2), kept(3), kept(4), g[0], kept(5), kept(6), d[0], d[1], d[2], p, fuse);
+    rope_attn_backward(q, kept[1], kept[2], kept[3], kept[4], g[0], kept[5], kept[6], d[0], d[1], d[2], p, fuse);
     return {d[0], d[1], d[2]};
   }
 };
@@ -396,15 +406,13 @@ Tensor heads_of(const Tensor& x, int64_t B, int64_t S, int64_t H) {
 struct QkvBwd : OpNode {
   AttnArgs p{};
   int64_t fuse = 0, B = 0, S = 0, H = 0, rows = -1;        // rows >= 0: the flattened form with padding rows
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor()};
-    OpScope scope;
-    const Tensor qkv = kept(0), cos = kept(5), sin = kept(6);
-    const Tensor q = cos.defined() ? kept(1) : qkv_part(qkv, 0, B, S, H), k = cos.defined() ? kept(2) : qkv_part(qkv, 1, B, S, H);
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor qkv = kept[0], cos = kept[5], sin = kept[6];
+    const Tensor q = cos.defined() ? kept[1] : qkv_part(qkv, 0, B, S, H), k = cos.defined() ? kept[2] : qkv_part(qkv, 1, B, S, H);
     const Tensor go = heads_of(g[0].contiguous(), B, S, H);
     const Tensor d = empty_cuda(qkv.sizes(), qkv.scalar_type(), qkv);
     if (rows > B * S) d.narrow(0, B * S, rows - B * S).zero_();
-    rope_attn_backward(q, k, qkv_part(qkv, 2, B, S, H), heads_of(kept(3), B, S, H), kept(4), go, cos, sin,
+    rope_attn_backward(q, k, qkv_part(qkv, 2, B, S, H), heads_of(kept[3], B, S, H), kept[4], go, cos, sin,
                        qkv_part(d, 0, B, S, H), qkv_part(d, 1, B, S, H), qkv_part(d, 2, B, S, H), p, fuse);
     return {d};
   }
@@ -520,10 +528,8 @@ struct NormBwd : OpNode {
   double eps = 0;
   std::vector<int64_t> shape;
   at::ScalarType wdtype, ydtype;
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor(), Tensor()};
-    OpScope scope;
-    const Tensor x = kept(0), w = kept(1), rstd = kept(2);
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor x = kept[0], w = kept[1], rstd = kept[2];
     const Tensor dy = rows_of(g[0].to(ydtype)), dx = empty_cuda({x.size(0), x.size(1)}, x.scalar_type(), x);
     const Tensor dw = norm_backward(x, w, rstd, dy, eps, y_kind(ydtype, x.scalar_type()), dx, Tensor(), Tensor());
     return {dx.view(shape), dw.to(wdtype)};
@@ -567,11 +573,9 @@ struct AddNormBwd : OpNode {
   double eps = 0;
   std::vector<int64_t> shape;
   at::ScalarType wdtype, bdtype;
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined() && !g[1].defined()) return {Tensor(), Tensor(), Tensor()};
-    OpScope scope;
+  variable_list backward(variable_list& g, const variable_list& kept) override {
     if (!g[1].defined()) return {g[0], g[0].to(bdtype), Tensor()};          // the normalised output went unused
-    const Tensor x = kept(0), w = kept(1), rstd = kept(2);
+    const Tensor x = kept[0], w = kept[1], rstd = kept[2];
     const int64_t rows = x.size(0), d = x.size(1);
     const Tensor dy = rows_of(g[1].to(bdtype)), ga = g[0].defined() ? rows_of(g[0].to(at::kFloat)) : Tensor();
     const Tensor dx = empty_cuda({rows, d}, at::kFloat, x), db = empty_cuda({rows, d}, bdtype, x);
@@ -612,10 +616,8 @@ std::tuple<Tensor, Tensor> add_rms_norm(const Tensor& x, const Tensor& branch, c
 }
 
 struct SwigluBwd : OpNode {
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor(), Tensor()};
-    OpScope scope;
-    const Tensor a = kept(0), b = kept(1), dy = g[0].to(a.scalar_type()).contiguous();
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor a = kept[0], b = kept[1], dy = g[0].to(a.scalar_type()).contiguous();
     const Tensor da = empty_cuda(a.sizes(), a.scalar_type(), a), db = empty_cuda(a.sizes(), a.scalar_type(), a);
     ulm_swiglu_args p{a.data_ptr(), b.data_ptr(), nullptr, dy.data_ptr(), da.data_ptr(), db.data_ptr(), a.numel(), code_of(a.scalar_type()), 0, stream_of(a)};
     check(ulm_swiglu_bwd(&p), "swiglu backward");
@@ -732,10 +734,8 @@ Tensor weight_grad(const Tensor& weight, const Tensor& dy, const Tensor& x) {
 
 struct LinearBwd : OpNode {
   at::ScalarType cd, x_dtype;
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor(), Tensor()};
-    OpScope scope;
-    const Tensor x = kept(0), weight = kept(1);
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor x = kept[0], weight = kept[1];
     const Tensor dy = g[0].reshape({-1, g[0].size(-1)}).to(cd);
     Tensor dx, dw;
     if (task_should_compute_output(0)) dx = at::mm(dy, cast_cached(weight, cd)).view(x.sizes()).to(x_dtype);
@@ -791,10 +791,8 @@ void swiglu_rows(const Tensor& ab, const Tensor& y, const Tensor& dy, const Tens
 
 struct GatedBwd : OpNode {
   at::ScalarType cd, x_dtype;
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor(), Tensor(), Tensor()};
-    OpScope scope;
-    const Tensor x = kept(0), w1 = kept(1), w3 = kept(2), ab = kept(3);
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor x = kept[0], w1 = kept[1], w3 = kept[2], ab = kept[3];
     const Tensor dy = g[0].reshape({-1, g[0].size(-1)}).to(cd).contiguous(), x2 = x.reshape({-1, x.size(-1)});
     const Tensor dab = empty_cuda(ab.sizes(), cd, ab);
     swiglu_rows(ab, Tensor(), dy, dab, true);
@@ -913,10 +911,8 @@ struct KeptCeBwd : OpNode {
   int64_t ignore_index = 0;
   at::ScalarType cd;
   std::atomic<bool> consumed{false};
-  variable_list apply(variable_list&& g) override {
-    if (!g[0].defined()) return {Tensor(), Tensor()};
-    OpScope scope;
-    const Tensor hidden = kept(0), weight = kept(1), target = kept(2), lse = kept(3), logits = kept(4), inv = kept(5), wc = kept(6), hc = kept(7);
+  variable_list backward(variable_list& g, const variable_list& kept) override {
+    const Tensor hidden = kept[0], weight = kept[1], target = kept[2], lse = kept[3], logits = kept[4], inv = kept[5], wc = kept[6], hc = kept[7];
     TORCH_CHECK(!consumed.exchange(true),
                 "chunked_cross_entropy: the kept logits were turned into their gradient in place by the first backward; a second "
                 "backward through the same graph is not supported");
