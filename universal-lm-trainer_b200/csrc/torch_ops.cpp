@@ -907,6 +907,27 @@ std::tuple<Tensor, Tensor> lm_head_score(const Tensor& h, const Tensor& w, const
   return {loss, hit};
 }
 
+// The kernel's form of ulm_ops.token_targets; empty where the tensors are not what it reads (device, type, shape)
+std::optional<std::tuple<Tensor, Tensor>> token_targets(const Tensor& ids, const Tensor& labels, int64_t padded, int64_t ignore_index) {
+  if (!ids.is_cuda() || labels.device() != ids.device() || ids.scalar_type() != at::kLong || labels.scalar_type() != at::kLong || ids.dim() != 2 ||
+      labels.sizes() != ids.sizes() || !ids.is_contiguous() || !labels.is_contiguous())
+    return std::nullopt;
+  const int64_t n = ids.size(0), L = ids.size(1);
+  TORCH_CHECK_VALUE(padded >= n * L, "token_targets: ", padded, " rows do not hold ", n, " x ", L, " tokens");
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(ids.device());
+  const Tensor out = empty_cuda({2, padded}, at::kLong, ids), flat = out.select(0, 0), target = out.select(0, 1);
+  check(ulm_token_targets(ids.data_ptr<int64_t>(), labels.data_ptr<int64_t>(), n, L, padded, ignore_index, flat.data_ptr<int64_t>(),
+                          target.data_ptr<int64_t>(), stream_of(ids)), "token_targets");
+  return std::make_tuple(flat, target);
+}
+
+// One int64 target per row of `hidden`, where the cross-entropy kernels can read it
+void check_target(const Tensor& hidden, const Tensor& target) {
+  TORCH_CHECK_VALUE(target.scalar_type() == at::kLong && target.device() == hidden.device() && target.numel() >= hidden.size(0),
+                    "chunked_cross_entropy takes one int64 target per row, on the device of hidden");
+}
+
 struct KeptCeBwd : OpNode {
   int64_t ignore_index = 0;
   at::ScalarType cd;
@@ -932,6 +953,7 @@ struct KeptCeBwd : OpNode {
 
 Tensor kept_cross_entropy(const Tensor& hidden, const Tensor& weight, const Tensor& target, int64_t ignore_index, at::ScalarType cd,
                           const OptTensor& denom_dev, double denom, bool fused) {
+  check_target(hidden, target);
   Tensor loss, lse, rows_loss, logits, inv, wc, hc;
   {
     OpScope scope;
@@ -998,5 +1020,7 @@ PYBIND11_MODULE(_ulm_torch, m) {
   m.def("gated_linear", &gated_linear, no_gil());
   m.def("lm_head_lse", &lm_head_lse, no_gil());
   m.def("lm_head_score", &lm_head_score, no_gil());
+  m.def("token_targets", &token_targets, no_gil());
+  m.def("check_target", &check_target);
   m.def("kept_cross_entropy", &kept_cross_entropy, no_gil());
 }

@@ -249,17 +249,26 @@ def chunked_cross_entropy(hidden, weight, target, ignore_index=0, chunk_rows=204
     if hidden.shape[0] * weight.shape[0] * 2 <= KEEP_LOGITS_BYTES:
         dev, host = (denominator, 0.0) if torch.is_tensor(denominator) else (None, float(denominator or 0.0))
         return N.ext().kept_cross_entropy(hidden, weight, target, int(ignore_index), compute_dtype, dev, host, FUSED_LM_HEAD)
+    N.ext().check_target(hidden, target)
     return _ChunkedCE.apply(hidden, weight, target, int(ignore_index), int(chunk_rows), compute_dtype, denominator)
 
 
 def token_targets(ids, labels, padded, ignore_index):
-    """The [n, L] int64 ``ids`` as ``padded`` flat rows (0 past the end) and the label each row predicts: the next token of
+    """The [n, L] ``ids`` as ``padded`` flat rows (0 past the end) and the label each row predicts: the next token of
     its sequence, ``ignore_index`` at a sequence's last position and on the padding rows."""
+    out = N.ext().token_targets(ids, labels, padded, int(ignore_index))
+    if out is not None:
+        return out
+    # other integer types, other devices, labels that broadcast: plain torch, whose errors come before any launch
+    if labels.is_floating_point():
+        raise ValueError('token_targets takes integer labels')
     n, L = ids.shape
-    out = torch.empty((2, padded), dtype=torch.long, device=ids.device)
-    N.check(N.lib().ulm_token_targets(ids.data_ptr(), labels.data_ptr(), n, L, padded, int(ignore_index), out[0].data_ptr(),
-                                      out[1].data_ptr(), _stream(ids)), 'token_targets')
-    return out[0], out[1]
+    flat = ids.reshape(-1)
+    if padded > n * L:
+        flat = torch.cat([flat, flat.new_zeros(padded - n * L)])
+    target = labels.new_full((padded,), ignore_index, dtype=torch.long)
+    target[:n * L].view(n, L)[:, :-1] = labels[:, 1:]
+    return flat, target
 
 
 def grad_clip_(flat_grad, sumsq, max_norm):
