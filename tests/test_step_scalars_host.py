@@ -44,3 +44,10 @@ def test_cross_entropy_refuses_targets_its_kernels_cannot_read(target, kept, mon
     monkeypatch.setattr(ulm_ops, 'KEEP_LOGITS_BYTES', ulm_ops.KEEP_LOGITS_BYTES if kept else 0)
     with pytest.raises(ValueError):
         ulm_ops.chunked_cross_entropy(torch.zeros(4, 64, dtype=torch.bfloat16), torch.zeros(64, 64), target, denominator=1.0)
+
+
+@pytest.mark.parametrize('flat,sumsq', [(torch.zeros(8), torch.zeros(1)), (torch.zeros(8, device='meta'), torch.zeros(1, device='meta')),
+                                        (torch.zeros(8, dtype=torch.float16), torch.zeros(1))])
+def test_grad_clip_refuses_what_its_kernel_cannot_read(flat, sumsq):
+    with pytest.raises(ValueError):
+        ulm_ops.grad_clip_(flat, sumsq, 1.0)

@@ -922,6 +922,16 @@ std::optional<std::tuple<Tensor, Tensor>> token_targets(const Tensor& ids, const
   return std::make_tuple(flat, target);
 }
 
+Tensor grad_clip(const Tensor& flat, const Tensor& sumsq, double max_norm) {
+  auto ok = [&](const Tensor& t) { return t.is_cuda() && t.device() == flat.device() && t.scalar_type() == at::kFloat && t.is_contiguous(); };
+  TORCH_CHECK_VALUE(ok(flat) && ok(sumsq) && sumsq.numel() >= 1, "grad_clip_ takes contiguous fp32 gradients and their squared norm on one CUDA device");
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(flat.device());
+  const Tensor norm = empty_cuda({}, at::kFloat, flat);
+  check(ulm_grad_clip(flat.data_ptr<float>(), flat.numel(), sumsq.data_ptr<float>(), (float)max_norm, norm.data_ptr<float>(), stream_of(flat)), "grad_clip");
+  return norm;
+}
+
 // One int64 target per row of `hidden`, where the cross-entropy kernels can read it
 void check_target(const Tensor& hidden, const Tensor& target) {
   TORCH_CHECK_VALUE(target.scalar_type() == at::kLong && target.device() == hidden.device() && target.numel() >= hidden.size(0),
@@ -1021,6 +1031,7 @@ PYBIND11_MODULE(_ulm_torch, m) {
   m.def("lm_head_lse", &lm_head_lse, no_gil());
   m.def("lm_head_score", &lm_head_score, no_gil());
   m.def("token_targets", &token_targets, no_gil());
+  m.def("grad_clip", &grad_clip, no_gil());
   m.def("check_target", &check_target);
   m.def("kept_cross_entropy", &kept_cross_entropy, no_gil());
 }

@@ -274,10 +274,7 @@ def token_targets(ids, labels, padded, ignore_index):
 def grad_clip_(flat_grad, sumsq, max_norm):
     """clip_grad_norm_ on the flat gradients, given their squared norm on the device: scales them by
     min(1, max_norm / (norm + 1e-6)) and returns the norm; no pass over memory when nothing is to be clipped."""
-    norm = torch.empty((), dtype=torch.float32, device=flat_grad.device)
-    N.check(N.lib().ulm_grad_clip(flat_grad.data_ptr(), flat_grad.numel(), sumsq.data_ptr(), float(max_norm), norm.data_ptr(),
-                                  _stream(flat_grad)), 'grad_clip')
-    return norm
+    return N.ext().grad_clip(flat_grad, sumsq, float(max_norm))
 
 
 _SUMSQ_SCRATCH = {}     # device index -> fp32 scratch for the per-CTA partial sums
