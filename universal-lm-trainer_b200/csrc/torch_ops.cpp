@@ -458,6 +458,7 @@ Tensor qkv_attn(const Tensor& qkv, int64_t H, const OptTensor& cos_o, const OptT
 // 356 us stand-alone, 336 inside).
 constexpr int64_t kRopeAloneElems = 20 << 20;
 std::tuple<Tensor, Tensor, Tensor> causal_attention(const Tensor& qkv_in, int64_t H, const OptTensor& cos_o, const OptTensor& sin_o, double scale) {
+  TORCH_CHECK_VALUE(cos_o.has_value() == sin_o.has_value(), "cos and sin must be given together");
   OpScope scope;
   const Tensor qkv = qkv_in.detach();
   TORCH_CHECK_VALUE(qkv.is_cuda() && is_16bit(qkv.scalar_type()) && qkv.dim() == 3 && qkv.is_contiguous() && qkv.size(2) == 3 * H * 64,
