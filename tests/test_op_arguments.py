@@ -9,3 +9,21 @@ import ulm_infer
 def test_causal_attention_wants_both_tables_or_none(half):
     with pytest.raises(ValueError, match='given together'):
         ulm_infer.causal_attention(torch.zeros(1, 4, 192, dtype=torch.float16), 1, **{half: torch.zeros(4, 64)})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('L', [67, 300])
+@pytest.mark.parametrize('rope', [True, False])
+@pytest.mark.parametrize('form', ['columns of a wider tensor', 'every other row', 'one sequence of a batch'])
+def test_causal_attention_reads_strided_projections_in_place(form, L, rope):
+    H, w = 2, 3 * 2 * 64
+    g = torch.Generator(device='cuda').manual_seed(L)
+    cos, sin = (torch.randn(L, 128, generator=g, device='cuda') for _ in range(2)) if rope else (None, None)
+    if form == 'columns of a wider tensor':
+        qkv = torch.randn(3, L, w + 64, generator=g, device='cuda').half()[..., :w]
+    elif form == 'every other row':
+        qkv = torch.randn(3, 2 * L, w, generator=g, device='cuda').half()[:, ::2]
+    else:
+        qkv = torch.randn(L, 3, w, generator=g, device='cuda').half().transpose(0, 1)[1:2]
+    for a, b in zip(ulm_infer.causal_attention(qkv, H, cos, sin), ulm_infer.causal_attention(qkv.contiguous(), H, cos, sin)):
+        assert torch.equal(a, b)

@@ -461,12 +461,17 @@ std::tuple<Tensor, Tensor, Tensor> causal_attention(const Tensor& qkv_in, int64_
   TORCH_CHECK_VALUE(cos_o.has_value() == sin_o.has_value(), "cos and sin must be given together");
   OpScope scope;
   const Tensor qkv = qkv_in.detach();
-  TORCH_CHECK_VALUE(qkv.is_cuda() && is_16bit(qkv.scalar_type()) && qkv.dim() == 3 && qkv.is_contiguous() && qkv.size(2) == 3 * H * 64,
-                    "causal_attention needs a contiguous CUDA fp16/bf16 [n, L, 3*n_heads*64] tensor");
+  TORCH_CHECK_VALUE(qkv.is_cuda() && is_16bit(qkv.scalar_type()) && qkv.dim() == 3 && qkv.size(2) == 3 * H * 64 && (qkv.is_contiguous() || qkv.stride(2) == 1),
+                    "causal_attention needs a CUDA fp16/bf16 [n, L, 3*n_heads*64] tensor with contiguous rows");
   c10::cuda::CUDAGuard dev(qkv.device());
   const int64_t B = qkv.size(0), S = qkv.size(1);
-  const Tensor q = qkv_part(qkv, 0, B, S, H), v = qkv_part(qkv, 2, B, S, H), out = empty_cuda({B, S, H * 64}, qkv.scalar_type(), qkv);
-  Tensor k = qkv_part(qkv, 1, B, S, H), cos, sin;
+  // rows that lie further apart (a slice of a wider tensor) are read in place
+  auto part = [&](int i) {
+    return qkv.is_contiguous() ? qkv_part(qkv, i, B, S, H)
+                               : qkv.as_strided({B, H, S, 64}, {qkv.stride(0), 64, qkv.stride(1), 1}, qkv.storage_offset() + i * H * 64);
+  };
+  const Tensor q = part(0), v = part(2), out = empty_cuda({B, S, H * 64}, qkv.scalar_type(), qkv);
+  Tensor k = part(1), cos, sin;
   const Tensor lse = empty_lse(q);
   const AttnArgs p{0.0, true, scale, 0};
   if (cos_o) {

@@ -26,7 +26,7 @@ import ulm_ops
 
 
 def causal_attention(qkv, n_heads, cos=None, sin=None, softmax_scale=None):
-    """qkv [n, L, 3*n_heads*64] 16-bit contiguous -> (attention output [n, L, n_heads*64], k, v) with k
+    """qkv [n, L, 3*n_heads*64] 16-bit, rows contiguous -> (attention output [n, L, n_heads*64], k, v) with k
     rotated, both as (n, n_heads, L, 64) views.  ``cos``/``sin``: the model's [1, L, >=64] or [L, >=64]
     fp32 RoPE tables (None: no rotation).  No autograd graph is built and nothing is saved."""
     return N.ext().causal_attention(qkv, n_heads, cos, sin, 64 ** -0.5 if softmax_scale is None else float(softmax_scale))
