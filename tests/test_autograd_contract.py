@@ -57,3 +57,10 @@ def test_checkpoint_with_library_ops_between():
     plain = run(block)
     for a, b in zip(run(lambda t: checkpoint(block, t, use_reentrant=False)), plain):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('shape', [(3, 4), (2, 3, 4)])
+def test_linear_has_second_derivatives(shape):
+    g = torch.Generator().manual_seed(5)
+    x, w = (torch.randn(s, generator=g, dtype=torch.double, requires_grad=True) for s in (shape, (5, 4)))
+    assert torch.autograd.gradgradcheck(ulm_ops.linear, (x, w))

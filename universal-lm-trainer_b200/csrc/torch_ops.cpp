@@ -80,6 +80,11 @@ struct OpNode : torch::autograd::Node {
   void keep(const Tensor& t, bool is_output = false) { saved.emplace_back(t, is_output); }
   // the gradients of the inputs, from those of the outputs (at least one is defined) and the tensors kept
   virtual variable_list backward(variable_list& g, const variable_list& kept) = 0;
+  // the same for a backward that is itself recorded (create_graph); the library's kernels have no derivative of their own
+  virtual variable_list backward_recorded(variable_list& g, const variable_list& kept) {
+    OpScope scope;
+    return backward(g, kept);
+  }
   variable_list apply(variable_list&& g) final {
     if (std::none_of(g.begin(), g.end(), [](const Tensor& t) { return t.defined(); })) return variable_list(num_outputs());
     variable_list kept;
@@ -88,6 +93,7 @@ struct OpNode : torch::autograd::Node {
       kept.reserve(saved.size());
       for (const auto& s : saved) kept.push_back(s.unpack(getptr()));
     }
+    if (at::GradMode::is_enabled()) return backward_recorded(g, kept);
     OpScope scope;
     return backward(g, kept);
   }
@@ -746,6 +752,16 @@ struct LinearBwd : OpNode {
     Tensor dx, dw;
     if (task_should_compute_output(0)) dx = at::mm(dy, cast_cached(weight, cd)).view(x.sizes()).to(x_dtype);
     if (task_should_compute_output(1)) dw = weight_grad(weight, dy, x.reshape({-1, x.size(-1)}));
+    return {dx, dw};
+  }
+  // two library GEMMs, which autograd can differentiate
+  variable_list backward_recorded(variable_list& g, const variable_list& kept) override {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast{c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)};
+    const Tensor x = kept[0], weight = kept[1];
+    const Tensor dy = g[0].reshape({-1, g[0].size(-1)}).to(cd);
+    Tensor dx, dw;
+    if (task_should_compute_output(0)) dx = at::mm(dy, cast_cached(weight, cd)).view(x.sizes()).to(x_dtype);
+    if (task_should_compute_output(1)) dw = at::mm(dy.t(), x.reshape({-1, x.size(-1)})).to(weight.scalar_type());
     return {dx, dw};
   }
 };
