@@ -64,3 +64,46 @@ def test_linear_has_second_derivatives(shape):
     g = torch.Generator().manual_seed(5)
     x, w = (torch.randn(s, generator=g, dtype=torch.double, requires_grad=True) for s in (shape, (5, 4)))
     assert torch.autograd.gradgradcheck(ulm_ops.linear, (x, w))
+
+
+def _tangent(x, w):
+    import torch.autograd.forward_ad as fwd
+    with fwd.dual_level():
+        return ulm_ops.linear(fwd.make_dual(x, torch.ones_like(x)), w)
+
+
+@pytest.mark.parametrize('transform', [
+    _tangent,
+    lambda x, w: torch.func.vmap(lambda t: ulm_ops.linear(t, w))(x),
+    lambda x, w: torch.func.grad(lambda t: ulm_ops.linear(t, w).sum())(x),
+    lambda x, w: torch.func.jvp(lambda t: ulm_ops.linear(t, w), (x,), (x,)),
+])
+def test_transforms_without_a_rule_are_refused(transform):
+    with pytest.raises((RuntimeError, NotImplementedError), match='autograd.Function'):
+        transform(torch.ones(3, 2, 16), _weights()[0])
+
+
+class _Traced(torch.nn.Module):
+    def __init__(self, device):
+        super().__init__()
+        self.w1, self.w3 = _weights(device=device)
+        self.scale = torch.nn.Parameter(torch.ones(16, device=device))
+        self.device = device
+
+    def forward(self, x):
+        if self.device == 'cpu':
+            return ulm_ops.linear(x, self.w1).relu()
+        h = ulm_ops.rms_norm(x, self.scale)
+        x, h = ulm_ops.add_rms_norm(x, ulm_ops.gated_linear(h, self.w1, self.w3).half(), self.scale)
+        return x + ulm_ops.swiglu(ulm_ops.linear(h.float(), self.w1), h.float())
+
+
+@pytest.mark.parametrize('device', ['cpu', pytest.param('cuda', marks=pytest.mark.gpu)])
+def test_traced_ops_run_again_on_other_inputs(device):
+    m = _Traced(device)
+    traced = torch.jit.trace(m, torch.randn(8, 16, device=device))
+    x = torch.randn(24, 16, device=device)
+    got, want = traced(x), m(x)
+    assert torch.equal(got, want)
+    for a, b in zip(torch.autograd.grad(got.sum(), m.w1), torch.autograd.grad(want.sum(), m.w1)):
+        assert torch.equal(a, b)

@@ -11,11 +11,13 @@
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/AutogradState.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <algorithm>
@@ -1019,6 +1021,28 @@ Tensor kept_cross_entropy(const Tensor& hidden, const Tensor& weight, const Tens
   return loss;
 }
 
+// ---------------------------------------------------------------------------
+// bindings
+// ---------------------------------------------------------------------------
+template <typename T> bool has_tangent(const T&) { return false; }
+bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+
+// A differentiable op.  A tracer, a functorch level or a forward-mode tangent would not notice a node made in C++: there
+// the call goes through a Python autograd function (ulm_recorded.py), which each of them knows how to record or refuse.
+template <typename R, typename... A>
+void def_op(pybind11::module_& m, const char* name, R (*f)(A...)) {
+  m.def(name, [name, f](A... a) -> pybind11::object {
+    if (torch::jit::tracer::isTracing() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) ||
+        (c10::AutogradState::get_tls_state().get_fw_grad_mode() && (has_tangent(a) || ...)))
+      return pybind11::module_::import("ulm_recorded").attr("Recorded").attr("apply")(name, a...);
+    auto run = [&]() -> R {
+      pybind11::gil_scoped_release nogil;
+      return f(a...);
+    };
+    return pybind11::cast(run());
+  });
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_ulm_torch, m) {
@@ -1028,14 +1052,14 @@ PYBIND11_MODULE(_ulm_torch, m) {
   m.def("fa_ready", &fa_ready);
   m.def("can_use", &can_use);
   m.def("rope_can_use", &rope_can_use);
-  m.def("rope", &rope, no_gil());
-  m.def("flash_attn", &flash_attn, no_gil());
-  m.def("rope_flash_attn", &rope_flash_attn, no_gil());
-  m.def("qkv_attn", &qkv_attn, no_gil());
+  def_op(m, "rope", &::rope);
+  def_op(m, "flash_attn", &::flash_attn);
+  def_op(m, "rope_flash_attn", &::rope_flash_attn);
+  def_op(m, "qkv_attn", &::qkv_attn);
   m.def("causal_attention", &causal_attention, no_gil());
-  m.def("rms_norm", &rms_norm, no_gil());
-  m.def("add_rms_norm", &add_rms_norm, no_gil());
-  m.def("swiglu", &swiglu, no_gil());
+  def_op(m, "rms_norm", &::rms_norm);
+  def_op(m, "add_rms_norm", &::add_rms_norm);
+  def_op(m, "swiglu", &::swiglu);
   m.def("set_wgrad_in_place", [](bool on) { return g_wgrad_in_place.exchange(on); });
   py::class_<WeightCopies, std::shared_ptr<WeightCopies>>(m, "WeightCopies")
       .def(py::init<std::vector<Tensor>, at::ScalarType>())
@@ -1048,12 +1072,12 @@ PYBIND11_MODULE(_ulm_torch, m) {
     Tensor g = weight_grad(w, dy, x);
     return g.defined() ? OptTensor(g) : std::nullopt;
   }, no_gil());
-  m.def("linear", &linear, no_gil());
-  m.def("gated_linear", &gated_linear, no_gil());
+  def_op(m, "linear", &::linear);
+  def_op(m, "gated_linear", &::gated_linear);
   m.def("lm_head_lse", &lm_head_lse, no_gil());
   m.def("lm_head_score", &lm_head_score, no_gil());
   m.def("token_targets", &token_targets, no_gil());
   m.def("grad_clip", &grad_clip, no_gil());
   m.def("check_target", &check_target);
-  m.def("kept_cross_entropy", &kept_cross_entropy, no_gil());
+  def_op(m, "kept_cross_entropy", &::kept_cross_entropy);
 }
