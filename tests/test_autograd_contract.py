@@ -107,3 +107,28 @@ def test_traced_ops_run_again_on_other_inputs(device):
     assert torch.equal(got, want)
     for a, b in zip(torch.autograd.grad(got.sum(), m.w1), torch.autograd.grad(want.sum(), m.w1)):
         assert torch.equal(a, b)
+
+
+class _Cut(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def test_an_input_no_gradient_reaches_has_a_zero_one():
+    x, w = torch.randn(3, 16, requires_grad=True), _weights()[0]
+    _Cut.apply(ulm_ops.linear(x, w)).sum().backward()
+    assert torch.equal(x.grad, torch.zeros(3, 16)) and torch.equal(w.grad, torch.zeros(16, 16))
+
+
+@pytest.mark.gpu
+def test_the_norm_weight_of_an_unused_norm_has_a_zero_gradient():
+    x, w = torch.randn(3, 64, device='cuda', requires_grad=True), torch.ones(64, device='cuda', requires_grad=True)
+    b = torch.randn(3, 64, device='cuda', dtype=torch.float16, requires_grad=True)
+    x_new, _ = ulm_ops.add_rms_norm(x, b, w)
+    dx, db, dw = torch.autograd.grad(x_new.sum(), [x, b, w])
+    assert torch.equal(dx, torch.ones_like(x)) and torch.equal(db, torch.ones_like(b)) and not dw.any() and dw.shape == w.shape

@@ -80,6 +80,12 @@ struct OpScope {
 struct OpNode : torch::autograd::Node {
   std::vector<torch::autograd::SavedVariable> saved;
   void keep(const Tensor& t, bool is_output = false) { saved.emplace_back(t, is_output); }
+  // the zero gradient of input i; undefined where none is asked for
+  Tensor zero_grad(size_t i) {
+    if (!task_should_compute_output(i)) return Tensor();
+    const torch::autograd::Edge& e = next_edge(i);
+    return e.function->input_metadata(e.input_nr).zeros_like();
+  }
   // the gradients of the inputs, from those of the outputs (at least one is defined) and the tensors kept
   virtual variable_list backward(variable_list& g, const variable_list& kept) = 0;
   // the same for a backward that is itself recorded (create_graph); the library's kernels have no derivative of their own
@@ -88,7 +94,12 @@ struct OpNode : torch::autograd::Node {
     return backward(g, kept);
   }
   variable_list apply(variable_list&& g) final {
-    if (std::none_of(g.begin(), g.end(), [](const Tensor& t) { return t.defined(); })) return variable_list(num_outputs());
+    if (std::none_of(g.begin(), g.end(), [](const Tensor& t) { return t.defined(); })) {
+      // an input that no gradient reaches has a zero one, not none: an optimiser treats the two differently
+      variable_list zeros;
+      for (size_t i = 0; i < num_outputs(); ++i) zeros.push_back(zero_grad(i));
+      return zeros;
+    }
     variable_list kept;
     {
       std::lock_guard<std::mutex> lock(mutex_);
@@ -277,7 +288,7 @@ struct RopeBwd : OpNode {
     if (has_k) rope_launch(in[0], in[1], out[0], out[1], cos, sin, true);
     else rope_launch(Tensor(), in[0], Tensor(), out[0], cos, sin, true);
     for (int i = 0; i < 2; ++i)
-      if (!out[i].defined() && task_should_compute_output(i)) out[i] = rope_out_like(n, i ? ks : qs, in[1 - i]).zero_();
+      if (!out[i].defined()) out[i] = zero_grad(i);
     return {out[0], out[1]};
   }
 };
@@ -588,7 +599,7 @@ struct AddNormBwd : OpNode {
   std::vector<int64_t> shape;
   at::ScalarType wdtype, bdtype;
   variable_list backward(variable_list& g, const variable_list& kept) override {
-    if (!g[1].defined()) return {g[0], g[0].to(bdtype), Tensor()};          // the normalised output went unused
+    if (!g[1].defined()) return {g[0], g[0].to(bdtype), zero_grad(2)};      // the normalised output went unused
     const Tensor x = kept[0], w = kept[1], rstd = kept[2];
     const int64_t rows = x.size(0), d = x.size(1);
     const Tensor dy = rows_of(g[1].to(bdtype)), ga = g[0].defined() ? rows_of(g[0].to(at::kFloat)) : Tensor();
