@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+import flash_attn_v100_cuda as fa
 import ulm_infer
 
 
@@ -27,3 +28,24 @@ def test_causal_attention_reads_strided_projections_in_place(form, L, rope):
         qkv = torch.randn(L, 3, w, generator=g, device='cuda').half().transpose(0, 1)[1:2]
     for a, b in zip(ulm_infer.causal_attention(qkv, H, cos, sin), ulm_infer.causal_attention(qkv.contiguous(), H, cos, sin)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize('qkv,kw', [
+    (torch.zeros(0, 5, 7, dtype=torch.float16), {}),                             # an empty tensor of another width
+    (torch.zeros(0, 5, 192), {}),                                                # of a type the op does not take
+    (torch.zeros(8, 192, dtype=torch.float16), dict(flat_shape=(0, -3))),        # negative sizes
+    (torch.zeros(8, 7, dtype=torch.float16), dict(flat_shape=(0, 4))),
+    (torch.zeros(0, 5, 192, dtype=torch.float16), dict(cos2d=torch.zeros(5, 64))),
+])
+def test_qkv_attention_checks_empty_inputs_like_others(qkv, kw):
+    with pytest.raises(ValueError):
+        fa.qkv_rope_flash_attn(qkv, 1, **kw)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('shape,kw', [((0, 5, 384), {}), ((3, 0, 384), {}), ((8, 384), dict(flat_shape=(0, 4)))])
+def test_qkv_attention_of_nothing_is_zero_and_differentiable(shape, kw):
+    qkv = torch.ones(shape, dtype=torch.float16, device='cuda', requires_grad=True)
+    out = fa.qkv_rope_flash_attn(qkv, 2, **kw)
+    assert out.shape == (*shape[:-1], 128) and not out.any()
+    assert not torch.autograd.grad(out.sum(), qkv)[0].any()

@@ -449,6 +449,11 @@ Tensor qkv_attn(const Tensor& qkv, int64_t H, const OptTensor& cos_o, const OptT
   TORCH_CHECK_VALUE(cos.defined() == sin.defined(), "cos2d and sin2d must be given together");
   TORCH_CHECK_VALUE(!cos.defined() || (table_ok(cos, S, qkv) && table_ok(sin, S, qkv)),
                     "RoPE tables must be fp32 (L,64) views on the same device, 16-byte aligned rows");
+  if (B * S == 0) {
+    auto n = qkv.sizes().vec();
+    n.back() = H * 64;
+    return at::zeros(n, qkv.options()) + 0 * qkv.sum();
+  }
   const AttnArgs p{dropout_p, causal, scale, seed};
   Tensor out, lse, qr, kr;
   {

@@ -306,11 +306,11 @@ def qkv_rope_flash_attn(qkv, n_heads, cos2d=None, sin2d=None, dropout_p: float =
     in (n, L, H, 64) order, and the backward kernels write dq, dk, dv straight into the three slices of one gradient
     tensor (autograd would otherwise concatenate them)."""
     n, L = (-1, -1) if flat_shape is None else flat_shape
+    if flat_shape is not None and min(n, L) < 0:
+        raise ValueError('flat_shape=(n, L) takes sizes')
     code = _fuse_code(fuse)
     if softmax_scale is None:
         softmax_scale = 64 ** -0.5
-    if qkv.numel() == 0 or (flat_shape is not None and n * L == 0):
-        return qkv.new_zeros((*qkv.shape[:-1], n_heads * 64)) + 0 * qkv.sum()
     return N.ext().qkv_attn(qkv, n_heads, cos2d, sin2d, dropout_p, bool(causal), softmax_scale, _seed_for(dropout_p), code, n, L)
 
 
