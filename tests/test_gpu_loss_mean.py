@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import _native as N
+import ulm_ops
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +40,20 @@ def test_loss_mean_is_rounded_once(rows):
     # an fp64 sum is exact to 2^-53 * rows: what remains is the one rounding to fp32
     want = float(losses.double().sum()) / rows
     assert abs(float(out[0]) - want) <= 2.0 ** -24 * want * (1 + 1e-6)
+
+
+@pytest.mark.parametrize('kept', [True, False])
+@pytest.mark.parametrize('denominator', [0, -4.0, float('nan'), 7, torch.tensor(5), torch.tensor([5.0]), torch.tensor([[2.0, 4.0]])])
+def test_cross_entropy_divides_by_the_denominator_it_is_given(denominator, kept, monkeypatch):
+    monkeypatch.setattr(ulm_ops, 'KEEP_LOGITS_BYTES', ulm_ops.KEEP_LOGITS_BYTES if kept else 0)
+    g = torch.Generator(device='cuda').manual_seed(1)
+    h, w = (torch.randn(s, 64, generator=g, device='cuda').half().requires_grad_() for s in (40, 128))
+    t = torch.randint(1, 128, (40,), generator=g, device='cuda')
+    total = ulm_ops.chunked_cross_entropy(h, w, t, denominator=1.0)
+    got = ulm_ops.chunked_cross_entropy(h, w, t, denominator=denominator)
+    want = total / (denominator.cuda() if torch.is_tensor(denominator) else denominator)
+    assert got.shape == want.shape and torch.allclose(got, want, rtol=1e-6, equal_nan=True)
+    if got.numel() == 1 and torch.isfinite(got).all():
+        # two 16-bit roundings of values that differ by a factor: a few half ulps of fp16
+        torch.testing.assert_close(torch.autograd.grad(got.sum(), h)[0].float(), (torch.autograd.grad(total, h)[0].float() / float(denominator)),
+                                   rtol=4e-3, atol=1e-6)

@@ -232,7 +232,7 @@ def chunked_cross_entropy(hidden, weight, target, ignore_index=0, chunk_rows=204
                           compute_dtype=None, denominator=None):
     """hidden [rows, d], weight [V, d] (the tied lm head), target int64 [rows]
     -> CE summed over targets != ignore_index and divided by their count
-    (train.py:2069-2082), or by ``denominator`` (a positive number or a tensor) when one is given.
+    (train.py:2069-2082), or by ``denominator`` (a number or a tensor) when one is given.
 
     The reference loops fc_out + F.cross_entropy over row chunks so that no fp32 [rows, V] tensor is ever alive
     (autograd still keeps each chunk's fp32 log-softmax).  Here only 16-bit logits ever exist.  Two forms, same values:
@@ -247,8 +247,16 @@ def chunked_cross_entropy(hidden, weight, target, ignore_index=0, chunk_rows=204
         return torch.zeros((), device=hidden.device, requires_grad=True)
     target = target.contiguous()
     if hidden.shape[0] * weight.shape[0] * 2 <= KEEP_LOGITS_BYTES:
-        dev, host = (denominator, 0.0) if torch.is_tensor(denominator) else (None, float(denominator or 0.0))
-        return N.ext().kept_cross_entropy(hidden, weight, target, int(ignore_index), compute_dtype, dev, host, FUSED_LM_HEAD)
+        dev = denominator.detach() if torch.is_tensor(denominator) else None
+        host, shaped = 0.0, dev is not None and dev.dim() > 0
+        if dev is None and denominator is not None:
+            host = float(denominator)
+            if not host > 0.0:                            # the kernel counts then; a division by this number was asked for
+                dev = torch.full((), host, dtype=torch.float32, device=hidden.device)
+        elif shaped:                                      # one sum, divided as the tensor's shape says
+            dev, host = None, 1.0
+        loss = N.ext().kept_cross_entropy(hidden, weight, target, int(ignore_index), compute_dtype, dev, host, FUSED_LM_HEAD)
+        return loss / denominator.detach().to(device=hidden.device, dtype=torch.float32) if shaped else loss
     N.ext().check_target(hidden, target)
     return _ChunkedCE.apply(hidden, weight, target, int(ignore_index), int(chunk_rows), compute_dtype, denominator)
 
