@@ -4,6 +4,7 @@ import torch
 
 import flash_attn_v100_cuda as fa
 import ulm_infer
+import ulm_model
 
 
 @pytest.mark.parametrize('half', ['cos', 'sin'])
@@ -49,3 +50,19 @@ def test_qkv_attention_of_nothing_is_zero_and_differentiable(shape, kw):
     out = fa.qkv_rope_flash_attn(qkv, 2, **kw)
     assert out.shape == (*shape[:-1], 128) and not out.any()
     assert not torch.autograd.grad(out.sum(), qkv)[0].any()
+
+
+def test_what_stands_in_for_a_dropout_is_called():
+    x, seen = torch.ones(3), []
+    hooked = torch.nn.Dropout(0.0)
+    hooked.register_forward_hook(lambda m, a, y: seen.append(1))
+
+    class Mine(torch.nn.Dropout):
+        def forward(self, t):
+            return t + 1
+
+    assert ulm_model._drop(torch.nn.Identity(), x) is x
+    assert torch.equal(ulm_model._drop(hooked, x), x) and seen == [1]
+    assert torch.equal(ulm_model._drop(Mine(0.0), x), x + 1)
+    assert ulm_model._drop(torch.nn.Dropout(0.0), x) is x and ulm_model._drop(torch.nn.Dropout(0.5).eval(), x) is x
+    assert not torch.equal(ulm_model._drop(torch.nn.Dropout(1.0), x), x)
