@@ -43,3 +43,25 @@ def test_score_gives_ties_to_the_lowest_column():
     t = torch.tensor([130, 131, 500, 899, 0] * 40, device='cuda')
     _, hit = ulm_ops.lm_head_score(h, w, t)
     assert hit.tolist() == [1, 0, 0, 0, 0] * 40
+
+
+@pytest.mark.parametrize('V', [1, 64, 300, 4100])
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16])
+def test_score_ranks_infinities_and_nans_as_argmax_does(V, dtype):
+    inf, nan = float('inf'), float('nan')
+    h = torch.zeros(1, 64, dtype=dtype)
+    h[0, 0] = 1
+    rows = torch.linspace(-1, 1, V).repeat(6, 1)          # finite; all -inf; +inf twice; one NaN; two; nothing but NaN
+    rows[1] = -inf
+    rows[2, [V // 3, V // 2]] = inf
+    rows[3, V - 1] = nan
+    rows[4, [V // 2, V - 1]] = nan
+    rows[5] = nan
+    for row in range(6):
+        w = torch.zeros(V, 64, dtype=dtype)
+        w[:, 0] = rows[row].to(dtype)
+        z = (h.float() @ w.float().t())[0]
+        for target in {int(z.argmax()), 0, V // 2, V - 1}:
+            _, hit = ulm_ops.lm_head_score(h.cuda(), w.cuda(), torch.tensor([target], device='cuda'))
+            assert bool(hit[0]) == (int(z.argmax()) == target), (row, target)
+    fa.check_status()

@@ -112,7 +112,7 @@ struct LmItems {
 };
 
 // TOP1 (scoring): instead of storing the logits the epilogue picks out what a score needs of them, the target's logit
-// (into z_target) and the column of the largest one (part_i, the lowest on ties).
+// (into z_target) and the column of the largest one (part_i, the lowest on ties; ~column of the first NaN if there is one).
 struct LmTop1 {
   const int64_t* target;
   int64_t ignore_index;
@@ -291,7 +291,7 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
             }
           }
           if constexpr (TOP1) {
-            if (mx > best) {                             // strictly: the lowest column keeps a tie
+            if (mx > best && best_i >= 0) {              // strictly: the lowest column keeps a tie
               int at = 0;
 #pragma unroll
               for (int c = 63; c >= 0; --c) at = __uint_as_float(acc[c]) == mx ? c : at;
@@ -306,6 +306,7 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
             }
           }
           // running statistics over the rounded values
+          [[maybe_unused]] bool nan_seen = false;
           const float m_new = fmaxf(m, mx * kLmLog2e);
           if (m_new > -INFINITY) {
             ssum *= ex2(m - m_new);                      // 2^(-inf) = 0 on the first tile
@@ -318,8 +319,20 @@ lmhead_lse_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant
               s2 += ex2(fmaf(__uint_as_float(acc[c + 2]), kLmLog2e, nm));
               s3 += ex2(fmaf(__uint_as_float(acc[c + 3]), kLmLog2e, nm));
             }
-            ssum += (s0 + s1) + (s2 + s3);
+            const float add = (s0 + s1) + (s2 + s3);
+            ssum += add;
             m = m_new;
+            if constexpr (TOP1) nan_seen = add != add;
+          }
+          if constexpr (TOP1) {
+            // a NaN counts as the largest, the first one if there are several (argmax's rule); its column is kept as ~column.
+            // Only sums that are NaN and blocks without a finite maximum can hold one: no cost on ordinary rows.
+            if ((nan_seen || !(m_new > -INFINITY)) && best_i >= 0) {
+              int at = 64;
+#pragma unroll
+              for (int c = 63; c >= 0; --c) at = __uint_as_float(acc[c]) != __uint_as_float(acc[c]) ? c : at;
+              if (at < 64) best_i = ~(col0 + at);
+            }
           }
         }
       }
@@ -353,16 +366,18 @@ lmhead_finish_kernel(const float* __restrict__ part_m, const float* __restrict__
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
   float m = -INFINITY;
-  [[maybe_unused]] int at = V;
+  [[maybe_unused]] int at = V, nan_at = V;
   for (int i = lane; i < n_parts; i += 32) {
     const float mi = part_m[r * n_parts + i];
     if constexpr (TOP1) {
       const int ai = part_i[r * n_parts + i];
-      if (mi > m || (mi == m && ai < at)) at = ai;
+      if (ai < 0) nan_at = min(nan_at, ~ai);
+      else if (mi > m || (mi == m && ai < at)) at = ai;
     }
     m = fmaxf(m, mi);
   }
   if constexpr (TOP1) {
+    nan_at = __reduce_min_sync(0xffffffffu, nan_at);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float mo = __shfl_xor_sync(0xffffffffu, m, o);
@@ -387,7 +402,8 @@ lmhead_finish_kernel(const float* __restrict__ part_m, const float* __restrict__
     const bool none = t == ignore_index || t < 0 || t >= V;
     if constexpr (TOP1) {
       loss[r] = none ? 0.f : l - loss[r];
-      hit[r] = !none && at == (int)t;
+      const int top = nan_at < V ? nan_at : at < V ? at : 0;      // a row of nothing but -inf: its first column
+      hit[r] = !none && top == (int)t;
     } else {
       loss[r] = none ? 0.f : l - Cvt<T>::to_f(logits[r * row_stride + t]);
     }
