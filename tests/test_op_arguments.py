@@ -1,4 +1,5 @@
 """Which arguments the ops take and which they refuse; refusals are decided on the host, before any launch."""
+import numpy as np
 import pytest
 import torch
 
@@ -66,3 +67,42 @@ def test_what_stands_in_for_a_dropout_is_called():
     assert torch.equal(ulm_model._drop(Mine(0.0), x), x + 1)
     assert ulm_model._drop(torch.nn.Dropout(0.0), x) is x and ulm_model._drop(torch.nn.Dropout(0.5).eval(), x) is x
     assert not torch.equal(ulm_model._drop(torch.nn.Dropout(1.0), x), x)
+
+
+@pytest.mark.parametrize('window', [[3, 4, 5], (3, 4, 5), [3.0, 4.0, 5.0], torch.tensor([3, 4, 5]), torch.tensor([3, 4, 5], dtype=torch.int32),
+                                    np.array([3, 4, 5], dtype=np.int32), np.array([3.0, 4.0, 5.0]), [torch.tensor(3), torch.tensor(4), torch.tensor(5)], range(3, 6)])
+def test_windows_of_any_sequence_type(window):
+    ids = ulm_infer._ids(window)
+    assert ids.dtype == np.int64 and ids.tolist() == [3, 4, 5]
+
+
+class _Embeds(torch.nn.Module):
+    def __init__(self, V, d):
+        super().__init__()
+        g = torch.Generator().manual_seed(V)
+        self.embedding, self.fc_out = torch.nn.Embedding(V, d), torch.nn.Linear(d, V, bias=False)
+        for p in self.parameters():
+            p.data = torch.randn(p.shape, generator=g)
+
+    def forward_hidden(self, ids):
+        return self.embedding(ids)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('V,d', [(100, 64), (96, 40)])
+@pytest.mark.parametrize('dtype', [torch.float32, torch.float16])
+@pytest.mark.parametrize('kind', ['lists', 'device tensors'])
+def test_scores_of_a_module_of_any_width_and_type(V, d, dtype, kind):
+    m = _Embeds(V, d).cuda()
+    g = torch.Generator().manual_seed(1)
+    windows = [torch.randint(0, V, (n,), generator=g).tolist() for n in (1, 2, 9, 30)]
+    windows[2][-1] = -100                                 # an ignored label: no loss and no token
+    got = ulm_infer.score_windows(m, windows if kind == 'lists' else [torch.tensor(w).cuda() for w in windows], 0, torch.device('cuda'), 3, 7, amp_dtype=dtype)
+    for i, w in enumerate(windows):
+        x, y = torch.tensor(w[:-1], dtype=torch.long), torch.tensor(w[1:], dtype=torch.long)
+        z = (m.embedding.weight.cpu()[x].to(dtype).float() @ m.fc_out.weight.detach().cpu().to(dtype).float().t()).to(dtype).float()
+        want = torch.nn.functional.cross_entropy(z, y, ignore_index=-100, reduction='sum') if len(y) else torch.zeros(())
+        assert got[1][i] == int((y != -100).sum())
+        # logits up to 30 with one rounding to fp16 each
+        assert abs(got[0][i] - float(want)) <= 2.0 ** -6 * max(1, len(y))
+        assert abs(got[2][i] - int((z.argmax(1) == y).sum())) <= (1 if dtype == torch.float16 else 0)
