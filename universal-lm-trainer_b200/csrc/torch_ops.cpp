@@ -9,6 +9,7 @@
 //
 // Nothing here computes: every kernel is the library's, plus the library GEMMs of the linear layers.
 #include <ATen/ATen.h>
+#include <ATen/ThreadLocalPythonObjects.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/AutogradState.h>
@@ -22,8 +23,10 @@
 
 #include <algorithm>
 #include <atomic>
+#include <functional>
 #include <memory>
 #include <mutex>
+#include <string>
 #include <unordered_map>
 #include <utility>
 #include <vector>
@@ -678,15 +681,58 @@ Tensor swiglu(const Tensor& a_in, const Tensor& b_in) {
 // ---------------------------------------------------------------------------
 // linear layers
 // ---------------------------------------------------------------------------
-std::atomic<bool> g_wgrad_in_place{false};
-
-// Scopes in which the 16-bit copy of a weight is made once and reused (the innermost one counts; an empty stack:
-// nothing is cached).  Keyed by the parameter's implementation object, which a cache entry keeps alive.
+// What `wgrad_in_place` and `weight_cast_scope` switch on belongs to the thread that entered them and to the backward
+// passes it starts there: it travels in the thread-local state that autograd hands to its workers.  Another thread, with
+// another model, sees neither.
+//
+// A cast scope keeps the 16-bit copy of a leaf weight and reuses it, on the stream that made it.  Keyed by the parameter's
+// implementation object, which an entry keeps alive.  A closed scope, which a worker may still hold, gives nothing.
 struct CastScope {
-  std::unordered_map<const c10::TensorImpl*, std::pair<Tensor, Tensor>> made;      // parameter, its copy
+  struct Entry { Tensor param, copy; int64_t stream; };
+  std::mutex mu;
+  bool open = true;
+  std::unordered_map<const c10::TensorImpl*, Entry> made;
 };
-std::mutex g_cast_mu;
-std::vector<std::unique_ptr<CastScope>> g_cast_scopes;
+struct OpContext : c10::SafePyObject {
+  bool wgrad_in_place = false;
+  std::shared_ptr<CastScope> casts;
+  OpContext() : SafePyObject(nullptr, nullptr) {}
+};
+using ContextPtr = std::shared_ptr<c10::SafePyObject>;
+const std::string kContextKey = "ulm_ops";
+ContextPtr context() {
+  using TLS = at::impl::ThreadLocalPythonObjects;
+  return TLS::contains(kContextKey) ? TLS::get(kContextKey) : nullptr;
+}
+const OpContext& context_of(const ContextPtr& c) {
+  static const OpContext none;
+  return c ? static_cast<const OpContext&>(*c) : none;
+}
+bool wgrad_in_place() { return context_of(context()).wgrad_in_place; }
+int64_t stream_id(const Tensor& t) { return t.is_cuda() ? (int64_t)c10::cuda::getCurrentCUDAStream(t.device().index()).id() : 0; }
+
+// The state a context manager found and puts back on leaving; `casts` is the scope it opened, if it did.
+struct ContextToken { ContextPtr before; std::shared_ptr<CastScope> casts; };
+ContextToken enter_context(const std::function<void(OpContext&)>& change) {
+  ContextToken t{context(), nullptr};
+  auto next = std::make_shared<OpContext>();
+  next->wgrad_in_place = context_of(t.before).wgrad_in_place;
+  next->casts = context_of(t.before).casts;
+  change(*next);
+  if (next->casts != context_of(t.before).casts) t.casts = next->casts;
+  at::impl::ThreadLocalPythonObjects::set(kContextKey, next);
+  return t;
+}
+void leave_context(ContextToken& t) {
+  if (t.casts) {
+    decltype(t.casts->made) gone;                        // the tensors are released outside the lock
+    std::lock_guard<std::mutex> lock(t.casts->mu);
+    t.casts->open = false;
+    gone.swap(t.casts->made);
+  }
+  at::impl::ThreadLocalPythonObjects::set(kContextKey, t.before ? t.before : std::make_shared<OpContext>());
+}
+
 // 16-bit copies of a fixed set of fp32 weights in one buffer, in the given order: one fused cast fills them all where a
 // scope would otherwise make each on first use (a launch and about 12 us of host time per weight), and weights that
 // follow one another in the list do so in memory, so that two projections of one input can run as one GEMM.  A training
@@ -712,45 +758,37 @@ struct WeightCopies {
   }
 };
 
-// `copies` (already refreshed) seeds the scope
-void cast_scope_push(const std::shared_ptr<WeightCopies>& copies) {
-  auto scope = std::make_unique<CastScope>();
+// `copies` (already refreshed, on the current stream) seeds the scope
+ContextToken enter_casts(const std::shared_ptr<WeightCopies>& copies) {
+  auto scope = std::make_shared<CastScope>();
   if (copies)
-    for (size_t i = 0; i < copies->params.size(); ++i) scope->made[copies->params[i].unsafeGetTensorImpl()] = {copies->params[i], copies->views[i]};
-  std::lock_guard<std::mutex> lock(g_cast_mu);
-  g_cast_scopes.push_back(std::move(scope));
-}
-void cast_scope_pop() {
-  std::unique_ptr<CastScope> gone;                       // its tensors are released outside the lock
-  std::lock_guard<std::mutex> lock(g_cast_mu);
-  TORCH_CHECK(!g_cast_scopes.empty(), "no weight-cast scope is active");
-  gone = std::move(g_cast_scopes.back());
-  g_cast_scopes.pop_back();
+    for (size_t i = 0; i < copies->params.size(); ++i)
+      scope->made[copies->params[i].unsafeGetTensorImpl()] = {copies->params[i], copies->views[i], stream_id(copies->views[i])};
+  return enter_context([&](OpContext& c) { c.casts = scope; });
 }
 Tensor cast_cached(const Tensor& weight, at::ScalarType dtype) {
   if (weight.scalar_type() == dtype) return weight;
+  const ContextPtr held = context();
+  const std::shared_ptr<CastScope>& scope = context_of(held).casts;
+  if (!scope || !weight.is_leaf()) return weight.detach().to(dtype);
   const c10::TensorImpl* key = weight.unsafeGetTensorImpl();
-  CastScope* scope = nullptr;
+  const int64_t stream = stream_id(weight);
   {
-    std::lock_guard<std::mutex> lock(g_cast_mu);
-    if (!g_cast_scopes.empty()) {
-      scope = g_cast_scopes.back().get();
-      auto it = scope->made.find(key);
-      if (it != scope->made.end() && it->second.second.scalar_type() == dtype && it->second.second.device() == weight.device()) return it->second.second;
-    }
+    std::lock_guard<std::mutex> lock(scope->mu);
+    auto it = scope->made.find(key);
+    if (it != scope->made.end() && it->second.copy.scalar_type() == dtype && it->second.copy.device() == weight.device() && it->second.stream == stream)
+      return it->second.copy;
   }
   const Tensor c = weight.detach().to(dtype);
-  if (scope) {
-    std::lock_guard<std::mutex> lock(g_cast_mu);
-    if (!g_cast_scopes.empty() && g_cast_scopes.back().get() == scope) scope->made[key] = {weight, c};
-  }
+  std::lock_guard<std::mutex> lock(scope->mu);
+  if (scope->open) scope->made.insert_or_assign(key, CastScope::Entry{weight, c, stream});
   return c;
 }
 
 // dW = dy^T x for autograd, or an undefined tensor after adding it into weight.grad in place
 Tensor weight_grad(const Tensor& weight, const Tensor& dy, const Tensor& x) {
   const bool half_gemm = dy.is_cuda() && is_16bit(dy.scalar_type());
-  if (g_wgrad_in_place.load(std::memory_order_relaxed) && half_gemm) {
+  if (half_gemm && wgrad_in_place()) {
     Tensor g = weight.grad();
     if (g.defined() && g.scalar_type() == at::kFloat && g.is_contiguous()) {
       at::addmm_out(g, g, dy.t(), x, at::kFloat);
@@ -847,7 +885,7 @@ struct GatedBwd : OpNode {
     const bool need1 = task_should_compute_output(1), need3 = task_should_compute_output(2);
     if (need1 && need3) {
       const Tensor g1 = w1.grad(), g3 = w3.grad();
-      if (g_wgrad_in_place.load(std::memory_order_relaxed) && is_16bit(cd) && g1.defined() && g3.defined() && g1.scalar_type() == at::kFloat) {
+      if (is_16bit(cd) && wgrad_in_place() && g1.defined() && g3.defined() && g1.scalar_type() == at::kFloat) {
         Tensor both = stacked(g1, g3);
         if (both.defined()) {
           at::addmm_out(both, both, dab.t(), x2, at::kFloat);
@@ -1076,12 +1114,12 @@ PYBIND11_MODULE(_ulm_torch, m) {
   def_op(m, "rms_norm", &::rms_norm);
   def_op(m, "add_rms_norm", &::add_rms_norm);
   def_op(m, "swiglu", &::swiglu);
-  m.def("set_wgrad_in_place", [](bool on) { return g_wgrad_in_place.exchange(on); });
+  py::class_<ContextToken>(m, "ContextToken").def("leave", &leave_context);
+  m.def("enter_wgrad_in_place", [](bool on) { return enter_context([on](OpContext& c) { c.wgrad_in_place = on; }); });
   py::class_<WeightCopies, std::shared_ptr<WeightCopies>>(m, "WeightCopies")
       .def(py::init<std::vector<Tensor>, at::ScalarType>())
       .def("refresh", &WeightCopies::refresh, no_gil());
-  m.def("cast_scope_push", &cast_scope_push, py::arg("copies") = nullptr);
-  m.def("cast_scope_pop", &cast_scope_pop, no_gil());
+  m.def("enter_casts", &enter_casts);
   m.def("cast_cached", &cast_cached, no_gil());
   m.def("weight_grad", [](const Tensor& w, const Tensor& dy, const Tensor& x) -> OptTensor {
     OpScope scope;

@@ -78,28 +78,29 @@ def wgrad_in_place(enabled=True):
     existing fp32 ``weight.grad`` with one GEMM (16-bit operands, fp32 accumulation and output, beta = 1)
     instead of returning a 16-bit product that autograd casts and adds in two more passes per parameter
     and micro-batch.  The caller owns the gradient buffers (they must exist, be zeroed per step, and no
-    post-accumulate hook may be waiting for these parameters): `ulm_dp.DataParallelStep` does."""
-    prev = N.ext().set_wgrad_in_place(bool(enabled))
+    post-accumulate hook may be waiting for these parameters): `ulm_dp.DataParallelStep` does.  It holds for the
+    calling thread and the backward passes it starts inside."""
+    token = N.ext().enter_wgrad_in_place(bool(enabled))
     try:
         yield
     finally:
-        N.ext().set_wgrad_in_place(prev)
+        token.leave()
 
 
 @contextlib.contextmanager
 def weight_cast_scope(copies=None):
-    """While active, `linear` keeps the 16-bit copy it makes of a weight and reuses it: the caller promises
+    """While active in the calling thread, `linear` keeps the 16-bit copy it makes of a weight and reuses it: the caller promises
     that the weights do not change inside the scope (one optimiser step's forward/backward calls).  Nothing
     is reused across scopes or outside one -- a parameter's version counter cannot be relied on for that
     (fused optimisers update parameters without bumping it).  ``copies``: a `weight_copies` object, which is
     refreshed here; without it each weight is cast on first use."""
     if copies is not None:
         copies.refresh()
-    N.ext().cast_scope_push(copies)
+    token = N.ext().enter_casts(copies)
     try:
         yield
     finally:
-        N.ext().cast_scope_pop()
+        token.leave()
 
 
 def weight_copies(weights, dtype):
