@@ -107,3 +107,37 @@ def test_a_copy_is_used_on_the_stream_that_made_it():
     torch.cuda.synchronize()
     casts = [sum(e.count for e in p.key_averages() if e.key == 'aten::_to_copy') for p in (main, other)]
     assert casts == [0, 1] and bool((y == 64).all())
+
+
+def test_the_cpu_step_needs_no_build(monkeypatch):
+    import _native as N
+    import ulm_dp
+
+    def missing():
+        raise RuntimeError('not built')
+
+    for name in ('ext', 'lib', '_load_ext', '_load'):
+        monkeypatch.setattr(N, name, missing)
+    monkeypatch.setattr(N, '_ext', None)
+    monkeypatch.setattr(N, '_ext_error', None, raising=False)
+
+    class Model(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.embedding, self.head = torch.nn.Embedding(11, 8), torch.nn.Linear(8, 11, bias=False)
+
+        def compute_loss(self, ids, ignore_index=0, chunk_rows=0, denominator=None):
+            z = ulm_ops.linear(self.embedding(ids[:, :-1]), self.head.weight)
+            return torch.nn.functional.cross_entropy(z.reshape(-1, 11), ids[:, 1:].reshape(-1), ignore_index=ignore_index, reduction='sum') / denominator
+
+    def post(flat, inv_scale, out):
+        flat.mul_(inv_scale)
+        out[0] += flat.square().sum()
+
+    torch.manual_seed(0)
+    model = Model()
+    before = model.head.weight.detach().clone()
+    cost = ulm_dp.CostModel.for_model(100.0, 8, 1, False)
+    step = ulm_dp.DataParallelStep(model, torch.optim.SGD(model.parameters(), 0.1), samples_per_step=4, grad_post=post, cost=cost)
+    loss, norm, skipped = step.step([torch.randint(1, 11, (4, 6))])
+    assert float(loss) > 0 and float(norm) > 0 and not skipped and not torch.equal(before, model.head.weight)

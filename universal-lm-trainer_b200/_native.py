@@ -31,6 +31,7 @@ _EXT_SOURCE = 'torch_ops.cpp'
 
 _lock = threading.Lock()
 _ext = None
+_ext_error = None
 _lib = None
 _error = None
 
@@ -281,6 +282,19 @@ def _load_ext():
             spec.loader.exec_module(mod)
             _ext = mod
     return _ext
+
+
+def have_ext() -> bool:
+    """Whether `ext` can be had; CPU code paths that need none of its kernels ask this first."""
+    global _ext_error
+    if _ext is not None:
+        return True
+    if _ext_error is None:
+        try:
+            _load_ext()
+        except Exception as e:                             # noqa: BLE001 - `ext` raises it to whoever needs the extension
+            _ext_error = e
+    return _ext is not None
 
 
 def available() -> bool:

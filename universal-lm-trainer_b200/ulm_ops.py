@@ -80,11 +80,12 @@ def wgrad_in_place(enabled=True):
     and micro-batch.  The caller owns the gradient buffers (they must exist, be zeroed per step, and no
     post-accumulate hook may be waiting for these parameters): `ulm_dp.DataParallelStep` does.  It holds for the
     calling thread and the backward passes it starts inside."""
-    token = N.ext().enter_wgrad_in_place(bool(enabled))
+    token = N.ext().enter_wgrad_in_place(bool(enabled)) if N.have_ext() else None
     try:
         yield
     finally:
-        token.leave()
+        if token is not None:
+            token.leave()
 
 
 @contextlib.contextmanager
@@ -96,11 +97,12 @@ def weight_cast_scope(copies=None):
     refreshed here; without it each weight is cast on first use."""
     if copies is not None:
         copies.refresh()
-    token = N.ext().enter_casts(copies)
+    token = N.ext().enter_casts(copies) if N.have_ext() else None
     try:
         yield
     finally:
-        token.leave()
+        if token is not None:
+            token.leave()
 
 
 def weight_copies(weights, dtype):
@@ -125,7 +127,10 @@ def gated_linear(x, w1, w3):
 
 def linear(x, weight):
     """``x @ weight.T`` for the model's bias-free projections (train.py:1925-1926, 1969-1971) in the autocast
-    dtype; see `wgrad_in_place` for what it does differently from ``nn.Linear`` in the backward."""
+    dtype; see `wgrad_in_place` for what it does differently from ``nn.Linear`` in the backward.  On the CPU it needs no
+    build of the library."""
+    if not x.is_cuda and not N.have_ext():
+        return nn.functional.linear(x, weight.to(x.dtype))
     return N.ext().linear(x, weight)
 
 
