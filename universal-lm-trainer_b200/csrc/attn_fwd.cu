@@ -38,7 +38,7 @@
 // except when the whole sequence is one query tile (S <= 128): then K belongs to this CTA
 // alone, its rows have the positions of Q's, and it is rotated with the same table values
 // in the same pass (kRopeQK).  One launch instead of two: at these sizes launches are the cost
-// (67 tokens x 12 heads: 14.2 -> 8.3 us a call).
+// (67 tokens x 12 heads: 14.2 -> 8.3 us a call).  Callers take it while the CTAs run in one wave.
 // Every barrier wait is bounded; on expiry the CTA records a status bit, drains
 // its loads, frees TMEM and returns.  Waits of the softmax warps are made warp-uniform
 // by a vote, because warp-wide instructions (TMEM loads, votes) follow them.

@@ -206,11 +206,14 @@ struct AttnArgs {
   double dropout_p; bool causal; double scale; int64_t seed;
 };
 
-// Longest sequence whose K the attention forward rotates itself (one query tile)
-constexpr int64_t kRopeQkRows = 128;
+// Whether the attention forward rotates Q and K itself: sequences of one query tile, and no more of them than run at a
+// time (two CTAs on each of 148 SMs).  Then the saved launch is what counts: 12 heads x 67 tokens x 1 sequence 7.2 us
+// against 8.2, x 24 (288 CTAs) 9.9 against 10.8.  With more, every further wave pays for the rotation at the start of its
+// CTAs: x 64 24.7 against 21.2, 16 heads x 256 sequences x 16 / 67 / 128 tokens 78 / 112 / 125 against 59 / 95 / 121 us.
+bool rope_in_tile(int64_t B, int64_t H, int64_t S) { return S <= 128 && B * H <= 2 * 148; }
 
 // -> (o, lse); with tables q comes unrotated and, where q_rot is defined, its rotated copy is written there; with k_rot
-// (S <= kRopeQkRows) k comes unrotated too
+// (S <= 128) k comes unrotated too
 void attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const AttnArgs& p,
                   const Tensor& cos = Tensor(), const Tensor& sin = Tensor(), const Tensor& q_rot = Tensor(), const Tensor& k_rot = Tensor()) {
   ulm_attn_fwd_args a{};
@@ -358,7 +361,7 @@ std::pair<Tensor, Tensor> rope_attn_forward(const Tensor& q, const Tensor& k, co
                                             const Tensor& o, const Tensor& lse, const AttnArgs& p, int64_t fuse) {
   const Tensor ko = rope_out_like(k.sizes(), k.strides(), k);
   Tensor qo;
-  if (q.size(2) <= kRopeQkRows) {                        // one query tile: its CTA rotates both, and a launch is saved
+  if (rope_in_tile(q.size(0), q.size(1), q.size(2))) {
     qo = rope_out_like(q.sizes(), q.strides(), q);
     attn_forward(q, k, v, o, lse, p, cos, sin, qo, ko);
   } else if (fuse == kFuseNone) {
@@ -479,10 +482,11 @@ Tensor qkv_attn(const Tensor& qkv, int64_t H, const OptTensor& cos_o, const OptT
   return out;
 }
 
-// Forward alone, nothing kept.  Up to one query tile Q and K are rotated inside the kernel.  Beyond that the launch that
-// rotates K takes Q along while the rotated copy stays in L2 (16 x 4096 x 1 prompt: 76 -> 72 us, x 4: 234 -> 228); from
-// about 20 M elements its traffic costs more than rotating Q inside the kernel, at the start of every CTA (12 x 4096 x 8:
-// 356 us stand-alone, 336 inside).
+// Forward alone, nothing kept.  Where Q and K are not rotated in their tile (rope_in_tile) the launch that rotates K takes Q
+// along while the rotated copy stays in L2, against Q rotated inside the kernel, at the start of every CTA: 2-15 % for
+// short sequences (12 heads x 67 x 128: 37.4 us against 40.7, x 300 x 64: 74.3 / 77.4), 0-4 % for long ones (16 x 4096 x 1:
+// 63.7 / 66.4, x 4: 234 / 240; 12 x 4096 x 6: 277 / 273, within the spread).  From about 20 M elements the two are equal
+// for short sequences (12 x 128 x 2048: 733 both) and the copy's traffic costs more for long ones (12 x 4096 x 8: 356 / 336).
 constexpr int64_t kRopeAloneElems = 20 << 20;
 std::tuple<Tensor, Tensor, Tensor> causal_attention(const Tensor& qkv_in, int64_t H, const OptTensor& cos_o, const OptTensor& sin_o, double scale) {
   TORCH_CHECK_VALUE(cos_o.has_value() == sin_o.has_value(), "cos and sin must be given together");
@@ -511,7 +515,7 @@ std::tuple<Tensor, Tensor, Tensor> causal_attention(const Tensor& qkv_in, int64_
     cos = table(*cos_o); sin = table(*sin_o);
     TORCH_CHECK_VALUE(rope_can_use(q, k, cos, sin), "causal_attention needs fp32 RoPE tables of at least 64 columns on the same device");
     const Tensor ko = rope_out_like(k.sizes(), k.strides(), k);
-    if (S <= kRopeQkRows) {
+    if (rope_in_tile(B, H, S)) {
       attn_forward(q, k, v, heads_of(out, B, S, H), lse, p, cos, sin, Tensor(), ko);
       return {out, ko, v};
     }
