@@ -20,20 +20,20 @@ def test_every_value(dtype):
     y, da, db = _gate(a, one, one)
     x, fi = a.double(), torch.finfo(dtype)
     s = torch.sigmoid(x)
-    t = torch.sigmoid(-x)
     ok = torch.isfinite(x)
 
     def bound(want, terms):
-        # half an ulp of the result (a fixed one among the subnormals) + the stated relative error of s, t and u, on the
-        # terms that are added; below a = -88 exp(-a) overflows fp32 and what is lost is under 2^-119
+        # half an ulp of the result (a fixed one among the subnormals) + the stated relative error of s and u, on the terms
+        # that are added; below a = -88 exp(-a) overflows fp32 and what is lost is under 2^-119
         ulp = 2.0 ** torch.floor(torch.log2(want.abs().clamp(min=fi.tiny))) * fi.eps
         return 0.5 * ulp * 1.01 + 2.0 ** -17 * terms + 2.0 ** -119
 
     u = x * s
     assert bool(((y - u).abs() <= bound(u, u.abs()))[ok].all())
     assert bool(((db - u).abs() <= bound(u, u.abs()))[ok].all())
-    want = s * (1 + x * t)
-    assert bool(((da - want).abs() <= bound(want, s * (1 + (x * t).abs())))[ok].all())
+    want = s * (1 + x * (1 - s))
+    # 1 - s has the error of the reciprocal's last place too: 2^-23, 2^-6 of the bound
+    assert bool(((da - want).abs() <= bound(want, s * (1 + x.abs() * (1 - s + 2.0 ** -6))))[ok].all())
     nan = torch.isnan(x) | (x == -torch.inf)             # silu(-inf) is -inf / inf in the divided form too
     assert bool(torch.isnan(y[nan]).all()) and float(y[x == torch.inf][0]) == torch.inf
 
@@ -51,5 +51,5 @@ def test_error_is_that_of_the_divided_formula(dtype, spread):
     sf, u = 1 / d, r(fa / d)
     ref = (r(u * b.float()), r(r(dy.float() * b.float()) * (sf * (1 + fa * (1 - sf)))), r(dy.float() * u))
     for x, e, f in zip(got, want, ref):
-        # 8 M independent roundings: flips of single ones leave the rms error within 1e-6 of itself
-        assert float((x - e).norm()) <= float((f.double() - e).norm()) * (1 + 1e-6)
+        # an error of 2^-19 beside fp16's rounding of rms 2^-11 / sqrt(12) adds up to sqrt(1 + 0.0135^2)
+        assert float((x - e).norm()) <= float((f.double() - e).norm()) * (1 + 1e-4)
