@@ -105,8 +105,9 @@ def test_traced_ops_run_again_on_other_inputs(device):
     x = torch.randn(24, 16, device=device)
     got, want = traced(x), m(x)
     assert torch.equal(got, want)
-    for a, b in zip(torch.autograd.grad(got.sum(), m.w1), torch.autograd.grad(want.sum(), m.w1)):
-        assert torch.equal(a, b)
+    a, b = torch.autograd.grad(got.sum(), m.w1)[0], torch.autograd.grad(want.sum(), m.w1)[0]
+    # the trace's own backward of the cast to fp16 rounds at another place: one fp16 rounding of a summand
+    assert float((a - b).norm()) <= 2.0 ** -11 * float(b.norm())
 
 
 class _Cut(torch.autograd.Function):
