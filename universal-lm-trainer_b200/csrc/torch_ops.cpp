@@ -239,9 +239,10 @@ void attn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
 }
 
 void attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o_in, const Tensor& lse, const Tensor& do_in,
-                   const Tensor& dq, const Tensor& dk, const Tensor& dv, const AttnArgs& p, const Tensor& cos = Tensor(), const Tensor& sin = Tensor()) {
+                   const Tensor& dq, const Tensor& dk, const Tensor& dv, const AttnArgs& p, const Tensor& cos = Tensor(), const Tensor& sin = Tensor(),
+                   int64_t mode = 7, const Tensor& delta_in = Tensor()) {
   const Tensor go = fa_ready(do_in) ? do_in : do_in.contiguous(), o = fa_ready(o_in) ? o_in : o_in.contiguous();
-  const Tensor delta = empty_cuda({q.size(0), q.size(1), q.size(2)}, at::kFloat, q);
+  const Tensor delta = delta_in.defined() ? delta_in : empty_cuda({q.size(0), q.size(1), q.size(2)}, at::kFloat, q);
   ulm_attn_bwd_args a{};
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.d_o = go.data_ptr();
   a.lse = lse.data_ptr<float>(); a.delta = delta.data_ptr<float>();
@@ -255,7 +256,7 @@ void attn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
   a.dk_sb = dk.stride(0); a.dk_sh = dk.stride(1); a.dk_ss = dk.stride(2);
   a.dv_sb = dv.stride(0); a.dv_sh = dv.stride(1); a.dv_ss = dv.stride(2);
   a.B = (int32_t)q.size(0); a.H = (int32_t)q.size(1); a.S = (int32_t)q.size(2);
-  a.dtype = code_of(q.scalar_type()); a.causal = p.causal; a.mode = 7;
+  a.dtype = code_of(q.scalar_type()); a.causal = p.causal; a.mode = (int32_t)mode;
   a.softmax_scale = (float)p.scale; a.dropout_p = (float)p.dropout_p; a.seed = (uint32_t)p.seed;
   a.status_dev = status_ptr(q); a.stream = stream_of(q);
   if (cos.defined()) {
@@ -530,6 +531,57 @@ std::tuple<Tensor, Tensor, Tensor> causal_attention(const Tensor& qkv_in, int64_
   }
   attn_forward(q, k, v, heads_of(out, B, S, H), lse, p, cos, sin);
   return {out, k, v};
+}
+
+// ---------------------------------------------------------------------------
+// single launches, as the reference's extension exposes them (tests and timings of one kernel)
+// ---------------------------------------------------------------------------
+std::tuple<Tensor, Tensor, OptTensor> single_forward(const Tensor& q, const Tensor& k, const Tensor& v, double dropout_p, bool causal, double scale, int64_t seed,
+                                                     const OptTensor& cos, const OptTensor& sin, bool want_q_rot, const OptTensor& o_out) {
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(q.device());
+  const Tensor o = o_out ? *o_out : empty_bshd(q.size(0), q.size(1), q.size(2), q), lse = empty_lse(q);
+  Tensor q_rot;
+  if (cos && want_q_rot) q_rot = empty_bshd(q.size(0), q.size(1), q.size(2), q);
+  attn_forward(q, k, v, o, lse, {dropout_p, causal, scale, seed}, cos.value_or(Tensor()), sin.value_or(Tensor()), q_rot);
+  return {o, lse, q_rot.defined() ? OptTensor(q_rot) : std::nullopt};
+}
+
+std::array<Tensor, 3> single_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go, double dropout_p,
+                                      bool causal, double scale, int64_t seed, int64_t mode, const OptTensor& delta, const OptTensor& cos, const OptTensor& sin,
+                                      const std::optional<std::array<Tensor, 3>>& out) {
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(q.device());
+  const std::array<Tensor, 3> d = out ? *out : empty_grads(q);
+  attn_backward(q, k, v, o, lse, go, d[0], d[1], d[2], {dropout_p, causal, scale, seed}, cos.value_or(Tensor()), sin.value_or(Tensor()), mode,
+                delta.value_or(Tensor()));
+  return d;
+}
+
+std::tuple<OptTensor, Tensor> single_rope(const OptTensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin, bool backward) {
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(k.device());
+  const Tensor ko = rope_out_like(k.sizes(), k.strides(), k), qo = q ? rope_out_like(q->sizes(), q->strides(), *q) : Tensor();
+  rope_launch(q.value_or(Tensor()), k, qo, ko, cos, sin, backward);
+  return {q ? OptTensor(qo) : std::nullopt, ko};
+}
+
+// o, lse, rotated q and k of unrotated q and k, and the gradients of those
+std::array<Tensor, 4> single_rope_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cos, const Tensor& sin, double dropout_p, bool causal,
+                                          double scale, int64_t seed, int64_t fuse) {
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(q.device());
+  const Tensor o = empty_bshd(q.size(0), q.size(1), q.size(2), q), lse = empty_lse(q);
+  auto [qr, kr] = rope_attn_forward(q, k, v, cos, sin, o, lse, {dropout_p, causal, scale, seed}, fuse);
+  return {o, lse, qr, kr};
+}
+std::array<Tensor, 3> single_rope_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& go, const Tensor& cos,
+                                           const Tensor& sin, double dropout_p, bool causal, double scale, int64_t seed, int64_t fuse) {
+  OpScope scope;
+  c10::cuda::CUDAGuard dev(q.device());
+  auto d = empty_grads(q);
+  rope_attn_backward(q, k, v, o, lse, go, cos, sin, d[0], d[1], d[2], {dropout_p, causal, scale, seed}, fuse);
+  return d;
 }
 
 // ---------------------------------------------------------------------------
@@ -1114,6 +1166,11 @@ PYBIND11_MODULE(_ulm_torch, m) {
   def_op(m, "flash_attn", &::flash_attn);
   def_op(m, "rope_flash_attn", &::rope_flash_attn);
   def_op(m, "qkv_attn", &::qkv_attn);
+  m.def("attn_forward", &single_forward, no_gil());
+  m.def("attn_backward", &single_backward, no_gil());
+  m.def("rope_launch", &single_rope, no_gil());
+  m.def("rope_attn_forward", &single_rope_forward, no_gil());
+  m.def("rope_attn_backward", &single_rope_backward, no_gil());
   m.def("causal_attention", &causal_attention, no_gil());
   def_op(m, "rms_norm", &::rms_norm);
   def_op(m, "add_rms_norm", &::add_rms_norm);

@@ -30,7 +30,6 @@ import _native as N
 
 _SEED_COUNTER = itertools.count(1)
 _STATUS = {}            # device index -> uint32[1] tensor the kernels OR their timeout bits into
-_16BIT = (torch.float16, torch.bfloat16)
 
 
 _last_seed = 0          # seed of the most recent forward (tests rebuild the dropout mask from it)
@@ -50,10 +49,6 @@ def is_available():
 
 def build_error():
     return N.build_error()
-
-
-def _dt(t):
-    return N.ULM_F16 if t.dtype == torch.float16 else N.ULM_BF16
 
 
 def _stream(t=None):
@@ -91,40 +86,12 @@ def can_use(q, k, v):
     return N.ext().can_use(q, k, v)
 
 
-def _empty_bshd(B, H, S, like):
-    """(B,H,S,64) tensor stored as (B,S,H,64)."""
-    return torch.empty((B, S, H, 64), dtype=like.dtype, device=like.device).transpose(1, 2)
-
-
-def _strides3(t):
-    return t.stride(0), t.stride(1), t.stride(2)
-
-
 def attn_forward(q, k, v, dropout_p, causal, softmax_scale, seed, cos=None, sin=None, want_q_rot=True, o_out=None):
     """The reference's ``fa_fwd`` (flash_attn_v100.cu:337-364): returns (o, lse, q_rot).
     With ``cos``/``sin`` (fp32 [S,64] views) q is taken unrotated and rotated inside the
     kernel; q_rot is the rotated copy the backward needs (None without tables).  ``o_out``: a
     preallocated (B,H,S,64) view to write the output into."""
-    lib = N.lib()
-    B, H, S, _ = q.shape
-    o = o_out if o_out is not None else _empty_bshd(B, H, S, q)
-    lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
-    q_rot = None
-    cos_p = sin_p = qr_p = None
-    cos_s = sin_s = 0
-    qr_s = (0, 0, 0)
-    if cos is not None:
-        cos_p, sin_p, cos_s, sin_s = cos.data_ptr(), sin.data_ptr(), cos.stride(0), sin.stride(0)
-        if want_q_rot:
-            q_rot = _empty_bshd(B, H, S, q)
-            qr_p, qr_s = q_rot.data_ptr(), _strides3(q_rot)
-    # positional construction: field by field assignment costs 4x as much host time per launch
-    a = N.AttnFwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
-                      *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(o),
-                      B, H, S, _dt(q), int(bool(causal)), float(softmax_scale), float(dropout_p), int(seed),
-                      _status(q.device).data_ptr(), _stream(), cos_p, sin_p, cos_s, sin_s, qr_p, *qr_s)
-    N.check(lib.ulm_attn_fwd(C.byref(a)), 'flash_attn_v100 forward')
-    return o, lse, q_rot
+    return N.ext().attn_forward(q, k, v, float(dropout_p), bool(causal), float(softmax_scale), int(seed), cos, sin, bool(want_q_rot), o_out)
 
 
 def _seed_for(dropout_p):
@@ -149,68 +116,12 @@ def attn_backward(q, k, v, o, lse, do, dropout_p, causal, softmax_scale, seed, m
     (dq, dk, dv); ``mode`` selects delta / dQ / dK,dV passes like its bitmask.
     With ``cos``/``sin`` q and k are the rotated tensors and dq, dk come back as the
     gradients of the unrotated ones (adjoint rotation in the kernels' epilogues)."""
-    lib = N.lib()
-    B, H, S, _ = q.shape
-    if not _fa_ready(do):
-        do = do.contiguous()
-    if not _fa_ready(o):
-        o = o.contiguous()
-    if out is None:
-        buf = torch.empty((3, B, S, H, 64), dtype=q.dtype, device=q.device)
-        dq, dk, dv = (buf[i].transpose(1, 2) for i in range(3))
-    else:
-        dq, dk, dv = out                                   # caller's (B,H,S,64) views, any 8-element-aligned strides
-    if delta is None:
-        delta = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
-    cos_p = sin_p = None
-    cos_s = sin_s = 0
-    if cos is not None:
-        cos_p, sin_p, cos_s, sin_s = cos.data_ptr(), sin.data_ptr(), cos.stride(0), sin.stride(0)
-    a = N.AttnBwdArgs(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-                      dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                      *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(o), *_strides3(do),
-                      *_strides3(dq), *_strides3(dk), *_strides3(dv),
-                      B, H, S, _dt(q), int(bool(causal)), int(mode), float(softmax_scale), float(dropout_p), int(seed),
-                      _status(q.device).data_ptr(), _stream(), cos_p, sin_p, cos_s, sin_s)
-    N.check(lib.ulm_attn_bwd(C.byref(a)), 'flash_attn_v100 backward')
-    return dq, dk, dv
+    return tuple(N.ext().attn_backward(q, k, v, o, lse, do, float(dropout_p), bool(causal), float(softmax_scale), int(seed), int(mode), delta, cos, sin, out))
 
 
-def _rope_out_like(x):
-    """Dense output in the input's memory order (fast_ops.cu:142-150): fused-qkv
-    views come back as (B,S,H,64)-ordered tensors, not 3x-sized copies."""
-    B, H, S, D = x.shape
-    dense = sum((n - 1) * s for n, s in zip(x.shape, x.stride())) + 1 == x.numel()
-    if dense:
-        return torch.empty_strided(x.shape, x.stride(), dtype=x.dtype, device=x.device)
-    if x.stride(1) == D and x.stride(2) >= H * D:
-        return torch.empty((B, S, H, D), dtype=x.dtype, device=x.device).transpose(1, 2)
-    return torch.empty((B, H, S, D), dtype=x.dtype, device=x.device)
-
-
-def _rope_launch(q, k, cos, sin, backward, shape_like=None, out=None):
-    """q may be None: only k is rotated then (and None comes back in q's place).  ``out`` = (qo, ko)
-    preallocated (B,H,S,64) views to write into."""
-    lib = N.lib()
-    ref_q, ref_k = shape_like if shape_like is not None else (q, k)
-    ko = out[1] if out is not None else _rope_out_like(ref_k)
-    a = N.RopeArgs()
-    a.k, a.ko = k.data_ptr(), ko.data_ptr()
-    a.k_sb, a.k_sh, a.k_ss = _strides3(k)
-    a.ko_sb, a.ko_sh, a.ko_ss = _strides3(ko)
-    qo = None
-    if q is not None:
-        qo = out[0] if out is not None else _rope_out_like(ref_q)
-        a.q, a.qo = q.data_ptr(), qo.data_ptr()
-        a.q_sb, a.q_sh, a.q_ss = _strides3(q)
-        a.qo_sb, a.qo_sh, a.qo_ss = _strides3(qo)
-    a.cos_tab, a.sin_tab = cos.data_ptr(), sin.data_ptr()
-    a.cos_stride, a.sin_stride = cos.stride(0), sin.stride(0)
-    a.B, a.H, a.S = k.shape[0], k.shape[1], k.shape[2]
-    a.dtype, a.backward = _dt(k), int(backward)
-    a.stream = _stream()
-    N.check(lib.ulm_rope(C.byref(a)), 'rope')
-    return qo, ko
+def _rope_launch(q, k, cos, sin, backward):
+    """The stand-alone kernel or its adjoint; q may be None: only k is rotated then (and None comes back in q's place)."""
+    return N.ext().rope_launch(q, k, cos, sin, bool(backward))
 
 
 class _RopeV100Cuda:
@@ -250,38 +161,21 @@ ROPE_FUSION = 'none'
 _FUSE = {'none': 0, 'fwd': 1, 'all': 2}
 
 
-def _rope_attn_forward(q, k, v, cos, sin, dropout_p, causal, softmax_scale, seed, fuse, o_out=None):
-    """-> (o, lse, q_rot, k_rot)"""
-    if fuse == 'none':
-        q_rot, k_rot = _rope_launch(q, k, cos, sin, backward=False)
-        o, lse, _ = attn_forward(q_rot, k_rot, v, dropout_p, causal, softmax_scale, seed, o_out=o_out)
-    else:
-        _, k_rot = _rope_launch(None, k, cos, sin, backward=False)
-        o, lse, q_rot = attn_forward(q, k_rot, v, dropout_p, causal, softmax_scale, seed, cos=cos, sin=sin, o_out=o_out)
-    return o, lse, q_rot, k_rot
-
-
-def _rope_attn_backward(q_rot, k_rot, v, o, lse, do, cos, sin, dropout_p, causal, softmax_scale, seed, fuse, out=None):
-    """-> (dq, dk, dv) of the UNROTATED q, k and of v; ``out`` = three preallocated (B,H,S,64) views."""
-    if fuse == 'all':
-        return attn_backward(q_rot, k_rot, v, o, lse, do, dropout_p, causal, softmax_scale, seed, cos=cos, sin=sin, out=out)
-    if out is None:
-        dqr, dkr, dv = attn_backward(q_rot, k_rot, v, o, lse, do, dropout_p, causal, softmax_scale, seed)
-        dq, dk = _rope_launch(dqr, dkr, cos, sin, backward=True)
-        return dq, dk, dv
-    B, H, S, _ = q_rot.shape
-    tmp = torch.empty((2, B, S, H, 64), dtype=q_rot.dtype, device=q_rot.device)
-    dqr, dkr = tmp[0].transpose(1, 2), tmp[1].transpose(1, 2)
-    attn_backward(q_rot, k_rot, v, o, lse, do, dropout_p, causal, softmax_scale, seed, out=(dqr, dkr, out[2]))
-    _rope_launch(dqr, dkr, cos, sin, backward=True, out=(out[0], out[1]))
-    return out
-
-
 def _fuse_code(fuse):
     code = _FUSE.get(ROPE_FUSION if fuse is None else fuse)
     if code is None:
         raise ValueError("fuse must be 'none', 'fwd' or 'all'")
     return code
+
+
+def _rope_attn_forward(q, k, v, cos, sin, dropout_p, causal, softmax_scale, seed, fuse):
+    """-> (o, lse, q_rot, k_rot): what `rope_flash_attn` launches, without a graph"""
+    return tuple(N.ext().rope_attn_forward(q, k, v, cos, sin, float(dropout_p), bool(causal), float(softmax_scale), int(seed), _fuse_code(fuse)))
+
+
+def _rope_attn_backward(q_rot, k_rot, v, o, lse, do, cos, sin, dropout_p, causal, softmax_scale, seed, fuse):
+    """-> (dq, dk, dv) of the UNROTATED q, k and of v"""
+    return tuple(N.ext().rope_attn_backward(q_rot, k_rot, v, o, lse, do, cos, sin, float(dropout_p), bool(causal), float(softmax_scale), int(seed), _fuse_code(fuse)))
 
 
 def rope_flash_attn(q, k, v, cos2d, sin2d, dropout_p: float = 0.0, causal: bool = True, softmax_scale=None, fuse=None):
