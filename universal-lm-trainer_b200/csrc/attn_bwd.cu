@@ -22,8 +22,7 @@
 // in score buffer pair t % kBufs and is turned into P/dS by compute group
 // t % kGroups (kGW warps each).  MMAs are issued by single-purpose threads, one
 // warp each: one issues S, one dP, into a buffer pair as soon as it is free; one
-// (dK/dV kernel: optionally two) issues the gradient MMAs out of it as soon as the
-// group has written P/dS.  tcgen05.mma blocks its issuing thread while the tensor
+// issues the gradient MMAs out of it as soon as the group has written P/dS.  tcgen05.mma blocks its issuing thread while the tensor
 // pipe is busy, so a thread's barrier waits add to its MMAs' time; with one issuer
 // per operand stream those waits overlap the other issuers' MMAs (one thread for
 // everything left the pipe idle during every hand-off; S and dP on one thread
@@ -53,7 +52,6 @@ constexpr int BR = 128;                 // rows owned by a CTA (queries or keys)
 constexpr int BT = 64;                  // rows of the streamed tile
 constexpr int kBufs = 3;                // score buffer pairs in TMEM; tile t lives in pair t % kBufs
 constexpr int kGroups = 3;              // compute groups; tile t is worked on by group t % kGroups
-constexpr int kGradIssuers = 1;         // dK/dV kernel: 1 = one thread issues dV and dK, 2 = one thread each
 constexpr int kStages = 6;              // streamed-tile ring (must exceed kBufs)
 static_assert(128 * kBufs + 128 <= 512, "score buffer pairs and accumulators must fit 512 TMEM columns");
 static_assert(kBufs == kGroups, "a buffer pair's barriers are awaited by one group only: successive phases of an mbarrier must be awaited in order");
@@ -63,16 +61,15 @@ static_assert(kBufs == kGroups, "a buffer pair's barriers are awaited by one gro
 // the dK/dV kernel gains 8 % with 8, the dQ kernel (less work per element, 72 instead of 128
 // registers) loses 2 %.
 constexpr int kGWdQ = 4, kGWdKV = 8;
-// Single-thread roles, one warp each, after the compute warps: TMA producer, the S issuer, the dP issuer,
-// then kGradIssuers gradient issuers (dK/dV kernel: dV and dK on one thread or on two; the dQ kernel uses
-// the first).
+// Single-thread roles, one warp each, after the compute warps: TMA producer, the S issuer, the dP issuer and
+// the gradient issuer (dK/dV kernel: dV and dK on one thread).
 template <int GW>
 struct Roles {
   static_assert(GW == 4 || GW == 8, "a compute group is one or two warps per TMEM sub-partition");
   static constexpr int kGroupThreads = 32 * GW;
   static constexpr int kProducerWarp = GW * kGroups, kMmaWarp = kProducerWarp + 1, kMma2Warp = kProducerWarp + 2,
-                       kGradWarp = kProducerWarp + 3, kGrad2Warp = kProducerWarp + 4;
-  static constexpr int kThreads = kGroupThreads * kGroups + (3 + kGradIssuers) * 32;
+                       kGradWarp = kProducerWarp + 3;
+  static constexpr int kThreads = kGroupThreads * kGroups + 4 * 32;
 };
 constexpr uint32_t kBigTile = BR * HD * 2;    // 16 KB
 constexpr uint32_t kSmallTile = BT * HD * 2;  //  8 KB
@@ -343,7 +340,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   constexpr int kGW = kGWdQ;
   using R = Roles<kGW>;
   [[maybe_unused]] constexpr int kGroupThreads = R::kGroupThreads, kProducerWarp = R::kProducerWarp, kMmaWarp = R::kMmaWarp,
-                kMma2Warp = R::kMma2Warp, kGradWarp = R::kGradWarp, kGrad2Warp = R::kGrad2Warp;
+                kMma2Warp = R::kMma2Warp, kGradWarp = R::kGradWarp;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQdObig = base;                               // [slot][Q|dO|O], 16 KB each; item n uses slot n & 1
@@ -694,7 +691,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   constexpr int kGW = kGWdKV;
   using R = Roles<kGW>;
   [[maybe_unused]] constexpr int kGroupThreads = R::kGroupThreads, kProducerWarp = R::kProducerWarp, kMmaWarp = R::kMmaWarp,
-                kMma2Warp = R::kMma2Warp, kGradWarp = R::kGradWarp, kGrad2Warp = R::kGrad2Warp;
+                kMma2Warp = R::kMma2Warp, kGradWarp = R::kGradWarp;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sKVbig = base;                                 // [slot][K|V], 16 KB each; item n uses slot n & 1
@@ -717,9 +714,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&ctl->kv_full[i], 1); mbar_init(&ctl->kv_free[i], 2); }
-    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->qdo_full[s], 1); mbar_init(&ctl->qdo_empty[s], kGradIssuers); }
-    for (int g = 0; g < kBufs; ++g) { mbar_init(&ctl->sdp_full[g], 2); mbar_init(&ctl->pds_ready[g], kGroupThreads); mbar_init(&ctl->buf_free[g], kGradIssuers); }
-    for (int g = 0; g < kGroups; ++g) mbar_init(&ctl->dkv_done[g], kGradIssuers);
+    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->qdo_full[s], 1); mbar_init(&ctl->qdo_empty[s], 1); }
+    for (int g = 0; g < kBufs; ++g) { mbar_init(&ctl->sdp_full[g], 2); mbar_init(&ctl->pds_ready[g], kGroupThreads); mbar_init(&ctl->buf_free[g], 1); }
+    for (int g = 0; g < kGroups; ++g) mbar_init(&ctl->dkv_done[g], 1);
     mbar_init(&ctl->acc_free, kGroupThreads);
     ctl->abort = 0;
     ctl->fail_bits = 0;
@@ -816,9 +813,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         mma_commit(&ctl->kv_free[slot]);                  // arrives once this thread's MMAs of the item have read K (V)
       }
     }
-  } else if (warp == kGradWarp || (warp == kGrad2Warp && kGradIssuers == 2)) {
-    if (elect_one()) {                                     // gradient MMAs: dV += P^T dO_i (first issuer), dK += dS^T Q_i (second)
-      const bool second = warp == kGrad2Warp;
+  } else if (warp == kGradWarp) {
+    if (elect_one()) {                                     // gradient MMAs: dV += P^T dO_i, dK += dS^T Q_i
       constexpr uint32_t idesc_a = make_idesc(Fmt<T>::v, BR, HD, 1);   // B = dO / Q tile read MN-major
       ItemIter items(n_items);
       uint32_t t = 0;
@@ -835,9 +831,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (!mbar_wait(&ctl->pds_ready[g], (t / kBufs) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); ok = false; break; }
           fence_after_sync();
 #pragma unroll
-          for (int w = 0; w < 3 - kGradIssuers; ++w) {
+          for (int w = 0; w < 2; ++w) {
             // dV reads P^T (packed over S^T) against the dO tile; dK reads dS^T (packed over dP^T) against the Q tile
-            const bool sec = kGradIssuers == 2 ? second : (w == 1);
+            const bool sec = w == 1;
             const uint64_t db = make_sdesc_sw128(smem_u32(sQdO + (size_t)s * 2 * kSmallTile + (sec ? 0 : kSmallTile)));
             const uint32_t t_acc = tmem_base + (sec ? cK : cV), t_a = tmem_base + 128 * g + (sec ? 64 : 0);
 #pragma unroll
@@ -891,68 +887,29 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const bool edge = CAUSAL && (i0 < n0 + BR - 1);   // some query of the tile precedes some key of the CTA
         auto tile_body = [&](auto edge_c) {                // masked / unmasked tiles as separate code (see the dQ kernel)
         constexpr bool EDGE = decltype(edge_c)::value;
-        if constexpr (kGW == 8) {
 #pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
-            uint32_t sv[16], pv[16], pp[8], pd[8];
-            const int col0 = my_half * 32 + ch * 16;
-            tmem_ld16(t_row + cS + col0, sv);
-            tmem_ld16(t_row + cP + col0, pv);
-            tmem_wait_ld();
-            float l4[4], d4[4];                            // statistics of 4 queries per 16-byte shared load
-#pragma unroll
-            for (int c = 0; c < 16; c += 2) {
-              float p2[2], d2[2];
-              if ((c & 3) == 0) {
-                *reinterpret_cast<float4*>(l4) = *reinterpret_cast<const float4*>(&ctl->lse2[g][col0 + c]);
-                *reinterpret_cast<float4*>(d4) = *reinterpret_cast<const float4*>(&ctl->dlt[g][col0 + c]);
-              }
-#pragma unroll
-              if constexpr (!DROPOUT) {
-                pair_ds(sv[c], sv[c + 1], pv[c], pv[c + 1], sc2, f2_pack(l4[c & 3], l4[(c + 1) & 3]), f2_pack(d4[c & 3], d4[(c + 1) & 3]),
-                        [&](int e) { return !EDGE || (i0 + col0 + c + e >= kc); }, d2, p2);
-              } else {
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int q = i0 + col0 + c + e;
-                float p = ex2(fmaf(__uint_as_float(sv[c + e]), scale2, l4[(c + e) & 3]));
-                if constexpr (EDGE) p = (q >= kc) ? p : 0.f;
-                float dp = __uint_as_float(pv[c + e]);
-                const bool keep = dropout_keep(seed_mix, q, kc, dropout_p);
-                p2[e] = keep ? p * inv_keep : 0.f;
-                dp = keep ? dp * inv_keep : 0.f;
-                d2[e] = p * (dp + d4[(c + e) & 3]);
-              }
-              }
-              pp[c >> 1] = Cvt<T>::pack2(p2[0], p2[1]);
-              pd[c >> 1] = Cvt<T>::pack2(d2[0], d2[1]);
-            }
-            st8(t_row + cS + my_half * 32 + ch * 8, pp);
-            st8(t_row + cP + my_half * 32 + ch * 8, pd);
-          }
-        } else {
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t sv[32], pv[32], pp[16], pd[16];
-          tmem_ld32(t_row + cS + hf * 32, sv);
-          tmem_ld32(t_row + cP + hf * 32, pv);
+        for (int ch = 0; ch < 2; ++ch) {
+          uint32_t sv[16], pv[16], pp[8], pd[8];
+          const int col0 = my_half * 32 + ch * 16;
+          tmem_ld16(t_row + cS + col0, sv);
+          tmem_ld16(t_row + cP + col0, pv);
           tmem_wait_ld();
-          float l4[4], d4[4];                              // statistics of 4 queries per 16-byte shared load
+          float l4[4], d4[4];                            // statistics of 4 queries per 16-byte shared load
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) {
+          for (int c = 0; c < 16; c += 2) {
             float p2[2], d2[2];
             if ((c & 3) == 0) {
-              *reinterpret_cast<float4*>(l4) = *reinterpret_cast<const float4*>(&ctl->lse2[g][hf * 32 + c]);
-              *reinterpret_cast<float4*>(d4) = *reinterpret_cast<const float4*>(&ctl->dlt[g][hf * 32 + c]);
+              *reinterpret_cast<float4*>(l4) = *reinterpret_cast<const float4*>(&ctl->lse2[g][col0 + c]);
+              *reinterpret_cast<float4*>(d4) = *reinterpret_cast<const float4*>(&ctl->dlt[g][col0 + c]);
             }
 #pragma unroll
             if constexpr (!DROPOUT) {
               pair_ds(sv[c], sv[c + 1], pv[c], pv[c + 1], sc2, f2_pack(l4[c & 3], l4[(c + 1) & 3]), f2_pack(d4[c & 3], d4[(c + 1) & 3]),
-                      [&](int e) { return !EDGE || (i0 + hf * 32 + c + e >= kc); }, d2, p2);
+                      [&](int e) { return !EDGE || (i0 + col0 + c + e >= kc); }, d2, p2);
             } else {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int q = i0 + hf * 32 + c + e;
+              const int q = i0 + col0 + c + e;
               float p = ex2(fmaf(__uint_as_float(sv[c + e]), scale2, l4[(c + e) & 3]));
               if constexpr (EDGE) p = (q >= kc) ? p : 0.f;
               float dp = __uint_as_float(pv[c + e]);
@@ -965,9 +922,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             pp[c >> 1] = Cvt<T>::pack2(p2[0], p2[1]);
             pd[c >> 1] = Cvt<T>::pack2(d2[0], d2[1]);
           }
-          st16(t_row + cS + hf * 16, pp);
-          st16(t_row + cP + hf * 16, pd);
-        }
+          st8(t_row + cS + my_half * 32 + ch * 8, pp);
+          st8(t_row + cP + my_half * 32 + ch * 8, pd);
         }
         };
         if (edge) tile_body(std::true_type{}); else tile_body(std::false_type{});
@@ -990,16 +946,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         T* v_item = dV + (int64_t)b * dv_sb + (int64_t)h * dv_sh + (int64_t)n0 * dv_ss;
         T* k_item = dK + (int64_t)b * dk_sb + (int64_t)h * dk_sh + (int64_t)n0 * dk_ss;
         uint4 vlo[4], klo[4];
-        [[maybe_unused]] uint4 vhi[4], khi[4];
-        if constexpr (kGW == 4) {
-          acc_to_16bit<T>(t_row + cV, 1.f, vlo);
-          acc_to_16bit<T>(t_row + cV + 32, 1.f, vhi);
-          acc_to_16bit<T>(t_row + cK, scale, klo);
-          acc_to_16bit<T>(t_row + cK + 32, scale, khi);
-        } else {
-          acc_to_16bit<T>(t_row + cV + my_half * 32, 1.f, vlo);
-          acc_to_16bit<T>(t_row + cK + my_half * 32, scale, klo);
-        }
+        [[maybe_unused]] uint4 khi[4];                     // a thread holds 32 columns: nothing in the other half
+        acc_to_16bit<T>(t_row + cV + my_half * 32, 1.f, vlo);
+        acc_to_16bit<T>(t_row + cK + my_half * 32, scale, klo);
         fence_before_sync();
         mbar_arrive(&ctl->acc_free);
         staged_store<T>(stage + (size_t)g * kRopeStageBytes, g, tg, r, my_half, vlo, v_item, dv_ss, S - n0);
