@@ -141,3 +141,21 @@ def test_the_cpu_step_needs_no_build(monkeypatch):
     step = ulm_dp.DataParallelStep(model, torch.optim.SGD(model.parameters(), 0.1), samples_per_step=4, grad_post=post, cost=cost)
     loss, norm, skipped = step.step([torch.randint(1, 11, (4, 6))])
     assert float(loss) > 0 and float(norm) > 0 and not skipped and not torch.equal(before, model.head.weight)
+
+
+@pytest.mark.gpu
+def test_the_copies_outlive_the_work_of_every_stream_that_used_them():
+    w = torch.nn.Parameter(torch.ones(1024, 1024, device='cuda'))
+    x = torch.ones(4, 1024, device='cuda', dtype=torch.float16)
+    copies = ulm_ops.weight_copies([w], torch.float16)
+    torch.cuda.synchronize()
+    side, where = torch.cuda.Stream(), copies.views[0].data_ptr()
+    with torch.no_grad(), torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)                    # about 0.1 s of clock cycles, in front of the copies' use
+        with ulm_ops.weight_cast_scope(copies):
+            y = ulm_ops.linear(x, w)
+    del copies
+    other = torch.full((1024, 1024), 2.0, device='cuda', dtype=torch.float16)
+    assert other.data_ptr() != where
+    torch.cuda.synchronize()
+    assert bool((y == 1024).all())

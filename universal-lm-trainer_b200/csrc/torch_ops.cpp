@@ -13,6 +13,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/AutogradState.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -810,6 +811,10 @@ struct WeightCopies {
   void refresh() {
     if (params.empty()) return;
     OpScope scope;
+    // the buffer outlives a step and may be filled and read on another stream than the one it was allocated on: what is
+    // queued there has to end before the allocator hands the memory out again
+    if (views[0].is_cuda())
+      c10::cuda::CUDACachingAllocator::recordStream(views[0].storage().data_ptr(), c10::cuda::getCurrentCUDAStream(views[0].device().index()));
     at::_foreach_copy_(views, params);
   }
 };
@@ -1179,6 +1184,7 @@ PYBIND11_MODULE(_ulm_torch, m) {
   m.def("enter_wgrad_in_place", [](bool on) { return enter_context([on](OpContext& c) { c.wgrad_in_place = on; }); });
   py::class_<WeightCopies, std::shared_ptr<WeightCopies>>(m, "WeightCopies")
       .def(py::init<std::vector<Tensor>, at::ScalarType>())
+      .def_readonly("views", &WeightCopies::views)
       .def("refresh", &WeightCopies::refresh, no_gil());
   m.def("enter_casts", &enter_casts);
   m.def("cast_cached", &cast_cached, no_gil());
