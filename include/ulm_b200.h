@@ -71,7 +71,7 @@ uint64_t ulm_launch_count(void);
  */
 typedef struct {
   const void* q; const void* k;        /* inputs (or dqo, dko when backward)  */
-  void* qo; void* ko;                  /* outputs                             */
+  void* qo; void* ko;                  /* outputs; may be the inputs, with the same strides */
   const float* cos_tab; const float* sin_tab;
   int64_t q_sb, q_sh, q_ss;
   int64_t k_sb, k_sh, k_ss;

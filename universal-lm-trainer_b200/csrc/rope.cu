@@ -19,10 +19,11 @@ constexpr int kHeadsPerThread = 4;
 // A thread owns 8 columns of the low half and their 8 partners in the high half (two 16-byte
 // vectors each way) of up to kHeadsPerThread heads of ONE position: the cos / sin values depend on
 // the position only, so they are loaded once and reused for every head -- per row two 16-byte loads
-// of data and two of tables instead of two and eight.
+// of data and two of tables instead of two and eight.  The output may be the input (the adjoint behind the attention
+// backward): a thread reads all that it rotates before it writes, and no __restrict__ says otherwise.
 template <typename T, bool BWD>
 __global__ void __launch_bounds__(kThreads)
-rope_kernel(const T* __restrict__ q, const T* __restrict__ k, T* __restrict__ qo, T* __restrict__ ko,
+rope_kernel(const T* q, const T* k, T* qo, T* ko,
             const float* __restrict__ cs, const float* __restrict__ sn,
             int64_t q_sb, int64_t q_sh, int64_t q_ss, int64_t k_sb, int64_t k_sh, int64_t k_ss,
             int64_t qo_sb, int64_t qo_sh, int64_t qo_ss, int64_t ko_sb, int64_t ko_sh, int64_t ko_ss,
