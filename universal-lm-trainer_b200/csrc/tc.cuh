@@ -72,11 +72,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 }
 
 // True in exactly one lane of a converged warp.  The single-thread roles (TMA producer, MMA issuers) branch on THIS
-// and not on `lane == 0`: the compiler knows that an elected region runs in one thread and keeps the matrix
-// descriptors and TMEM addresses of tcgen05 instructions in uniform registers.  Behind a lane comparison every
-// tcgen05.mma and tcgen05.commit costs its issuer 46-54 clk of moves and waits, more than the tensor pipe needs for
-// the 128x64x16 products it is fed (32 clk with A in TMEM, 48 with both operands in shared memory); elected, an MMA
-// issues in under 10 clk and a commit in 5 (measured, one issuing thread, back to back).
+// and not on `lane == 0`.  Measured, one issuing thread, back to back: behind a lane comparison a tcgen05.mma or a
+// tcgen05.commit costs its issuer 46-54 clk, more than the tensor pipe needs for the 128x64x16 products it is fed (32 clk
+// with A in TMEM, 48 with both operands in shared memory); elected, an MMA issues in under 10 clk and a commit in 5.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
