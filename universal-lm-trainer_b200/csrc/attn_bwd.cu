@@ -17,7 +17,7 @@
 //   dK/dV kernel: CTA = 128 keys (thread r = key r), walks query tiles of 64 from
 //                the diagonal down, transposed view: S^T = K Q^T, dP^T = V dO^T,
 //                dV += P^T dO, dK += dS^T Q.
-// One CTA per SM owns all 512 TMEM columns.  Streamed tiles are independent of
+// dK/dV kernel: one CTA per SM owns all 512 TMEM columns (the dQ kernel's CTAs share an SM, see there).  Streamed tiles are independent of
 // each other (the softmax statistics come from the forward pass), so tile t lives
 // in score buffer pair t % kBufs and is turned into P/dS by compute group
 // t % kGroups (kGW warps each).  MMAs are issued by single-purpose threads, one
@@ -25,8 +25,7 @@
 // issues the gradient MMAs out of it as soon as the group has written P/dS.  tcgen05.mma blocks its issuing thread while the tensor
 // pipe is busy, so a thread's barrier waits add to its MMAs' time; with one issuer
 // per operand stream those waits overlap the other issuers' MMAs (one thread for
-// everything left the pipe idle during every hand-off; S and dP on one thread
-// cost the dQ kernel 12 %).  Each accumulator has exactly one issuer, so the
+// everything left the pipe idle during every hand-off).  Each accumulator has exactly one issuer, so the
 // summation order, and with it the result, is the same on every run.  All barrier
 // waits are bounded (status bit + clean exit on expiry); the compute warps make the
 // outcome of a wait warp-uniform by a vote, because warp-wide TMEM loads follow.
@@ -58,9 +57,8 @@ static_assert(kBufs == kGroups, "a buffer pair's barriers are awaited by one gro
 // Warps per compute group: 4 (a thread per row of the tile) or 8 (two threads per row, 32 columns each).
 // A single warp issues about one instruction every two clocks on its dependent chains, so a second
 // warp per sub-partition nearly halves the time a group holds a tile; measured at B=8,H=12,S=4096:
-// the dK/dV kernel gains 8 % with 8, the dQ kernel (less work per element, 72 instead of 128
-// registers) loses 2 %.
-constexpr int kGWdQ = 4, kGWdKV = 8;
+// the dK/dV kernel gains 8 % with 8.
+constexpr int kGWdKV = 8;
 // Single-thread roles, one warp each, after the compute warps: TMA producer, the S issuer, the dP issuer and
 // the gradient issuer (dK/dV kernel: dV and dK on one thread).
 template <int GW>
@@ -145,6 +143,25 @@ __device__ __forceinline__ bool group_wait(int g, bool poller, uint64_t* bar, ui
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(any) : "r"(fail), "r"(g + 1), "n"(32 * GW) : "memory");
   return any == 0;
+}
+
+// All lanes of a warp learn together whether the wait succeeded.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
+// The threads of compute group g learn together whether any of them says yes.
+template <int GW>
+__device__ __forceinline__ bool group_any(int g, bool yes) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "bar.red.or.pred p, %2, %3, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(any) : "r"((uint32_t)yes), "r"(g + 1), "n"(32 * GW) : "memory");
+  return any != 0;
 }
 
 // Tables of the fused RoPE adjoint (unused when ROPE is false).
@@ -299,7 +316,7 @@ attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO, float* __re
 }
 
 // ---------------------------------------------------------------------------
-// Persistent CTAs.  Both tensor-core kernels launch one CTA per SM, which walks a static list of
+// Persistent CTAs.  The dK/dV kernel launches one CTA per SM, which walks a static list of
 // work items (one item = one (batch*head, tile of 128 rows)).  Items are numbered heaviest first
 // and dealt to the CTAs in boustrophedon order -- round r gives CTA c item r*G + c on even rounds
 // and r*G + G-1-c on odd ones -- which balances the CTAs' totals to within one item of the mean
@@ -311,343 +328,241 @@ attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO, float* __re
 // ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // dQ kernel
-// TMEM columns: buffer pair b holds S at 128b and dP at 128b+64 (dS is packed over S);
-// the dQ accumulator sits at 128*kBufs.
+// One CTA per work item (128 query rows of one (batch, head)), two CTAs per SM, so that one CTA's exponentials run
+// under the other's waits, loads and stores, and a CTA's start-up and epilogue under the other's tiles.
+// TMEM columns: S at 0, dP at 64, packed dS at 128, the dQ accumulator at 192.  A compute thread owns a query row: it takes the
+// 64 + 64 values of its row into registers and hands both buffers back at once, so the next tile's S and dP are
+// there when it has written this tile's dS, into columns that the previous tile's gradient MMAs have long read.
+// What bounds it: issue slots and the SFU (64 exponentials a thread and tile), then the synchronisation around a tile, whose
+// instructions queue behind the exponentials.  Against one persistent CTA per SM with three score buffer pairs, which waited a round
+// trip through the tensor core for every pair (us, start -> now): B8 H12 S4096 bf16 376 -> 335, B24 H12 S1363 fp16 180 -> 162,
+// B4 H12 S201 8.6 -> 7.6, B64 H12 S300 64 -> 64, B1 H16 S4096 68 -> 71 (512 CTAs are not quite two waves).
 // ---------------------------------------------------------------------------
+constexpr int kStagesQ = 3;                // K/V tile ring
+constexpr int kThreadsQ = 32 * (4 + 2);    // compute warps, producer warp, MMA warp
 struct CtlQ {
-  uint64_t qdo_full[2], qdo_free[2], kv_full[kStages], kv_empty[kStages], sdp_full[kBufs], ds_ready[kBufs], buf_free[kBufs],
-      dq_done[kGroups], acc_free;
+  uint64_t qdo_full, kv_full[kStagesQ], kv_empty[kStagesQ], sdp_full, sdp_free, ds_ready, dq_done;
   uint32_t tmem_base;
   int abort;
   uint32_t fail_bits;
 };
-constexpr size_t kCtlBytes = 4096;        // control block (barriers, per-tile statistics), padded so that what follows stays 128-byte aligned
-static_assert(sizeof(CtlQ) <= kCtlBytes, "control block");
-constexpr size_t kStageBytes = (size_t)kGroups * kRopeStageBytes;   // staging tiles: the dK/dV kernel's, and the dQ kernel's ROPE variants'
-constexpr size_t kSmemQ = 1024 + 6 * (size_t)kBigTile + (size_t)kStages * 2 * kSmallTile + kCtlBytes;
+constexpr uint32_t kTmemColsQ = 256, kColDP = 64, kColDS = 128, kColDQ = 192;
+constexpr size_t kSmemQ = 1024 + 3 * (size_t)kBigTile + (size_t)kStagesQ * 2 * kSmallTile + sizeof(CtlQ);
 
 // FUSE_DELTA: the kernel also loads the item's O tile, computes delta = rowsum(O * dO) for its 128 rows
-// itself (each compute group for its own use, from shared memory) and writes it to DELTA for the dK/dV
-// kernel that follows on the stream; otherwise DELTA is an input.
+// itself and writes it to DELTA for the dK/dV kernel that follows on the stream; otherwise DELTA is an input.
 template <typename T, bool CAUSAL, bool DROPOUT, bool FUSE_DELTA, bool ROPE>
-__global__ void __launch_bounds__(Roles<kGWdQ>::kThreads, 1)
+__global__ void __launch_bounds__(kThreadsQ, 2)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                    const __grid_constant__ CUtensorMap tmO,
                    const float* __restrict__ LSE, float* __restrict__ DELTA, T* __restrict__ dQ,
-                   int64_t dq_sb, int64_t dq_sh, int64_t dq_ss, int S, int H, int BH, float scale, float scale2,
+                   int64_t dq_sb, int64_t dq_sh, int64_t dq_ss, int S, int H, float scale, float scale2,
                    float dropout_p, uint32_t seed, uint32_t* status, const RopeTab rt) {
-  constexpr int kGW = kGWdQ;
-  using R = Roles<kGW>;
-  [[maybe_unused]] constexpr int kGroupThreads = R::kGroupThreads, kProducerWarp = R::kProducerWarp, kMmaWarp = R::kMmaWarp,
-                kMma2Warp = R::kMma2Warp, kGradWarp = R::kGradWarp;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQdObig = base;                               // [slot][Q|dO|O], 16 KB each; item n uses slot n & 1
-  uint8_t* sKV = base + 6 * kBigTile;                    // [stage][K|V], 8 KB each
-  CtlQ* ctl = reinterpret_cast<CtlQ*>(sKV + (size_t)kStages * 2 * kSmallTile);
-  [[maybe_unused]] uint8_t* stage = reinterpret_cast<uint8_t*>(ctl) + kCtlBytes;   // ROPE only: kGroups staging tiles
+  uint8_t* sQ = base;                                    // dQ is staged here once the scores are done
+  uint8_t* sdO = base + kBigTile;
+  uint8_t* sO = base + 2 * kBigTile;
+  uint8_t* sKV = base + 3 * kBigTile;                    // [stage][K|V], 8 KB each
+  CtlQ* ctl = reinterpret_cast<CtlQ*>(sKV + (size_t)kStagesQ * 2 * kSmallTile);
   volatile int* abort_flag = &ctl->abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
+  const int qt = (int)gridDim.y - 1 - (int)blockIdx.y;   // the last query tile is the heaviest under the causal mask: scheduled first
+  const int m0 = qt * BR;
   const int n_all = (S + BT - 1) / BT;
-  const int n_qt = (S + BR - 1) / BR;
-  const int n_items = BH * n_qt;
-  // item -> (batch*head, first query row, key tiles): the last query tile is the heaviest under the causal mask
-  auto decode = [&](int idx, int& bh, int& m0, int& nkv) {
-    const int lvl = idx / BH;
-    bh = idx - lvl * BH;
-    m0 = (n_qt - 1 - lvl) * BR;
-    const int n_causal = (m0 + BR) / BT;
-    nkv = CAUSAL ? (n_causal < n_all ? n_causal : n_all) : n_all;
-  };
+  const int n_causal = (m0 + BR) / BT;
+  const int nkv = CAUSAL ? (n_causal < n_all ? n_causal : n_all) : n_all;
 
   if (threadIdx.x == 0) {
-    // a slot is free again once the S and dP issuers' MMAs have read it and, when the compute threads read it
-    // too (FUSE_DELTA), once every one of them is done with the item
-    for (int i = 0; i < 2; ++i) { mbar_init(&ctl->qdo_full[i], 1); mbar_init(&ctl->qdo_free[i], 2 + (FUSE_DELTA ? kGroups * kGroupThreads : 0)); }
-    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->kv_full[s], 1); mbar_init(&ctl->kv_empty[s], 1); }
-    for (int g = 0; g < kBufs; ++g) { mbar_init(&ctl->sdp_full[g], 2); mbar_init(&ctl->ds_ready[g], kGroupThreads); mbar_init(&ctl->buf_free[g], 1); }
-    for (int g = 0; g < kGroups; ++g) mbar_init(&ctl->dq_done[g], 1);
-    mbar_init(&ctl->acc_free, kGroupThreads);
+    mbar_init(&ctl->qdo_full, 1);
+    for (int s = 0; s < kStagesQ; ++s) { mbar_init(&ctl->kv_full[s], 1); mbar_init(&ctl->kv_empty[s], 1); }
+    mbar_init(&ctl->sdp_full, 1);
+    mbar_init(&ctl->sdp_free, 4);
+    mbar_init(&ctl->ds_ready, 4);
+    mbar_init(&ctl->dq_done, 1);
     ctl->abort = 0;
     ctl->fail_bits = 0;
     fence_mbar_init();
   }
-  if (warp == kMmaWarp) { tmem_alloc(&ctl->tmem_base, kTmemCols); tmem_relinquish(); }
+  if (warp == 5) { tmem_alloc(&ctl->tmem_base, kTmemColsQ); tmem_relinquish(); }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);   // warp-uniform
-  constexpr uint32_t cQ = 128 * kBufs;
 
-  if (warp == kProducerWarp) {
+  if (warp == 4) {
+    // ------------------------------ TMA producer ------------------------------
     if (elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
       if (FUSE_DELTA) tma_prefetch_desc(&tmO);
-      ItemIter items(n_items);
-      uint32_t t = 0;                                     // tiles issued so far, over all items
-      int n = 0, idx;
-      bool ok = true;
-      for (; ok && items.next(idx); ++n) {
-        int bh, m0, nkv;
-        decode(idx, bh, m0, nkv);
-        const int b = bh / H, h = bh - b * H, slot = n & 1;
-        // the slot's previous Q/dO (item n-2) must have been read by the last S and dP MMAs of that item
-        if (n >= 2 && !mbar_wait(&ctl->qdo_free[slot], ((n >> 1) - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); break; }
-        uint8_t* big = sQdObig + (size_t)slot * 3 * kBigTile;
-        mbar_expect_tx(&ctl->qdo_full[slot], (FUSE_DELTA ? 3 : 2) * kBigTile);
-        tma_load_4d(big, &tmQ, &ctl->qdo_full[slot], 0, m0, h, b);
-        tma_load_4d(big + kBigTile, &tmdO, &ctl->qdo_full[slot], 0, m0, h, b);
-        if (FUSE_DELTA) tma_load_4d(big + 2 * kBigTile, &tmO, &ctl->qdo_full[slot], 0, m0, h, b);
-        for (int j = 0; j < nkv; ++j, ++t) {
-          const uint32_t s = t % kStages;
-          if (t >= kStages && !mbar_wait(&ctl->kv_empty[s], ((t / kStages) - 1) & 1, abort_flag)) {
-            atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA);
-            ok = false;
-            break;
-          }
-          uint8_t* dst = sKV + (size_t)s * 2 * kSmallTile;
-          mbar_expect_tx(&ctl->kv_full[s], 2 * kSmallTile);
-          tma_load_4d(dst, &tmK, &ctl->kv_full[s], 0, j * BT, h, b);
-          tma_load_4d(dst + kSmallTile, &tmV, &ctl->kv_full[s], 0, j * BT, h, b);
-        }
+      mbar_expect_tx(&ctl->qdo_full, (FUSE_DELTA ? 3 : 2) * kBigTile);
+      tma_load_4d(sQ, &tmQ, &ctl->qdo_full, 0, m0, h, b);
+      tma_load_4d(sdO, &tmdO, &ctl->qdo_full, 0, m0, h, b);
+      if (FUSE_DELTA) tma_load_4d(sO, &tmO, &ctl->qdo_full, 0, m0, h, b);
+      int j = 0;
+      for (; j < nkv; ++j) {
+        const int s = j % kStagesQ;
+        if (j >= kStagesQ && !mbar_wait(&ctl->kv_empty[s], ((j / kStagesQ) - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); break; }
+        uint8_t* dst = sKV + (size_t)s * 2 * kSmallTile;
+        mbar_expect_tx(&ctl->kv_full[s], 2 * kSmallTile);
+        tma_load_4d(dst, &tmK, &ctl->kv_full[s], 0, j * BT, h, b);
+        tma_load_4d(dst + kSmallTile, &tmV, &ctl->kv_full[s], 0, j * BT, h, b);
       }
       if (*abort_flag) {   // let our own copies land before the CTA's shared memory goes away
-        const int n_loaded = ok ? n : n + 1;              // items whose Q/dO loads were issued
-        for (int m = n_loaded > 2 ? n_loaded - 2 : 0; m < n_loaded; ++m) {
+        auto drain = [](uint64_t* full, uint32_t parity) {
           const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try(&ctl->qdo_full[m & 1], (m >> 1) & 1))
+          while (!mbar_try(full, parity))
             if (globaltimer_ns() - t0 > kWaitLimitNs) break;
-        }
-        for (uint32_t u = t > (uint32_t)kStages ? t - kStages : 0; u < t; ++u) {
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try(&ctl->kv_full[u % kStages], (u / kStages) & 1))
-            if (globaltimer_ns() - t0 > kWaitLimitNs) break;
-        }
+        };
+        drain(&ctl->qdo_full, 0);
+        for (int u = j > kStagesQ ? j - kStagesQ : 0; u < j; ++u) drain(&ctl->kv_full[u % kStagesQ], (u / kStagesQ) & 1);
       }
     }
-  } else if (warp == kMmaWarp || warp == kMma2Warp) {
-    if (elect_one()) {                                     // score MMAs: S_j = Q K_j^T (first issuer), dP_j = dO V_j^T (second)
-      const bool second = warp == kMma2Warp;
+  } else if (warp == 5) {
+    // ------------------------------ MMA issuer --------------------------------
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc(Fmt<T>::v, BR, BT, 0);   // 128 x 64, both K-major
-      ItemIter items(n_items);
-      uint32_t t = 0;
-      int n = 0, idx;
-      bool ok = true;
-      for (; ok && items.next(idx); ++n) {
-        int bh, m0, nkv;
-        decode(idx, bh, m0, nkv);
-        const int slot = n & 1;
-        if (!mbar_wait(&ctl->qdo_full[slot], (n >> 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD); break; }
-        const uint64_t da = make_sdesc_sw128(smem_u32(sQdObig + (size_t)slot * 3 * kBigTile + (second ? kBigTile : 0)));
-        for (int j = 0; j < nkv; ++j, ++t) {
-          const uint32_t s = t % kStages, g = t % kBufs;
-          // the buffer pair still holds dS of tile t-kBufs until the gradient MMAs have read it
-          if (t >= kBufs && !mbar_wait(&ctl->buf_free[g], ((t / kBufs) - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; break; }
-          if (!mbar_wait(&ctl->kv_full[s], (t / kStages) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD); ok = false; break; }
-          fence_after_sync();
-          const uint64_t db = make_sdesc_sw128(smem_u32(sKV + (size_t)s * 2 * kSmallTile + (second ? kSmallTile : 0)));
-          const uint32_t t_dst = tmem_base + 128 * g + (second ? 64 : 0);
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) mma_ss(t_dst, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc_s, kk > 0);
-          mma_commit(&ctl->sdp_full[g]);
-        }
-        mma_commit(&ctl->qdo_free[slot]);                 // arrives once this thread's MMAs of the item have read Q (dO)
-      }
-    }
-  } else if (warp == kGradWarp) {
-    if (elect_one()) {                                     // gradient MMAs: dQ += dS_j K_j
       constexpr uint32_t idesc_q = make_idesc(Fmt<T>::v, BR, HD, 1);   // 128 x 64, B = K tile read MN-major
-      ItemIter items(n_items);
-      uint32_t t = 0;
-      int n = 0, idx;
-      bool ok = true;
-      for (; ok && items.next(idx); ++n) {
-        int bh, m0, nkv;
-        decode(idx, bh, m0, nkv);
-        // the accumulator still holds the previous item's dQ until its epilogue has read it
-        if (n >= 1 && !mbar_wait(&ctl->acc_free, (n - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); break; }
+      bool ok = mbar_wait(&ctl->qdo_full, 0, abort_flag);
+      if (!ok) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD);
+      const uint64_t dq = make_sdesc_sw128(smem_u32(sQ)), ddo = make_sdesc_sw128(smem_u32(sdO));
+      auto issue_scores = [&](int j) -> bool {             // S_j = Q K_j^T, dP_j = dO V_j^T
+        const int s = j % kStagesQ;
+        if (!mbar_wait(&ctl->kv_full[s], (j / kStagesQ) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD); return false; }
         fence_after_sync();
-        for (int j = 0; j < nkv; ++j, ++t) {
-          const uint32_t s = t % kStages, g = t % kBufs;
-          if (!mbar_wait(&ctl->ds_ready[g], (t / kBufs) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); ok = false; break; }
-          fence_after_sync();
-          const uint64_t dk = make_sdesc_sw128(smem_u32(sKV + (size_t)s * 2 * kSmallTile));
+        const uint64_t dk = make_sdesc_sw128(smem_u32(sKV + (size_t)s * 2 * kSmallTile)), dv = dk + (kSmallTile >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BT / 16; ++kk)           // 16 keys = 2048 bytes of K, 8 TMEM columns of dS
-            mma_ts(tmem_base + cQ, tmem_base + 128 * g + packed_col<kGW>(kk), dk + (uint64_t)(kk * (2048 >> 4)), idesc_q, (j > 0 || kk > 0) ? 1u : 0u);
-          mma_commit(&ctl->buf_free[g]);
-          mma_commit(&ctl->kv_empty[s]);
+        for (int kk = 0; kk < HD / 16; ++kk) mma_ss(tmem_base, dq + (uint64_t)(kk * 2), dk + (uint64_t)(kk * 2), idesc_s, kk > 0);
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; ++kk) mma_ss(tmem_base + kColDP, ddo + (uint64_t)(kk * 2), dv + (uint64_t)(kk * 2), idesc_s, kk > 0);
+        mma_commit(&ctl->sdp_full);
+        return true;
+      };
+      if (ok) ok = issue_scores(0);
+      for (int j = 0; ok && j < nkv; ++j) {
+        const int s = j % kStagesQ;
+        if (j + 1 < nkv) {                                 // the compute warps free S and dP long before they have this tile's dS
+          if (!mbar_wait(&ctl->sdp_free, j & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); break; }
+          if (!issue_scores(j + 1)) break;
         }
-        // the group that took the item's last tile runs its epilogue; one barrier per group, because a
-        // barrier's successive phases must be awaited by the same threads in order
-        if (ok) mma_commit(&ctl->dq_done[(t - 1) % kGroups]);
+        if (!mbar_wait(&ctl->ds_ready, j & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); break; }
+        fence_after_sync();
+        const uint64_t dk = make_sdesc_sw128(smem_u32(sKV + (size_t)s * 2 * kSmallTile));
+#pragma unroll
+        for (int kk = 0; kk < BT / 16; ++kk)               // 16 keys = 2048 bytes of K, 8 TMEM columns of dS
+          mma_ts(tmem_base + kColDQ, tmem_base + kColDS + (uint32_t)(kk * 8), dk + (uint64_t)(kk * (2048 >> 4)), idesc_q, (j > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(&ctl->dq_done);
+        mma_commit(&ctl->kv_empty[s]);
       }
     }
-  } else if (warp < kProducerWarp) {
-    const int g = warp / kGW;                            // compute group
-    const int r = ((warp & 3) << 5) | lane;              // query row within the tile == TMEM lane
-    const int my_half = (warp % kGW) >> 2;               // with two threads per row: which 32 of the tile's 64 columns
-    const bool poller = warp % kGW == 0;                 // the group's warp that polls barriers (group_wait)
-    const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+  } else {
+    // ------------------------------ compute warps -----------------------------
+    const int r = warp * 32 + lane;                      // query row within the tile == TMEM lane
+    const int grow = m0 + r;
+    const uint32_t t_row = tmem_base + ((uint32_t)(warp * 32) << 16);
+    const uint32_t seed_mix = (seed * 0x9E3779B1u) ^ (((uint32_t)bh + 1u) * 0x27D4EB2Fu);
     const float inv_keep = DROPOUT ? 1.f / (1.f - dropout_p) : 1.f;
-    ItemIter items(n_items);
-    uint32_t t0 = 0;                                     // tile counter at the start of the item
-    uint32_t epilogues = 0;                              // epilogues this group has run: the phase of its dq_done barrier
-    int n = 0, idx;
+    const float lse2 = grow < S ? LSE[(int64_t)bh * S + grow] * kLog2e : INFINITY;
     bool ok = true;
-    for (; ok && items.next(idx); ++n) {
-      int bh, m0, nkv;
-      decode(idx, bh, m0, nkv);
-      const int b = bh / H, h = bh - b * H;
-      const int grow = m0 + r;
-      const uint32_t seed_mix = (seed * 0x9E3779B1u) ^ (((uint32_t)bh + 1u) * 0x27D4EB2Fu);
-      const float lse2 = grow < S ? LSE[(int64_t)bh * S + grow] * kLog2e : INFINITY;
-      const int j_first = (int)((g + kGroups - t0 % kGroups) % kGroups);   // tile t belongs to group t % kGroups, counted over all items
-      float dlt = 0.f;
-      if (FUSE_DELTA) {
-        // Every compute thread awaits every item's load and then releases the slot (qdo_free counts all of
-        // them), whether its group has a tile in the item or not: the producer cannot refill a slot before
-        // the slowest group is past it, so no thread ever meets a barrier two phases ahead of the one it
-        // waits for (it would wait for the wrong one -- a deadlock seen with >3 short items per CTA).
-        if (!group_wait<kGW>(g, poller, &ctl->qdo_full[n & 1], (n >> 1) & 1, abort_flag, &ctl->fail_bits, ULM_STATUS_TIMEOUT_LOAD)) { ok = false; break; }
-        if (j_first < nkv) {
-          // row r of a 128-byte-swizzled tile: 16-byte chunk c sits at chunk position c ^ (r & 7)
-          const uint8_t* go = sQdObig + (size_t)(n & 1) * 3 * kBigTile + kBigTile + (size_t)r * 128;
-          const uint8_t* oo = go + kBigTile;
+    float dlt = 0.f;
+    if (FUSE_DELTA) {
+      ok = warp_wait(&ctl->qdo_full, 0, abort_flag);
+      if (!ok && lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD);
+      if (ok) {
+        // row r of a 128-byte-swizzled tile: 16-byte chunk c sits at chunk position c ^ (r & 7)
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const int off = (c ^ (r & 7)) << 4;
-            const uint4 gv = *reinterpret_cast<const uint4*>(go + off);
-            const uint4 ov = *reinterpret_cast<const uint4*>(oo + off);
-            const uint32_t* gw = reinterpret_cast<const uint32_t*>(&gv);
-            const uint32_t* ow = reinterpret_cast<const uint32_t*>(&ov);
+        for (int c = 0; c < 8; ++c) {
+          const int off = r * 128 + ((c ^ (r & 7)) << 4);
+          const uint4 gv = *reinterpret_cast<const uint4*>(sdO + off);
+          const uint4 ov = *reinterpret_cast<const uint4*>(sO + off);
+          const uint32_t* gw = reinterpret_cast<const uint32_t*>(&gv);
+          const uint32_t* ow = reinterpret_cast<const uint32_t*>(&ov);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float2 a2 = Cvt<T>::unpack2(ow[i]), g2 = Cvt<T>::unpack2(gw[i]);
-              dlt = fmaf(a2.x, g2.x, dlt);
-              dlt = fmaf(a2.y, g2.y, dlt);
-            }
+          for (int i = 0; i < 4; ++i) {
+            const float2 a2 = Cvt<T>::unpack2(ow[i]), g2 = Cvt<T>::unpack2(gw[i]);
+            dlt = fmaf(a2.x, g2.x, dlt);
+            dlt = fmaf(a2.y, g2.y, dlt);
           }
-          // the group that owns the item's first tile publishes delta for the dK/dV kernel
-          if (j_first == 0 && (kGW == 4 || my_half == 0) && grow < S) DELTA[(int64_t)bh * S + grow] = dlt;
         }
-        mbar_arrive(&ctl->qdo_free[n & 1]);
-      } else {
-        dlt = grow < S ? DELTA[(int64_t)bh * S + grow] : 0.f;
+        if (grow < S) DELTA[(int64_t)bh * S + grow] = dlt;
       }
-      [[maybe_unused]] const uint64_t sc2 = f2_pack(scale2, scale2), nl2 = f2_pack(-lse2, -lse2), nd2 = f2_pack(-dlt, -dlt);
-      for (int j = j_first; j < nkv; j += kGroups) {
-        const uint32_t t = t0 + (uint32_t)j;
-        const uint32_t bf = t % kBufs;
-        const uint32_t cS = 128 * bf, cP = 128 * bf + 64;
-        if (!group_wait<kGW>(g, poller, &ctl->sdp_full[bf], (t / kBufs) & 1, abort_flag, &ctl->fail_bits, ULM_STATUS_TIMEOUT_MMA)) { ok = false; break; }
-        fence_after_sync();
-        const int c0 = j * BT;
-        const bool edge = (CAUSAL && c0 + BT - 1 > m0) || (c0 + BT > S);
-        // The masked and the unmasked form of a tile are separate code: as one body the compiler predicates the
-        // mask's compare-and-select per element, and predicated-off instructions still take issue slots in the
-        // tiles that need no mask (all but one or two per item).
-        auto tile_body = [&](auto edge_c) {
+    } else {
+      dlt = grow < S ? DELTA[(int64_t)bh * S + grow] : 0.f;
+    }
+    [[maybe_unused]] const uint64_t sc2 = f2_pack(scale2, scale2), nl2 = f2_pack(-lse2, -lse2), nd2 = f2_pack(-dlt, -dlt);
+    for (int j = 0; ok && j < nkv; ++j) {
+      if (!warp_wait(&ctl->sdp_full, j & 1, abort_flag)) { if (lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; break; }
+      fence_after_sync();
+      uint32_t sv[2][32], pv[2][32], pk[32];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) { tmem_ld32(t_row + hf * 32, sv[hf]); tmem_ld32(t_row + kColDP + hf * 32, pv[hf]); }
+      tmem_wait_ld();
+      fence_before_sync();
+      warp_arrive(&ctl->sdp_free);                       // both are in registers: the next tile's may come
+      const int c0 = j * BT;
+      const int lim = (CAUSAL && grow < S ? grow : S - 1) - c0;   // last visible key of this row within the tile
+      // The masked and the unmasked form of a tile are separate code: as one body the compiler predicates the
+      // mask's compare-and-select per element, and predicated-off instructions still take issue slots in the
+      // tiles that need no mask (all but one or two per item).
+      auto tile_body = [&](auto edge_c) {
         constexpr bool EDGE = decltype(edge_c)::value;
-        if constexpr (kGW == 8) {
-          // two threads per row: this one takes columns [32 my_half, +32) in two chunks of 16 and packs dS
-          // over its own scores
-  #pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
-            uint32_t sv[16], pv[16], pk[8];
-            const int col0 = my_half * 32 + ch * 16;
-            tmem_ld16(t_row + cS + col0, sv);
-            tmem_ld16(t_row + cP + col0, pv);
-            tmem_wait_ld();
-  #pragma unroll
-            for (int c = 0; c < 16; c += 2) {
-              float d2[2];
-              if constexpr (!DROPOUT) {
-                pair_ds(sv[c], sv[c + 1], pv[c], pv[c + 1], sc2, nl2, nd2,
-                        [&](int e) { const int col = c0 + col0 + c + e; return !EDGE || ((col < S) && (!CAUSAL || col <= grow)); }, d2);
-              } else {
-  #pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int col = c0 + col0 + c + e;
-                float p = ex2(fmaf(__uint_as_float(sv[c + e]), scale2, -lse2));
-                if constexpr (EDGE) p = ((col < S) && (!CAUSAL || col <= grow)) ? p : 0.f;
-                float dp = __uint_as_float(pv[c + e]);
-                dp = dropout_keep(seed_mix, grow, col, dropout_p) ? dp * inv_keep : 0.f;
-                d2[e] = p * (dp - dlt);
-              }
-              }
-              pk[c >> 1] = Cvt<T>::pack2(d2[0], d2[1]);
-            }
-            st8(t_row + cS + my_half * 32 + ch * 8, pk);
-          }
-        } else {
-  #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t sv[32], pv[32], pk[16];
-          tmem_ld32(t_row + cS + hf * 32, sv);
-          tmem_ld32(t_row + cP + hf * 32, pv);
-          tmem_wait_ld();
-  #pragma unroll
-          for (int c = 0; c < 32; c += 2) {
-            float d2[2];
-            if constexpr (!DROPOUT) {
-              pair_ds(sv[c], sv[c + 1], pv[c], pv[c + 1], sc2, nl2, nd2,
-                      [&](int e) { const int col = c0 + hf * 32 + c + e; return !EDGE || ((col < S) && (!CAUSAL || col <= grow)); }, d2);
-            } else {
-  #pragma unroll
+#pragma unroll
+        for (int c = 0; c < BT; c += 2) {
+          float d2[2];
+          const uint32_t s0 = sv[c >> 5][c & 31], s1 = sv[c >> 5][(c & 31) + 1], g0 = pv[c >> 5][c & 31], g1 = pv[c >> 5][(c & 31) + 1];
+          if constexpr (!DROPOUT) {
+            pair_ds(s0, s1, g0, g1, sc2, nl2, nd2, [&](int e) { return !EDGE || c + e <= lim; }, d2);
+          } else {
+#pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int col = c0 + hf * 32 + c + e;
-              float p = ex2(fmaf(__uint_as_float(sv[c + e]), scale2, -lse2));
-              if constexpr (EDGE) p = ((col < S) && (!CAUSAL || col <= grow)) ? p : 0.f;
-              float dp = __uint_as_float(pv[c + e]);
-              dp = dropout_keep(seed_mix, grow, col, dropout_p) ? dp * inv_keep : 0.f;
+              float p = ex2(fmaf(__uint_as_float(e ? s1 : s0), scale2, -lse2));
+              if constexpr (EDGE) p = c + e <= lim ? p : 0.f;
+              float dp = __uint_as_float(e ? g1 : g0);
+              dp = dropout_keep(seed_mix, grow, c0 + c + e, dropout_p) ? dp * inv_keep : 0.f;
               d2[e] = p * (dp - dlt);
             }
-            }
-            pk[c >> 1] = Cvt<T>::pack2(d2[0], d2[1]);
           }
-          st16(t_row + cS + hf * 16, pk);   // packed dS columns [hf*16, hf*16+16)
+          pk[c >> 1] = Cvt<T>::pack2(d2[0], d2[1]);
         }
+      };
+      if ((CAUSAL && c0 + BT - 1 > m0 + warp * 32) || c0 + BT > S) tile_body(std::true_type{}); else tile_body(std::false_type{});
+      // dS_{j-1} must have been read; its MMAs were issued a tile ago
+      if (j > 0 && !warp_wait(&ctl->dq_done, (j - 1) & 1, abort_flag)) { if (lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; break; }
+      fence_after_sync();
+      tmem_st32(t_row + kColDS, pk);
+      tmem_wait_st();
+      fence_before_sync();
+      warp_arrive(&ctl->ds_ready);
+    }
+    // epilogue: the four warps go through it together or not at all (its staging tile is shared)
+    const int tg = (int)threadIdx.x;
+    [[maybe_unused]] RopeQuad tab[RopeTasks<4>::n];
+    if constexpr (ROPE) rope_prefetch_pass<4>(tab, rt, m0, 0, tg, S);   // ahead of the wait for the last gradient MMAs
+    if (ok && !warp_wait(&ctl->dq_done, (nkv - 1) & 1, abort_flag)) { if (lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; }
+    if (!group_any<4>(0, !ok)) {
+      fence_after_sync();
+      uint4 lo[4], hi[4];
+      acc_to_16bit<T>(t_row + kColDQ, scale, lo);
+      acc_to_16bit<T>(t_row + kColDQ + 32, scale, hi);
+      T* item_out = dQ + (int64_t)b * dq_sb + (int64_t)h * dq_sh + (int64_t)m0 * dq_ss;
+      if constexpr (ROPE) {
+        rope_adjoint_store<T, 4>(sQ, 0, tg, r, 0, lo, hi, item_out, dq_ss, m0, S, rt, tab);
+      } else {
+        // through this warp's rows of the Q tile, so that the stores are coalesced whatever the layout
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          *reinterpret_cast<uint4*>(sQ + r * 128 + ((c ^ (r & 7)) << 4)) = lo[c];
+          *reinterpret_cast<uint4*>(sQ + r * 128 + (((4 + c) ^ (r & 7)) << 4)) = hi[c];
         }
-        };
-        if (edge) tile_body(std::true_type{}); else tile_body(std::false_type{});
-        tmem_wait_st();
-        fence_before_sync();
-        mbar_arrive(&ctl->ds_ready[bf]);
-      }
-      t0 += (uint32_t)nkv;
-      if (!ok) break;
-      // The group that worked on the item's last tile runs the epilogue: its next tile reuses that tile's buffer
-      // pair, which is free no sooner than the item's last gradient MMA, so it has nothing else to do meanwhile.
-      if ((t0 - 1) % kGroups == (uint32_t)g) {
-        // Fused RoPE adjoint: the first pass's table values are fetched into registers BEFORE the wait for the
-        // last gradient MMA (the group has nothing else to do then), so their latency is off the path between
-        // "accumulator complete" and "accumulator released".
-        const int tg = (int)threadIdx.x - g * kGroupThreads;
-        [[maybe_unused]] RopeQuad tab[RopeTasks<kGW>::n];
-        if constexpr (ROPE) rope_prefetch_pass<kGW>(tab, rt, m0, 0, tg, S);
-        if (!group_wait<kGW>(g, poller, &ctl->dq_done[g], epilogues++ & 1, abort_flag, &ctl->fail_bits, ULM_STATUS_TIMEOUT_MMA)) { ok = false; break; }
-        fence_after_sync();
-        // read and round everything first, hand the accumulator back, rotate (ROPE) and store afterwards
-        T* item_out = dQ + (int64_t)b * dq_sb + (int64_t)h * dq_sh + (int64_t)m0 * dq_ss;
-        uint4 lo[4];
-        [[maybe_unused]] uint4 hi[4];
-        if constexpr (kGW == 4) {
-          acc_to_16bit<T>(t_row + cQ, scale, lo);
-          acc_to_16bit<T>(t_row + cQ + 32, scale, hi);
-        } else {
-          acc_to_16bit<T>(t_row + cQ + my_half * 32, scale, lo);
-        }
-        fence_before_sync();
-        mbar_arrive(&ctl->acc_free);
-        if constexpr (ROPE) {
-          rope_adjoint_store<T, kGW>(stage + (size_t)g * kRopeStageBytes, g, tg, r, my_half, lo, hi, item_out, dq_ss, m0, S, rt, tab);
-        } else if (grow < S) {
-          T* orow = item_out + (int64_t)r * dq_ss;
-          if constexpr (kGW == 4) { store_32<T>(orow, lo); store_32<T>(orow + 32, hi); }
-          else store_32<T>(orow + my_half * 32, lo);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = warp * 32 + i * 4 + (lane >> 3), c = lane & 7;
+          const uint4 u = *reinterpret_cast<const uint4*>(sQ + row * 128 + ((c ^ (row & 7)) << 4));
+          if (m0 + row < S) *reinterpret_cast<uint4*>(item_out + (int64_t)row * dq_ss + c * 8) = u;
         }
       }
     }
@@ -655,9 +570,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   fence_before_sync();
   __syncthreads();
-  if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
+  if (warp == 5) tmem_dealloc(tmem_base, kTmemColsQ);
   if (threadIdx.x == 0 && ctl->fail_bits && status) atomicOr(status, ctl->fail_bits);
 }
+
+constexpr size_t kCtlBytes = 4096;        // control block (barriers, per-tile statistics), padded so that what follows stays 128-byte aligned
+constexpr size_t kStageBytes = (size_t)kGroups * kRopeStageBytes;   // the dK/dV kernel's staging tiles
 
 // ---------------------------------------------------------------------------
 // dK / dV kernel
@@ -999,10 +917,9 @@ int launch_bwd(const ulm_attn_bwd_args* a, int device, const Maps& m) {
   const unsigned grid = items < (unsigned)sm_count() ? items : (unsigned)sm_count();
   if (a->mode & 2) {
     auto go = [&](auto kern, std::atomic<bool>* attr) -> int {
-      const size_t smem = kSmemQ + (ROPE ? kStageBytes : 0);
-      if (int r = ensure_smem_attr(kern, smem, device, attr, "ulm_attn_bwd(dq)")) return r;
-      kern<<<grid, Roles<kGWdQ>::kThreads, smem, st>>>(m.q128, m.k64, m.v64, m.do128, m.o128, a->lse, a->delta, (T*)a->dq,
-                                                          a->dq_sb, a->dq_sh, a->dq_ss, a->S, a->H, (int)BH, a->softmax_scale, scale2,
+      if (int r = ensure_smem_attr(kern, kSmemQ, device, attr, "ulm_attn_bwd(dq)")) return r;
+      kern<<<dim3(BH, nt), kThreadsQ, kSmemQ, st>>>(m.q128, m.k64, m.v64, m.do128, m.o128, a->lse, a->delta, (T*)a->dq,
+                                                          a->dq_sb, a->dq_sh, a->dq_ss, a->S, a->H, a->softmax_scale, scale2,
                                                           a->dropout_p, a->seed, a->status_dev, rt);
       return check_launch("ulm_attn_bwd(dq)");
     };
