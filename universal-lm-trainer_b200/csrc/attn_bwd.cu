@@ -17,18 +17,12 @@
 //   dK/dV kernel: CTA = 128 keys (thread r = key r), walks query tiles of 64 from
 //                the diagonal down, transposed view: S^T = K Q^T, dP^T = V dO^T,
 //                dV += P^T dO, dK += dS^T Q.
-// dK/dV kernel: one CTA per SM owns all 512 TMEM columns (the dQ kernel's CTAs share an SM, see there).  Streamed tiles are independent of
-// each other (the softmax statistics come from the forward pass), so tile t lives
-// in score buffer pair t % kBufs and is turned into P/dS by compute group
-// t % kGroups (kGW warps each).  MMAs are issued by single-purpose threads, one
-// warp each: one issues S, one dP, into a buffer pair as soon as it is free; one
-// issues the gradient MMAs out of it as soon as the group has written P/dS.  tcgen05.mma blocks its issuing thread while the tensor
-// pipe is busy, so a thread's barrier waits add to its MMAs' time; with one issuer
-// per operand stream those waits overlap the other issuers' MMAs (one thread for
-// everything left the pipe idle during every hand-off).  Each accumulator has exactly one issuer, so the
-// summation order, and with it the result, is the same on every run.  All barrier
-// waits are bounded (status bit + clean exit on expiry); the compute warps make the
-// outcome of a wait warp-uniform by a vote, because warp-wide TMEM loads follow.
+// In both a thread owns a row: it takes the tile's S and dP of its row into registers and releases their TMEM columns at
+// once, and P / dS go to columns of their own, so no tile waits for the round trip "P / dS written -> gradient MMAs -> columns
+// free -> scores".  Two warps of compute share a scheduler (two CTAs in the dQ kernel, two groups in the dK/dV kernel).  Each
+// accumulator has exactly one issuing thread, so the summation order, and with it the result, is the same on every run.  All
+// barrier waits are bounded (status bit + clean exit on expiry); the compute warps make the outcome of a wait warp-uniform
+// by a vote, because warp-wide TMEM loads follow.
 //
 // Fused RoPE adjoint (template parameter ROPE): q and k are the rotated tensors; the
 // dQ and dK epilogues round their result to 16 bits, hand the accumulator back, and
@@ -49,26 +43,18 @@ using namespace tc;
 constexpr int HD = 64;
 constexpr int BR = 128;                 // rows owned by a CTA (queries or keys)
 constexpr int BT = 64;                  // rows of the streamed tile
-constexpr int kBufs = 3;                // score buffer pairs in TMEM; tile t lives in pair t % kBufs
-constexpr int kGroups = 3;              // compute groups; tile t is worked on by group t % kGroups
-constexpr int kStages = 6;              // streamed-tile ring (must exceed kBufs)
-static_assert(128 * kBufs + 128 <= 512, "score buffer pairs and accumulators must fit 512 TMEM columns");
-static_assert(kBufs == kGroups, "a buffer pair's barriers are awaited by one group only: successive phases of an mbarrier must be awaited in order");
-// Warps per compute group: 4 (a thread per row of the tile) or 8 (two threads per row, 32 columns each).
-// A single warp issues about one instruction every two clocks on its dependent chains, so a second
-// warp per sub-partition nearly halves the time a group holds a tile; measured at B=8,H=12,S=4096:
-// the dK/dV kernel gains 8 % with 8.
-constexpr int kGWdKV = 8;
-// Single-thread roles, one warp each, after the compute warps: TMA producer, the S issuer, the dP issuer and
-// the gradient issuer (dK/dV kernel: dV and dK on one thread).
-template <int GW>
-struct Roles {
-  static_assert(GW == 4 || GW == 8, "a compute group is one or two warps per TMEM sub-partition");
-  static constexpr int kGroupThreads = 32 * GW;
-  static constexpr int kProducerWarp = GW * kGroups, kMmaWarp = kProducerWarp + 1, kMma2Warp = kProducerWarp + 2,
-                       kGradWarp = kProducerWarp + 3;
-  static constexpr int kThreads = kGroupThreads * kGroups + 4 * 32;
-};
+constexpr int kGroups = 2;              // dK/dV kernel: compute groups; tile t is worked on by group t % kGroups, in that group's TMEM columns
+constexpr int kGroupWarps = 4, kGroupThreads = 32 * kGroupWarps;   // a thread per row of the tile
+constexpr int kStages = 6;              // dK/dV kernel: streamed-tile ring
+static_assert(192 * kGroups + 128 <= 512, "score buffers, packed operands and accumulators must fit 512 TMEM columns");
+// The other roles of the dK/dV kernel, one warp each, after the compute warps: TMA producer, the S issuer, the dP issuer and the
+// gradient issuer (dV and dK); then the warpgroup that writes finished gradients out.
+constexpr int kProducerWarp = kGroupWarps * kGroups, kMmaWarp = kProducerWarp + 1, kMma2Warp = kProducerWarp + 2, kGradWarp = kProducerWarp + 3,
+              kStoreWarp = kProducerWarp + 4;
+constexpr int kThreadsKV = 32 * (kStoreWarp + 4);
+constexpr int kRegsCompute = 184, kRegsIssue = 56, kRegsStore = 88;   // per thread, by warpgroup
+static_assert(kGroups * kGroupThreads * kRegsCompute + 128 * (kRegsIssue + kRegsStore) <= 65536 / kThreadsKV / 8 * 8 * kThreadsKV,
+              "the register split must fit what the CTA is launched with");
 constexpr uint32_t kBigTile = BR * HD * 2;    // 16 KB
 constexpr uint32_t kSmallTile = BT * HD * 2;  //  8 KB
 constexpr uint32_t kTmemCols = 512;
@@ -87,14 +73,6 @@ __device__ __forceinline__ bool dropout_keep(uint32_t seed_mix, int row, int col
   return ((h >> 8) * (1.0f / 16777216.0f)) >= p;
 }
 
-// TMEM column (relative to the buffer) of the packed 16-bit A operand for k-step kk: 8 columns per 16
-// streamed rows.  With one thread per row the 64 rows pack into columns [0,32); with two threads per
-// row each half packs over its own scores, rows [0,32) into columns [0,16) and rows [32,64) into [32,48).
-template <int GW>
-__device__ __forceinline__ constexpr uint32_t packed_col(int kk) {
-  return GW == 8 ? (uint32_t)((kk >> 1) * 32 + (kk & 1) * 8) : (uint32_t)(kk * 8);
-}
-
 // dS of two neighbouring score elements without dropout, two-wide fp32 arithmetic (one issue slot per pair, same
 // rounding as the scalar operations): p = 2^(s*scale2 - lse2), dS = p * (dP - delta); nl and nd hold the NEGATED
 // statistics of the two elements.  keep(e) says whether element e is inside the mask.
@@ -103,7 +81,7 @@ __device__ __forceinline__ void pair_ds(uint32_t s0, uint32_t s1, uint32_t dp0, 
                                         Keep keep, float (&d)[2], float* p_out = nullptr) {
   float x0, x1;
   f2_unpack(f2_fma(f2_pack(__uint_as_float(s0), __uint_as_float(s1)), sc2, nl), x0, x1);
-  float p0 = ex2(x0), p1 = ex2(x1);
+  float p0 = ex2_ordered(x0), p1 = ex2_ordered(x1);
   p0 = keep(0) ? p0 : 0.f;
   p1 = keep(1) ? p1 : 0.f;
   if (p_out) { p_out[0] = p0; p_out[1] = p1; }
@@ -114,35 +92,8 @@ template <typename T> struct Fmt { static constexpr int v = 0; };
 template <> struct Fmt<__nv_bfloat16> { static constexpr int v = 1; };
 
 template <int GW>
-__device__ __forceinline__ void group_sync(int g) {      // the threads of compute group g
+__device__ __forceinline__ void group_sync(int g) {      // the 32 GW threads of group g
   asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(32 * GW) : "memory");
-}
-
-// A compute group's wait for an mbarrier.  One warp polls; the others block in the group's named barrier.  The
-// barrier's OR-reduction hands every thread of the group the same verdict, so a group leaves as a whole and no
-// warp is left behind in a later group barrier when a wait times out.  (Eight warps polling issued more than half
-// of the kernel's instructions; taking them away did not change the run time, so the polling was not what the
-// working groups were short of.)
-template <int GW>
-__device__ __forceinline__ bool group_wait(int g, bool poller, uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                           uint32_t* fail_bits, uint32_t bit) {
-  uint32_t fail = 0;
-  if (poller) {
-    if (!mbar_wait(bar, parity, abort_flag)) {
-      fail = 1;
-      if ((threadIdx.x & 31) == 0) atomicOr(fail_bits, bit);
-    } else if (*abort_flag) {
-      fail = 1;
-    }
-  }
-  uint32_t any;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.or.pred p, %2, %3, q;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(any) : "r"(fail), "r"(g + 1), "n"(32 * GW) : "memory");
-  return any == 0;
 }
 
 // All lanes of a warp learn together whether the wait succeeded.
@@ -151,7 +102,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
-// The threads of compute group g learn together whether any of them says yes.
+// The threads of group g learn together whether any of them says yes.
 template <int GW>
 __device__ __forceinline__ bool group_any(int g, bool yes) {
   uint32_t any;
@@ -162,6 +113,11 @@ __device__ __forceinline__ bool group_any(int g, bool yes) {
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(any) : "r"((uint32_t)yes), "r"(g + 1), "n"(32 * GW) : "memory");
   return any != 0;
+}
+
+// Four floats from shared memory, kept in program order with respect to other such calls and the exponentials
+__device__ __forceinline__ void lds_f4(const float* p, float* v) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(smem_u32(p)));
 }
 
 // Tables of the fused RoPE adjoint (unused when ROPE is false).
@@ -258,33 +214,26 @@ __device__ __forceinline__ void rope_adjoint_store(uint8_t* stage, int g, int tg
   }
 }
 
-// The plain store of a 128-row gradient tile of the dK/dV kernel, through the same staging tile: threads that wrote their
-// own halves of rows would spread every store instruction over 32 cache lines, and the group that runs an item's epilogue is
-// awaited by the next item's tiles.  Same box, row stores -> staged, with the next item's K and V requested earlier: dK/dV
-// kernel B8 H12 S4096 480 -> 474 us, B24 H12 S1363 231 -> 224 us, B64 H12 S300 76 -> 71 us.  (The dQ kernel, whose epilogue
-// group holds whole rows, gains nothing: 376 -> 381 us.)
+// The plain store of a gradient tile held one row per thread: each warp passes its 32 rows through 4 KB of its own, so that the
+// stores are coalesced whatever the layout (a thread that wrote its own row would spread every store instruction over 32 lines).
+constexpr uint32_t kWarpStageBytes = 32 * 128;
 template <typename T>
-__device__ __forceinline__ void staged_store(uint8_t* stage, int g, int tg, int r, int my_half, const uint4 (&v)[4], T* item_out,
+__device__ __forceinline__ void staged_store(uint8_t* stage, int lane, const uint4 (&lo)[4], const uint4 (&hi)[4], T* warp_out,
                                              int64_t row_stride, int rows) {
-  constexpr int GW = kGWdKV;
-#pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-    if ((r >> 6) == pass) {
-      const int rr = r & 63;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(stage + rr * 128 + (((my_half * 4 + c) ^ (rr & 7)) << 4)) = v[c];
-    }
-    group_sync<GW>(g);
-#pragma unroll
-    for (int j = 0; j < kRopeStageRows * 8 / (32 * GW); ++j) {
-      const int idx = j * 32 * GW + tg, rr = idx >> 3, c = idx & 7, row = kRopeStageRows * pass + rr;
-      const uint4 u = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((c ^ (rr & 7)) << 4));
-      if (row < rows) *reinterpret_cast<uint4*>(item_out + (int64_t)row * row_stride + c * 8) = u;
-    }
-    group_sync<GW>(g);                                    // the tile is rewritten by the next pass / the next epilogue
+  for (int c = 0; c < 4; ++c) {
+    *reinterpret_cast<uint4*>(stage + lane * 128 + ((c ^ (lane & 7)) << 4)) = lo[c];
+    *reinterpret_cast<uint4*>(stage + lane * 128 + (((4 + c) ^ (lane & 7)) << 4)) = hi[c];
   }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = i * 4 + (lane >> 3), c = lane & 7;
+    const uint4 u = *reinterpret_cast<const uint4*>(stage + row * 128 + ((c ^ (row & 7)) << 4));
+    if (row < rows) *reinterpret_cast<uint4*>(warp_out + (int64_t)row * row_stride + c * 8) = u;
+  }
+  __syncwarp();                                           // the rows are rewritten by the next store
 }
-static_assert(kGWdKV == 8, "staged_store: two threads per row");
 
 // ---------------------------------------------------------------------------
 // delta[bh, s] = sum_d O[s, d] * dO[s, d]   (fp32), 8 threads per row
@@ -324,7 +273,7 @@ attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO, float* __re
 // tile counter that keeps counting across items, so the producer prefetches the next item's resident
 // tiles (double-buffered) and first streamed tiles, and the S and dP issuers fill free score buffers
 // with them, while the last tiles of the current item are still being worked on.  Only the gradient
-// issuer pauses between items, until the epilogue group has read the accumulators out of TMEM.
+// issuer pauses between items, until the accumulators have been read out of TMEM.
 // ---------------------------------------------------------------------------
 // ---------------------------------------------------------------------------
 // dQ kernel
@@ -551,19 +500,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if constexpr (ROPE) {
         rope_adjoint_store<T, 4>(sQ, 0, tg, r, 0, lo, hi, item_out, dq_ss, m0, S, rt, tab);
       } else {
-        // through this warp's rows of the Q tile, so that the stores are coalesced whatever the layout
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          *reinterpret_cast<uint4*>(sQ + r * 128 + ((c ^ (r & 7)) << 4)) = lo[c];
-          *reinterpret_cast<uint4*>(sQ + r * 128 + (((4 + c) ^ (r & 7)) << 4)) = hi[c];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = warp * 32 + i * 4 + (lane >> 3), c = lane & 7;
-          const uint4 u = *reinterpret_cast<const uint4*>(sQ + row * 128 + ((c ^ (row & 7)) << 4));
-          if (m0 + row < S) *reinterpret_cast<uint4*>(item_out + (int64_t)row * dq_ss + c * 8) = u;
-        }
+        staged_store<T>(sQ + warp * kWarpStageBytes, lane, lo, hi, item_out + (int64_t)(warp * 32) * dq_ss, dq_ss, S - m0 - warp * 32);
       }
     }
   }
@@ -574,31 +511,39 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (threadIdx.x == 0 && ctl->fail_bits && status) atomicOr(status, ctl->fail_bits);
 }
 
-constexpr size_t kCtlBytes = 4096;        // control block (barriers, per-tile statistics), padded so that what follows stays 128-byte aligned
-constexpr size_t kStageBytes = (size_t)kGroups * kRopeStageBytes;   // the dK/dV kernel's staging tiles
-
 // ---------------------------------------------------------------------------
 // dK / dV kernel
 // A work item is one (batch*head, key tile of 128); key tile 0 meets the most query tiles under the
 // causal mask, so items are numbered by key tile, ascending.
-// TMEM columns: buffer pair b holds S^T at 128b and dP^T at 128b+64 (P^T and dS^T
-// are packed over them); the dV and dK accumulators sit at 128*kBufs and +64, so
-// kBufs = 3 uses all 512 columns.
+// Two compute groups of four warps take alternate query tiles, each in TMEM columns of its own.  A compute thread owns a key row: it
+// takes the 64 + 64 values of its row into registers and hands both buffers back at once, so the group's next S^T and dP^T are there
+// when it has written this tile's P^T and dS^T, into columns that the gradient MMAs of its previous tile have long read.
+// Finished gradients leave through a warpgroup of its own: done by a compute group, the 6,500 clk between an item's last gradient
+// MMA and its stores held up the tiles of the next item, 12 % of the kernel's time at S = 4096.
+// What bounds it: 1,330 of a group's 1,900 clk per tile are arithmetic (issue slots and the SFU, shared with the other
+// group), the rest synchronisation whose instructions queue behind the exponentials.  Against three groups of eight warps over three
+// score buffer pairs, P and dS packed over the scores (us, start -> now): B8 H12 S4096 bf16 475 -> 446, B24 H12 S1363 fp16
+// 222 -> 200, B64 H12 S300 68 -> 61, B1 H16 S4096 84 -> 76, B4 H12 S201 8.8 -> 8.7, B1 H12 S67 6.7 -> 6.9.  The groups taking
+// strict turns with their exponentials: 489 (turns of 1,000 clk each leave no more than they give).
 // ---------------------------------------------------------------------------
 struct CtlKV {
-  uint64_t kv_full[2], kv_free[2], qdo_full[kStages], qdo_empty[kStages], sdp_full[kBufs], pds_ready[kBufs], buf_free[kBufs],
-      dkv_done[kGroups], acc_free;
+  uint64_t kv_full[2], kv_free[2], qdo_full[kStages], qdo_empty[kStages], sdp_full[kGroups], sdp_free[kGroups], pds_ready[kGroups],
+      grad_done[kGroups], dkv_done, acc_free;
   uint32_t tmem_base;
   int abort;
   uint32_t fail_bits;
-  alignas(16) float lse2[kGroups][BT];   // per-query statistics of each group's current tile (read as float4)
-  alignas(16) float dlt[kGroups][BT];
+  alignas(16) float stat[kStages][2][BT];   // per-query statistics of each streamed tile: -lse in log2 units, -delta (read as float4)
 };
+constexpr size_t kCtlBytes = 4096;        // padded so that what follows stays 128-byte aligned
 static_assert(sizeof(CtlKV) <= kCtlBytes, "control block");
-constexpr size_t kSmemKV = 1024 + 4 * (size_t)kBigTile + (size_t)kStages * 2 * kSmallTile + kCtlBytes + kStageBytes;
+constexpr uint32_t kGroupStageBytes = 4 * kWarpStageBytes;   // staging tile of the storing warps: 32 rows each, or a RoPE pass
+static_assert(kGroupStageBytes >= kRopeStageBytes, "the RoPE adjoint's pass fits the staging tile");
+constexpr size_t kSmemKV = 1024 + 4 * (size_t)kBigTile + (size_t)kStages * 2 * kSmallTile + kCtlBytes + kGroupStageBytes;
+constexpr uint32_t kColG = 192;           // columns of a group: S^T at 0, dP^T at 64, packed P^T at 128, packed dS^T at 160
+constexpr uint32_t kColV = kColG * kGroups, kColK = kColV + 64;
 
 template <typename T, bool CAUSAL, bool DROPOUT, bool ROPE>
-__global__ void __launch_bounds__(Roles<kGWdKV>::kThreads, 1)
+__global__ void __launch_bounds__(kThreadsKV, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                     const float* __restrict__ LSE, const float* __restrict__ DELTA,
@@ -606,16 +551,12 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     int64_t dk_sb, int64_t dk_sh, int64_t dk_ss, int64_t dv_sb, int64_t dv_sh, int64_t dv_ss,
                     int S, int H, int BH, float scale, float scale2, float dropout_p, uint32_t seed, uint32_t* status,
                     const RopeTab rt) {
-  constexpr int kGW = kGWdKV;
-  using R = Roles<kGW>;
-  [[maybe_unused]] constexpr int kGroupThreads = R::kGroupThreads, kProducerWarp = R::kProducerWarp, kMmaWarp = R::kMmaWarp,
-                kMma2Warp = R::kMma2Warp, kGradWarp = R::kGradWarp;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sKVbig = base;                                 // [slot][K|V], 16 KB each; item n uses slot n & 1
   uint8_t* sQdO = base + 4 * kBigTile;                    // [stage][Q|dO], 8 KB each
   CtlKV* ctl = reinterpret_cast<CtlKV*>(sQdO + (size_t)kStages * 2 * kSmallTile);
-  uint8_t* stage = reinterpret_cast<uint8_t*>(ctl) + kCtlBytes;   // kGroups staging tiles
+  uint8_t* stage = reinterpret_cast<uint8_t*>(ctl) + kCtlBytes;   // the storing warps' staging tile
   volatile int* abort_flag = &ctl->abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -632,10 +573,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&ctl->kv_full[i], 1); mbar_init(&ctl->kv_free[i], 2); }
-    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->qdo_full[s], 1); mbar_init(&ctl->qdo_empty[s], 1); }
-    for (int g = 0; g < kBufs; ++g) { mbar_init(&ctl->sdp_full[g], 2); mbar_init(&ctl->pds_ready[g], kGroupThreads); mbar_init(&ctl->buf_free[g], 1); }
-    for (int g = 0; g < kGroups; ++g) mbar_init(&ctl->dkv_done[g], 1);
-    mbar_init(&ctl->acc_free, kGroupThreads);
+    for (int s = 0; s < kStages; ++s) { mbar_init(&ctl->qdo_full[s], 2); mbar_init(&ctl->qdo_empty[s], 1); }
+    for (int g = 0; g < kGroups; ++g) {
+      mbar_init(&ctl->sdp_full[g], 2); mbar_init(&ctl->sdp_free[g], kGroupWarps); mbar_init(&ctl->pds_ready[g], kGroupWarps);
+      mbar_init(&ctl->grad_done[g], 1);
+    }
+    mbar_init(&ctl->dkv_done, 1);
+    mbar_init(&ctl->acc_free, 4);
     ctl->abort = 0;
     ctl->fail_bits = 0;
     fence_mbar_init();
@@ -645,61 +589,124 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, ctl->tmem_base, 0);   // warp-uniform
-  constexpr uint32_t cV = 128 * kBufs, cK = 128 * kBufs + 64;
 
+  if (warp >= kStoreWarp) {
+    // ------------------------------ gradients out -----------------------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsStore));
+    const int sub = warp & 3, tg = (int)threadIdx.x & 127;
+    const int r = tg;                                     // key row within the tile == TMEM lane
+    const uint32_t t_row = tmem_base + ((uint32_t)(sub * 32) << 16);
+    uint8_t* w_stage = stage + sub * kWarpStageBytes;
+    ItemIter items(n_items);
+    int idx;
+    for (int n = 0; items.next(idx); ++n) {
+      int bh, n0, i_begin, nq;
+      decode(idx, bh, n0, i_begin, nq);
+      const int b = bh / H, h = bh - b * H;
+      // Fused RoPE adjoint on dK: the first pass's table values are fetched BEFORE the wait for the last gradient MMAs.
+      [[maybe_unused]] RopeQuad tab[RopeTasks<4>::n];
+      if constexpr (ROPE) rope_prefetch_pass<4>(tab, rt, n0, 0, tg, S);
+      const bool ok = warp_wait(&ctl->dkv_done, n & 1, abort_flag);
+      if (!ok && lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA);
+      if (group_any<4>(0, !ok)) break;                    // the four warps leave together: their staging tile is shared
+      fence_after_sync();
+      // read and round everything first, hand the accumulators back, rotate dK (ROPE) and store afterwards
+      T* v_item = dV + (int64_t)b * dv_sb + (int64_t)h * dv_sh + (int64_t)n0 * dv_ss;
+      T* k_item = dK + (int64_t)b * dk_sb + (int64_t)h * dk_sh + (int64_t)n0 * dk_ss;
+      uint4 vlo[4], vhi[4], klo[4], khi[4];
+      acc_to_16bit<T>(t_row + kColV, 1.f, vlo);
+      acc_to_16bit<T>(t_row + kColV + 32, 1.f, vhi);
+      acc_to_16bit<T>(t_row + kColK, scale, klo);
+      acc_to_16bit<T>(t_row + kColK + 32, scale, khi);
+      fence_before_sync();
+      warp_arrive(&ctl->acc_free);
+      const int w0 = sub * 32;
+      staged_store<T>(w_stage, lane, vlo, vhi, v_item + (int64_t)w0 * dv_ss, dv_ss, S - n0 - w0);
+      if constexpr (ROPE) {
+        group_sync<4>(0);                                 // the staging tile changes from a warp's to the group's
+        rope_adjoint_store<T, 4>(stage, 0, tg, r, 0, klo, khi, k_item, dk_ss, n0, S, rt, tab);
+      } else {
+        staged_store<T>(w_stage, lane, klo, khi, k_item + (int64_t)w0 * dk_ss, dk_ss, S - n0 - w0);
+      }
+    }
+  } else if (warp >= kProducerWarp) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
   if (warp == kProducerWarp) {
-    if (elect_one()) {
-      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
-      ItemIter items(n_items);
-      uint32_t t = 0;                                     // tiles issued so far, over all items
-      int idx, idx_next, n_loaded = 0;                    // n_loaded: items whose K/V loads were issued
-      auto load_item = [&](int item) -> bool {
-        int bh, n0, i_begin, nq;
-        decode(item, bh, n0, i_begin, nq);
-        const int b = bh / H, h = bh - b * H, slot = n_loaded & 1;
-        // the slot's previous K/V (two items ago) must have been read by the last S and dP MMAs of that item
-        if (n_loaded >= 2 && !mbar_wait(&ctl->kv_free[slot], ((n_loaded >> 1) - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); return false; }
+    // The whole warp: one lane issues the copies, all of them bring the tiles' statistics (4-byte values at any offset, which TMA does
+    // not take), fetched a tile ahead of the slot they go to.
+    const bool leader = elect_one();
+    if (leader) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO); }
+    ItemIter items(n_items);
+    uint32_t t = 0;                                       // tiles issued so far, over all items
+    int idx, idx_next, n_loaded = 0;                      // n_loaded: items whose K/V loads were issued
+    auto load_item = [&](int item) -> bool {
+      int bh, n0, i_begin, nq;
+      decode(item, bh, n0, i_begin, nq);
+      const int b = bh / H, h = bh - b * H, slot = n_loaded & 1;
+      // the slot's previous K/V (two items ago) must have been read by the last S and dP MMAs of that item
+      if (n_loaded >= 2 && !warp_wait(&ctl->kv_free[slot], ((n_loaded >> 1) - 1) & 1, abort_flag)) { if (leader) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); return false; }
+      if (leader) {
         uint8_t* big = sKVbig + (size_t)slot * 2 * kBigTile;
         mbar_expect_tx(&ctl->kv_full[slot], 2 * kBigTile);
         tma_load_4d(big, &tmK, &ctl->kv_full[slot], 0, n0, h, b);
         tma_load_4d(big + kBigTile, &tmV, &ctl->kv_full[slot], 0, n0, h, b);
-        ++n_loaded;
-        return true;
+      }
+      ++n_loaded;
+      return true;
+    };
+    bool have = items.next(idx);
+    bool ok = have && load_item(idx);
+    for (; ok && have; idx = idx_next) {
+      int bh, n0, i_begin, nq;
+      decode(idx, bh, n0, i_begin, nq);
+      const int b = bh / H, h = bh - b * H;
+      have = items.next(idx_next);
+      float f_lse[BT / 32], f_dlt[BT / 32];
+      auto fetch_stats = [&](int it) {
+#pragma unroll
+        for (int e = 0; e < BT / 32; ++e) {
+          const int q = (i_begin + it) * BT + 32 * e + lane, qc = q < S ? q : S - 1;
+          f_lse[e] = LSE[(int64_t)bh * S + qc];
+          f_dlt[e] = DELTA[(int64_t)bh * S + qc];
+        }
       };
-      bool have = items.next(idx);
-      bool ok = have && load_item(idx);
-      for (; ok && have; idx = idx_next) {
-        int bh, n0, i_begin, nq;
-        decode(idx, bh, n0, i_begin, nq);
-        const int b = bh / H, h = bh - b * H;
-        have = items.next(idx_next);
-        for (int it = 0; it < nq; ++it, ++t) {
-          const uint32_t s = t % kStages;
-          if (t >= kStages && !mbar_wait(&ctl->qdo_empty[s], ((t / kStages) - 1) & 1, abort_flag)) {
-            atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA);
-            ok = false;
-            break;
-          }
+      fetch_stats(0);
+      for (int it = 0; it < nq; ++it, ++t) {
+        const uint32_t s = t % kStages;
+        if (t >= kStages && !warp_wait(&ctl->qdo_empty[s], ((t / kStages) - 1) & 1, abort_flag)) {
+          if (leader) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA);
+          ok = false;
+          break;
+        }
+        if (leader) {
           uint8_t* dst = sQdO + (size_t)s * 2 * kSmallTile;
           mbar_expect_tx(&ctl->qdo_full[s], 2 * kSmallTile);
           tma_load_4d(dst, &tmQ, &ctl->qdo_full[s], 0, (i_begin + it) * BT, h, b);
           tma_load_4d(dst + kSmallTile, &tmdO, &ctl->qdo_full[s], 0, (i_begin + it) * BT, h, b);
-          // the next item's resident tiles are requested behind the third tile of this one: the previous item is done with
-          // their slot by then
-          if (have && it == (nq > 3 ? 2 : nq - 1) && !load_item(idx_next)) { ok = false; ++t; break; }
         }
+#pragma unroll
+        for (int e = 0; e < BT / 32; ++e) {
+          const bool in = (i_begin + it) * BT + 32 * e + lane < S;
+          ctl->stat[s][0][32 * e + lane] = in ? -(f_lse[e] * kLog2e) : -INFINITY;
+          ctl->stat[s][1][32 * e + lane] = in ? -f_dlt[e] : 0.f;
+        }
+        warp_arrive(&ctl->qdo_full[s]);
+        if (it + 1 < nq) fetch_stats(it + 1);
+        // the next item's resident tiles are requested behind the third tile of this one: the previous item is done with
+        // their slot by then
+        if (have && it == (nq > 3 ? 2 : nq - 1) && !load_item(idx_next)) { ok = false; ++t; break; }
       }
-      if (*abort_flag) {   // let our own copies land before the CTA's shared memory goes away
-        for (int m = n_loaded > 2 ? n_loaded - 2 : 0; m < n_loaded; ++m) {
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try(&ctl->kv_full[m & 1], (m >> 1) & 1))
-            if (globaltimer_ns() - t0 > kWaitLimitNs) break;
-        }
-        for (uint32_t u = t > (uint32_t)kStages ? t - kStages : 0; u < t; ++u) {
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try(&ctl->qdo_full[u % kStages], (u / kStages) & 1))
-            if (globaltimer_ns() - t0 > kWaitLimitNs) break;
-        }
+    }
+    if (*abort_flag && leader) {   // let our own copies land before the CTA's shared memory goes away
+      for (int m = n_loaded > 2 ? n_loaded - 2 : 0; m < n_loaded; ++m) {
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try(&ctl->kv_full[m & 1], (m >> 1) & 1))
+          if (globaltimer_ns() - t0 > kWaitLimitNs) break;
+      }
+      for (uint32_t u = t > (uint32_t)kStages ? t - kStages : 0; u < t; ++u) {
+        const uint64_t t0 = globaltimer_ns();
+        while (!mbar_try(&ctl->qdo_full[u % kStages], (u / kStages) & 1))
+          if (globaltimer_ns() - t0 > kWaitLimitNs) break;
       }
     }
   } else if (warp == kMmaWarp || warp == kMma2Warp) {
@@ -717,13 +724,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (!mbar_wait(&ctl->kv_full[slot], (n >> 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD); break; }
         const uint64_t da = make_sdesc_sw128(smem_u32(sKVbig + (size_t)slot * 2 * kBigTile + (second ? kBigTile : 0)));
         for (int it = 0; it < nq; ++it, ++t) {
-          const uint32_t s = t % kStages, g = t % kBufs;
-          // the buffer pair still holds P/dS of tile t-kBufs until the gradient MMAs have read it
-          if (t >= kBufs && !mbar_wait(&ctl->buf_free[g], ((t / kBufs) - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; break; }
+          const uint32_t s = t % kStages, g = t % kGroups;
+          // the group has the values of its previous tile in registers
+          if (t >= kGroups && !mbar_wait(&ctl->sdp_free[g], ((t / kGroups) - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); ok = false; break; }
           if (!mbar_wait(&ctl->qdo_full[s], (t / kStages) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_LOAD); ok = false; break; }
           fence_after_sync();
           const uint64_t db = make_sdesc_sw128(smem_u32(sQdO + (size_t)s * 2 * kSmallTile + (second ? kSmallTile : 0)));
-          const uint32_t t_dst = tmem_base + 128 * g + (second ? 64 : 0);
+          const uint32_t t_dst = tmem_base + kColG * g + (second ? 64 : 0);
 #pragma unroll
           for (int kk = 0; kk < HD / 16; ++kk) mma_ss(t_dst, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc_s, kk > 0);
           mma_commit(&ctl->sdp_full[g]);
@@ -745,137 +752,119 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (n >= 1 && !mbar_wait(&ctl->acc_free, (n - 1) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); break; }
         fence_after_sync();
         for (int it = 0; it < nq; ++it, ++t) {
-          const uint32_t s = t % kStages, g = t % kBufs;
-          if (!mbar_wait(&ctl->pds_ready[g], (t / kBufs) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); ok = false; break; }
+          const uint32_t s = t % kStages, g = t % kGroups;
+          if (!mbar_wait(&ctl->pds_ready[g], (t / kGroups) & 1, abort_flag)) { atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_SOFTMAX); ok = false; break; }
           fence_after_sync();
 #pragma unroll
           for (int w = 0; w < 2; ++w) {
-            // dV reads P^T (packed over S^T) against the dO tile; dK reads dS^T (packed over dP^T) against the Q tile
+            // dV reads P^T against the dO tile; dK reads dS^T against the Q tile
             const bool sec = w == 1;
             const uint64_t db = make_sdesc_sw128(smem_u32(sQdO + (size_t)s * 2 * kSmallTile + (sec ? 0 : kSmallTile)));
-            const uint32_t t_acc = tmem_base + (sec ? cK : cV), t_a = tmem_base + 128 * g + (sec ? 64 : 0);
+            const uint32_t t_acc = tmem_base + (sec ? kColK : kColV), t_a = tmem_base + kColG * g + (sec ? 160 : 128);
 #pragma unroll
             for (int kk = 0; kk < BT / 16; ++kk)
-              mma_ts(t_acc, t_a + packed_col<kGW>(kk), db + (uint64_t)(kk * (2048 >> 4)), idesc_a, (it > 0 || kk > 0) ? 1u : 0u);
+              mma_ts(t_acc, t_a + (uint32_t)(kk * 8), db + (uint64_t)(kk * (2048 >> 4)), idesc_a, (it > 0 || kk > 0) ? 1u : 0u);
           }
-          mma_commit(&ctl->buf_free[g]);
+          mma_commit(&ctl->grad_done[g]);
           mma_commit(&ctl->qdo_empty[s]);
         }
-        // the group that took the item's last tile runs its epilogue (see there); one barrier per group, because a
-        // barrier's successive phases must be awaited by the same threads in order
-        if (ok) mma_commit(&ctl->dkv_done[(t - 1) % kGroups]);
+        if (ok) mma_commit(&ctl->dkv_done);
       }
     }
-  } else if (warp < kProducerWarp) {
-    const int g = warp / kGW;
-    const int r = ((warp & 3) << 5) | lane;               // key row within the tile == TMEM lane
-    const int tg = (int)threadIdx.x - g * kGroupThreads;  // thread index within the group
-    const int my_half = (warp % kGW) >> 2;                // with two threads per row: which 32 of the tile's 64 columns
-    const bool poller = warp % kGW == 0;                  // the group's warp that polls barriers (group_wait)
-    const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCompute));
+    const int g = warp / kGroupWarps;
+    const int sub = warp & 3;                             // TMEM sub-partition = scheduler
+    const int r = sub * 32 + lane;                        // key row within the tile == TMEM lane
+    const uint32_t t_grp = tmem_base + ((uint32_t)(sub * 32) << 16) + kColG * g;
     [[maybe_unused]] const uint64_t sc2 = f2_pack(scale2, scale2);
     const float inv_keep = DROPOUT ? 1.f / (1.f - dropout_p) : 1.f;
     ItemIter items(n_items);
     uint32_t t0 = 0;                                      // tile counter at the start of the item
-    uint32_t epilogues = 0;                               // epilogues this group has run: the phase of its dkv_done barrier
-    int n = 0, idx;
+    uint32_t mine = 0;                                    // tiles this group has worked on: the phase of its barriers
+    int idx;
     bool ok = true;
-    for (; ok && items.next(idx); ++n) {
+    while (ok && items.next(idx)) {
       int bh, n0, i_begin, nq;
       decode(idx, bh, n0, i_begin, nq);
-      const int b = bh / H, h = bh - b * H;
       const int kc = n0 + r;                              // this thread's key
       const uint32_t seed_mix = (seed * 0x9E3779B1u) ^ (((uint32_t)bh + 1u) * 0x27D4EB2Fu);
       // tile t belongs to group t % kGroups, counted over all items
-      for (int it = (int)((g + kGroups - t0 % kGroups) % kGroups); it < nq; it += kGroups) {
-        const uint32_t t = t0 + (uint32_t)it;
+      for (int it = (int)((g + kGroups - t0 % kGroups) % kGroups); it < nq; it += kGroups, ++mine) {
         const int i0 = (i_begin + it) * BT;
-        const uint32_t bf = t % kBufs;
-        const uint32_t cS = 128 * bf, cP = 128 * bf + 64;
-        {   // per-query softmax statistics of this tile, shared by the group's key rows
-          const int c = tg & (BT - 1);
-          const int q = i0 + c;
-          group_sync<kGW>(g);                                  // everyone is done with the previous tile's values
-          if (tg < BT) ctl->lse2[g][c] = q < S ? -(LSE[(int64_t)bh * S + q] * kLog2e) : -INFINITY;   // both stored negated
-          else if (tg < 2 * BT) ctl->dlt[g][c] = q < S ? -DELTA[(int64_t)bh * S + q] : 0.f;
-        }
-        // the group barrier inside the wait also publishes the statistics
-        if (!group_wait<kGW>(g, poller, &ctl->sdp_full[bf], (t / kBufs) & 1, abort_flag, &ctl->fail_bits, ULM_STATUS_TIMEOUT_MMA)) { ok = false; break; }
+        const float* w_lse = ctl->stat[(t0 + (uint32_t)it) % kStages][0];
+        const float* w_dlt = w_lse + BT;
+        if (!warp_wait(&ctl->sdp_full[g], mine & 1, abort_flag)) { if (lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; break; }
         fence_after_sync();
-        const bool edge = CAUSAL && (i0 < n0 + BR - 1);   // some query of the tile precedes some key of the CTA
-        auto tile_body = [&](auto edge_c) {                // masked / unmasked tiles as separate code (see the dQ kernel)
-        constexpr bool EDGE = decltype(edge_c)::value;
+        // The statistics are read two chunks of queries ahead of their use: a shared-memory load queues behind the
+        // exponentials that were issued before it.
+        constexpr int kStat = 4;
+        float st[3][2 * kStat];
+        auto load_stats = [&](int cc) {
 #pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-          uint32_t sv[16], pv[16], pp[8], pd[8];
-          const int col0 = my_half * 32 + ch * 16;
-          tmem_ld16(t_row + cS + col0, sv);
-          tmem_ld16(t_row + cP + col0, pv);
-          tmem_wait_ld();
-          float l4[4], d4[4];                            // statistics of 4 queries per 16-byte shared load
-#pragma unroll
-          for (int c = 0; c < 16; c += 2) {
-            float p2[2], d2[2];
-            if ((c & 3) == 0) {
-              *reinterpret_cast<float4*>(l4) = *reinterpret_cast<const float4*>(&ctl->lse2[g][col0 + c]);
-              *reinterpret_cast<float4*>(d4) = *reinterpret_cast<const float4*>(&ctl->dlt[g][col0 + c]);
-            }
-#pragma unroll
-            if constexpr (!DROPOUT) {
-              pair_ds(sv[c], sv[c + 1], pv[c], pv[c + 1], sc2, f2_pack(l4[c & 3], l4[(c + 1) & 3]), f2_pack(d4[c & 3], d4[(c + 1) & 3]),
-                      [&](int e) { return !EDGE || (i0 + col0 + c + e >= kc); }, d2, p2);
-            } else {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int q = i0 + col0 + c + e;
-              float p = ex2(fmaf(__uint_as_float(sv[c + e]), scale2, l4[(c + e) & 3]));
-              if constexpr (EDGE) p = (q >= kc) ? p : 0.f;
-              float dp = __uint_as_float(pv[c + e]);
-              const bool keep = dropout_keep(seed_mix, q, kc, dropout_p);
-              p2[e] = keep ? p * inv_keep : 0.f;
-              dp = keep ? dp * inv_keep : 0.f;
-              d2[e] = p * (dp + d4[(c + e) & 3]);
-            }
-            }
-            pp[c >> 1] = Cvt<T>::pack2(p2[0], p2[1]);
-            pd[c >> 1] = Cvt<T>::pack2(d2[0], d2[1]);
+          for (int v = 0; v < kStat; v += 4) {
+            lds_f4(w_lse + cc * kStat + v, st[cc % 3] + v);
+            lds_f4(w_dlt + cc * kStat + v, st[cc % 3] + kStat + v);
           }
-          st8(t_row + cS + my_half * 32 + ch * 8, pp);
-          st8(t_row + cP + my_half * 32 + ch * 8, pd);
-        }
         };
-        if (edge) tile_body(std::true_type{}); else tile_body(std::false_type{});
+        uint32_t sv[2][32], pv[2][32], pp[16], pd[16];
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) { tmem_ld32(t_grp + hf * 32, sv[hf]); tmem_ld32(t_grp + 64 + hf * 32, pv[hf]); }
+        load_stats(0);
+        load_stats(1);
+        tmem_wait_ld();
+        fence_before_sync();
+        warp_arrive(&ctl->sdp_free[g]);                   // both are in registers: the group's next tile may come
+        const int first = kc - i0;                        // the first query of the tile that sees this key
+        auto tile_body = [&](auto edge_c) {                // masked / unmasked tiles as separate code (see the dQ kernel)
+          constexpr bool EDGE = decltype(edge_c)::value;
+#pragma unroll
+          for (int cc = 0; cc < BT / kStat; ++cc) {
+            if (cc + 2 < BT / kStat) load_stats(cc + 2);
+            const float* l8 = st[cc % 3];
+            const float* d8 = st[cc % 3] + kStat;
+#pragma unroll
+            for (int i = 0; i < kStat; i += 2) {
+              const int c = cc * kStat + i;
+              float p2[2], d2[2];
+              const uint32_t s0 = sv[c >> 5][c & 31], s1 = sv[c >> 5][(c & 31) + 1], g0 = pv[c >> 5][c & 31], g1 = pv[c >> 5][(c & 31) + 1];
+              if constexpr (!DROPOUT) {
+                pair_ds(s0, s1, g0, g1, sc2, f2_pack(l8[i], l8[i + 1]), f2_pack(d8[i], d8[i + 1]),
+                        [&](int e) { return !EDGE || c + e >= first; }, d2, p2);
+              } else {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                  float p = ex2(fmaf(__uint_as_float(e ? s1 : s0), scale2, l8[i + e]));
+                  if constexpr (EDGE) p = c + e >= first ? p : 0.f;
+                  float dp = __uint_as_float(e ? g1 : g0);
+                  const bool keep = dropout_keep(seed_mix, i0 + c + e, kc, dropout_p);
+                  p2[e] = keep ? p * inv_keep : 0.f;
+                  dp = keep ? dp * inv_keep : 0.f;
+                  d2[e] = p * (dp + d8[i + e]);
+                }
+              }
+              pp[(c >> 1) & 15] = Cvt<T>::pack2(p2[0], p2[1]);
+              pd[(c >> 1) & 15] = Cvt<T>::pack2(d2[0], d2[1]);
+            }
+            if (cc == BT / kStat / 2 - 1) {
+              // the group's previous P^T and dS^T must have been read; their MMAs were issued a tile ago
+              if (mine > 0 && !warp_wait(&ctl->grad_done[g], (mine - 1) & 1, abort_flag)) { if (lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; }
+              fence_after_sync();
+              st16(t_grp + 128, pp);
+              st16(t_grp + 160, pd);
+            }
+          }
+          st16(t_grp + 144, pp);
+          st16(t_grp + 176, pd);
+        };
+        if (CAUSAL && i0 < n0 + sub * 32 + 31) tile_body(std::true_type{}); else tile_body(std::false_type{});   // some query of the tile precedes some key of the warp
+        if (!ok) break;
         tmem_wait_st();
         fence_before_sync();
-        mbar_arrive(&ctl->pds_ready[bf]);
+        warp_arrive(&ctl->pds_ready[g]);
       }
       t0 += (uint32_t)nq;
-      if (!ok) break;
-      // The group that worked on the item's last tile runs the epilogue: its next tile reuses that tile's buffer
-      // pair, which is free no sooner than the item's last gradient MMA, so it has nothing else to do meanwhile.
-      if ((t0 - 1) % kGroups == (uint32_t)g) {
-        // Fused RoPE adjoint on dK: the first pass's table values are fetched into registers BEFORE the wait for
-        // the last gradient MMAs (see the dQ kernel's epilogue).
-        [[maybe_unused]] RopeQuad tab[RopeTasks<kGW>::n];
-        if constexpr (ROPE) rope_prefetch_pass<kGW>(tab, rt, n0, 0, tg, S);
-        if (!group_wait<kGW>(g, poller, &ctl->dkv_done[g], epilogues++ & 1, abort_flag, &ctl->fail_bits, ULM_STATUS_TIMEOUT_MMA)) { ok = false; break; }
-        fence_after_sync();
-        // read and round everything first, hand the accumulators back, rotate dK (ROPE) and store afterwards
-        T* v_item = dV + (int64_t)b * dv_sb + (int64_t)h * dv_sh + (int64_t)n0 * dv_ss;
-        T* k_item = dK + (int64_t)b * dk_sb + (int64_t)h * dk_sh + (int64_t)n0 * dk_ss;
-        uint4 vlo[4], klo[4];
-        [[maybe_unused]] uint4 khi[4];                     // a thread holds 32 columns: nothing in the other half
-        acc_to_16bit<T>(t_row + cV + my_half * 32, 1.f, vlo);
-        acc_to_16bit<T>(t_row + cK + my_half * 32, scale, klo);
-        fence_before_sync();
-        mbar_arrive(&ctl->acc_free);
-        staged_store<T>(stage + (size_t)g * kRopeStageBytes, g, tg, r, my_half, vlo, v_item, dv_ss, S - n0);
-        if constexpr (ROPE) {
-          rope_adjoint_store<T, kGW>(stage + (size_t)g * kRopeStageBytes, g, tg, r, my_half, klo, khi, k_item, dk_ss, n0, S, rt, tab);
-        } else {
-          staged_store<T>(stage + (size_t)g * kRopeStageBytes, g, tg, r, my_half, klo, k_item, dk_ss, S - n0);
-        }
-      }
     }
   }
 
@@ -933,7 +922,7 @@ int launch_bwd(const ulm_attn_bwd_args* a, int device, const Maps& m) {
     static std::atomic<bool> attr[kMaxDevices];
     const size_t smem = kSmemKV;
     if ((rc = ensure_smem_attr(kern, smem, device, attr, "ulm_attn_bwd(dkv)"))) return rc;
-    kern<<<grid, Roles<kGWdKV>::kThreads, smem, st>>>(m.q64, m.k128, m.v128, m.do64, a->lse, a->delta, (T*)a->dk, (T*)a->dv,
+    kern<<<grid, kThreadsKV, smem, st>>>(m.q64, m.k128, m.v128, m.do64, a->lse, a->delta, (T*)a->dk, (T*)a->dv,
                                           a->dk_sb, a->dk_sh, a->dk_ss, a->dv_sb, a->dv_sh, a->dv_ss,
                                           a->S, a->H, (int)BH, a->softmax_scale, scale2, a->dropout_p, a->seed, a->status_dev, rt);
     if ((rc = check_launch("ulm_attn_bwd(dkv)"))) return rc;

@@ -229,6 +229,13 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// The same, kept in program order with respect to other such calls
+__device__ __forceinline__ float ex2_ordered(float x) {
+  float y;
+  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Two-wide fp32 arithmetic (one issue slot for two lanes of work) and the three-input maximum.
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
   uint64_t r;
