@@ -423,7 +423,7 @@ rmsnorm_bwd_kernel(const BwdParams p) {
   }
 }
 
-// The same backward for wide fp32 rows (more than 16 elements per lane: d = 768, 1024 in the training layout, an
+// The same backward for wide fp32 rows (more than 16 elements per lane: d = 768 in the training layout, an
 // fp32 residual stream with a 16-bit dy).  One warp per row needs the raw x, dy and g_add of the row plus the dw
 // accumulators in registers at once, which at 128 registers leaves no room for a second row in flight; here TWO
 // warps share a row (NVH vectors per lane each), twelve warps a CTA, so that 24 warps per SM each have a whole
@@ -548,6 +548,143 @@ rmsnorm_bwd_split_kernel(const BwdParams p) {
   }
 }
 
+// The same for rows of 769 to 1024 elements: FOUR warps share a row, two vectors per lane, and every lane requests x and dy of its
+// part of the NEXT row before it works on this one (g_add, needed last, comes with the row's own turn), so that loads are in
+// flight while the warps reduce and store.  With two warps a row of this width fills the registers (and spills), and nothing can be
+// requested ahead.  32768 x 1024, fused add, L2 flushed: 97.5 -> 88 us (5.5 -> 6.1 TB/s).  Rows of up to 768 keep two
+// warps: three a row with the same lookahead took 70.6 us against 70.0 (32768 x 768), 13.2 / 12.5 (5000 x 768), 40.7 / 38.5 (20000 x 640).
+constexpr int kQuadWarps = 4;
+
+template <typename TW, typename TY, bool ADD>
+__global__ void __launch_bounds__(kSplitThreads, 2)
+rmsnorm_bwd_quad_kernel(const BwdParams p) {
+  constexpr int N = 4, NV = 2, WPR = kQuadWarps, kGroups = kSplitWarps / WPR;
+  static_assert(kSplitWarps % WPR == 0, "whole rows per CTA");
+  extern __shared__ float s_dw[];                      // [kSplitWarps][d], then the groups' exchange slots
+  float* s_red = s_dw + (size_t)kSplitWarps * p.d;     // [2 phases][2 quantities][kSplitWarps]
+  const float* __restrict__ x = static_cast<const float*>(p.x);
+  const TW* __restrict__ w = static_cast<const TW*>(p.w);
+  const TY* __restrict__ dy = static_cast<const TY*>(p.dy);
+  const float* __restrict__ ga = static_cast<const float*>(p.g_add);
+  float* __restrict__ dx = static_cast<float*>(p.dx);
+  TY* __restrict__ db = static_cast<TY*>(p.d_branch);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int group = warp / WPR, part = warp % WPR;
+  const int nvec = p.d / N;
+  const float inv_d = 1.f / (float)p.d;
+  float acc[NV][N];
+#pragma unroll
+  for (int it = 0; it < NV; ++it)
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc[it][j] = 0.f;
+  auto row_sum = [&](float v, int phase, int q) {      // sum of v over the warps of the row
+    v = warp_sum(v);
+    float* slot = s_red + ((phase * 2 + q) * kSplitWarps);
+    if (lane == 0) slot[warp] = v;
+    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(32 * WPR) : "memory");
+    float t = slot[WPR * group];
+#pragma unroll
+    for (int i = 1; i < WPR; ++i) t += slot[WPR * group + i];
+    return t;
+  };
+  struct Row {
+    uint4 x[NV];
+    uint2 g[NV];
+    float rstd;
+  };
+  auto request = [&](Row& t, int64_t r) {              // vectors past the end are zeros
+#pragma unroll
+    for (int it = 0; it < NV; ++it) {
+      const int vi = (part * NV + it) * 32 + lane;
+      t.x[it] = make_uint4(0u, 0u, 0u, 0u);
+      t.g[it] = make_uint2(0u, 0u);
+      if (vi < nvec) {
+        t.x[it] = *reinterpret_cast<const uint4*>(x + r * p.x_stride + vi * N);
+        t.g[it] = *reinterpret_cast<const uint2*>(dy + r * p.dy_stride + vi * N);
+      }
+    }
+    t.rstd = p.rstd ? p.rstd[r] : 0.f;
+  };
+  int phase = 0;
+  const int64_t step = (int64_t)gridDim.x * kGroups;
+  int64_t r = (int64_t)blockIdx.x * kGroups + group;
+  Row cur, next;
+  if (r < p.rows) request(cur, r);
+  for (; r < p.rows; r += step, phase ^= 1) {
+    [[maybe_unused]] float4 ar[NV];                    // needed last: requested with the row's own turn
+    if constexpr (ADD) {
+#pragma unroll
+      for (int it = 0; it < NV; ++it) {
+        const int vi = (part * NV + it) * 32 + lane;
+        ar[it] = ga && vi < nvec ? *reinterpret_cast<const float4*>(ga + r * p.gadd_stride + vi * N) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    if (r + step < p.rows) request(next, r + step);
+    float inv = cur.rstd;
+    if (!p.rstd) {
+      float ss = 0.f;
+#pragma unroll
+      for (int it = 0; it < NV; ++it) {
+        float xv[N];
+        unpack_raw<float, N>(cur.x[it], xv);
+#pragma unroll
+        for (int j = 0; j < N; ++j) ss += xv[j] * xv[j];
+      }
+      inv = rsqrtf(row_sum(ss, phase, 0) * inv_d + p.eps);
+    }
+    float dot = 0.f;
+#pragma unroll
+    for (int it = 0; it < NV; ++it) {
+      const int vi = (part * NV + it) * 32 + lane;
+      float wv[N] = {0.f, 0.f, 0.f, 0.f}, xv[N], gv[N];
+      if (vi < nvec) load_w<TW, N>(w, vi * N, wv);       // from L1, each time: registers are what bounds the rows in flight
+      unpack_raw<float, N>(cur.x[it], xv);
+      unpack_graw<TY, N>(cur.g[it], gv);
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const float xh = xv[j] * inv;
+        acc[it][j] += gv[j] * xh;
+        dot += gv[j] * wv[j] * xh;
+      }
+    }
+    const float dm = row_sum(dot, phase, 1) * inv_d;
+#pragma unroll
+    for (int it = 0; it < NV; ++it) {
+      const int vi = (part * NV + it) * 32 + lane;
+      if (vi < nvec) {
+        float wv[N], xv[N], gv[N], o[N];
+        load_w<TW, N>(w, vi * N, wv);
+        unpack_raw<float, N>(cur.x[it], xv);
+        unpack_graw<TY, N>(cur.g[it], gv);
+#pragma unroll
+        for (int j = 0; j < N; ++j) o[j] = inv * (gv[j] * wv[j] - xv[j] * inv * dm);
+        if constexpr (ADD) {
+          o[0] += ar[it].x; o[1] += ar[it].y; o[2] += ar[it].z; o[3] += ar[it].w;
+          if (db) store_n<TY, N>(db + r * p.dbranch_stride + vi * N, o);
+        }
+        store_n<float, N>(dx + r * p.dx_stride + vi * N, o);
+      }
+    }
+    cur = next;
+  }
+#pragma unroll
+  for (int it = 0; it < NV; ++it) {
+    const int vi = (part * NV + it) * 32 + lane;
+    if (vi < nvec) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) s_dw[warp * p.d + vi * N + j] = acc[it][j];
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < p.d; c += kSplitThreads) {
+    const int h = (c / N) / (32 * NV);                 // the part of every group that owns this column
+    float t = 0.f;
+#pragma unroll
+    for (int gi = 0; gi < kGroups; ++gi) t += s_dw[(WPR * gi + h) * p.d + c];
+    p.partial[(int64_t)blockIdx.x * p.d + c] = t;
+  }
+}
+
 // dw[c] = sum over the partial rows, in a fixed order: a CTA takes 32 columns, its 32 x 32 threads each add
 // every 32nd partial row of one column (coalesced 128-byte reads, short independent chains), and the 32
 // sub-sums of a column are added in index order.
@@ -633,15 +770,16 @@ void launch_fwd(const FwdParams& p, int nv, cudaStream_t st) {
 template <typename T, typename TW, typename TY, bool ADD>
 void launch_bwd(const BwdParams& p, int nv, int64_t blocks, size_t smem, cudaStream_t st) {
   if constexpr (sizeof(T) == 4 && sizeof(TY) == 2) {
-    if (nv == 6 || nv == 8) {                          // wide fp32 rows: two warps per row
-      const int64_t want = (p.rows + kSplitWarps / 2 - 1) / (kSplitWarps / 2);
+    if (nv == 6 || nv == 8) {                          // wide fp32 rows: two or four warps per row
+      const int per_cta = kSplitWarps / (nv == 6 ? 2 : kQuadWarps);
+      const int64_t want = (p.rows + per_cta - 1) / per_cta;
       const int64_t grid = want < blocks ? want : blocks;       // never more CTAs than partial rows were provided
       const size_t sm = ((size_t)kSplitWarps * p.d + 4 * kSplitWarps) * sizeof(float);
       auto launch = [&](auto kern) {
         if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         kern<<<(unsigned)grid, kSplitThreads, sm, st>>>(p);
       };
-      if (nv == 6) launch(rmsnorm_bwd_split_kernel<TW, TY, 3, ADD>); else launch(rmsnorm_bwd_split_kernel<TW, TY, 4, ADD>);
+      if (nv == 6) launch(rmsnorm_bwd_split_kernel<TW, TY, 3, ADD>); else launch(rmsnorm_bwd_quad_kernel<TW, TY, ADD>);
       return;
     }
   }
