@@ -10,9 +10,9 @@
 //
 // Machine mapping (both tensor-core kernels): TMA-staged 128-byte-swizzled
 // tiles, tcgen05.mma with fp32 accumulators in TMEM, the 16-bit P / dS operands
-// written back into TMEM over the scores they came from and consumed as the A
-// operand, so no intermediate ever touches shared or global memory.
-//   dQ kernel:   CTA = 128 query rows (thread r of a group = row r = TMEM lane r),
+// written back into TMEM and consumed as the A operand, so no intermediate
+// ever touches shared or global memory.
+//   dQ kernel:   CTA = 128 query rows (compute thread r = row r = TMEM lane r),
 //                walks key tiles of 64: S and dP (128x64 each) -> dS -> dQ += dS K.
 //   dK/dV kernel: CTA = 128 keys (thread r = key r), walks query tiles of 64 from
 //                the diagonal down, transposed view: S^T = K Q^T, dP^T = V dO^T,
@@ -91,10 +91,8 @@ __device__ __forceinline__ void pair_ds(uint32_t s0, uint32_t s1, uint32_t dp0, 
 template <typename T> struct Fmt { static constexpr int v = 0; };
 template <> struct Fmt<__nv_bfloat16> { static constexpr int v = 1; };
 
-template <int GW>
-__device__ __forceinline__ void group_sync(int g) {      // the 32 GW threads of group g
-  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(32 * GW) : "memory");
-}
+// The four warps that share a staging tile (the dQ kernel's compute warps, the dK/dV kernel's storing warps)
+__device__ __forceinline__ void quad_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // All lanes of a warp learn together whether the wait succeeded.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -102,16 +100,15 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
-// The threads of group g learn together whether any of them says yes.
-template <int GW>
-__device__ __forceinline__ bool group_any(int g, bool yes) {
+// The threads of those four warps learn together whether any of them says yes.
+__device__ __forceinline__ bool quad_any(bool yes) {
   uint32_t any;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.or.pred p, %2, %3, q;\n\t"
+      "bar.red.or.pred p, 1, 128, q;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(any) : "r"((uint32_t)yes), "r"(g + 1), "n"(32 * GW) : "memory");
+      : "=r"(any) : "r"((uint32_t)yes) : "memory");
   return any != 0;
 }
 
@@ -141,43 +138,34 @@ __device__ __forceinline__ void acc_to_16bit(uint32_t taddr, float f, uint4 (&ou
   }
 }
 
-// 32 consecutive 16-bit columns of a gradient row held as four 16-byte vectors
-template <typename T>
-__device__ __forceinline__ void store_32(T* dst, const uint4 (&v)[4]) {
-#pragma unroll
-  for (int v4 = 0; v4 < 4; ++v4) *reinterpret_cast<uint4*>(dst + v4 * 8) = v[v4];
-}
-
 // ---------------------------------------------------------------------------
-// Fused RoPE adjoint of a 128-row gradient tile held one row per thread (or per thread pair).
+// Fused RoPE adjoint of a 128-row gradient tile held one row per thread by four warps.
 // A thread that owned a row would have to read its own table row: 32 different 128-byte lines per warp
 // load, which makes the load/store unit the cost.  So the rounded 16-bit rows go through a small shared
-// staging tile (64 rows x 128 bytes per compute group, 128-byte swizzle) and are picked up again with
+// staging tile (64 rows x 128 bytes, 128-byte swizzle) and are picked up again with
 // eight threads per row (rope_math.cuh): table loads and the final global stores are then fully
 // coalesced.  Two passes of 64 rows; the tables of pass 0 are prefetched into registers before the wait
 // for the accumulator (see the callers), those of pass 1 while pass 0 is being worked on.
 // ---------------------------------------------------------------------------
 constexpr int kRopeStageRows = 64;
-constexpr uint32_t kRopeStageBytes = kRopeStageRows * 128;          // per compute group
-template <int GW> struct RopeTasks { static constexpr int n = kRopeStageRows * 8 / (32 * GW); };   // per thread and pass
+constexpr uint32_t kRopeStageBytes = kRopeStageRows * 128;
+constexpr int kRopeTasks = kRopeStageRows * 8 / 128;                // per thread and pass
 
-template <int GW>
-__device__ __forceinline__ void rope_prefetch_pass(RopeQuad (&tab)[RopeTasks<GW>::n], const RopeTab& rt, int row0, int pass, int tg, int S) {
+__device__ __forceinline__ void rope_prefetch_pass(RopeQuad (&tab)[kRopeTasks], const RopeTab& rt, int row0, int pass, int tg, int S) {
 #pragma unroll
-  for (int j = 0; j < RopeTasks<GW>::n; ++j) {
-    const int idx = j * 32 * GW + tg;
+  for (int j = 0; j < kRopeTasks; ++j) {
+    const int idx = j * 128 + tg;
     const int row = row0 + kRopeStageRows * pass + (idx >> 3);
     const int pos = row < S ? row : S - 1;
     rope_load_quad(tab[j], rt.cos_tab + (int64_t)pos * rt.cos_stride, rt.sin_tab + (int64_t)pos * rt.sin_stride, idx & 7);
   }
 }
 
-// `lo` / `hi`: columns [0,32) / [32,64) of this thread's row r (GW == 4), or `lo` alone = the 32 columns of half
-// `my_half` (GW == 8).  `item_out` points at row 0 of the item in the output tensor.
-template <typename T, int GW>
-__device__ __forceinline__ void rope_adjoint_store(uint8_t* stage, int g, int tg, int r, int my_half, const uint4 (&lo)[4], const uint4 (&hi)[4],
+// `lo` / `hi`: columns [0,32) / [32,64) of this thread's row r.  `item_out` points at row 0 of the item in the output tensor.
+template <typename T>
+__device__ __forceinline__ void rope_adjoint_store(uint8_t* stage, int tg, int r, const uint4 (&lo)[4], const uint4 (&hi)[4],
                                                    T* item_out, int64_t row_stride, int row0, int S, const RopeTab& rt,
-                                                   RopeQuad (&tab)[RopeTasks<GW>::n]) {
+                                                   RopeQuad (&tab)[kRopeTasks]) {
 #pragma unroll
   for (int pass = 0; pass < 2; ++pass) {
     if ((r >> 6) == pass) {
@@ -185,18 +173,14 @@ __device__ __forceinline__ void rope_adjoint_store(uint8_t* stage, int g, int tg
       uint8_t* srow = stage + rr * 128;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        if constexpr (GW == 4) {
-          *reinterpret_cast<uint4*>(srow + ((c ^ (rr & 7)) << 4)) = lo[c];
-          *reinterpret_cast<uint4*>(srow + (((4 + c) ^ (rr & 7)) << 4)) = hi[c];
-        } else {
-          *reinterpret_cast<uint4*>(srow + (((my_half * 4 + c) ^ (rr & 7)) << 4)) = lo[c];
-        }
+        *reinterpret_cast<uint4*>(srow + ((c ^ (rr & 7)) << 4)) = lo[c];
+        *reinterpret_cast<uint4*>(srow + (((4 + c) ^ (rr & 7)) << 4)) = hi[c];
       }
     }
-    group_sync<GW>(g);
+    quad_sync();
 #pragma unroll
-    for (int j = 0; j < RopeTasks<GW>::n; ++j) {
-      const int idx = j * 32 * GW + tg;
+    for (int j = 0; j < kRopeTasks; ++j) {
+      const int idx = j * 128 + tg;
       const int row = idx >> 3, cg = idx & 7;
       const uint2 glo = *reinterpret_cast<const uint2*>(stage + swz_quad_offset(row, cg));
       const uint2 ghi = *reinterpret_cast<const uint2*>(stage + swz_quad_offset(row, cg + 8));
@@ -209,8 +193,8 @@ __device__ __forceinline__ void rope_adjoint_store(uint8_t* stage, int g, int tg
         *reinterpret_cast<uint2*>(dst + 32 + 4 * cg) = ohi;
       }
     }
-    if (pass == 0) rope_prefetch_pass<GW>(tab, rt, row0, 1, tg, S);
-    group_sync<GW>(g);                                    // the tile is rewritten by the next pass / the next epilogue
+    if (pass == 0) rope_prefetch_pass(tab, rt, row0, 1, tg, S);
+    quad_sync();                                    // the tile is rewritten by the next pass / the next epilogue
   }
 }
 
@@ -488,17 +472,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     // epilogue: the four warps go through it together or not at all (its staging tile is shared)
     const int tg = (int)threadIdx.x;
-    [[maybe_unused]] RopeQuad tab[RopeTasks<4>::n];
-    if constexpr (ROPE) rope_prefetch_pass<4>(tab, rt, m0, 0, tg, S);   // ahead of the wait for the last gradient MMAs
+    [[maybe_unused]] RopeQuad tab[kRopeTasks];
+    if constexpr (ROPE) rope_prefetch_pass(tab, rt, m0, 0, tg, S);   // ahead of the wait for the last gradient MMAs
     if (ok && !warp_wait(&ctl->dq_done, (nkv - 1) & 1, abort_flag)) { if (lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA); ok = false; }
-    if (!group_any<4>(0, !ok)) {
+    if (!quad_any(!ok)) {
       fence_after_sync();
       uint4 lo[4], hi[4];
       acc_to_16bit<T>(t_row + kColDQ, scale, lo);
       acc_to_16bit<T>(t_row + kColDQ + 32, scale, hi);
       T* item_out = dQ + (int64_t)b * dq_sb + (int64_t)h * dq_sh + (int64_t)m0 * dq_ss;
       if constexpr (ROPE) {
-        rope_adjoint_store<T, 4>(sQ, 0, tg, r, 0, lo, hi, item_out, dq_ss, m0, S, rt, tab);
+        rope_adjoint_store<T>(sQ, tg, r, lo, hi, item_out, dq_ss, m0, S, rt, tab);
       } else {
         staged_store<T>(sQ + warp * kWarpStageBytes, lane, lo, hi, item_out + (int64_t)(warp * 32) * dq_ss, dq_ss, S - m0 - warp * 32);
       }
@@ -604,11 +588,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       decode(idx, bh, n0, i_begin, nq);
       const int b = bh / H, h = bh - b * H;
       // Fused RoPE adjoint on dK: the first pass's table values are fetched BEFORE the wait for the last gradient MMAs.
-      [[maybe_unused]] RopeQuad tab[RopeTasks<4>::n];
-      if constexpr (ROPE) rope_prefetch_pass<4>(tab, rt, n0, 0, tg, S);
+      [[maybe_unused]] RopeQuad tab[kRopeTasks];
+      if constexpr (ROPE) rope_prefetch_pass(tab, rt, n0, 0, tg, S);
       const bool ok = warp_wait(&ctl->dkv_done, n & 1, abort_flag);
       if (!ok && lane == 0) atomicOr(&ctl->fail_bits, (uint32_t)ULM_STATUS_TIMEOUT_MMA);
-      if (group_any<4>(0, !ok)) break;                    // the four warps leave together: their staging tile is shared
+      if (quad_any(!ok)) break;                    // the four warps leave together: their staging tile is shared
       fence_after_sync();
       // read and round everything first, hand the accumulators back, rotate dK (ROPE) and store afterwards
       T* v_item = dV + (int64_t)b * dv_sb + (int64_t)h * dv_sh + (int64_t)n0 * dv_ss;
@@ -623,8 +607,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int w0 = sub * 32;
       staged_store<T>(w_stage, lane, vlo, vhi, v_item + (int64_t)w0 * dv_ss, dv_ss, S - n0 - w0);
       if constexpr (ROPE) {
-        group_sync<4>(0);                                 // the staging tile changes from a warp's to the group's
-        rope_adjoint_store<T, 4>(stage, 0, tg, r, 0, klo, khi, k_item, dk_ss, n0, S, rt, tab);
+        quad_sync();                                 // the staging tile changes from a warp's to the group's
+        rope_adjoint_store<T>(stage, tg, r, klo, khi, k_item, dk_ss, n0, S, rt, tab);
       } else {
         staged_store<T>(w_stage, lane, klo, khi, k_item + (int64_t)w0 * dk_ss, dk_ss, S - n0 - w0);
       }
