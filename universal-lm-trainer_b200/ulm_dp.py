@@ -426,8 +426,8 @@ class DataParallelStep:
         self.heartbeat = heartbeat                        # optional StepHeartbeat, checked before each step
         # False (default): ONE all-reduce of the whole flat buffer after the last backward.  True: bucket
         # all-reduces issued from gradient-ready hooks during the last backward.  Measured on 2 B200 (100M preset,
-        # weak): overlapped 166.8 ms/step, not overlapped 117.9 ms/step.  The attention backward kernels are
-        # persistent, one CTA per SM with all of its shared memory and TMEM; a collective kernel that sits on a few
+        # weak): overlapped 166.8 ms/step, not overlapped 117.9 ms/step.  The attention backward kernels were
+        # persistent then (dK/dV still is), one CTA per SM with all of its shared memory and TMEM; a collective kernel that sits on a few
         # SMs waiting for its peer turns their single wave into two (the rank that reaches the collective first
         # lost 50 ms of forward/backward time per step), which costs far more than the 3-6 ms the all-reduce takes
         # on its own.
