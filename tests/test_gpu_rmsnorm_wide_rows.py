@@ -1,11 +1,18 @@
 """Residual add + RMSNorm backward for rows of 769 to 1024 elements (four warps a row, x and dy of the next row requested ahead): ragged
-widths, row counts around a CTA's three rows and around one pass of the grid (888 rows), with and without a gradient at the sum."""
+widths, row counts around a CTA's three rows and around one pass of the full grid (296 CTAs, 888 rows), with and without a gradient at
+the sum."""
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
+
+@pytest.mark.parametrize('rows,parts', [(0, 1), (1, 1), (3, 1), (4, 2), (512, 171), (885, 295), (886, 296), (888, 296), (100000, 296)])
+def test_partial_rows_cover_a_cta_per_three_rows(rows, parts):
+    """The grid is capped by the partial rows: with fewer, rows wait for a CTA while SMs have none."""
+    import _native
+    assert _native.lib().ulm_rmsnorm_bwd_partial_rows(rows) == parts
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize('rows,d', [(1, 1024), (2, 772), (3, 900), (4, 1020), (887, 1024), (889, 772), (1777, 1024), (2665, 1000)])
 @pytest.mark.parametrize('with_sum', [True, False])

@@ -554,6 +554,12 @@ rmsnorm_bwd_split_kernel(const BwdParams p) {
 // requested ahead.  32768 x 1024, fused add, L2 flushed: 97.5 -> 88 us (5.5 -> 6.1 TB/s).  Rows of up to 768 keep two
 // warps: three a row with the same lookahead took 70.6 us against 70.0 (32768 x 768), 13.2 / 12.5 (5000 x 768), 40.7 / 38.5 (20000 x 640).
 constexpr int kQuadWarps = 4;
+// Rows a CTA takes a pass, the fewest of all the backward kernels: the partial rows are provided for it, and the grid follows it.
+// With a CTA per eight rows, as for the one-warp form, the two CTAs that an SM holds were not filled below 2368 rows, and each
+// made three passes.  Backward and weight reduction, us, with two warps a row / four and a CTA per eight rows / per three:
+// 64 x 1024 9.2 / 7.6 / 5.7, 514 10.6 / 8.8 / 7.3, 889 11.2 / 9.2 / 8.1, 2000 14.7 / 11.7 / 11.6, 2664 16.6 / 12.7 / 12.7,
+// 257 x 772 9.8 / 8.0 / 6.6.
+constexpr int kFewestRowsPerCta = kSplitWarps / kQuadWarps;
 
 template <typename TW, typename TY, bool ADD>
 __global__ void __launch_bounds__(kSplitThreads, 2)
@@ -713,9 +719,9 @@ int check_kind(const char* who, int kind, int x_dtype) {
   return ULM_OK;
 }
 
-// upper bound on the CTAs of the backward = partial rows the caller provides
-int64_t bwd_grid(int64_t rows) {
-  const int64_t want = (rows + kWarps - 1) / kWarps;
+// CTAs of a backward launch with one CTA per `per_cta` rows, two per SM at most; each fills one partial row
+int64_t bwd_grid(int64_t rows, int per_cta) {
+  const int64_t want = (rows + per_cta - 1) / per_cta;
   const int64_t cap = 2 * kNumSMs;
   return want < 1 ? 1 : (want < cap ? want : cap);
 }
@@ -771,13 +777,10 @@ template <typename T, typename TW, typename TY, bool ADD>
 void launch_bwd(const BwdParams& p, int nv, int64_t blocks, size_t smem, cudaStream_t st) {
   if constexpr (sizeof(T) == 4 && sizeof(TY) == 2) {
     if (nv == 6 || nv == 8) {                          // wide fp32 rows: two or four warps per row
-      const int per_cta = kSplitWarps / (nv == 6 ? 2 : kQuadWarps);
-      const int64_t want = (p.rows + per_cta - 1) / per_cta;
-      const int64_t grid = want < blocks ? want : blocks;       // never more CTAs than partial rows were provided
       const size_t sm = ((size_t)kSplitWarps * p.d + 4 * kSplitWarps) * sizeof(float);
       auto launch = [&](auto kern) {
         if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        kern<<<(unsigned)grid, kSplitThreads, sm, st>>>(p);
+        kern<<<(unsigned)blocks, kSplitThreads, sm, st>>>(p);
       };
       if (nv == 6) launch(rmsnorm_bwd_split_kernel<TW, TY, 3, ADD>); else launch(rmsnorm_bwd_quad_kernel<TW, TY, ADD>);
       return;
@@ -800,7 +803,7 @@ void launch_bwd(const BwdParams& p, int nv, int64_t blocks, size_t smem, cudaStr
 }  // namespace
 }  // namespace ulm
 
-extern "C" int64_t ulm_rmsnorm_bwd_partial_rows(int64_t rows) { return ulm::bwd_grid(rows); }
+extern "C" int64_t ulm_rmsnorm_bwd_partial_rows(int64_t rows) { return ulm::bwd_grid(rows, ulm::kFewestRowsPerCta); }
 
 extern "C" int ulm_rmsnorm_fwd(const ulm_rmsnorm_fwd_args* a) {
   using namespace ulm;
@@ -862,11 +865,8 @@ int rmsnorm_bwd_launch(const ulm_rmsnorm_bwd_args* a, float* partial, const char
   cudaStream_t st = (cudaStream_t)a->stream;
   const int n = a->x_dtype == ULM_F32 ? 4 : 8;
   const int nv = pick_nv((a->d / n + 31) / 32);          // d <= 1024: at most 8 vectors per lane
-  const int r_iter = bwd_rows_per_iter(nv * n);
-  int64_t blocks = (a->rows + (int64_t)kWarps * r_iter - 1) / ((int64_t)kWarps * r_iter);
-  const int64_t cap = bwd_grid(a->rows);
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
+  const bool quad = nv == 8 && a->x_dtype == ULM_F32 && a->dy_kind != ULM_Y_SAME;   // rmsnorm_bwd_quad_kernel (launch_bwd)
+  const int64_t blocks = bwd_grid(a->rows, quad ? kFewestRowsPerCta : kWarps);
   const size_t smem = (size_t)kWarps * a->d * sizeof(float);
   if (a->rows > 0) {
     BwdParams p{a->x, a->w, a->dy, a->rstd, a->g_add, a->dx, a->d_branch, partial,
@@ -952,8 +952,8 @@ extern "C" int ulm_rmsnorm_bwd_static(const ulm_rmsnorm_bwd_args* a) {
   if (!a) return fail(ULM_ERR_ARG, "%s: null args", who);
   if (a->d > kStaticMaxD)
     return fail(ULM_ERR_TOO_LARGE, "%s: d=%d exceeds the built-in scratch (rows of at most %d elements)", who, a->d, kStaticMaxD);
-  if (bwd_grid(a->rows) > kStaticMaxParts)
-    return fail(ULM_ERR_TOO_LARGE, "%s: %lld partial rows exceed the built-in scratch (%d)", who, (long long)bwd_grid(a->rows), kStaticMaxParts);
+  if (bwd_grid(a->rows, kFewestRowsPerCta) > kStaticMaxParts)
+    return fail(ULM_ERR_TOO_LARGE, "%s: %lld partial rows exceed the built-in scratch (%d)", who, (long long)bwd_grid(a->rows, kFewestRowsPerCta), kStaticMaxParts);
   if (a->rows > 0 && a->x) {                              // the tensors must live on the current device
     cudaPointerAttributes at;
     int dev = -1;
