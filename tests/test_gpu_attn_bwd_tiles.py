@@ -5,13 +5,16 @@ import torch
 
 
 UNIT = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}   # unit roundoff
+LEAST = {torch.float16: 2.0 ** -14, torch.bfloat16: 2.0 ** -126, torch.float32: 0.0}   # smallest normal number
 
 
 def attention_grads(q, k, v, do, causal, lse_of=None):
     """fp64 dQ, dK, dV and, for every row of each, the rms size of its rounding error per unit roundoff.  The kernels round P (forward: for
     O; backward: for dV), O, dS and each gradient once, everything else is fp32; a rounding has an rms of at most 1 / sqrt(3) of the
-    unit roundoff, roundings are independent, and what P and O get in the forward pass reaches dS through delta = sum(O dO) = sum(P dP).
+    unit roundoff (of the smallest normal number where a value is smaller: a last key's dS of 1e-5 was off by eleven times what its own size
+    gives in fp16), roundings are independent, and what P and O get in the forward pass reaches dS through delta = sum(O dO) = sum(P dP).
     `lse_of`: for every query row, the row whose softmax statistics are taken for it (None: its own)."""
+    least = LEAST[q.dtype] ** 2
     q, k, v, do = (t.double() for t in (q, k, v, do))
     S = q.shape[2]
     s = q @ k.transpose(-1, -2) * 0.125
@@ -28,10 +31,11 @@ def attention_grads(q, k, v, do, causal, lse_of=None):
     dq, dk, dv = ds @ k * 0.125, ds.transpose(-1, -2) @ q * 0.125, p.transpose(-1, -2) @ do
     sq = lambda t: t.square().sum(-1, keepdim=True)      # noqa: E731
     var_delta = ((p @ v) * do).square().sum(-1, keepdim=True) + (p * dp).square().sum(-1, keepdim=True)
-    var_q = (ds.square() @ sq(k) + var_delta * sq(p @ k)) / 64 + sq(dq)
-    var_k = (ds.square() + p.square() * var_delta).transpose(-1, -2) @ sq(q) / 64 + sq(dk)
-    var_v = p.square().transpose(-1, -2) @ sq(do) + sq(dv)
-    return (dq, dk, dv), [(x.squeeze(-1) / 3).sqrt() for x in (var_q, var_k, var_v)]
+    var_ds, var_p = (torch.where(p > 0, x.square() + least, 0.0) for x in (ds, p))
+    var_q = (var_ds @ sq(k) + var_delta * sq(p @ k)) / 64 + sq(dq)
+    var_k = (var_ds + p.square() * var_delta).transpose(-1, -2) @ sq(q) / 64 + sq(dk)
+    var_v = var_p.transpose(-1, -2) @ sq(do) + sq(dv)
+    return (dq, dk, dv), [((x.squeeze(-1) + 64 * least) / 3).sqrt() for x in (var_q, var_k, var_v)]
 
 
 def row_error(got, want, rms):
