@@ -52,7 +52,10 @@ static_assert(192 * kGroups + 128 <= 512, "score buffers, packed operands and ac
 constexpr int kProducerWarp = kGroupWarps * kGroups, kMmaWarp = kProducerWarp + 1, kMma2Warp = kProducerWarp + 2, kGradWarp = kProducerWarp + 3,
               kStoreWarp = kProducerWarp + 4;
 constexpr int kThreadsKV = 32 * (kStoreWarp + 4);
-constexpr int kRegsCompute = 184, kRegsIssue = 56, kRegsStore = 88;   // per thread, by warpgroup
+// Per thread, by warpgroup.  The plain kernels spill 100-170 bytes all the same, the ones with the RoPE adjoint 370-410: there a storing
+// thread holds both rounded rows (64 registers) beside the tables' values (64).  168 / 56 / 120, 176 / 56 / 104 and 200 / 40 / 72
+// were slower.
+constexpr int kRegsCompute = 184, kRegsIssue = 56, kRegsStore = 88;
 static_assert(kGroups * kGroupThreads * kRegsCompute + 128 * (kRegsIssue + kRegsStore) <= 65536 / kThreadsKV / 8 * 8 * kThreadsKV,
               "the register split must fit what the CTA is launched with");
 constexpr uint32_t kBigTile = BR * HD * 2;    // 16 KB
@@ -249,27 +252,17 @@ attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO, float* __re
 }
 
 // ---------------------------------------------------------------------------
-// Persistent CTAs.  The dK/dV kernel launches one CTA per SM, which walks a static list of
-// work items (one item = one (batch*head, tile of 128 rows)).  Items are numbered heaviest first
-// and dealt to the CTAs in boustrophedon order -- round r gives CTA c item r*G + c on even rounds
-// and r*G + G-1-c on odd ones -- which balances the CTAs' totals to within one item of the mean
-// without a global counter.  Every role walks the same list, and all ring / buffer indices run on a
-// tile counter that keeps counting across items, so the producer prefetches the next item's resident
-// tiles (double-buffered) and first streamed tiles, and the S and dP issuers fill free score buffers
-// with them, while the last tiles of the current item are still being worked on.  Only the gradient
-// issuer pauses between items, until the accumulators have been read out of TMEM.
-// ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // dQ kernel
 // One CTA per work item (128 query rows of one (batch, head)), two CTAs per SM, so that one CTA's exponentials run
 // under the other's waits, loads and stores, and a CTA's start-up and epilogue under the other's tiles.
 // TMEM columns: S at 0, dP at 64, packed dS at 128, the dQ accumulator at 192.  A compute thread owns a query row: it takes the
 // 64 + 64 values of its row into registers and hands both buffers back at once, so the next tile's S and dP are
 // there when it has written this tile's dS, into columns that the previous tile's gradient MMAs have long read.
-// What bounds it: issue slots and the SFU (64 exponentials a thread and tile), then the synchronisation around a tile, whose
-// instructions queue behind the exponentials.  Against one persistent CTA per SM with three score buffer pairs, which waited a round
-// trip through the tensor core for every pair (us, start -> now): B8 H12 S4096 bf16 376 -> 335, B24 H12 S1363 fp16 180 -> 162,
-// B4 H12 S201 8.6 -> 7.6, B64 H12 S300 64 -> 64, B1 H16 S4096 68 -> 71 (512 CTAs are not quite two waves).
+// What bounds it: the SFU (64 exponentials a thread and tile; 61 % of its peak at B8 H12 S4096, tensor pipe 45 %, issue slots
+// 41 %), then the synchronisation around a tile, whose instructions queue behind the exponentials.  Against one persistent CTA per SM
+// with three score buffer pairs, which waited a round trip through the tensor core for every pair, on one box (us): B8 H12 S4096 bf16
+// 371 -> 335, B24 H12 S1363 fp16 179 -> 162, B4 H12 S201 8.6 -> 7.5, B1 H12 S67 6.6 -> 5.8, B64 H12 S300 64 -> 64, B1 H16 S4096
+// 69 -> 70.5 (512 CTAs are not quite two waves).
 // ---------------------------------------------------------------------------
 constexpr int kStagesQ = 3;                // K/V tile ring
 constexpr int kThreadsQ = 32 * (4 + 2);    // compute warps, producer warp, MMA warp
@@ -498,17 +491,24 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // ---------------------------------------------------------------------------
 // dK / dV kernel
 // A work item is one (batch*head, key tile of 128); key tile 0 meets the most query tiles under the
-// causal mask, so items are numbered by key tile, ascending.
+// causal mask, so items are numbered by key tile, ascending: heaviest first.
+// Persistent: one CTA per SM walks a static list of items, dealt in boustrophedon order (ItemIter), which balances the CTAs' totals to
+// within one item of the mean without a global counter.  Every role walks the same list, and all ring / buffer indices run on a
+// tile counter that keeps counting across items, so the producer prefetches the next item's resident tiles (double-buffered) and
+// first streamed tiles, and the S and dP issuers fill free score buffers with them, while the last tiles of the current item are
+// still being worked on.  Only the gradient issuer pauses between items, until the accumulators have been read out of TMEM.
 // Two compute groups of four warps take alternate query tiles, each in TMEM columns of its own.  A compute thread owns a key row: it
 // takes the 64 + 64 values of its row into registers and hands both buffers back at once, so the group's next S^T and dP^T are there
 // when it has written this tile's P^T and dS^T, into columns that the gradient MMAs of its previous tile have long read.
 // Finished gradients leave through a warpgroup of its own: done by a compute group, the 6,500 clk between an item's last gradient
 // MMA and its stores held up the tiles of the next item, 12 % of the kernel's time at S = 4096.
-// What bounds it: 1,330 of a group's 1,900 clk per tile are arithmetic (issue slots and the SFU, shared with the other
-// group), the rest synchronisation whose instructions queue behind the exponentials.  Against three groups of eight warps over three
-// score buffer pairs, P and dS packed over the scores (us, start -> now): B8 H12 S4096 bf16 475 -> 446, B24 H12 S1363 fp16
-// 222 -> 200, B64 H12 S300 68 -> 61, B1 H16 S4096 84 -> 76, B4 H12 S201 8.8 -> 8.7, B1 H12 S67 6.7 -> 6.9.  The groups taking
-// strict turns with their exponentials: 489 (turns of 1,000 clk each leave no more than they give).
+// What bounds it: at B8 H12 S4096 a CTA runs 730,000 clk, 2,130 for each of a group's 342 tiles.  1,900 of them are the group's loop,
+// of which 1,330 are arithmetic (issue slots and the SFU, shared with the other group) and the rest synchronisation whose
+// instructions queue behind the exponentials; 230 a tile, 3,800 an item, are the change of item, start-up and the end.  The SFU is
+// at 48 % of its peak, the tensor pipe at 48 %, issue slots at 49 %.  Against three groups of eight warps over three score buffer
+// pairs, P and dS packed over the scores, on one box (us): B8 H12 S4096 bf16 470 -> 450, B24 H12 S1363 fp16 222 -> 202, B64 H12
+// S300 68.7 -> 61.5, B1 H16 S4096 85 -> 76.5, B4 H12 S201 8.9 -> 8.6, B1 H12 S67 6.8 -> 6.7, B1 H2 S32 6.0 -> 6.2.  The groups
+// taking strict turns with their exponentials: 489 (turns of 1,000 clk each leave no more than they give).
 // ---------------------------------------------------------------------------
 struct CtlKV {
   uint64_t kv_full[2], kv_free[2], qdo_full[kStages], qdo_empty[kStages], sdp_full[kGroups], sdp_free[kGroups], pds_ready[kGroups],

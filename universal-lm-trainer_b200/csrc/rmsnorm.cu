@@ -553,6 +553,7 @@ rmsnorm_bwd_split_kernel(const BwdParams p) {
 // flight while the warps reduce and store.  With two warps a row of this width fills the registers (and spills), and nothing can be
 // requested ahead.  32768 x 1024, fused add, L2 flushed: 97.5 -> 88 us (5.5 -> 6.1 TB/s).  Rows of up to 768 keep two
 // warps: three a row with the same lookahead took 70.6 us against 70.0 (32768 x 768), 13.2 / 12.5 (5000 x 768), 40.7 / 38.5 (20000 x 640).
+// (One template for both forms slows the two-warp one: 69.2 -> 70.4 us at 32768 x 768.)
 constexpr int kQuadWarps = 4;
 // Rows a CTA takes a pass, the fewest of all the backward kernels: the partial rows are provided for it, and the grid follows it.
 // With a CTA per eight rows, as for the one-warp form, the two CTAs that an SM holds were not filled below 2368 rows, and each

@@ -154,9 +154,11 @@ def flash_attn_v100(q, k, v, dropout_p: float = 0.0, causal: bool = True, softma
 #   'none'  stand-alone RoPE kernel on q and k, plain attention kernels, stand-alone RoPE adjoint kernel
 #   'fwd'   Q rotated inside the attention forward (K through the stand-alone kernel), backward as 'none'
 #   'all'   as 'fwd', and the adjoint applied in the dQ / dK epilogues of the backward kernels
-# Measured at B=8, H=12, S=4096 on B200 the forward fusion costs what it saves (the rotation sits on each
-# CTA's start-up path) and the backward fusion costs more than the launch it removes (the epilogue of a
-# persistent in-order pipeline is on its critical path), so 'none' is the default; profiles/ has the numbers.
+# The kernels of one call on B200, us, none / fwd / all: 8x12x4096 bf16 1158 / 1160-1190 / 1256-1261, 24x12x1363 fp16 586-611 / 584-600 /
+# 604-616, 64x12x300 bf16 222-227 / 234 / 263-266, 4x12x201 fp16 30.5 / 31.6 / 32.0.  The forward fusion costs what it saves (the
+# rotation sits on each CTA's start-up path).  The backward fusion costs more than the launch it removes, although the dQ epilogue
+# runs under the SM's other CTA and the dK epilogue in a warpgroup of its own, whose registers spill.  So 'none' is the default; where
+# the host is the limit (4x12x201) 'all', with fewer launches, is 5 % faster a call.
 ROPE_FUSION = 'none'
 _FUSE = {'none': 0, 'fwd': 1, 'all': 2}
 
