@@ -56,7 +56,7 @@ FWD_FLOPS = 4.0 * B * H * S * S * D / 2.0           # causal-halved QK^T + PV
 STEP_FLOPS = 3.5 * FWD_FLOPS                         # backward counted as 2.5 x forward
 METRIC = 'causal attn fwd+bwd TFLOP/s (S=4096,D=64)'
 kRepeats = 3                                          # timed regions are taken this many times (outlier guard)
-NCU_TRAFFIC = {'attn_fwd': 453.2e6, 'attn_bwd_dq': 738.8e6, 'attn_bwd_dkv': 691.1e6}
+NCU_TRAFFIC = {'attn_fwd': 517.1e6, 'attn_bwd_dq': 612.4e6, 'attn_bwd_dkv': 704.5e6}
 WORKLOAD = 'configs[1]: RoPE (768-wide table) + causal attention fwd+bwd, B=8 H=12 S=4096 D=64, unrotated q,k in, gradients of unrotated q,k and v out'
 
 
