@@ -260,7 +260,7 @@ attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO, float* __re
 // there when it has written this tile's dS, into columns that the previous tile's gradient MMAs have long read.
 // What bounds it: the SFU (64 exponentials a thread and tile; 61 % of its peak at B8 H12 S4096, tensor pipe 45 %, issue slots
 // 41 %), then the synchronisation around a tile, whose instructions queue behind the exponentials.  Against one persistent CTA per SM
-// with three score buffer pairs, which waited a round trip through the tensor core for every pair, on one box (us): B8 H12 S4096 bf16
+// with three score buffer pairs, which waited a round trip through the tensor core for every pair, on one GPU (us): B8 H12 S4096 bf16
 // 371 -> 335, B24 H12 S1363 fp16 179 -> 162, B4 H12 S201 8.6 -> 7.5, B1 H12 S67 6.6 -> 5.8, B64 H12 S300 64 -> 64, B1 H16 S4096
 // 69 -> 70.5 (512 CTAs are not quite two waves).
 // ---------------------------------------------------------------------------
@@ -506,7 +506,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // of which 1,330 are arithmetic (issue slots and the SFU, shared with the other group) and the rest synchronisation whose
 // instructions queue behind the exponentials; 230 a tile, 3,800 an item, are the change of item, start-up and the end.  The SFU is
 // at 48 % of its peak, the tensor pipe at 48 %, issue slots at 49 %.  Against three groups of eight warps over three score buffer
-// pairs, P and dS packed over the scores, on one box (us): B8 H12 S4096 bf16 470 -> 450, B24 H12 S1363 fp16 222 -> 202, B64 H12
+// pairs, P and dS packed over the scores, on one GPU (us): B8 H12 S4096 bf16 470 -> 450, B24 H12 S1363 fp16 222 -> 202, B64 H12
 // S300 68.7 -> 61.5, B1 H16 S4096 85 -> 76.5, B4 H12 S201 8.9 -> 8.6, B1 H12 S67 6.8 -> 6.7, B1 H2 S32 6.0 -> 6.2.  The groups
 // taking strict turns with their exponentials: 489 (turns of 1,000 clk each leave no more than they give).
 // ---------------------------------------------------------------------------
